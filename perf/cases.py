@@ -230,3 +230,117 @@ def tolerance(case):
     if case["kind"] == "mlp":
         return {"rel": 4e-3}
     return {"rel": {"bf16": 1.6e-3, "fp16": 1e-4, "fp32": 4e-6}[case["dtype"]]}
+
+
+# ------------------------------------------------------------------------------------------ in 64 bits
+_E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
+_E2M1_MIDDLE = (0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0)  # a tie goes to the even code: up behind the odd ones
+
+
+def _divided(a, b):
+    """a / b in fp32, rounded once (a Python number as the divisor would become a product)."""
+    return a / torch.as_tensor(b, dtype=torch.float32, device=a.device).expand_as(a)
+
+
+def _tiled(scales):
+    """Scale bytes [rows, columns] in the 128 x 4 tiles that the tensor cores read, zero padded."""
+    rows, cols = scales.shape
+    r, c = (rows + 127) // 128, (cols + 3) // 4
+    full = torch.zeros(r * 128, c * 4, dtype=torch.uint8, device=scales.device)
+    full[:rows, :cols] = scales
+    return full.view(r, 4, 32, c, 4).permute(0, 3, 2, 1, 4).reshape(r * 128, c * 4)
+
+
+def _dynamic_scale(x):
+    """amax / (448 * 6), divided in x's own type."""
+    return _divided(x.abs().amax().float(), 2688.0).to(x.dtype).float()
+
+
+def _nvfp4(x, scale):
+    """(codes 0..15 as uint8, E4M3 scales of 16 elements) of a part of x's rows."""
+    v = x.float().view(x.shape[0], -1, 16)
+    amax = v.abs().amax(-1)
+    block = _divided(_divided(amax, 6.0), scale).clamp(max=448.0).to(torch.float8_e4m3fn)
+    total = (scale * block.float()).unsqueeze(-1)
+    q = torch.where(total == 0, torch.zeros_like(v), v / torch.where(total == 0, 1.0, total).expand_as(v))
+    a = q.abs()
+    code = torch.zeros(a.shape, dtype=torch.uint8, device=x.device)
+    for i, middle in enumerate(_E2M1_MIDDLE):
+        code += (a >= middle) if i % 2 else (a > middle)
+    return (code | (torch.signbit(q).to(torch.uint8) << 3)).view(x.shape), block
+
+
+def _mxfp8(x):
+    """(E4M3 data, E8M0 scale bytes of 32 elements) of a part of x's rows."""
+    v = x.float().view(x.shape[0], -1, 32)
+    amax = v.abs().amax(-1)
+    mantissa, exponent = torch.frexp(_divided(amax, 448.0).clamp(min=2.0 ** -127))
+    e = (exponent - (mantissa == 0.5).to(exponent.dtype) + 127).clamp(0, 254)
+    data = torch.ldexp(v, (127 - e).unsqueeze(-1)).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+    return data.view(x.shape), torch.where(amax == 0, 0, e).to(torch.uint8)
+
+
+def _stored(x, layout, scale=None):
+    """What the quantized x stands for, in 64 bits."""
+    out = torch.empty(x.shape, dtype=torch.float64, device=x.device)
+    lut = torch.tensor(_E2M1, dtype=torch.float64, device=x.device)
+    for r in range(0, x.shape[0], 2048):
+        part = x[r:r + 2048]
+        if layout == "nvfp4":
+            code, block = _nvfp4(part, scale)
+            value = lut[(code & 7).long()] * (1.0 - 2.0 * (code >> 3).double())
+            factor, size = block.double() * scale.double(), 16
+        else:
+            data, e = _mxfp8(part)
+            value, size = data.double(), 32
+            factor = torch.where(e == 0, 0.0, torch.ldexp(torch.ones_like(e, dtype=torch.float64), e.int() - 127))
+        out[r:r + 2048] = (value.view(part.shape[0], -1, size) * factor.unsqueeze(-1)).view(part.shape)
+    return out
+
+
+def _linear(x, w, bias, layout, x_scale=None):
+    """The linear layer on what x (dense) and w (dense) are stored as."""
+    if layout == "nvfp4":
+        xs, ws = _dynamic_scale(x) if x_scale is None else x_scale, _dynamic_scale(w)
+        y = _stored(x, layout, xs) @ _stored(w, layout, ws).T
+    else:
+        y = _stored(x, layout) @ _stored(w, layout).T
+    return y if bias is None else y.add_(bias.double())
+
+
+def _rounded_gelu(h, dtype):
+    """GELU (tanh form) between the two layers of an MLP: from and to the layers' type."""
+    out = torch.empty(h.shape, dtype=dtype, device=h.device)
+    for r in range(0, h.shape[0], 2048):
+        out[r:r + 2048] = torch.nn.functional.gelu(h[r:r + 2048].to(dtype).double(), approximate="tanh").to(dtype)
+    return out
+
+
+def exact(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(int(seed))
+    kind, layout, dtype = case["kind"], case["layout"], DTYPE[case["dtype"]]
+    m, n, k, with_bias = case["m"], case["n"], case["k"], case["bias"]
+    with torch.inference_mode():
+        if kind in ("quantize", "dequantize"):
+            x = _weight(gen, m, k, dtype)
+            if kind == "dequantize":
+                return _stored(x, layout, _dynamic_scale(x) if layout == "nvfp4" else None)
+            if layout == "nvfp4":
+                scale = _scale(x) if case["static"] else _dynamic_scale(x)
+                parts = [_nvfp4(x[r:r + 2048], scale) for r in range(0, m, 2048)]
+                codes = torch.cat([(c[:, 0::2] << 4) | c[:, 1::2] for c, _ in parts])
+                codes = torch.nn.functional.pad(codes, (0, 0, 0, -m % 16))
+                return codes, _tiled(torch.cat([b.view(torch.uint8) for _, b in parts])), scale.double()
+            parts = [_mxfp8(x[r:r + 2048]) for r in range(0, m, 2048)]
+            data = torch.cat([d.view(torch.uint8) for d, _ in parts])
+            return torch.nn.functional.pad(data, (0, 0, 0, -m % 32)), _tiled(torch.cat([e for _, e in parts]))
+        x = _activation(gen, m, k, dtype)
+        x_scale = _scale(x) if case["static"] and kind != "gemm" else None
+        if kind == "mlp":
+            fc1, fc2 = _dense_linear(gen, n, k, dtype, with_bias), _dense_linear(gen, k, n, dtype, with_bias)
+            # the calibration's hidden scale and the pass's own hidden tensor, each rounded where the layers round
+            sample = _rounded_gelu(_linear(x[:1024], fc1.weight, fc1.bias, layout, x_scale), dtype)
+            hidden = _rounded_gelu(_linear(x, fc1.weight, fc1.bias, layout, x_scale), dtype)
+            return _linear(hidden, fc2.weight, fc2.bias, layout, _dynamic_scale(sample))
+        lin = _dense_linear(gen, n, k, dtype, with_bias)
+        return _linear(x, lin.weight, lin.bias, layout, x_scale)
