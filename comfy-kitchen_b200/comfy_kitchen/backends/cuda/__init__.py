@@ -211,6 +211,7 @@ def quantize_mxfp8(x: torch.Tensor, pad_32x: bool = False) -> tuple[torch.Tensor
 
 
 _scale_scratch: dict = {}
+_retired_workspaces: list = []  # outgrown buffers stay alive: a captured CUDA graph may still point at them
 
 
 def _scale_scratch_for(device, stream: int, need: int) -> torch.Tensor:
@@ -325,36 +326,11 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        ws_ptr, ws_bytes = _gemm_workspace(lib, False, m, n, k, dev)
-        _check(lib.ck_scaled_mm_nvfp4_ws(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), _ptr(tsa), _ptr(tsb),
-                                         _ptr(alpha_t), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
-                                         ws_ptr, ws_bytes, _stream(dev)), "scaled_mm_nvfp4")
+        _check(lib.ck_scaled_mm_nvfp4(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), _ptr(tsa), _ptr(tsb),
+                                      _ptr(alpha_t), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
+                                      _stream(dev)), "scaled_mm_nvfp4")
     del bias_keep
     return out
-
-
-_gemm_workspaces: dict = {}
-_retired_workspaces: list = []  # outgrown buffers stay alive: a captured CUDA graph may still point at them
-
-
-def _gemm_workspace(lib, is_mxfp8: bool, m: int, n: int, k: int, device):
-    """(pointer, bytes) of the split-K workspace for this shape on the current stream, or (None, 0).
-
-    The library decides (few activation rows, or few output tiles and a long K); the buffer is
-    cached per device and stream and only ever grows, so steady-state calls allocate nothing."""
-    need = int(lib.ck_scaled_mm_workspace_bytes(int(is_mxfp8), m, n, k))
-    if need == 0:
-        return None, 0
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    ws = _gemm_workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        if ws is not None:
-            _retired_workspaces.append(ws)
-        # zero-filled: the head of the workspace holds arrival counters that must start at zero
-        # (every call leaves them at zero again)
-        ws = torch.zeros(max(need, 1 << 22), dtype=torch.uint8, device=device)
-        _gemm_workspaces[key] = ws
-    return ws.data_ptr(), ws.numel()
 
 
 def _pointer_array(ptrs):
@@ -593,10 +569,8 @@ def scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tenso
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        ws_ptr, ws_bytes = _gemm_workspace(lib, True, m, n, k, dev)
-        _check(lib.ck_scaled_mm_mxfp8_ws(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), bias_ptr, bias_code,
-                                         _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, ws_ptr, ws_bytes, _stream(dev)),
-               "scaled_mm_mxfp8")
+        _check(lib.ck_scaled_mm_mxfp8(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), bias_ptr, bias_code,
+                                      _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, _stream(dev)), "scaled_mm_mxfp8")
     del bias_keep
     return out
 

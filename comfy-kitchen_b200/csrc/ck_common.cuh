@@ -39,17 +39,12 @@ int sm_count();
 // Device address of the GEMM kernels' status word on the current device (ck_gemm.cu).
 int gemm_status_word(int** out);
 
-// Caller-owned GEMM workspace: the first kWorkspaceTicketBytes hold the arrival counters of the
-// small-M path (zero before the first use, left zero by every call); partial tiles of either
-// split-K path follow.
-constexpr int64_t kWorkspaceTicketBytes = 65536;
-
 // GEMMs with few activation rows (ck_gemm_smallm.cu).
 bool small_m_applies(int64_t M, int64_t N, int64_t K);
-int64_t small_m_workspace_bytes(bool is_mxfp8, int64_t M, int64_t N, int64_t K);
+int small_m_max_splits(int64_t N, int k_bytes);
 int scaled_mm_small_m(bool is_mxfp8, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
                       const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
-                      int64_t M, int64_t N, int64_t K, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
+                      int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 
 // ---- programmatic dependent launch ------------------------------------------------------
 // The streaming kernels and the GEMMs of this library are launched with programmatic stream

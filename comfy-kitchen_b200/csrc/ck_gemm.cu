@@ -1,5 +1,5 @@
-// Block-scaled GEMM entry points (scaled_mm_nvfp4 / scaled_mm_mxfp8, fused linear, split-K with a
-// workspace, all-gather variants): shape-based choice of the kernel configuration of
+// Block-scaled GEMM entry points (scaled_mm_nvfp4 / scaled_mm_mxfp8, fused linear, split-K,
+// all-gather variants): shape-based choice of the kernel configuration of
 // ck_gemm_kernel.cuh, argument validation, and the device status word.
 #include "ck_gemm_kernel.cuh"
 
@@ -64,86 +64,34 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
 // ---------------------------------------------------------------------------
 // split-K
 // ---------------------------------------------------------------------------
-struct SplitPlan {
-  int splits;
-  int k_stages_per_split;
-};
-
-// More than one split only when the 128 x 128 tiles leave at least half of the SMs idle and K is
-// long enough (>= 16 pipeline stages) for the extra pass over the partial tiles to pay.
-SplitPlan plan_splits(int64_t M, int64_t N, int k_bytes) {
+// Few 128 x 128 tiles and a long K: the K range of a tile is spread over a cluster of CTAs that add
+// their partial tiles through distributed shared memory (ck_gemm_kernel.cuh).  At most as many CTAs
+// per tile as leave every CTA six pipeline stages and let all clusters run at once; 1 = no split.
+int max_splits(int64_t M, int64_t N, int k_bytes) {
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
-  SplitPlan plan = {1, k_stages};
-  if (tiles * 2 > sm_count() || k_stages < 16) return plan;
+  if (tiles * 2 > sm_count() || k_stages < 16) return 1;
+  int splits = min(kMaxSplits, k_stages / 6);
   const int64_t by_sms = sm_count() / tiles;
-  int splits = min(kMaxOutputs, k_stages / 6);
   if (by_sms < splits) splits = static_cast<int>(by_sms);
-  if (splits < 2) return plan;
-  plan.k_stages_per_split = static_cast<int>(ceil_div(k_stages, splits));
-  plan.splits = static_cast<int>(ceil_div(k_stages, plan.k_stages_per_split));
-  return plan;
+  return max(splits, 1);
 }
 
-// out = cast(alpha * (partial_0 + partial_1 + ...) + bias), four consecutive columns per thread;
-// the partials are added in index order, so the result does not depend on scheduling.
-template <typename OutT>
-__global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* partials, int splits, int64_t mn, int n_cols, const float* alpha_ptr, const float* tsa,
-                     const float* tsb, const void* bias, int bias_dtype, OutT* out) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
-  if (i >= mn) return;
-  float alpha = 1.0f;
-  if (alpha_ptr != nullptr) {
-    alpha = ld_f32_dependent(alpha_ptr);
-  } else if (tsa != nullptr && tsb != nullptr) {
-    alpha = ld_f32_dependent(tsa) * ld_f32_dependent(tsb);
+template <Kind KIND, typename OutT>
+int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, int splits, bool* launched, cudaStream_t stream) {
+  *launched = false;
+  const int64_t tiles = ceil_div(p.M, kTileM) * ceil_div(p.N, 128);
+  const int k_stages = static_cast<int>(ceil_div(p.k_bytes, kStageKBytes));
+  for (; splits > 1; --splits) {
+    int clusters = 0;
+    if (int rc = split_clusters<KIND, 128, 2, 5, OutT, 1, false>(splits, &clusters)) return rc;
+    if (clusters >= tiles) break;
   }
-  float4 acc = *reinterpret_cast<const float4*>(partials + i);
-  for (int sidx = 1; sidx < splits; ++sidx) {
-    const float4 v = *reinterpret_cast<const float4*>(partials + sidx * mn + i);
-    acc.x += v.x;
-    acc.y += v.y;
-    acc.z += v.z;
-    acc.w += v.w;
-  }
-  const int n = static_cast<int>(i % n_cols);
-  float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  if (bias != nullptr) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = load_bias(bias, bias_dtype, n + j);
-  }
-  const float r[4] = {fmaf(acc.x, alpha, b[0]), fmaf(acc.y, alpha, b[1]), fmaf(acc.z, alpha, b[2]), fmaf(acc.w, alpha, b[3])};
-  if constexpr (std::is_same<OutT, float>::value) {
-    *reinterpret_cast<float4*>(out + i) = make_float4(r[0], r[1], r[2], r[3]);
-  } else {
-    uint2 o;
-    o.x = pack_pair<OutT>(r[0], r[1]);
-    o.y = pack_pair<OutT>(r[2], r[3]);
-    *reinterpret_cast<uint2*>(out + i) = o;
-  }
-}
-
-int launch_splitk_reduce(const float* partials, int splits, int64_t M, int64_t N, const GemmParams& p, cudaStream_t stream) {
-  const int64_t mn = M * N;
-  const dim3 grid(static_cast<unsigned>(ceil_div(mn / 4, 256))), block(256);
-  const int n_cols = static_cast<int>(N);
-  switch (p.out_dtype) {
-    case CK_DTYPE_BF16:
-      CK_CUDA(launch_pdl(splitk_reduce_kernel<__nv_bfloat16>, grid, block, 0, stream, partials, splits, mn, n_cols, p.alpha, p.tsa,
-                         p.tsb, p.bias, p.bias_dtype, static_cast<__nv_bfloat16*>(p.out)));
-      break;
-    case CK_DTYPE_F16:
-      CK_CUDA(launch_pdl(splitk_reduce_kernel<__half>, grid, block, 0, stream, partials, splits, mn, n_cols, p.alpha, p.tsa, p.tsb,
-                         p.bias, p.bias_dtype, static_cast<__half*>(p.out)));
-      break;
-    default:
-      CK_CUDA(launch_pdl(splitk_reduce_kernel<float>, grid, block, 0, stream, partials, splits, mn, n_cols, p.alpha, p.tsa, p.tsb,
-                         p.bias, p.bias_dtype, static_cast<float*>(p.out)));
-  }
-  return CK_OK;
+  if (splits < 2) return CK_OK;
+  p.k_stages_per_split = static_cast<int>(ceil_div(k_stages, splits));
+  p.splits = static_cast<int>(ceil_div(k_stages, p.k_stages_per_split));
+  *launched = true;
+  return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1>(ops, p, os, stream);
 }
 
 struct FusedArgs {
@@ -158,7 +106,7 @@ template <Kind KIND>
 int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
               const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
               int64_t M, int64_t N, int64_t K, void* stream, const FusedArgs& fused = FusedArgs(),
-              const OutputSpec* out_spec = nullptr, void* workspace = nullptr, int64_t workspace_bytes = 0) {
+              const OutputSpec* out_spec = nullptr) {
   CK_REQUIRE(a && b && sfa && sfb, "%s: null pointer", op);
   CK_REQUIRE(out != nullptr || (fused.enabled && fused.rq_codes != nullptr), "%s: no output requested", op);
   if (fused.enabled) {
@@ -227,36 +175,22 @@ int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, con
     os.pitch = N;
     os.col_offset = 0;
   }
-  // Few activation rows: the weight-streaming path (operands swapped, K split over all SMs).
-  // CK_GEMM_CONFIG=9 forces it, any other forced configuration keeps it off.
-  if (!fused.enabled && out_spec == nullptr && small_m_applies(M, N, K) && (forced_config() == 0 || forced_config() == 9)) {
-    return scaled_mm_small_m(KIND == Kind::kMxfp8, a, b, sfa, sfb, tsa, tsb, alpha, bias, bias_dtype, out, out_dtype, M, N, K,
-                             workspace, workspace_bytes, s);
-  }
-  // Split-K for problems with few tiles and a long K (small M): the tiles' K ranges are spread
-  // over otherwise idle SMs as separate work items that store raw fp32 partial tiles to the
-  // caller's workspace; a second kernel adds them in a fixed order and applies alpha and bias.
-  if (workspace != nullptr && !fused.enabled && out_spec == nullptr && forced_config() == 0) {
-    const SplitPlan plan = plan_splits(M, N, p.k_bytes);
-    const int64_t need = kWorkspaceTicketBytes + static_cast<int64_t>(plan.splits) * M * N * 4;
-    if (plan.splits > 1 && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && (N * 4) % 16 == 0) {
-      workspace = static_cast<uint8_t*>(workspace) + kWorkspaceTicketBytes;  // the counters of the small-M path stay untouched
-      GemmParams ps = p;
-      ps.tsa = ps.tsb = ps.alpha = nullptr;
-      ps.bias = nullptr;
-      ps.out = workspace;
-      ps.out_dtype = CK_DTYPE_F32;
-      ps.splits = plan.splits;
-      ps.k_stages_per_split = plan.k_stages_per_split;
-      void* parts[kMaxOutputs] = {};
-      for (int i = 0; i < plan.splits; ++i) parts[i] = static_cast<uint8_t*>(workspace) + static_cast<int64_t>(i) * M * N * 4;
-      OutputSpec ws_spec;
-      ws_spec.ptrs = parts;
-      ws_spec.n = plan.splits;
-      ws_spec.pitch = N;
-      ws_spec.col_offset = 0;
-      if (int rc = launch_config<KIND, 128, 2, 5, 1, float, false, 1>(ops, ps, ws_spec, s)) return rc;
-      return launch_splitk_reduce(static_cast<const float*>(workspace), plan.splits, M, N, p, s);
+  if (!fused.enabled && out_spec == nullptr) {
+    // Few activation rows: the weight-streaming path (operands swapped, K split over all SMs).
+    // CK_GEMM_CONFIG=9 forces it, any other forced configuration keeps it off.
+    if (small_m_applies(M, N, K) && (forced_config() == 0 || forced_config() == 9)) {
+      return scaled_mm_small_m(KIND == Kind::kMxfp8, a, b, sfa, sfb, tsa, tsb, alpha, bias, bias_dtype, out, out_dtype, M, N, K, s);
+    }
+    // the rows of the result are written four columns at a time
+    if (const int splits = max_splits(M, N, p.k_bytes); splits > 1 && forced_config() == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+      bool launched = false;
+      int rc = CK_OK;
+      switch (out_dtype) {
+        case CK_DTYPE_BF16: rc = launch_split<KIND, __nv_bfloat16>(ops, p, os, splits, &launched, s); break;
+        case CK_DTYPE_F16: rc = launch_split<KIND, __half>(ops, p, os, splits, &launched, s); break;
+        default: rc = launch_split<KIND, float>(ops, p, os, splits, &launched, s);
+      }
+      if (rc != CK_OK || launched) return rc;
     }
   }
   if constexpr (KIND == Kind::kNvfp4) {
@@ -314,28 +248,28 @@ extern "C" int ck_linear_nvfp4_fused(const void* a, const void* b, const void* s
                                          bias_dtype, out, out_dtype, M, N, K, stream, f);
 }
 
+// The split-K clusters exchange their partial tiles on chip: the workspace of these entry points is
+// accepted and not used.  The size stays non-zero for the shapes whose K is split.
 extern "C" int64_t ck_scaled_mm_workspace_bytes(int is_mxfp8, int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0 || M >= (1ll << 30) || N >= (1ll << 30) || K >= (1ll << 30)) return 0;
-  if (ck::small_m_applies(M, N, K)) return ck::small_m_workspace_bytes(is_mxfp8 != 0, M, N, K);
-  const ck::SplitPlan plan = ck::plan_splits(M, N, static_cast<int>(is_mxfp8 ? K : K / 2));
-  return plan.splits > 1 ? ck::kWorkspaceTicketBytes + static_cast<int64_t>(plan.splits) * M * N * 4 : 0;
+  const int k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
+  const int splits = ck::small_m_applies(M, N, K) ? ck::small_m_max_splits(N, k_bytes) : ck::max_splits(M, N, k_bytes);
+  return splits > 1 ? 256 : 0;
 }
 
 extern "C" int ck_scaled_mm_nvfp4_ws(const void* a, const void* b, const void* sfa, const void* sfb,
                                      const float* tensor_scale_a, const float* tensor_scale_b, const float* alpha,
                                      const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M, int64_t N,
-                                     int64_t K, void* workspace, int64_t workspace_bytes, void* stream) {
+                                     int64_t K, void* /*workspace*/, int64_t /*workspace_bytes*/, void* stream) {
   return ck::scaled_mm<ck::Kind::kNvfp4>("scaled_mm_nvfp4", a, b, sfa, sfb, tensor_scale_a, tensor_scale_b, alpha, bias,
-                                         bias_dtype, out, out_dtype, M, N, K, stream, ck::FusedArgs(), nullptr, workspace,
-                                         workspace_bytes);
+                                         bias_dtype, out, out_dtype, M, N, K, stream);
 }
 
 extern "C" int ck_scaled_mm_mxfp8_ws(const void* a, const void* b, const void* sfa, const void* sfb, const void* bias,
                                      int bias_dtype, void* out, int out_dtype, int64_t M, int64_t N, int64_t K,
-                                     void* workspace, int64_t workspace_bytes, void* stream) {
+                                     void* /*workspace*/, int64_t /*workspace_bytes*/, void* stream) {
   return ck::scaled_mm<ck::Kind::kMxfp8>("scaled_mm_mxfp8", a, b, sfa, sfb, nullptr, nullptr, nullptr, bias, bias_dtype,
-                                         out, out_dtype, M, N, K, stream, ck::FusedArgs(), nullptr, workspace,
-                                         workspace_bytes);
+                                         out, out_dtype, M, N, K, stream);
 }
 
 extern "C" int ck_scaled_mm_nvfp4_allgather(const void* a, const void* b, const void* sfa, const void* sfb,

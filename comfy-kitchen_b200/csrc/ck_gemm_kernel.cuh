@@ -18,8 +18,9 @@
 //             the accumulator into registers, hand it back at once, then alpha * acc + bias,
 //             convert, stage the rows in swizzled shared memory and write them with TMA stores
 //             while the next tile computes.  The fused variant applies GELU and
-//             re-quantizes to NVFP4 instead; split-K items store raw fp32 partial tiles to a
-//             workspace; the all-gather variant stores every tile into all ranks' results.
+//             re-quantizes to NVFP4 instead; the CTAs of a split-K cluster leave raw fp32 partial
+//             tiles in shared memory, which the cluster adds; the all-gather variant stores every
+//             tile into all ranks' results.
 // With NUM_ACC == 2 the epilogue of tile i overlaps the main loop of tile i+1 entirely.
 //
 // All synchronisation is by mbarriers with bounded waits (ck_sm100.cuh): a protocol error
@@ -118,6 +119,8 @@ struct Config {
                                                              KIND == Kind::kNvfp4 ? 0u : 1u, kTileRows, TILE_N);
 };
 
+constexpr int kMaxSplits = 8;       // CTAs of a split-K cluster (the portable cluster size)
+
 struct GemmParams {
   const uint8_t* sfa;      // A scales, tiled layout, [ceil(M/128)][sf_col_tiles] tiles of 512 bytes
   const uint8_t* sfb;      // B scales, same layout over N
@@ -137,10 +140,8 @@ struct GemmParams {
   int raster;              // order in which workers walk the tiles: 0 = down the rows first, 1 = along the columns first
   int out_tma;             // the output qualifies for TMA stores (16-byte aligned base and pitch)
   int n_out;               // destinations of every output tile (1, or one per GPU of an all-gather)
-  int splits;              // split-K: work items per tile (1 = off); item s of a tile covers pipeline stages
-  int k_stages_per_split;  //   [s * k_stages_per_split, ...) and stores its raw fp32 partial to destination s
-  float* partials;         // swapped-operand split-K: raw fp32 partial tiles, [item][epilogue warp][its slice]
-  unsigned int* tickets;   //   and one arrival counter per tile and epilogue warp (zero between launches)
+  int splits;              // split-K: CTAs per tile (1 = off), one thread-block cluster; CTA s of it covers pipeline stages
+  int k_stages_per_split;  //   [s * k_stages_per_split, ...) and the cluster adds the raw fp32 partial tiles in its shared memory
   int* status;             // device status word: set non-zero when a wait gave up
   int trace_launch;        // sequence number of the launch (timeline builds only)
   // fused epilogue (FUSED kernels only)
@@ -345,10 +346,7 @@ __device__ __forceinline__ float load_bias(const void* bias, int dtype, int n) {
 // [N, K] and "B" (the MMA's N dimension, TILE_N >= M) is the small activation [M, K] - so that a GEMM
 // with few activation rows fills the 128-row MMA dimension with weight rows and streams the weight
 // once.  p.M / p.N are then the weight's and the activation's row counts, the output is written
-// transposed (out[b_row][a_row]), the bias runs along the A rows, and a tile's K range may be split
-// over several CTAs that add their raw fp32 partial tiles through a workspace: every CTA stores its
-// partial and takes a ticket, the one that takes the last ticket adds all partials in split order
-// (deterministic) and writes the result - nobody waits for anybody.
+// transposed (out[b_row][a_row]) and the bias runs along the A rows.
 template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE, bool SWAP = false>
 __global__ void __launch_bounds__(num_threads(FUSED, TILE_N), (SWAP && TILE_N <= 128) ? 2 : 1)
 block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -360,6 +358,9 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   constexpr int kNumEpilogueWarps = epilogue_warps(FUSED, TILE_N);
   constexpr int kThreads = num_threads(FUSED, TILE_N);
   static_assert(TILE_N <= 32 * kNumEpilogueWarps, "one bias value per epilogue thread");
+  // configurations whose tiles may be split along K over the CTAs of a cluster
+  constexpr bool kCanSplit = CTAS == 1 && !FUSED && (SWAP || TILE_N == 128);
+  static_assert(!kCanSplit || kTileM * TILE_N * 4 <= Cfg::kRingBytes, "a partial tile fits in the operand ring");
   // Everything the kernel does until a role's griddepcontrol.wait is independent of the kernel
   // before it in the stream, so the next kernel may be scheduled as early as resources allow.
   pdl_launch_dependents();
@@ -681,7 +682,6 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint32_t tile_it = 0;
     for (int item = worker; item < num_items; item += num_workers, ++tile_it) {
       const int tile = item / splits;
-      const int split = item - tile * splits;
       const int tile_m = tile_row_block(p, tile);
       const int tile_n = tile_col_block(p, tile);
       const int row = tile_m * Cfg::kTileRows + static_cast<int>(cta_rank) * kTileM + quarter * 32 + lane;
@@ -709,53 +709,17 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
         if (warp == 2) CK_TRACE(8);
         if (splits > 1) {
-          // Each epilogue warp settles its own 32 rows x kColsPerWarp slice of the tile with the same
-          // warps of the CTAs that hold the tile's other K ranges: store the raw partial slice (16-byte
-          // units laid out so that the 32 lanes of a store are contiguous), take a ticket of the slice's
-          // counter with release / acquire semantics, and if it was the last one add all partials in
-          // split order.  No CTA-wide barrier, no waiting.
-          constexpr int kUnits = kColsPerWarp / 4;                      // 16-byte units per row of the slice
-          constexpr int kSliceFloats = 32 * kColsPerWarp;
-          const int slice = warp - 2;
-          const auto slice_of = [&](int it) {
-            return p.partials + (static_cast<int64_t>(it) * kNumEpilogueWarps + slice) * kSliceFloats;
-          };
-          float4* mine = reinterpret_cast<float4*>(slice_of(item));
-#pragma unroll
-          for (int u = 0; u < kUnits; ++u) {
-            const int c = u / 8, j = u % 8;
-            mine[u * 32 + lane] = make_float4(__uint_as_float(buf[c][4 * j]), __uint_as_float(buf[c][4 * j + 1]),
-                                              __uint_as_float(buf[c][4 * j + 2]), __uint_as_float(buf[c][4 * j + 3]));
-          }
-          __syncwarp();  // the lanes' stores are ordered before lane 0's release below
-          unsigned int ticket = 0;
-          unsigned int* counter = p.tickets + tile * kNumEpilogueWarps + slice;
-          if (lane == 0) {
-            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
-            if (ticket == static_cast<unsigned int>(splits - 1)) *counter = 0;  // all arrived: ready for the next launch
-          }
-          ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-          if (warp == 2) CK_TRACE(12);
-          if (ticket != static_cast<unsigned int>(splits - 1)) continue;
+          // Raw partial to the CTA's own shared memory, [column][128 rows]; added below by the cluster.
+          float* part = reinterpret_cast<float*>(smem) + r_in_tile;
 #pragma unroll
           for (int c = 0; c < kChunks; ++c) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) buf[c][i] = 0u;
-          }
-          for (int sidx = 0; sidx < splits; ++sidx) {
-            const float4* theirs = reinterpret_cast<const float4*>(slice_of(tile * splits + sidx));
-            float4 t[kUnits];
-#pragma unroll
-            for (int u = 0; u < kUnits; ++u) t[u] = __ldcg(theirs + u * 32 + lane);
-#pragma unroll
-            for (int u = 0; u < kUnits; ++u) {
-              const int c = u / 8, j = u % 8;
-              buf[c][4 * j + 0] = __float_as_uint(__uint_as_float(buf[c][4 * j + 0]) + t[u].x);
-              buf[c][4 * j + 1] = __float_as_uint(__uint_as_float(buf[c][4 * j + 1]) + t[u].y);
-              buf[c][4 * j + 2] = __float_as_uint(__uint_as_float(buf[c][4 * j + 2]) + t[u].z);
-              buf[c][4 * j + 3] = __float_as_uint(__uint_as_float(buf[c][4 * j + 3]) + t[u].w);
+            for (int i = 0; i < 32; ++i) {
+              const int col = c0 + c * 32 + i;
+              if (n0 + col < p.N) part[col * kTileM] = __uint_as_float(buf[c][i]);
             }
           }
+          continue;
         }
         if (warp == 2) CK_TRACE(13);
         if (a_row < p.M) {
@@ -791,7 +755,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // fetches one value of the next tile before it waits for the accumulator, so the load's
       // latency hides behind that wait.
       float* bias_s = smem_bias + (tile_it % 3) * TILE_N;
-      const bool with_bias = p.bias != nullptr && splits == 1;
+      const bool with_bias = p.bias != nullptr;
       if (tile_it == 0) {
         if (et < TILE_N) bias_s[et] = (with_bias && n0 + et < p.N) ? load_bias(p.bias, p.bias_dtype, n0 + et) : 0.0f;
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNumEpilogueWarps) : "memory");  // epilogue warps only
@@ -841,6 +805,23 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           mbar_arrive_cluster(acc_empty_leader + acc * 8);  // the leader's barrier counts both CTAs' warps
         } else {
           mbar_arrive(&acc_empty_bar[acc]);
+        }
+      }
+      if constexpr (kCanSplit) {
+        if (splits > 1) {
+          // Raw partial to the CTA's own shared memory: row r at r * TILE_N * 4 bytes, its 16-byte unit u
+          // at position u ^ (r % 8) (the eight rows of a store phase meet eight different bank groups).
+          const int r = quarter * 32 + lane;
+          const uint32_t part_row = smem_u32(smem) + r * (TILE_N * 4);
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int u = (c0 + c * 32) / 4 + j;
+              st_shared_128(part_row + ((u ^ (r & 7)) << 4), buf[c][4 * j], buf[c][4 * j + 1], buf[c][4 * j + 2], buf[c][4 * j + 3]);
+            }
+          }
+          continue;
         }
       }
       if (has_next) {
@@ -911,12 +892,8 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 __syncwarp();
                 const int col = n0 + c0 + (c / kChunksPerBox) * kBoxCols;
                 if (lane == 0 && row0 < p.M && col < p.N) {
-                  if (splits > 1) {
-                    tma_store_2d_addr(&maps_out.m[split], stage_box, col, row0);  // this item's partial
-                  } else {
-                    // the same staged box goes to every destination (peer stores cross NVLink)
-                    for (int d = 0; d < p.n_out; ++d) tma_store_2d_addr(&maps_out.m[d], stage_box, col, row0);
-                  }
+                  // the same staged box goes to every destination (peer stores cross NVLink)
+                  for (int d = 0; d < p.n_out; ++d) tma_store_2d_addr(&maps_out.m[d], stage_box, col, row0);
                 }
                 // (an empty group when nothing was stored keeps the ring's group count in step)
                 if (lane == 0) bulk_commit_group();
@@ -1058,6 +1035,110 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           bulk_wait_group_read0();
         }
       }
+    }
+  }
+
+  // ------------------------------------------------------------------ split-K: the cluster adds its partial tiles
+  // Every CTA of the cluster ran one item (the host launches tiles * splits CTAs); its partial lies in
+  // its own operand ring, which is idle: all loads have landed and all MMAs have retired before the
+  // accumulator was published.  Each CTA reads its share of the tile from all of them over distributed
+  // shared memory and adds in split order, so the result does not depend on scheduling; no workspace,
+  // no second kernel, no counters to keep zero - and so the one-call linears split as well.  Measured
+  // against partial tiles through L2 (graph replays, us; linear = quantize + GEMM in one call, which
+  // had no workspace and ran unsplit): MXFP8 1 x 3072 x 12288 linear 30.1 -> 12.5, 256 rows 33.0 -> 24.4;
+  // NVFP4 1 x 1024 x 15360 GEMM 8.7 -> 6.3, linear 21.8 -> 8.1; 64 x 3072 x 12288 11.3 -> 9.6.  A cluster
+  // must find its SMs in one part of the chip: where three CTAs per tile no longer fit at once, two are
+  // used (256 x 3072 x 12288 GEMM: 13.0 -> 14.4 with NVFP4, 17.0 -> 20.8 with MXFP8).
+  if constexpr (kCanSplit) {
+    if (splits > 1) {
+      __syncwarp();
+      cluster_sync_all();
+      if (warp >= 2) {
+        const int rank = static_cast<int>(cluster_cta_rank());
+        const int tile = worker / splits;
+        const uint32_t part = smem_u32(smem);
+        float alpha = 1.0f;
+        if (p.alpha != nullptr) {
+          alpha = ld_f32_dependent(p.alpha);
+        } else if (p.tsa != nullptr && p.tsb != nullptr) {
+          alpha = ld_f32_dependent(p.tsa) * ld_f32_dependent(p.tsb);
+        }
+        uint32_t base[kMaxSplits];
+#pragma unroll
+        for (int i = 0; i < kMaxSplits; ++i) base[i] = map_to_cta(part, i < splits ? i : 0);
+        if constexpr (SWAP) {
+          // a unit = 32 weight rows (a coalesced run of the output) of one activation row
+          OutT* out = static_cast<OutT*>(p.out);
+          const int units = 4 * p.N;
+          for (int u = rank + splits * (warp - 2); u < units; u += splits * kNumEpilogueWarps) {
+            const int col = u >> 2;
+            const int r = (u & 3) * 32 + lane;
+            const int a_row = tile_row_block(p, tile) * kTileM + r;
+            const float bias_v = (p.bias != nullptr && a_row < p.M) ? load_bias(p.bias, p.bias_dtype, a_row) : 0.0f;
+            float v[kMaxSplits];
+#pragma unroll
+            for (int i = 0; i < kMaxSplits; ++i) {
+              if (i < splits) v[i] = ld_shared_cluster_f32(base[i] + (col * kTileM + r) * 4);
+            }
+            float acc = v[0];
+#pragma unroll
+            for (int i = 1; i < kMaxSplits; ++i) {
+              if (i < splits) acc += v[i];
+            }
+            const float y = fmaf(acc, alpha, bias_v);
+            if (a_row < p.M) {
+              OutT* dst = out + static_cast<int64_t>(col) * p.M + a_row;
+              if constexpr (std::is_same<OutT, __nv_bfloat16>::value) {
+                *dst = __float2bfloat16_rn(y);
+              } else if constexpr (std::is_same<OutT, __half>::value) {
+                *dst = __float2half_rn(y);
+              } else {
+                *dst = y;
+              }
+            }
+          }
+        } else {
+          // a warp takes one row of the tile, a lane four neighbouring columns
+          const int row0 = tile_row_block(p, tile) * kTileM;
+          const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
+          const bool in_cols = col < p.N;  // N % 8 == 0: a group of four never straddles the edge
+          float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          if (p.bias != nullptr && in_cols) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = load_bias(p.bias, p.bias_dtype, col + j);
+          }
+          const int rows = min(kTileM, p.M - row0);
+          for (int r = rank + splits * (warp - 2); r < rows; r += splits * kNumEpilogueWarps) {
+            const uint32_t off = r * (TILE_N * 4) + ((lane ^ (r & 7)) << 4);
+            float4 v[kMaxSplits];
+#pragma unroll
+            for (int i = 0; i < kMaxSplits; ++i) {
+              if (i < splits) v[i] = ld_shared_cluster_f32x4(base[i] + off);
+            }
+            float4 acc = v[0];
+#pragma unroll
+            for (int i = 1; i < kMaxSplits; ++i) {
+              if (i < splits) {
+                acc.x += v[i].x;
+                acc.y += v[i].y;
+                acc.z += v[i].z;
+                acc.w += v[i].w;
+              }
+            }
+            const float y[4] = {fmaf(acc.x, alpha, b[0]), fmaf(acc.y, alpha, b[1]), fmaf(acc.z, alpha, b[2]), fmaf(acc.w, alpha, b[3])};
+            if (in_cols) {
+              OutT* dst = static_cast<OutT*>(p.out) + static_cast<int64_t>(row0 + r) * p.N + col;
+              if constexpr (sizeof(OutT) == 2) {
+                *reinterpret_cast<uint2*>(dst) = make_uint2(pack_pair<OutT>(y[0], y[1]), pack_pair<OutT>(y[2], y[3]));
+              } else {
+                *reinterpret_cast<float4*>(dst) = make_float4(y[0], y[1], y[2], y[3]);
+              }
+            }
+          }
+        }
+      }
+      __syncwarp();
+      cluster_sync_all();  // no CTA leaves while another may still read its partial
     }
   }
 
@@ -1218,6 +1299,36 @@ struct Operands {
   const void* b;
 };
 
+// Clusters of `splits` CTAs of this configuration that can run at once on the current device.
+template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, typename OutT, int OUT_STAGE, bool SWAP>
+int split_clusters(int splits, int* out) {
+  using Cfg = Config<KIND, TILE_N, NUM_ACC, STAGES, 1, OUT_STAGE>;
+  static std::atomic<int> cached[64][kMaxSplits + 1];
+  int dev = 0;
+  CK_CUDA(cudaGetDevice(&dev));
+  int n = (dev >= 0 && dev < 64) ? cached[dev][splits].load(std::memory_order_relaxed) : 0;
+  if (n == 0) {
+    auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, 1, OutT, false, OUT_STAGE, SWAP>;
+    CK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(num_threads(false, TILE_N));
+    cfg.gridDim = dim3(static_cast<unsigned>(sm_count() / splits * splits));
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+    if (n < 1) n = 1;
+    if (dev >= 0 && dev < 64) cached[dev][splits].store(n, std::memory_order_relaxed);
+  }
+  *out = n;
+  return CK_OK;
+}
+
 template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE = 0, bool SWAP = false>
 int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaStream_t stream) {
   using Cfg = Config<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OUT_STAGE>;
@@ -1242,7 +1353,7 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS;
+  attr[0].val.clusterDim.x = CTAS == 1 ? p.splits : CTAS;  // split-K: the CTAs of one tile are a cluster
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1264,6 +1375,7 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
     if (dev >= 0 && dev < 64) max_workers[dev].store(resident, std::memory_order_release);
   }
   int workers = min(p.tiles_m * p.tiles_n * p.splits, resident);
+  if (p.splits > 1) workers = p.tiles_m * p.tiles_n * p.splits;  // one item per CTA
 #ifdef CK_GEMM_TRACE
   if (const char* e = getenv("CK_GEMM_MAX_WORKERS")) workers = min(workers, atoi(e));
   static std::atomic<int> launch_seq{0};
@@ -1293,14 +1405,13 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
     // TMA stores need 16-byte aligned bases and row pitch.  A single dense [M, N] result whose rows
     // start on 32-byte boundaries is written straight from registers instead (256-bit stores, whole
     // sectors): measured 1-3 % faster than staging it for TMA stores, whose shared-memory traffic
-    // slows the next tile's main loop.  Partial tiles of a split and multi-destination stores
-    // (all-gather) go through the staged path.
+    // slows the next tile's main loop.  Multi-destination stores (all-gather) go through the staged path.
     bool ok = p.out != nullptr && (os.pitch * static_cast<int64_t>(sizeof(OutT))) % 16 == 0 &&
               (os.col_offset * static_cast<int64_t>(sizeof(OutT))) % 16 == 0;
     for (int d = 0; ok && d < os.n; ++d) ok = os.ptrs[d] != nullptr && reinterpret_cast<uintptr_t>(os.ptrs[d]) % 16 == 0;
-    const bool direct = os.n == 1 && p.splits == 1 && os.plain(p.N) && p.out != nullptr &&
+    const bool direct = os.n == 1 && os.plain(p.N) && p.out != nullptr &&
                         (static_cast<int64_t>(p.N) * sizeof(OutT)) % 32 == 0 && reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
-    ok = ok && !direct;
+    ok = ok && !direct && p.splits == 1;  // a split-K cluster writes its result itself
     if (ok) {
       for (int d = 0; d < os.n; ++d) {
         void* base = static_cast<uint8_t*>(os.ptrs[d]) + os.col_offset * static_cast<int64_t>(sizeof(OutT));
