@@ -28,6 +28,7 @@ __all__ = [
     "linear_nvfp4_from_float",
     "linear_mxfp8_from_float",
     "nvfp4_tensor_scale",
+    "quantize_nvfp4_dynamic",
     "check_device_status",
 ]
 
@@ -49,6 +50,8 @@ _SIGNATURES = {
     "ck_device_supported": [_I],
     "ck_debug_set_exact_division": [_I],
     "ck_quantize_nvfp4": [_P, _I, _P, _P, _P, _L, _L, _L, _L, _I, _P],
+    "ck_quantize_nvfp4_dynamic_scratch_bytes": [_L],
+    "ck_quantize_nvfp4_dynamic": [_P, _I, _P, _P, _P, _L, _L, _L, _L, _I, _P, _L, _P],
     "ck_quantize_mxfp8": [_P, _I, _P, _P, _L, _L, _L, _L, _P],
     "ck_scaled_mm_nvfp4": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _L, _L, _L, _P],
     "ck_scaled_mm_mxfp8": [_P, _P, _P, _P, _P, _I, _P, _I, _L, _L, _L, _P],
@@ -74,6 +77,7 @@ _SIGNATURES = {
     "ck_dequantize_mxfp8": [_P, _P, _P, _I, _L, _L, _P],
 }
 _RESTYPE = {"ck_last_error": ctypes.c_char_p, "ck_nvfp4_tensor_scale_scratch_bytes": ctypes.c_int64,
+            "ck_quantize_nvfp4_dynamic_scratch_bytes": ctypes.c_int64,
             "ck_scaled_mm_workspace_bytes": ctypes.c_int64, "ck_linear_nvfp4_from_float_workspace_bytes": ctypes.c_int64,
             "ck_linear_mxfp8_from_float_workspace_bytes": ctypes.c_int64}
 
@@ -246,6 +250,31 @@ def nvfp4_tensor_scale(x: torch.Tensor) -> torch.Tensor:
         _check(lib.ck_nvfp4_tensor_scale(_ptr(x), DTYPE_TO_CODE[x.dtype], n, _ptr(out), _ptr(scratch), scratch.numel(),
                                          stream), "nvfp4_tensor_scale")
     return out
+
+
+def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
+                           hi_first: bool = True) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """``scale = nvfp4_tensor_scale(x)`` and ``quantize_nvfp4(x, scale)`` in one library call (same bits):
+    ``(codes, block_scales, scale)``.  The reduction leaves partial maxima that the quantizer finishes."""
+    lib = load_library()
+    x = _plain(x)
+    assert x.is_contiguous(), "Input tensor must be contiguous"
+    rows, cols = x.shape
+    if pad_16x:
+        out_rows, out_cols = roundup(rows, 16), roundup(cols, 16)
+    else:
+        out_rows, out_cols = rows, cols
+        assert out_cols % 16 == 0, f"num_cols must be divisible by 16, got {out_cols}"
+    stream = _stream(x.device)
+    scratch = _scale_scratch_for(x.device, stream, lib.ck_quantize_nvfp4_dynamic_scratch_bytes(rows * cols))
+    scale = torch.empty((), dtype=torch.float32, device=x.device)
+    qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
+    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.uint8)
+    with _on_device(x.device):
+        _check(lib.ck_quantize_nvfp4_dynamic(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(scale), _ptr(qx), _ptr(sx), rows, cols, out_rows,
+                                             out_cols, int(bool(hi_first)), _ptr(scratch), scratch.numel(), stream),
+               "quantize_nvfp4_dynamic")
+    return qx, sx.view(torch.float8_e4m3fn), scale
 
 
 def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_scales: torch.Tensor,
@@ -456,7 +485,7 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     if ws is None or ws.numel() < need:
         if ws is not None:
             _retired_workspaces.append(ws)
-        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
+        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=dev)
         _linear_workspaces[key] = ws
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
@@ -486,7 +515,7 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     out_dtype = out_dtype or (x.dtype if x.dtype in (torch.float16, torch.bfloat16) else torch.bfloat16)
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     need = int(lib.ck_linear_mxfp8_from_float_workspace_bytes(m, k))
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream, "mxfp8")  # not shared with the NVFP4 path (its zeroed head)
+    key = (dev, torch.cuda.current_stream(dev).cuda_stream, "mxfp8")
     ws = _linear_workspaces.get(key)
     if ws is None or ws.numel() < need:
         if ws is not None:

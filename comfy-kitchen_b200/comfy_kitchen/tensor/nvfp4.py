@@ -46,17 +46,16 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
         if tensor.dim() != 2:
             raise ValueError(f"NVFP4 requires 2D tensor, got {tensor.dim()}D")
         orig_shape = tuple(tensor.shape)
+        pad = cls.get_padded_shape(orig_shape) != orig_shape
+        backend = direct_backend(tensor) if tensor.is_contiguous() else None
         if scale is None or (isinstance(scale, str) and scale == "recalculate"):
-            fused = direct_backend(tensor) if tensor.is_contiguous() else None
-            if fused is not None and tensor.dtype in (torch.bfloat16, torch.float16, torch.float32):
-                scale = fused.nvfp4_tensor_scale(tensor)  # one kernel for abs, amax and the division
-            else:
-                scale = torch.amax(tensor.abs()) / (F8_E4M3_MAX * F4_E2M1_MAX)
+            if backend is not None and tensor.dtype in (torch.bfloat16, torch.float16, torch.float32) and tensor.numel() > 0:
+                qdata, block_scale, scale = backend.quantize_nvfp4_dynamic(tensor, pad_16x=pad)
+                return qdata, cls.Params(scale=scale, orig_dtype=tensor.dtype, orig_shape=orig_shape, block_scale=block_scale)
+            scale = torch.amax(tensor.abs()) / (F8_E4M3_MAX * F4_E2M1_MAX)
         if not isinstance(scale, torch.Tensor):
             scale = torch.tensor(scale)
         scale = scale.to(device=tensor.device, dtype=torch.float32)
-        pad = cls.get_padded_shape(orig_shape) != orig_shape
-        backend = direct_backend(tensor) if tensor.is_contiguous() else None
         if backend is not None:
             qdata, block_scale = backend.quantize_nvfp4(tensor, scale, pad_16x=pad)
         else:

@@ -8,7 +8,7 @@
 // the partials, writes the scale and resets the counter, so the scratch area needs to be
 // zeroed only once, before its first use.  Scratch layout: word 0 = ticket counter,
 // words 64.. = one float per block (the gap keeps the counter on its own 256-byte line).
-#include "ck_common.cuh"
+#include "ck_quant_math.cuh"
 
 #include <mutex>
 #include <type_traits>
@@ -21,39 +21,7 @@ constexpr int kElemsPerThread = 64;
 constexpr int kChunk = kThreads * kElemsPerThread;  // elements per block
 constexpr int kPartialOffset = 64;                  // words
 
-template <typename T>
-__device__ __forceinline__ float round_to_input_dtype(float v) {
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    return __bfloat162float(__float2bfloat16_rn(v));
-  } else if constexpr (std::is_same<T, __half>::value) {
-    return __half2float(__float2half_rn(v));
-  } else {
-    return v;
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ float abs_max_of_vec(const Vec256& raw) {
-  float m = 0.0f;
-  if constexpr (sizeof(T) == 2) {
-    // |x| of a 16-bit float is its bit pattern without the sign, and for non-negative
-    // floats of one format the integer order of the bit patterns is the numeric order:
-    // reduce the eight packed pairs as unsigned 16-bit integers, convert once.
-    uint32_t p = raw.w[0] & 0x7FFF7FFFu;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) p = __vmaxu2(p, raw.w[i] & 0x7FFF7FFFu);
-    const uint32_t top = max(p & 0xFFFFu, p >> 16);
-    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      m = __uint_as_float(top << 16);
-    } else {
-      m = __half2float(__ushort_as_half(static_cast<unsigned short>(top)));
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(__uint_as_float(raw.w[i])));
-  }
-  return m;
-}
+using quant::abs_max_of_vec;
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -123,9 +91,43 @@ nvfp4_tensor_scale_kernel(const T* x, int64_t n, float* scale_out, unsigned int*
     float amax = warp_max[0];
 #pragma unroll
     for (int w = 1; w < kThreads / 32; ++w) amax = fmaxf(amax, warp_max[w]);
-    // amax / (448 * 6) in the input dtype (a true division, then rounded), then float32
-    *scale_out = round_to_input_dtype<T>(__fdiv_rn(amax, 2688.0f));
+    *scale_out = quant::nvfp4_scale_of_amax<T>(amax);
     scratch[0] = 0;  // ready for the next call
+  }
+}
+
+// Reduction pass in front of a quantizer that finishes the maximum itself (ck_quantize.cu): one partial
+// maximum per block, no arrival counter and no last block to wait for, and so no scratch that has to
+// start at zero.  The grid is what fits the device (four blocks per SM), each block strides over the
+// input with eight 256-bit loads per thread in flight.
+constexpr int kPartialVecs = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 4)
+amax_partials_kernel(const T* x, int64_t n_vecs, float* partials) {
+  constexpr int kPerVec = 32 / sizeof(T);
+  pdl_launch_dependents();
+  float m = 0.0f;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * kPartialVecs;
+  pdl_wait();  // x may be the output of the kernel before this one
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * kThreads * kPartialVecs + threadIdx.x; base < n_vecs; base += step) {
+    Vec256 raw[kPartialVecs];
+#pragma unroll
+    for (int v = 0; v < kPartialVecs; ++v) {
+      raw[v] = base + v * kThreads < n_vecs ? ld_global_stream_256(x + (base + v * kThreads) * kPerVec) : Vec256{};
+    }
+#pragma unroll
+    for (int v = 0; v < kPartialVecs; ++v) m = fmaxf(m, abs_max_of_vec<T>(raw[v]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  __shared__ float warp_max[kThreads / 32];
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < kThreads / 32; ++w) m = fmaxf(m, warp_max[w]);
+    partials[blockIdx.x] = m;
   }
 }
 
@@ -190,6 +192,22 @@ int static_scratch_for_device(unsigned int** out) {
 }
 
 }  // namespace
+
+int64_t amax_partials_max() { return 4 * static_cast<int64_t>(sm_count()); }
+
+int launch_amax_partials(const void* x, int dtype, int64_t n_vecs, float* partials, int* n_partials, cudaStream_t s) {
+  const int64_t blocks = ceil_div(n_vecs, static_cast<int64_t>(kThreads) * kPartialVecs);
+  const int64_t grid = blocks < amax_partials_max() ? blocks : amax_partials_max();
+  *n_partials = static_cast<int>(grid);
+  const dim3 g(static_cast<unsigned>(grid)), b(kThreads);
+  switch (dtype) {
+    case CK_DTYPE_BF16: CK_CUDA(launch_pdl(amax_partials_kernel<__nv_bfloat16>, g, b, 0, s, static_cast<const __nv_bfloat16*>(x), n_vecs, partials)); break;
+    case CK_DTYPE_F16: CK_CUDA(launch_pdl(amax_partials_kernel<__half>, g, b, 0, s, static_cast<const __half*>(x), n_vecs, partials)); break;
+    default: CK_CUDA(launch_pdl(amax_partials_kernel<float>, g, b, 0, s, static_cast<const float*>(x), n_vecs, partials));
+  }
+  return CK_OK;
+}
+
 }  // namespace ck
 
 extern "C" int ck_nvfp4_tensor_scale_noalloc(const void* input, int input_dtype, int64_t num_elements,

@@ -2,7 +2,7 @@
 //
 // The layout path of the reference runs this as separate operator calls
 // (comfy_kitchen/tensor/nvfp4.py:51-82 quantize, then :214-264 linear), each with its own
-// Python dispatch.  Here the three kernels are enqueued by one C call, chained with
+// Python dispatch.  Here the kernels are enqueued by one C call, chained with
 // programmatic dependent launch; the quantized activation lives in a caller-owned workspace
 // and is still in L2 when the GEMM's loads start.
 #include "ck_common.cuh"
@@ -15,8 +15,6 @@ struct FromFloatLayout {
 };
 
 // Workspace layout: tensor-scale scratch | dynamic tensor scale | codes [M, K/2] | tiled block scales.
-// The scratch comes first and has a fixed size: it must read as zero at the start of every call, and
-// only a region that no other part of any shape's layout ever overlaps stays that way.
 constexpr int64_t kScaleScratchBytes = 256 * 1024;  // covers 2^30 elements
 
 FromFloatLayout from_float_layout(int64_t M, int64_t K) {
@@ -34,7 +32,7 @@ FromFloatLayout from_float_layout(int64_t M, int64_t K) {
 
 extern "C" int64_t ck_linear_nvfp4_from_float_workspace_bytes(int64_t M, int64_t K, int dynamic_scale) {
   if (M <= 0 || K <= 0 || K % 32 != 0 || M >= (1ll << 30) || K >= (1ll << 30)) return 0;
-  if (dynamic_scale != 0 && ck_nvfp4_tensor_scale_scratch_bytes(M * K) > ck::kScaleScratchBytes) return 0;
+  if (dynamic_scale != 0 && ck_quantize_nvfp4_dynamic_scratch_bytes(M * K) > ck::kScaleScratchBytes) return 0;
   return ck::from_float_layout(M, K).total;
 }
 
@@ -48,7 +46,7 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
   CK_REQUIRE(K % 32 == 0, "linear_nvfp4_from_float: K=%lld must be a multiple of 32", (long long)K);
   CK_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 256 == 0, "linear_nvfp4_from_float: workspace must be 256-byte aligned");
   const bool dynamic = x_scale == nullptr;
-  CK_REQUIRE(!dynamic || ck_nvfp4_tensor_scale_scratch_bytes(M * K) <= kScaleScratchBytes,
+  CK_REQUIRE(!dynamic || ck_quantize_nvfp4_dynamic_scratch_bytes(M * K) <= kScaleScratchBytes,
              "linear_nvfp4_from_float: %lld x %lld elements are too many for the dynamic scale of this entry point",
              (long long)M, (long long)K);
   const FromFloatLayout l = from_float_layout(M, K);
@@ -60,10 +58,13 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
   const float* scale = x_scale;
   if (dynamic) {
     float* dyn = reinterpret_cast<float*>(ws + l.scale_off);
-    if (int rc = ck_nvfp4_tensor_scale(x, x_dtype, M * K, dyn, ws + l.scratch_off, kScaleScratchBytes, stream)) return rc;
+    if (int rc = ck_quantize_nvfp4_dynamic(x, x_dtype, dyn, codes, scales, M, K, M, K, /*hi_first=*/1, ws + l.scratch_off,
+                                           kScaleScratchBytes, stream))
+      return rc;
     scale = dyn;
+  } else if (int rc = ck_quantize_nvfp4(x, x_dtype, scale, codes, scales, M, K, M, K, /*hi_first=*/1, stream)) {
+    return rc;
   }
-  if (int rc = ck_quantize_nvfp4(x, x_dtype, scale, codes, scales, M, K, M, K, /*hi_first=*/1, stream)) return rc;
   return ck_scaled_mm_nvfp4(codes, w_codes, scales, w_block_scales, scale, w_scale, nullptr, bias, bias_dtype, out,
                             out_dtype, M, N, K, stream);
 }

@@ -319,5 +319,48 @@ __device__ __forceinline__ void nvfp4_block_packed(const uint32_t (&w)[8], const
   scale_byte = r.scale_byte;
 }
 
+// ---------------------------------------------------------------------------
+// dynamic per-tensor scale
+// ---------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ float round_to_input_dtype(float v) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    return __bfloat162float(__float2bfloat16_rn(v));
+  } else if constexpr (std::is_same<T, __half>::value) {
+    return __half2float(__float2half_rn(v));
+  } else {
+    return v;
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ float abs_max_of_vec(const Vec256& raw) {
+  float m = 0.0f;
+  if constexpr (sizeof(T) == 2) {
+    // |x| of a 16-bit float is its bit pattern without the sign, and for non-negative
+    // floats of one format the integer order of the bit patterns is the numeric order:
+    // reduce the eight packed pairs as unsigned 16-bit integers, convert once.
+    uint32_t p = raw.w[0] & 0x7FFF7FFFu;
+#pragma unroll
+    for (int i = 1; i < 8; ++i) p = __vmaxu2(p, raw.w[i] & 0x7FFF7FFFu);
+    const uint32_t top = max(p & 0xFFFFu, p >> 16);
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      m = __uint_as_float(top << 16);
+    } else {
+      m = __half2float(__ushort_as_half(static_cast<unsigned short>(top)));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(__uint_as_float(raw.w[i])));
+  }
+  return m;
+}
+
+// The dynamic per-tensor scale: amax / (448 * 6) in the input dtype (a true division, then rounded), then float32.
+template <typename T>
+__device__ __forceinline__ float nvfp4_scale_of_amax(float amax) {
+  return round_to_input_dtype<T>(__fdiv_rn(amax, 2688.0f));
+}
+
 }  // namespace quant
 }  // namespace ck

@@ -126,69 +126,143 @@ quantize_nvfp4_kernel(const T* x, const float* global_scale, uint8_t* __restrict
   store_scale_quad(scales, row, sc, sc_pad >> 2, scale_byte, sc < sc_pad);
 }
 
-// Streaming variant for 16-bit inputs whose rows are whole pairs of scale blocks (32
-// elements) and need no padding of the data: a thread owns two adjacent blocks of one row
-// (two 256-bit loads, one 128-bit code store), the two lanes that share a 4-byte scale group
-// merge with one shuffle, per-thread constants (tensor scale, its reciprocal) are set up
-// once, and a block of 32 x 8 threads walks row groups with a grid stride so that every SM
-// holds the same amount of work.
-constexpr int kPairRows = 16;  // rows per thread block; 32 lanes x 2 blocks x 16 = 1024 columns per warp
+// Where a launch of the streaming quantizer takes its per-tensor scale from.
+struct ScaleSource {
+  const float* given;      // static scale, or null: amax(|x|) / 2688 of this very input, from
+  const float* partials;   //   the maxima a reduction pass left (ck_amax.cu), or, when there are none,
+  int n_partials;          //   the whole (small) input, which every block then reads for itself
+  int64_t n_vecs;          // 32-byte units of the input
+  float* out;              // the dynamic scale for whoever needs it next
+};
 
-template <typename T, bool kHiFirst>
+// amax(|x|) / (448 * 6) of the whole input, by every block for itself (all threads return it).  NaNs
+// are dropped the way nvfp4_tensor_scale_kernel drops them: both reduce the same 32-byte units.
+template <typename T>
+__device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSource& src, int tid, int threads) {
+  float m = 0.0f;
+  if (src.n_partials > 0) {
+    for (int i = tid; i < src.n_partials; i += threads) m = fmaxf(m, ld_f32_dependent(src.partials + i));
+  } else {
+    constexpr int kPerVec = 32 / sizeof(T);
+    for (int64_t i = tid; i < src.n_vecs; i += 4 * threads) {
+      Vec256 raw[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        raw[j] = i + j * threads < src.n_vecs ? ld_global_stream_256(x + (i + j * threads) * kPerVec) : Vec256{};
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) m = fmaxf(m, abs_max_of_vec<T>(raw[j]));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  __shared__ float warp_max[32];
+  if ((tid & 31) == 0) warp_max[tid >> 5] = m;
+  __syncthreads();
+  m = (tid & 31) < threads / 32 ? warp_max[tid & 31] : 0.0f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  return nvfp4_scale_of_amax<T>(m);
+}
+
+// Streaming kernel for inputs whose rows are whole 64-byte units (two scale blocks of a 16-bit type,
+// one of fp32) and whose columns need no padding: a thread owns one unit of one row (two 256-bit
+// loads, one 128- or 64-bit code store), the lanes that share a 4-byte scale group merge by shuffle,
+// per-thread constants (tensor scale, its reciprocal) are set up once, and a block of 32 x kPairRows
+// threads walks row groups with a grid stride so that every SM holds the same amount of work.  Rows
+// past data_rows (padding) have zero codes and scales.
+//
+// The row groups are walked from the last to the first.  With a dynamic scale the reduction pass has
+// just read the input front to back, and what L2 still holds of it is its end; the GEMM that follows
+// starts with the first rows, the ones written last here.
+//
+// Bound by HBM for large inputs and by launches and latency for small ones: finishing the dynamic scale
+// here takes the reduction's last-block tail (and for small inputs the reduction kernel) off the chain.
+// Measured, whole calls: 8 x 3072 dynamic linear 39.5 -> 34.8 us; 1003 padded rows through the tensor
+// subclass 86.3 -> 70.5 (padded rows took scalar loads before: 6.4 us for 6 MB); an fp32 weight of
+// 12288 x 3072 with its dynamic scale 56.8 -> 52.4.
+constexpr int kPairRows = 16;  // rows per thread block
+
+template <typename T, bool kHiFirst, bool kDynamic>
 __global__ void __launch_bounds__(32 * kPairRows, 2)
-quantize_nvfp4_pair_kernel(const T* x, const float* global_scale,
-                           uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int rows, int cols,
-                           int rows_pad, int sc_pad, int row_groups) {
+quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
+                             int data_rows, int rows, int cols, int rows_pad, int sc_pad, int row_groups) {
+  constexpr int kElems = 64 / sizeof(T);  // elements of a thread's unit
+  constexpr int kBlocks = kElems / 16;    // scale blocks of a thread's unit
   pdl_launch_dependents();
-  const int pc = blockIdx.y * 32 + threadIdx.x;  // scale columns 2*pc and 2*pc + 1
-  const bool has_data = pc < (cols >> 5);
-  const bool has_scale = (threadIdx.x & 1) == 0 && 2 * pc < sc_pad;
+  const int pc = blockIdx.y * 32 + threadIdx.x;  // unit within the row
+  const bool has_data = pc < cols / kElems;
+  const bool has_scale = (threadIdx.x & (4 / kBlocks - 1)) == 0 && kBlocks * pc < sc_pad;
   // Ahead of the dependency wait: ask L2 for this block's first two row groups.  A prefetch only
   // warms the cache (L2 is the point of coherence: what the previous kernel still writes is seen
   // by the loads after the wait), and it takes the DRAM latency of the first loads off the
   // critical path of a kernel that only runs for a few microseconds.
+  const int first = row_groups - 1 - static_cast<int>(blockIdx.x);
   if (has_data && (threadIdx.x & 1) == 0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int row = (blockIdx.x + i * gridDim.x) * kPairRows + threadIdx.y;
-      if (row < rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * 32);  // one 128-byte line per lane pair
+      const int row = (first - i * static_cast<int>(gridDim.x)) * kPairRows + static_cast<int>(threadIdx.y);
+      if (row >= 0 && row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
     }
   }
   pdl_wait();  // the tensor scale and x may come from the kernel before this one
-  const TensorScale ts = make_tensor_scale(ld_f32_dependent(global_scale));
   const int col_tiles = sc_pad >> 2;
   const int code_pitch = cols >> 1;
   // The loads of the next row group are issued before the arithmetic of the current one, so
   // memory stays busy while the warps compute.
   Vec256 a = {}, b = {};
   {
-    const int row = blockIdx.x * kPairRows + threadIdx.y;
-    if (has_data && row < rows) {
-      const T* src = x + static_cast<int64_t>(row) * cols + pc * 32;
-      a = ld_global_stream_256(src);
-      b = ld_global_stream_256(src + 16);
+    const int row = first * kPairRows + threadIdx.y;
+    if (has_data && row < data_rows) {
+      const T* at = x + static_cast<int64_t>(row) * cols + pc * kElems;
+      a = ld_global_stream_256(at);
+      b = ld_global_stream_256(at + kElems / 2);
     }
   }
-  for (int rg = blockIdx.x; rg < row_groups; rg += gridDim.x) {
+  float g;
+  if constexpr (kDynamic) {
+    g = block_dynamic_scale(x, src, threadIdx.y * 32 + threadIdx.x, 32 * kPairRows);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *src.out = g;
+  } else {
+    g = ld_f32_dependent(src.given);
+  }
+  [[maybe_unused]] const TensorScale ts = make_tensor_scale(g);
+  for (int rg = first; rg >= 0; rg -= gridDim.x) {
     const int row = rg * kPairRows + threadIdx.y;
-    const int next_row = row + gridDim.x * kPairRows;
+    const int next_row = row - static_cast<int>(gridDim.x) * kPairRows;
     Vec256 an = {}, bn = {};
-    if (has_data && next_row < rows) {
-      const T* src = x + static_cast<int64_t>(next_row) * cols + pc * 32;
-      an = ld_global_stream_256(src);
-      bn = ld_global_stream_256(src + 16);
+    if (has_data && next_row >= 0 && next_row < data_rows) {
+      const T* at = x + static_cast<int64_t>(next_row) * cols + pc * kElems;
+      an = ld_global_stream_256(at);
+      bn = ld_global_stream_256(at + kElems / 2);
     }
     uint32_t sb = 0;
     if (has_data && row < rows) {
-      uint32_t w0, w1, w2, w3, s0, s1;
-      nvfp4_block_packed<T, kHiFirst>(a.w, ts, w0, w1, s0);
-      nvfp4_block_packed<T, kHiFirst>(b.w, ts, w2, w3, s1);
-      *reinterpret_cast<uint4*>(codes + static_cast<int64_t>(row) * code_pitch + pc * 16) = make_uint4(w0, w1, w2, w3);
-      sb = s0 | (s1 << 8);
+      uint8_t* const dst = codes + static_cast<int64_t>(row) * code_pitch + pc * (kElems / 2);
+      uint32_t w0, w1, s0;
+      if constexpr (kBlocks == 2) {
+        uint32_t w2, w3, s1;
+        nvfp4_block_packed<T, kHiFirst>(a.w, ts, w0, w1, s0);
+        nvfp4_block_packed<T, kHiFirst>(b.w, ts, w2, w3, s1);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w0, w1, w2, w3);
+        sb = s0 | (s1 << 8);
+      } else {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[i] = __uint_as_float(a.w[i]);
+          v[8 + i] = __uint_as_float(b.w[i]);
+        }
+        nvfp4_block<true>(v, g, kHiFirst, w0, w1, s0);
+        *reinterpret_cast<uint2*>(dst) = make_uint2(w0, w1);
+        sb = s0;
+      }
     }
-    const uint32_t word = sb | (__shfl_xor_sync(0xFFFFFFFFu, sb, 1) << 16);
+    uint32_t word = sb;
+    if constexpr (kBlocks == 1) word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1) << 8;
+    word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2 / kBlocks) << 16;
     if (has_scale && row < rows_pad) {
-      *reinterpret_cast<uint32_t*>(scales + swizzled_scale_offset(row, 2 * pc, col_tiles)) = word;
+      *reinterpret_cast<uint32_t*>(scales + swizzled_scale_offset(row, kBlocks * pc, col_tiles)) = word;
     }
     a = an;
     b = bn;
@@ -226,15 +300,17 @@ quantize_mxfp8_kernel(const T* x, uint8_t* __restrict__ data, uint8_t* __restric
   const int64_t n_sc = num_cols >> 5;
   if constexpr (kVec) {
     // ahead of the dependency wait: ask L2 for the thread pair's 128-byte line (warms the cache only)
-    if (row < num_rows && sc < n_sc && (threadIdx.x & 1) == 0) prefetch_l2(x + row * orig_cols + sc * 32);
+    if (row < orig_rows && sc < n_sc && (threadIdx.x & 1) == 0) prefetch_l2(x + row * orig_cols + sc * 32);
   }
   pdl_wait();
   uint32_t scale_byte = 0;
   if (row < num_rows && sc < n_sc) {
-    float lo[16], hi[16];
+    float lo[16] = {}, hi[16] = {};
     if constexpr (kVec) {
-      load16_vec(x + row * orig_cols + sc * 32, lo);
-      load16_vec(x + row * orig_cols + sc * 32 + 16, hi);
+      if (row < orig_rows) {  // rows may be padded (zeros), columns not
+        load16_vec(x + row * orig_cols + sc * 32, lo);
+        load16_vec(x + row * orig_cols + sc * 32 + 16, hi);
+      }
     } else {
       load16_guarded(x, row, sc * 32, orig_rows, orig_cols, lo);
       load16_guarded(x, row, sc * 32 + 16, orig_rows, orig_cols, hi);
@@ -285,6 +361,45 @@ bool use_exact_division() {
   return env;
 }
 
+// The streaming kernel takes rows of whole 64-byte units (rows may be padded, columns not), with
+// aligned input and codes.
+template <typename T>
+bool streaming_applies(const void* input, const void* codes, int64_t orig_rows, int64_t orig_cols, int64_t num_rows, int64_t num_cols) {
+  return orig_cols == num_cols && orig_rows <= num_rows && num_cols % (64 / static_cast<int64_t>(sizeof(T))) == 0 &&
+         reinterpret_cast<uintptr_t>(input) % 32 == 0 && reinterpret_cast<uintptr_t>(codes) % 16 == 0 &&
+         num_rows < (1 << 30) && num_cols < (1 << 30) && !use_exact_division();
+}
+
+template <typename T>
+int launch_streaming(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
+                     int64_t num_cols, int hi_first, cudaStream_t stream) {
+  const int64_t sc_pad = round_up(num_cols / 16, 4);
+  const int rows_pad = static_cast<int>(round_up(num_rows, 128));
+  const int row_groups = rows_pad / kPairRows;
+  const int col_chunks = static_cast<int>(ceil_div(sc_pad, 32 * (4 / static_cast<int>(sizeof(T)))));
+  CK_REQUIRE(col_chunks <= 65535, "quantize_nvfp4: tensor too large for one launch");
+  const bool dynamic = src.given == nullptr;
+  auto kernel = dynamic ? (hi_first ? quantize_nvfp4_stream_kernel<T, true, true> : quantize_nvfp4_stream_kernel<T, false, true>)
+                        : (hi_first ? quantize_nvfp4_stream_kernel<T, true, false> : quantize_nvfp4_stream_kernel<T, false, false>);
+  // All blocks resident at once and all of the same length: the grid is the number of
+  // row groups divided into the fewest equal passes that fit the device.
+  static std::atomic<int> blocks_per_sm[4] = {{0}, {0}, {0}, {0}};
+  std::atomic<int>& known = blocks_per_sm[(hi_first ? 1 : 0) + (dynamic ? 2 : 0)];
+  int per_sm = known.load(std::memory_order_relaxed);
+  if (per_sm == 0) {
+    CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kPairRows, 0));
+    per_sm = max(per_sm, 1);
+    known.store(per_sm, std::memory_order_relaxed);
+  }
+  const int per_wave = max(1, sm_count() * per_sm / col_chunks);
+  const int waves = static_cast<int>(ceil_div(row_groups, per_wave));
+  const int grid_x = static_cast<int>(ceil_div(row_groups, waves));
+  const dim3 grid(static_cast<unsigned>(grid_x), static_cast<unsigned>(col_chunks)), block(32, kPairRows);
+  CK_CUDA(launch_pdl(kernel, grid, block, 0, stream, x, src, codes, scales, static_cast<int>(orig_rows), static_cast<int>(num_rows),
+                     static_cast<int>(num_cols), rows_pad, static_cast<int>(sc_pad), row_groups));
+  return CK_OK;
+}
+
 template <typename T>
 int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, int64_t orig_rows, int64_t orig_cols,
                  int64_t num_rows, int64_t num_cols, int hi_first, cudaStream_t stream) {
@@ -292,39 +407,19 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
   const int64_t grid_rows = round_up(num_rows, 128) / kRowsPerBlock;
   const int64_t grid_cols = ceil_div(sc_pad, kColsPerBlock);
   CK_REQUIRE(grid_rows <= 0x7FFFFFFF && grid_cols <= 65535, "quantize_nvfp4: tensor too large for one launch");
+  const T* x = static_cast<const T*>(input);
+  uint8_t* c = static_cast<uint8_t*>(codes);
+  uint8_t* s = static_cast<uint8_t*>(scales);
+  if (streaming_applies<T>(input, codes, orig_rows, orig_cols, num_rows, num_cols)) {
+    ScaleSource src = {};
+    src.given = gs;
+    return launch_streaming<T>(x, src, c, s, orig_rows, num_rows, num_cols, hi_first, stream);
+  }
   const dim3 grid(static_cast<unsigned>(grid_rows), static_cast<unsigned>(grid_cols)), block(kColsPerBlock, kRowsPerBlock);
   // vector path: every 16-element run is inside the input and 32-byte aligned
   const bool vec = (orig_rows == num_rows) && (orig_cols == num_cols) &&
                    (reinterpret_cast<uintptr_t>(input) % 32 == 0);
-  const T* x = static_cast<const T*>(input);
-  uint8_t* c = static_cast<uint8_t*>(codes);
-  uint8_t* s = static_cast<uint8_t*>(scales);
   const bool exact = use_exact_division();
-  if constexpr (sizeof(T) == 2) {
-    if (vec && !exact && num_cols % 32 == 0 && reinterpret_cast<uintptr_t>(codes) % 16 == 0 &&
-        num_rows < (1 << 30) && num_cols < (1 << 30)) {
-      const int rows_pad = static_cast<int>(round_up(num_rows, 128));
-      const int row_groups = rows_pad / kPairRows;
-      const int col_chunks = static_cast<int>(ceil_div(sc_pad, 64));
-      auto kernel = hi_first ? quantize_nvfp4_pair_kernel<T, true> : quantize_nvfp4_pair_kernel<T, false>;
-      // All blocks resident at once and all of the same length: the grid is the number of
-      // row groups divided into the fewest equal passes that fit the device.
-      static std::atomic<int> blocks_per_sm[2] = {{0}, {0}};
-      int per_sm = blocks_per_sm[hi_first ? 1 : 0].load(std::memory_order_relaxed);
-      if (per_sm == 0) {
-        CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kPairRows, 0));
-        per_sm = max(per_sm, 1);
-        blocks_per_sm[hi_first ? 1 : 0].store(per_sm, std::memory_order_relaxed);
-      }
-      const int per_wave = max(1, sm_count() * per_sm / col_chunks);
-      const int waves = static_cast<int>(ceil_div(row_groups, per_wave));
-      const int grid_x = static_cast<int>(ceil_div(row_groups, waves));
-      const dim3 pgrid(static_cast<unsigned>(grid_x), static_cast<unsigned>(col_chunks)), pblock(32, kPairRows);
-      CK_CUDA(launch_pdl(kernel, pgrid, pblock, 0, stream, x, gs, c, s, static_cast<int>(num_rows),
-                         static_cast<int>(num_cols), rows_pad, static_cast<int>(sc_pad), row_groups));
-      return CK_OK;
-    }
-  }
 #define CK_LAUNCH(VEC, FAST)                                                                                  \
   CK_CUDA(launch_pdl(quantize_nvfp4_kernel<T, VEC, FAST>, grid, block, 0, stream, x, gs, c, s, orig_rows, orig_cols, \
                      num_rows, num_cols, sc_pad, hi_first))
@@ -338,6 +433,36 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
   return CK_OK;
 }
 
+// Inputs of at most this many bytes: every block of the quantizer takes the maximum of the whole input
+// itself (a few 16 KiB passes out of L2) instead of waiting for a reduction kernel.
+constexpr int64_t kWholeInputBytes = 64 * 1024;
+constexpr int64_t kDynamicScratchHead = 256;
+
+template <typename T>
+int launch_nvfp4_dynamic(const void* input, int dtype, float* scale_out, void* codes, void* scales, int64_t orig_rows,
+                         int64_t orig_cols, int64_t num_rows, int64_t num_cols, int hi_first, void* scratch,
+                         int64_t scratch_bytes, cudaStream_t stream) {
+  const int64_t n = orig_rows * orig_cols;
+  if (streaming_applies<T>(input, codes, orig_rows, orig_cols, num_rows, num_cols)) {
+    const T* x = static_cast<const T*>(input);
+    ScaleSource src = {};
+    src.out = scale_out;
+    src.n_vecs = n / (32 / static_cast<int64_t>(sizeof(T)));
+    if (n * static_cast<int64_t>(sizeof(T)) > kWholeInputBytes) {
+      // behind the arrival counter of the one-kernel reduction, which may share this scratch and wants it zero
+      float* partials = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kDynamicScratchHead);
+      if (int rc = launch_amax_partials(x, dtype, src.n_vecs, partials, &src.n_partials, stream)) return rc;
+      src.partials = partials;
+    }
+    return launch_streaming<T>(x, src, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), orig_rows, num_rows, num_cols,
+                               hi_first, stream);
+  }
+  // the one-kernel reduction keeps an arrival counter at the head of its scratch, which has to start at zero
+  CK_CUDA(cudaMemsetAsync(scratch, 0, sizeof(unsigned int), stream));
+  if (int rc = ck_nvfp4_tensor_scale(input, dtype, n, scale_out, scratch, scratch_bytes, stream)) return rc;
+  return launch_nvfp4<T>(input, scale_out, codes, scales, orig_rows, orig_cols, num_rows, num_cols, hi_first, stream);
+}
+
 template <typename T>
 int launch_mxfp8(const void* input, void* data, void* scales, int64_t orig_rows, int64_t orig_cols, int64_t num_rows,
                  int64_t num_cols, cudaStream_t stream) {
@@ -346,7 +471,7 @@ int launch_mxfp8(const void* input, void* data, void* scales, int64_t orig_rows,
   const int64_t grid_cols = ceil_div(sc_pad, kColsPerBlock);
   CK_REQUIRE(grid_rows <= 0x7FFFFFFF && grid_cols <= 65535, "quantize_mxfp8: tensor too large for one launch");
   const dim3 grid(static_cast<unsigned>(grid_rows), static_cast<unsigned>(grid_cols)), block(kColsPerBlock, kRowsPerBlock);
-  const bool vec = (orig_rows == num_rows) && (orig_cols == num_cols) &&
+  const bool vec = (orig_cols == num_cols) &&
                    (reinterpret_cast<uintptr_t>(input) % 32 == 0) && (reinterpret_cast<uintptr_t>(data) % 32 == 0);
   const T* x = static_cast<const T*>(input);
   uint8_t* d = static_cast<uint8_t*>(data);
@@ -410,6 +535,38 @@ extern "C" int ck_quantize_nvfp4(const void* input, int input_dtype, const float
                                  hi_first, s);
     default:
       return fail(CK_ERR_INVALID_ARGUMENT, "quantize_nvfp4: unsupported input dtype code %d", input_dtype);
+  }
+}
+
+extern "C" int64_t ck_quantize_nvfp4_dynamic_scratch_bytes(int64_t num_elements) {
+  const int64_t partials = ck::kDynamicScratchHead + ck::amax_partials_max() * 4, general = ck_nvfp4_tensor_scale_scratch_bytes(num_elements);
+  return num_elements <= 0 ? 0 : (general > partials ? general : partials);
+}
+
+extern "C" int ck_quantize_nvfp4_dynamic(const void* input, int input_dtype, float* scale_out, void* codes, void* block_scales,
+                                         int64_t orig_rows, int64_t orig_cols, int64_t num_rows, int64_t num_cols, int hi_first,
+                                         void* scratch, int64_t scratch_bytes, void* stream) {
+  using namespace ck;
+  if (int rc = check_quant_shapes("quantize_nvfp4_dynamic", 16, input, codes, block_scales, orig_rows, orig_cols, num_rows, num_cols))
+    return rc;
+  CK_REQUIRE(scale_out != nullptr && scratch != nullptr, "quantize_nvfp4_dynamic: null scale_out or scratch");
+  CK_REQUIRE(reinterpret_cast<uintptr_t>(codes) % 8 == 0, "quantize_nvfp4_dynamic: codes must be 8-byte aligned");
+  CK_REQUIRE(reinterpret_cast<uintptr_t>(scratch) % 4 == 0 && scratch_bytes >= ck_quantize_nvfp4_dynamic_scratch_bytes(orig_rows * orig_cols),
+             "quantize_nvfp4_dynamic: scratch of %lld bytes, %lld needed (4-byte aligned)", (long long)scratch_bytes,
+             (long long)ck_quantize_nvfp4_dynamic_scratch_bytes(orig_rows * orig_cols));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (input_dtype) {
+    case CK_DTYPE_BF16:
+      return launch_nvfp4_dynamic<__nv_bfloat16>(input, input_dtype, scale_out, codes, block_scales, orig_rows, orig_cols, num_rows,
+                                                 num_cols, hi_first, scratch, scratch_bytes, s);
+    case CK_DTYPE_F16:
+      return launch_nvfp4_dynamic<__half>(input, input_dtype, scale_out, codes, block_scales, orig_rows, orig_cols, num_rows, num_cols,
+                                          hi_first, scratch, scratch_bytes, s);
+    case CK_DTYPE_F32:
+      return launch_nvfp4_dynamic<float>(input, input_dtype, scale_out, codes, block_scales, orig_rows, orig_cols, num_rows, num_cols,
+                                         hi_first, scratch, scratch_bytes, s);
+    default:
+      return fail(CK_ERR_INVALID_ARGUMENT, "quantize_nvfp4_dynamic: unsupported input dtype code %d", input_dtype);
   }
 }
 

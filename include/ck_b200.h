@@ -116,6 +116,20 @@ CK_API int ck_nvfp4_tensor_scale(const void* input, int input_dtype, int64_t num
                           void* scratch, int64_t scratch_bytes, void* stream);
 
 /*
+ * ck_nvfp4_tensor_scale and ck_quantize_nvfp4 with that scale, bit for bit, enqueued by one call: the
+ * reduction over the input leaves one partial maximum per block and the quantizer finishes it (inputs of
+ * at most 64 KiB take no reduction kernel at all).  The scale goes to *scale_out (device memory).
+ * `scratch`: device memory, 4-byte aligned, at least ck_quantize_nvfp4_dynamic_scratch_bytes(orig_rows *
+ * orig_cols) bytes, with no requirement on its contents; a first word that was zero is zero again.
+ */
+CK_API int64_t ck_quantize_nvfp4_dynamic_scratch_bytes(int64_t num_elements);
+CK_API int ck_quantize_nvfp4_dynamic(const void* input, int input_dtype, float* scale_out,
+                      void* codes, void* block_scales,
+                      int64_t orig_rows, int64_t orig_cols,
+                      int64_t num_rows, int64_t num_cols, int hi_first,
+                      void* scratch, int64_t scratch_bytes, void* stream);
+
+/*
  * Same result as ck_nvfp4_tensor_scale, for callers that cannot hand in a scratch buffer
  * because they must not allocate device memory at that point: plugins that live inside a
  * host application with a fixed memory budget, or serving loops where a cudaMalloc would
@@ -201,15 +215,13 @@ CK_API int ck_linear_nvfp4_fused(const void* a, const void* b, const void* sfa, 
  * them) and multiplied with a pre-quantized weight:
  *   out[M,N] = cast( deq(quantize(x)) . deq(w)^T * (x_scale * w_scale) + bias )
  * x_scale: the activation's per-tensor scale in device memory, or NULL for the dynamic scale
- * amax(|x|)/2688 of ck_nvfp4_tensor_scale (one more kernel).  The kernels are enqueued back to
+ * amax(|x|)/2688 of ck_nvfp4_tensor_scale (one more kernel unless x is small).  The kernels are enqueued back to
  * back on `stream` and chained with programmatic dependent launch; results are bit-identical to
  * calling ck_nvfp4_tensor_scale, ck_quantize_nvfp4 and ck_scaled_mm_nvfp4 one after the other.
  * The quantized activation is written to `workspace` (device memory, 256-byte aligned, at least
  * ck_linear_nvfp4_from_float_workspace_bytes(M, K, x_scale == NULL) bytes; 0 = this shape is not
- * supported).  The first 256 KiB of the workspace are the scale kernel's scratch: they must have
- * been zero-filled once before the first call with a dynamic scale and are left zeroed by every
- * call, whatever the shapes of the calls that share the workspace; calls that can overlap on the
- * GPU need separate workspaces.  K % 32 == 0, N % 8 == 0; with a dynamic scale M x K <= 2^30.
+ * supported).  Its contents need no preparation; calls that can overlap on the GPU need separate
+ * workspaces.  K % 32 == 0, N % 8 == 0; with a dynamic scale M x K <= 2^30.
  * Replaces the sequence QuantizedTensor.from_float -> F.linear of the reference
  * (comfy_kitchen/tensor/nvfp4.py:51-82 followed by tensor/nvfp4.py:214-264; the caller side is
  * samples/nvfp4_linear.py:77-80).
