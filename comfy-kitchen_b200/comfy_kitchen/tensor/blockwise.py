@@ -18,6 +18,8 @@ from .base import QuantizedTensor, dequantize_args, register_layout_op
 
 logger = logging.getLogger(__name__)
 
+_backend = None  # the CUDA backend module, once a call has needed it
+
 
 def strict_mode() -> bool:
     """CK_STRICT=1: a failing fast path raises instead of silently falling back to dequantization."""
@@ -50,9 +52,10 @@ def direct_backend(*tensors):
         # __torch_dispatch__) have no data pointer: only plain tensors may skip the dispatcher
         if (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter) or not t.is_cuda:
             return None
-    from comfy_kitchen.backends import cuda as backend
-
-    return backend if backend.is_loaded() else None
+    global _backend
+    if _backend is None:
+        from comfy_kitchen.backends import cuda as _backend  # not at import: the backend imports this package
+    return _backend if _backend.is_loaded() else None
 
 
 def crop(result: torch.Tensor, rows: int, cols: int) -> torch.Tensor:
