@@ -90,6 +90,35 @@ __host__ __device__ __forceinline__ int64_t swizzled_scale_offset(int64_t r, int
   return tile * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4 + (c & 3);
 }
 
+#ifdef __CUDACC__
+// ---- two fp32 operations in one instruction (sm_100): each half rounds like its scalar form ----
+__device__ __forceinline__ uint64_t as_b64(float2 v) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+  return r;
+}
+__device__ __forceinline__ float2 as_float2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float2 fma_x2(float2 a, float2 b, float2 c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(as_b64(a)), "l"(as_b64(b)), "l"(as_b64(c)));
+  return as_float2(r);
+}
+__device__ __forceinline__ float2 mul_x2(float2 a, float2 b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(as_b64(a)), "l"(as_b64(b)));
+  return as_float2(r);
+}
+__device__ __forceinline__ float2 add_x2(float2 a, float2 b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(as_b64(a)), "l"(as_b64(b)));
+  return as_float2(r);
+}
+#endif
+
 // ---- 256-bit global memory access (sm_100) ------------------------------------
 struct __align__(32) Vec256 {
   uint32_t w[8];

@@ -333,6 +333,22 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   return x * r;
 }
 
+// The same for two values: the multiplies and adds as packed pairs (same roundings, same bits).  The fused
+// epilogue is bound by its instruction count (33 per element measured, 10.4 k cycles a tile against the
+// 6.3 k of its main loop); with the pairs here, in the drain and in the quantizer's products the MLP pair
+// 4608 x 12288 x 3072 goes from 188.7 to 177.2 us (163.0 to 154.5 on a cool chip).
+__device__ __forceinline__ float2 gelu_tanh_x2(float2 x) {
+  const float2 w = fma_x2(make_float2(-0.10294324f, -0.10294324f), mul_x2(x, x), make_float2(-2.3022082f, -2.3022082f));
+  const float2 u = mul_x2(x, w);
+  float2 t, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(u.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(u.y));
+  t = add_x2(t, make_float2(1.0f, 1.0f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(t.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(t.y));
+  return mul_x2(x, r);
+}
+
 __device__ __forceinline__ float load_bias(const void* bias, int dtype, int n) {
   if (dtype == CK_DTYPE_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[n]);
   if (dtype == CK_DTYPE_F16) return __half2float(static_cast<const __half*>(bias)[n]);
@@ -787,9 +803,9 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const float2* b2 = reinterpret_cast<const float2*>(bias_s + c0 + c * 32);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float2 b = b2[i];
-            pk[c][i] = pack_pair<OutT>(fmaf(__uint_as_float(buf[0][2 * i]), alpha, b.x),
-                                       fmaf(__uint_as_float(buf[0][2 * i + 1]), alpha, b.y));
+            const float2 y = fma_x2(make_float2(__uint_as_float(buf[0][2 * i]), __uint_as_float(buf[0][2 * i + 1])),
+                                    make_float2(alpha, alpha), b2[i]);
+            pk[c][i] = pack_pair<OutT>(y.x, y.y);
           }
         }
       } else {
@@ -935,9 +951,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               if (p.activation == CK_ACT_GELU_TANH) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  float a, b;
-                  unpack_pair<OutT>(pk[c][i], a, b);
-                  pk[c][i] = pack_pair<OutT>(gelu_tanh(a), gelu_tanh(b));
+                  float2 x;
+                  unpack_pair<OutT>(pk[c][i], x.x, x.y);
+                  x = gelu_tanh_x2(x);
+                  pk[c][i] = pack_pair<OutT>(x.x, x.y);
                 }
               }
               if (p.out != nullptr) {

@@ -257,10 +257,17 @@ __device__ __noinline__ uint2 nvfp4_codes_exact(uint32_t w0, uint32_t w1, uint32
 // 8 products v[i] * y -> one word of codes (nibble order as requested)
 template <bool kHiFirst>
 __device__ __forceinline__ uint32_t scaled_e2m1_word(const float* v, float y) {
+  float q[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 p = mul_x2(make_float2(v[2 * i], v[2 * i + 1]), make_float2(y, y));
+    q[2 * i] = p.x;
+    q[2 * i + 1] = p.y;
+  }
   if constexpr (kHiFirst) {
-    return f32x8_to_e2m1_word(v[0] * y, v[1] * y, v[2] * y, v[3] * y, v[4] * y, v[5] * y, v[6] * y, v[7] * y);
+    return f32x8_to_e2m1_word(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
   } else {
-    return f32x8_to_e2m1_word(v[1] * y, v[0] * y, v[3] * y, v[2] * y, v[5] * y, v[4] * y, v[7] * y, v[6] * y);
+    return f32x8_to_e2m1_word(q[1], q[0], q[3], q[2], q[5], q[4], q[7], q[6]);
   }
 }
 
