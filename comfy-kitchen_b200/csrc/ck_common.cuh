@@ -133,6 +133,16 @@ __device__ __forceinline__ Vec256 ld_global_stream_256(const void* p) {
   return r;
 }
 
+// The same load for data that this library will not read again: its lines are the first to leave L2.
+__device__ __forceinline__ Vec256 ld_global_last_use_256(const void* p) {
+  Vec256 r;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::evict_first.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]),
+                 "=r"(r.w[6]), "=r"(r.w[7])
+               : "l"(p));
+  return r;
+}
+
 // Scalar read of a value the previous kernel in the stream may have produced (a tensor scale,
 // alpha).  Kernels launched with programmatic stream serialization start before their predecessor
 // has finished; a read-only-cache load (__ldg, or what the compiler makes of a const __restrict__
