@@ -255,6 +255,16 @@ def nvfp4_tensor_scale(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
+_WHOLE_INPUT_BYTES = 64 << 10  # inputs up to here take no reduction kernel (ck_quantize_nvfp4_dynamic)
+
+
+def _call_workspace(need: int, device) -> torch.Tensor:
+    """Device memory of this one call, from the caching allocator's pool of the current stream: the next
+    allocation that gets the same block is ordered behind this call's kernels, and a captured call's block
+    belongs to its graph.  (Never empty: the library reports an unsupported shape itself.)"""
+    return torch.empty(max(need, 1), dtype=torch.uint8, device=device)
+
+
 def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
                            hi_first: bool = True) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """``scale = nvfp4_tensor_scale(x)`` and ``quantize_nvfp4(x, scale)`` in one library call (same bits):
@@ -269,7 +279,13 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
         out_rows, out_cols = rows, cols
         assert out_cols % 16 == 0, f"num_cols must be divisible by 16, got {out_cols}"
     stream = _stream(x.device)
-    scratch = _scale_scratch_for(x.device, stream, _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols))
+    need = _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
+    if rows * cols * x.element_size() <= _WHOLE_INPUT_BYTES:
+        scratch = _scale_scratch_for(x.device, stream, need)  # nothing is kept in it between two launches
+    else:
+        # The partial maxima go from one launch to the next: a buffer that another thread of this stream (or
+        # another graph captured on it) also uses could be written by its reduction in between.
+        scratch = _call_workspace(need, x.device)
     scale = torch.empty((), dtype=torch.float32, device=x.device)
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
     sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)
@@ -457,9 +473,6 @@ def check_device_status(what: str = "kernel") -> None:
         raise RuntimeError(f"{what}: rank {b.value - 1} did not arrive at the cross-GPU barrier in time; the result is invalid")
 
 
-_linear_workspaces: dict = {}
-
-
 @functools.lru_cache(maxsize=512)
 def _workspace_bytes(function: str, *shape: int) -> int:
     return int(getattr(_lib, function)(*shape))
@@ -473,8 +486,8 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     ``x`` [M, K] float; ``w_codes`` uint8 [N, K/2] with its tiled E4M3 ``w_block_scales`` and fp32
     ``w_scale``; ``x_scale`` a static per-tensor scale or None for ``amax(|x|)/2688``.  Same bits
     as ``quantize_nvfp4`` followed by ``scaled_mm_nvfp4``.  The quantized activation goes to a
-    workspace cached per device and stream (grow-only; outgrown buffers are kept alive because a
-    captured CUDA graph may still point at them)."""
+    workspace of this call: it passes from one launch to the next, and threads that share a stream
+    may interleave their launches."""
     lib = load_library()
     x, w_codes, w_block_scales = _plain(x), _plain(w_codes), _plain(w_block_scales)
     assert x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor"
@@ -490,13 +503,7 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     need = _workspace_bytes("ck_linear_nvfp4_from_float_workspace_bytes", m, k, int(sx is None))
     stream = _stream(dev)
-    key = (dev, stream)
-    ws = _linear_workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        if ws is not None:
-            _retired_workspaces.append(ws)
-        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-        _linear_workspaces[key] = ws
+    ws = _call_workspace(need, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
         _check(lib.ck_linear_nvfp4_from_float(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(sx), _ptr(w_codes), _ptr(w_block_scales),
@@ -511,7 +518,7 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     """MXFP8 linear on a dense activation in one library call: quantize -> GEMM.  ``x`` [M, K] float;
     ``w_data`` float8_e4m3fn [N, K] with its tiled E8M0 ``w_block_scales``.  Same bits as
     ``quantize_mxfp8`` followed by ``scaled_mm_mxfp8``; the quantized activation goes to a workspace
-    cached per device and stream."""
+    of this call, as in :func:`linear_nvfp4_from_float`."""
     lib = load_library()
     x, w_data, w_block_scales = _plain(x), _plain(w_data), _plain(w_block_scales)
     assert x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor"
@@ -526,13 +533,7 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     need = _workspace_bytes("ck_linear_mxfp8_from_float_workspace_bytes", m, k)
     stream = _stream(dev)
-    key = (dev, stream, "mxfp8")
-    ws = _linear_workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        if ws is not None:
-            _retired_workspaces.append(ws)
-        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-        _linear_workspaces[key] = ws
+    ws = _call_workspace(need, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
         _check(lib.ck_linear_mxfp8_from_float(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(w_data), _ptr(w_block_scales), bias_ptr,
