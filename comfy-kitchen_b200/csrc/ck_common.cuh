@@ -39,8 +39,8 @@ int sm_count();
 // Device address of the GEMM kernels' status word on the current device (ck_gemm.cu).
 int gemm_status_word(int** out);
 
-// Partial maxima of |x| (n_vecs 32-byte units), one per block of the launch, at most amax_partials_max() (ck_amax.cu).
-int64_t amax_partials_max();
+// Partial maxima of |x| (n_vecs 32-byte units), amax_partials(n_vecs) of them (ck_amax.cu).
+int64_t amax_partials(int64_t n_vecs);
 int launch_amax_partials(const void* x, int dtype, int64_t n_vecs, float* partials, int* n_partials, cudaStream_t s);
 
 // GEMMs with few activation rows (ck_gemm_smallm.cu).

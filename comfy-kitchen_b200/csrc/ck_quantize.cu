@@ -141,7 +141,13 @@ template <typename T>
 __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSource& src, int tid, int threads) {
   float m = 0.0f;
   if (src.n_partials > 0) {
-    for (int i = tid; i < src.n_partials; i += threads) m = fmaxf(m, ld_f32_dependent(src.partials + i));
+    for (int i = tid; i < src.n_partials; i += 8 * threads) {  // eight loads in flight: there may be thousands
+      float p[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) p[j] = i + j * threads < src.n_partials ? ld_f32_dependent(src.partials + i + j * threads) : 0.0f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, p[j]);
+    }
   } else {
     constexpr int kPerVec = 32 / sizeof(T);
     for (int64_t i = tid; i < src.n_vecs; i += 4 * threads) {
@@ -543,8 +549,11 @@ extern "C" int ck_quantize_nvfp4(const void* input, int input_dtype, const float
 }
 
 extern "C" int64_t ck_quantize_nvfp4_dynamic_scratch_bytes(int64_t num_elements) {
-  const int64_t partials = ck::kDynamicScratchHead + ck::amax_partials_max() * 4, general = ck_nvfp4_tensor_scale_scratch_bytes(num_elements);
-  return num_elements <= 0 ? 0 : (general > partials ? general : partials);
+  if (num_elements <= 0) return 0;
+  // the most of all types (fp32 has eight elements to a 32-byte unit) and of both routes
+  const int64_t partials = ck::kDynamicScratchHead + 4 * ck::amax_partials(ck::ceil_div(num_elements, 8));
+  const int64_t general = ck_nvfp4_tensor_scale_scratch_bytes(num_elements);
+  return general > partials ? general : partials;
 }
 
 extern "C" int ck_quantize_nvfp4_dynamic(const void* input, int input_dtype, float* scale_out, void* codes, void* block_scales,

@@ -1,0 +1,31 @@
+"""Size queries of the C ABI (no GPU needed)."""
+from __future__ import annotations
+
+import pytest
+
+from test_abi_cpu import lib_path  # noqa: F401  (a fixture)
+
+
+@pytest.fixture(scope="module")
+def lib(lib_path):  # noqa: F811
+    import ctypes
+
+    lib = ctypes.CDLL(lib_path)
+    for name in ("ck_quantize_nvfp4_dynamic_scratch_bytes", "ck_nvfp4_tensor_scale_scratch_bytes"):
+        getattr(lib, name).argtypes, getattr(lib, name).restype = [ctypes.c_int64], ctypes.c_int64
+    return lib
+
+
+@pytest.mark.parametrize("n", [1, 16, 16384, 16385, 592 * 16384, 592 * 16384 + 1, 4096 * 3072, 16384 * 8192, 1 << 30, 1 << 33])
+def test_dynamic_scratch_depends_on_the_input_alone(lib, n):
+    """One fp32 partial per 64 KiB of the input up to 592 of them, per 32 KiB beyond, at most 16384, behind a
+    256-byte head (or what the one-kernel scale wants): no term in the SM count of whichever device happens
+    to be current.  The input may be fp32."""
+    partials = -(-4 * n // 65536)
+    if partials > 592:
+        partials = min(-(-4 * n // 32768), 16384)
+    assert lib.ck_quantize_nvfp4_dynamic_scratch_bytes(n) == max(256 + 4 * partials, lib.ck_nvfp4_tensor_scale_scratch_bytes(n))
+
+
+def test_dynamic_scratch_of_nothing(lib):
+    assert lib.ck_quantize_nvfp4_dynamic_scratch_bytes(0) == 0 == lib.ck_quantize_nvfp4_dynamic_scratch_bytes(-5)
