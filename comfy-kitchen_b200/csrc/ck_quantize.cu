@@ -178,9 +178,9 @@ __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSour
 // threads walks row groups with a grid stride so that every SM holds the same amount of work.  Rows
 // past data_rows (padding) have zero codes and scales.
 //
-// The row groups are walked from the last to the first.  With a dynamic scale the reduction pass has
-// just read the input front to back, and what L2 still holds of it is its end; the GEMM that follows
-// starts with the first rows, the ones written last here.
+// The row groups are walked in order, which is also the order of the reduction pass: walked backwards (for
+// what the reduction pass left in L2) a static scale pays 0.3 us at 1024 x 3072 (4.72 against 4.43, inputs
+// not in L2) and three layers on one 4096 x 3072 input 85.0 against 83.9; a dynamic one gains nothing.
 //
 // This is the input's last read: its lines are marked first to leave L2 (evict_first), so that they make room
 // for each other and not push out what the reduction pass left there or the codes the GEMM reads next
@@ -207,12 +207,12 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
   // warms the cache (L2 is the point of coherence: what the previous kernel still writes is seen
   // by the loads after the wait), and it takes the DRAM latency of the first loads off the
   // critical path of a kernel that only runs for a few microseconds.
-  const int first = row_groups - 1 - static_cast<int>(blockIdx.x);
+  const int first = static_cast<int>(blockIdx.x);
   if (has_data && (threadIdx.x & 1) == 0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int row = (first - i * static_cast<int>(gridDim.x)) * kPairRows + static_cast<int>(threadIdx.y);
-      if (row >= 0 && row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
+      const int row = (first + i * static_cast<int>(gridDim.x)) * kPairRows + static_cast<int>(threadIdx.y);
+      if (row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
     }
   }
   pdl_wait();  // the tensor scale and x may come from the kernel before this one
@@ -237,11 +237,11 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
     g = ld_f32_dependent(src.given);
   }
   [[maybe_unused]] const TensorScale ts = make_tensor_scale(g);
-  for (int rg = first; rg >= 0; rg -= gridDim.x) {
+  for (int rg = first; rg < row_groups; rg += gridDim.x) {
     const int row = rg * kPairRows + threadIdx.y;
-    const int next_row = row - static_cast<int>(gridDim.x) * kPairRows;
+    const int next_row = row + static_cast<int>(gridDim.x) * kPairRows;
     Vec256 an = {}, bn = {};
-    if (has_data && next_row >= 0 && next_row < data_rows) {
+    if (has_data && next_row < data_rows) {
       const T* at = x + static_cast<int64_t>(next_row) * cols + pc * kElems;
       an = ld_global_last_use_256(at);
       bn = ld_global_last_use_256(at + kElems / 2);
