@@ -422,7 +422,12 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
   const T* x = static_cast<const T*>(input);
   uint8_t* c = static_cast<uint8_t*>(codes);
   uint8_t* s = static_cast<uint8_t*>(scales);
-  if (streaming_applies<T>(input, codes, orig_rows, orig_cols, num_rows, num_cols)) {
+  // Small fp32 inputs: the kernel below has twice the blocks of half the threads (not in L2, it / streaming:
+  // 128 x 1024 1.69 / 1.85 us, 77 x 4096 2.11 / 2.27, 512 x 1024 1.99 / 2.29; beyond the line 256 x 3072 2.62 / 2.45,
+  // 128 x 8192 3.06 / 2.53).  16-bit types and padded rows stream at every size.
+  constexpr int64_t kStreamFp32Elements = 640 * 1024;
+  const bool small_fp32 = sizeof(T) == 4 && orig_rows == num_rows && round_up(num_rows, 128) * num_cols < kStreamFp32Elements;
+  if (!small_fp32 && streaming_applies<T>(input, codes, orig_rows, orig_cols, num_rows, num_cols)) {
     ScaleSource src = {};
     src.given = gs;
     return launch_streaming<T>(x, src, c, s, orig_rows, num_rows, num_cols, hi_first, stream);

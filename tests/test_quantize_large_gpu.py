@@ -27,3 +27,18 @@ def test_large_input_equals_its_parts(cuda_device, rows, cols, dtype, where):
         tiles = want_scales.view(torch.uint8).flatten()
         at = start * block_scales.shape[1]
         assert torch.equal(block_scales.view(torch.uint8).flatten()[at:at + tiles.numel()], tiles)
+
+
+# padded rows x columns on both sides of the line between the two kernels of small fp32 inputs, and padded rows
+@pytest.mark.parametrize("rows, cols", [(1, 16), (128, 5104), (128, 5120), (100, 5120), (33, 5136), (640, 1008), (640, 1024), (7, 48)])
+def test_fp32_kernels_agree(cuda_device, rows, cols):
+    from comfy_kitchen.backends import cuda as backend
+
+    gen = torch.Generator(device=cuda_device).manual_seed(rows + cols)
+    x = torch.randn(rows, cols, generator=gen, device=cuda_device, dtype=torch.float32)
+    want_codes, want_scales, scale = backend.quantize_nvfp4_dynamic(x)  # streams at every size
+    codes, block_scales = backend.quantize_nvfp4(x, scale)
+    assert torch.equal(codes, want_codes) and torch.equal(block_scales.view(torch.uint8), want_scales.view(torch.uint8))
+    padded, padded_scales = backend.quantize_nvfp4(x, scale, pad_16x=True)
+    assert torch.equal(padded[:rows], codes) and not padded[rows:].any()
+    assert torch.equal(padded_scales.view(torch.uint8), block_scales.view(torch.uint8))
