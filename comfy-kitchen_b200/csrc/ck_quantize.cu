@@ -182,9 +182,9 @@ __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSour
 // what the reduction pass left in L2) a static scale pays 0.3 us at 1024 x 3072 (4.72 against 4.43, inputs
 // not in L2) and three layers on one 4096 x 3072 input 85.0 against 83.9; a dynamic one gains nothing.
 //
-// This is the input's last read: its lines are marked first to leave L2 (evict_first), so that they make room
-// for each other and not push out what the reduction pass left there or the codes the GEMM reads next
-// (fp32 weight of 12288 x 3072 with its dynamic scale: 52.3 -> 51.1 us; bf16 batches and few rows unchanged).
+// kMark: the input's lines are marked first to leave L2 (evict_first), so that they make room for each other
+// and not push out the codes, which the GEMM reads next.  By the rule in launch_streaming: not for inputs that
+// stay in L2, where the next layer on the same activation finds them.
 //
 // Bound by HBM for large inputs and by launches and latency for small ones: finishing the dynamic scale
 // here takes the reduction's last-block tail (and for small inputs the reduction kernel) off the chain.
@@ -193,7 +193,13 @@ __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSour
 // 12288 x 3072 with its dynamic scale 56.8 -> 52.4.
 constexpr int kPairRows = 16;  // rows per thread block
 
-template <typename T, bool kHiFirst, bool kDynamic>
+template <bool kMark>
+__device__ __forceinline__ Vec256 ld_stream_unit(const void* p) {
+  if constexpr (kMark) return ld_global_last_use_256(p);
+  return ld_global_stream_256(p);
+}
+
+template <typename T, bool kHiFirst, bool kDynamic, bool kMark>
 __global__ void __launch_bounds__(32 * kPairRows, 2)
 quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
                              int data_rows, int rows, int cols, int rows_pad, int sc_pad, int row_groups) {
@@ -233,8 +239,8 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
     const int row = first * kPairRows + threadIdx.y;
     if (has_data && row < data_rows) {
       const T* at = x + static_cast<int64_t>(row) * cols + pc * kElems;
-      a = ld_global_last_use_256(at);
-      b = ld_global_last_use_256(at + kElems / 2);
+      a = ld_stream_unit<kMark>(at);
+      b = ld_stream_unit<kMark>(at + kElems / 2);
     }
   }
   if constexpr (!kDynamic) g = ld_f32_dependent(src.given);
@@ -245,8 +251,8 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
     Vec256 an = {}, bn = {};
     if (has_data && next_row < data_rows) {
       const T* at = x + static_cast<int64_t>(next_row) * cols + pc * kElems;
-      an = ld_global_last_use_256(at);
-      bn = ld_global_last_use_256(at + kElems / 2);
+      an = ld_stream_unit<kMark>(at);
+      bn = ld_stream_unit<kMark>(at + kElems / 2);
     }
     uint32_t sb = 0;
     if (has_data && row < rows) {
@@ -382,21 +388,19 @@ bool streaming_applies(const void* input, const void* codes, int64_t orig_rows, 
          num_rows < (1 << 30) && num_cols < (1 << 30) && !use_exact_division();
 }
 
-template <typename T>
-int launch_streaming(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
-                     int64_t num_cols, int hi_first, cudaStream_t stream) {
+template <typename T, bool kDynamic, bool kMark>
+int launch_streaming_as(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
+                        int64_t num_cols, int hi_first, cudaStream_t stream) {
   const int64_t sc_pad = round_up(num_cols / 16, 4);
   const int rows_pad = static_cast<int>(round_up(num_rows, 128));
   const int row_groups = rows_pad / kPairRows;
   const int col_chunks = static_cast<int>(ceil_div(sc_pad, 32 * (4 / static_cast<int>(sizeof(T)))));
   CK_REQUIRE(col_chunks <= 65535, "quantize_nvfp4: tensor too large for one launch");
-  const bool dynamic = src.given == nullptr;
-  auto kernel = dynamic ? (hi_first ? quantize_nvfp4_stream_kernel<T, true, true> : quantize_nvfp4_stream_kernel<T, false, true>)
-                        : (hi_first ? quantize_nvfp4_stream_kernel<T, true, false> : quantize_nvfp4_stream_kernel<T, false, false>);
+  auto kernel = hi_first ? quantize_nvfp4_stream_kernel<T, true, kDynamic, kMark> : quantize_nvfp4_stream_kernel<T, false, kDynamic, kMark>;
   // All blocks resident at once and all of the same length: the grid is the number of
   // row groups divided into the fewest equal passes that fit the device.
-  static std::atomic<int> blocks_per_sm[4] = {{0}, {0}, {0}, {0}};
-  std::atomic<int>& known = blocks_per_sm[(hi_first ? 1 : 0) + (dynamic ? 2 : 0)];
+  static std::atomic<int> blocks_per_sm[2] = {{0}, {0}};
+  std::atomic<int>& known = blocks_per_sm[hi_first ? 1 : 0];
   int per_sm = known.load(std::memory_order_relaxed);
   if (per_sm == 0) {
     CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kPairRows, 0));
@@ -410,6 +414,20 @@ int launch_streaming(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t
   CK_CUDA(launch_pdl(kernel, grid, block, 0, stream, x, src, codes, scales, static_cast<int>(orig_rows), static_cast<int>(num_rows),
                      static_cast<int>(num_cols), rows_pad, static_cast<int>(sc_pad), row_groups));
   return CK_OK;
+}
+
+// Inputs of more than a quarter of L2 are marked as long as their codes and scales fit in half of it (64 MiB:
+// 227 MiB of a 16-bit type, 455 of fp32).  Measured marked / not: three linears on one bf16 activation of
+// 24 MiB 91.6 / 89.5 us, of 48 MiB 179.7 / 181.5; fp32 weights of 144 MiB 24.7 / 28.7, of 384 MiB 71.6 / 76.6, of
+// 576 MiB 124 / 115; the reduction and quantizer on 384 MiB of bf16 184.8 / 175.4.
+template <typename T>
+int launch_streaming(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
+                     int64_t num_cols, int hi_first, cudaStream_t stream) {
+  const int64_t bytes = orig_rows * num_cols * static_cast<int64_t>(sizeof(T)), written = num_rows * num_cols / 16 * 9;
+  const bool mark = bytes > (32ll << 20) && written <= (64ll << 20);
+  auto launch = src.given == nullptr ? (mark ? launch_streaming_as<T, true, true> : launch_streaming_as<T, true, false>)
+                                     : (mark ? launch_streaming_as<T, false, true> : launch_streaming_as<T, false, false>);
+  return launch(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream);
 }
 
 template <typename T>

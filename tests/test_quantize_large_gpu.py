@@ -8,8 +8,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# 2100 x 4096 fp32 is 33 MiB, 1050 chunks; 88000 x 3072 bf16 is 516 MiB, more than 16384 chunks of 32 KiB
-@pytest.mark.parametrize("rows, cols, dtype", [(2100, 4096, torch.float32), (7300, 3072, torch.bfloat16), (88000, 3072, torch.bfloat16)])
+# 2100 x 4096 fp32 is 33 MiB in 525 chunks; 38900 x 3072 has 64.1 MiB of codes and scales; 88000 x 3072 bf16 is 516 MiB, more than 16384 chunks of 32 KiB
+@pytest.mark.parametrize("rows, cols, dtype", [(2100, 4096, torch.float32), (7300, 3072, torch.bfloat16), (38900, 3072, torch.bfloat16), (88000, 3072, torch.bfloat16)])
 @pytest.mark.parametrize("where", ["first", "last", "middle"])
 def test_large_input_equals_its_parts(cuda_device, rows, cols, dtype, where):
     from comfy_kitchen.backends import cuda as backend
