@@ -278,6 +278,11 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     else:
         out_rows, out_cols = rows, cols
         assert out_cols % 16 == 0, f"num_cols must be divisible by 16, got {out_cols}"
+    if out_cols != cols or cols % (64 // x.element_size()) or x.data_ptr() % 32:
+        # Not the streaming quantizer's form: the one-kernel scale, whose cached scratch is zero already.  (The
+        # one call would clear its counter first: another launch in front of the other two.)
+        scale = nvfp4_tensor_scale(x)
+        return (*quantize_nvfp4(x, scale, pad_16x=pad_16x, hi_first=hi_first), scale)
     stream = _stream(x.device)
     need = _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
     if rows * cols * x.element_size() <= _WHOLE_INPUT_BYTES:
@@ -502,6 +507,8 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     sx = None if x_scale is None else _scalar_f32(x_scale, dev, "x_scale")
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     need = _workspace_bytes("ck_linear_nvfp4_from_float_workspace_bytes", m, k, int(sx is None))
+    if sx is None and need and x.data_ptr() % 32:
+        sx = nvfp4_tensor_scale(x)  # as in quantize_nvfp4_dynamic
     stream = _stream(dev)
     ws = _call_workspace(need, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)

@@ -479,6 +479,12 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
 constexpr int64_t kWholeInputBytes = 64 * 1024;
 constexpr int64_t kDynamicScratchHead = 256;
 
+__global__ void clear_word_kernel(unsigned int* word) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (threadIdx.x == 0) *word = 0;
+}
+
 template <typename T>
 int launch_nvfp4_dynamic(const void* input, int dtype, float* scale_out, void* codes, void* scales, int64_t orig_rows,
                          int64_t orig_cols, int64_t num_rows, int64_t num_cols, int hi_first, void* scratch,
@@ -498,8 +504,10 @@ int launch_nvfp4_dynamic(const void* input, int dtype, float* scale_out, void* c
     return launch_streaming<T>(x, src, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), orig_rows, num_rows, num_cols,
                                hi_first, stream);
   }
-  // the one-kernel reduction keeps an arrival counter at the head of its scratch, which has to start at zero
-  CK_CUDA(cudaMemsetAsync(scratch, 0, sizeof(unsigned int), stream));
+  // The one-kernel reduction keeps an arrival counter at the head of its scratch, which has to start at zero: cleared
+  // by a kernel, since a memset node would break the chain of dependent launches (8 x 3072 off by one element:
+  // 11.6 us with it, 8.3 so, 7.6 for the two calls on a scratch that is zero).
+  CK_CUDA(launch_pdl(clear_word_kernel, dim3(1), dim3(32), 0, stream, static_cast<unsigned int*>(scratch)));
   if (int rc = ck_nvfp4_tensor_scale(input, dtype, n, scale_out, scratch, scratch_bytes, stream)) return rc;
   return launch_nvfp4<T>(input, scale_out, codes, scales, orig_rows, orig_cols, num_rows, num_cols, hi_first, stream);
 }
