@@ -15,7 +15,7 @@ struct FromFloatLayout {
 };
 
 // Workspace layout: tensor-scale scratch | dynamic tensor scale | codes [M, K/2] | tiled block scales.
-constexpr int64_t kScaleScratchBytes = 256 * 1024;  // covers 2^30 elements
+constexpr int64_t kScaleScratchBytes = 256 + 256 * 1024;  // 2^30 elements: 65536 partials behind the head
 
 FromFloatLayout from_float_layout(int64_t M, int64_t K) {
   FromFloatLayout l{};

@@ -13,6 +13,8 @@ def lib(lib_path):  # noqa: F811
     lib = ctypes.CDLL(lib_path)
     for name in ("ck_quantize_nvfp4_dynamic_scratch_bytes", "ck_nvfp4_tensor_scale_scratch_bytes"):
         getattr(lib, name).argtypes, getattr(lib, name).restype = [ctypes.c_int64], ctypes.c_int64
+    lib.ck_linear_nvfp4_from_float_workspace_bytes.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int]
+    lib.ck_linear_nvfp4_from_float_workspace_bytes.restype = ctypes.c_int64
     return lib
 
 
@@ -29,3 +31,12 @@ def test_dynamic_scratch_depends_on_the_input_alone(lib, n):
 
 def test_dynamic_scratch_of_nothing(lib):
     assert lib.ck_quantize_nvfp4_dynamic_scratch_bytes(0) == 0 == lib.ck_quantize_nvfp4_dynamic_scratch_bytes(-5)
+
+
+@pytest.mark.parametrize("m, k, supported", [(1 << 15, 1 << 15, True), (1 << 20, 1 << 10, True), ((1 << 20) + 16, 1 << 10, False),
+                                             (1 << 15, (1 << 15) + 32, False)])
+def test_linear_takes_up_to_2_30_elements_with_a_dynamic_scale(lib, m, k, supported):
+    """The limit that the header states, and a chunk of the reduction (16384 elements) or more above it."""
+    assert (lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, 1) > 0) == supported
+    assert lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, 0) > 0
+    assert lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, 0) % 256 == 0
