@@ -11,6 +11,7 @@ from __future__ import annotations
 import torch
 
 from .float_utils import roundup
+from .registry import registry
 
 # dtype codes shared with the C ABI (comfy_kitchen/backends/eager/quantization.py:31-39)
 DTYPE_CODE_TO_DTYPE = {
@@ -27,15 +28,38 @@ _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
 
 
 def _impl(name: str, kwargs: dict):
-    from .registry import registry
-
     return registry.get_implementation(name, kwargs=kwargs)(**kwargs)
 
 
+# What Python code can register in front of the kernels below, for tensors that need no gradient.
+_KEYS_IN_FRONT = ("CUDA", "AutocastCUDA", "AutogradCUDA", "ADInplaceOrView", "BackendSelect")
+_registrations = getattr(torch.library, "_impls", None)  # "namespace/operator/key" of every kernel registered from Python
+_own: dict = {}  # operator -> (its definition, the kernels it was defined with, the registrations that would precede them)
+
+
+def _remember(op) -> None:
+    name = op._name
+    _own[name] = (op, dict(op._backend_fns), frozenset(f"comfy_kitchen/{name}/{key}" for key in _KEYS_IN_FRONT))
+
+
+def replaced(name: str) -> bool:
+    """True when somebody has registered a kernel of their own for the operator (``torch.library.impl``,
+    ``register_kernel``, ``register_autocast``) or switched this one off: the dispatcher finds it.  A kernel
+    registered from C++ code leaves no trace that is cheap to see; calls through ``torch.ops`` find it."""
+    known = _own.get(name)
+    if known is None or _registrations is None:
+        return True
+    op, kernels, in_front = known
+    return not in_front.isdisjoint(_registrations) or op._backend_fns != kernels or bool(op._disabled_kernel)
+
+
 def dispatcher_adds_nothing(tensors, optional=()) -> bool:
-    """True when calling an operator through the torch dispatcher would only call its implementation:
-    plain CUDA tensors of no autograd graph, and nobody who watches or rewrites operator calls (tracing,
-    ``torch.compile``, a profiler, a torch function or dispatch mode, functorch, forward-mode autograd).
+    """True when calling an operator that nobody replaced (:func:`replaced`) through the torch dispatcher
+    would only call its implementation: plain CUDA tensors of no autograd graph, and nobody who watches or
+    rewrites operator calls (tracing, ``torch.compile``, a profiler, a torch function or dispatch mode,
+    functorch, forward-mode autograd).  An observer without a profiler
+    (``ExecutionTraceObserver`` on its own) cannot be asked for: it sees the call's allocations and not the
+    operator's name.
 
     The call then goes to the registry at once.  The custom-op layer (schema, autograd and view
     wrappers, output alias checks) costs more host time than a GEMM of a few hundred rows takes on the
@@ -136,3 +160,9 @@ def _op_scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.T
 @_op_scaled_mm_mxfp8.register_fake
 def _(a, b, block_scale_a, block_scale_b, bias, output_dtype_code):
     return a.new_empty((a.shape[0], b.shape[0]), dtype=DTYPE_CODE_TO_DTYPE[output_dtype_code])
+
+
+if _registrations is not None and hasattr(_op_quantize_nvfp4, "_backend_fns") and hasattr(_op_quantize_nvfp4, "_disabled_kernel"):
+    for _op in (_op_quantize_nvfp4, _op_dequantize_nvfp4, _op_scaled_mm_nvfp4, _op_quantize_mxfp8, _op_dequantize_mxfp8,
+                _op_scaled_mm_mxfp8):
+        _remember(_op)
