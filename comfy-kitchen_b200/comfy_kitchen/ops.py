@@ -55,9 +55,9 @@ def replaced(name: str) -> bool:
 
 def dispatcher_adds_nothing(tensors, optional=()) -> bool:
     """True when calling an operator that nobody replaced (:func:`replaced`) through the torch dispatcher
-    would only call its implementation: plain CUDA tensors of no autograd graph, and nobody who watches or
-    rewrites operator calls (tracing, ``torch.compile``, a profiler, a torch function or dispatch mode,
-    functorch, forward-mode autograd).  An observer without a profiler
+    would only call its implementation: plain CUDA tensors of no autograd graph, without a pending negation
+    or zero, and nobody who watches or rewrites operator calls (tracing, ``torch.compile``, a profiler, a
+    torch function or dispatch mode, functorch, forward-mode autograd).  An observer without a profiler
     (``ExecutionTraceObserver`` on its own) cannot be asked for: it sees the call's allocations and not the
     operator's name.
 
@@ -73,10 +73,11 @@ def dispatcher_adds_nothing(tensors, optional=()) -> bool:
         return False
     grad = torch.is_grad_enabled()
     for t in tensors:
-        if type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad):
+        if type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad) or t.is_neg() or t._is_zerotensor():
             return False
     for t in optional:
-        if t is not None and (type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad)):
+        if t is not None and (type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad) or t.is_neg() or
+                              t._is_zerotensor()):
             return False
     return True
 
