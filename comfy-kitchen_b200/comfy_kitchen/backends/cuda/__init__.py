@@ -49,6 +49,7 @@ _SIGNATURES = {
     "ck_abi_version": [],
     "ck_last_error": [],
     "ck_device_supported": [_I],
+    "ck_debug_gemm_splits": [_I, _I, _L, _L, _L],
     "ck_debug_set_exact_division": [_I],
     "ck_quantize_nvfp4": [_P, _I, _P, _P, _P, _L, _L, _L, _L, _I, _P],
     "ck_quantize_nvfp4_dynamic_scratch_bytes": [_L],

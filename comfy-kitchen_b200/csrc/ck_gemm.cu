@@ -77,21 +77,40 @@ int max_splits(int64_t M, int64_t N, int k_bytes) {
   return max(splits, 1);
 }
 
+// CTAs per tile: the most whose clusters all run at once (1 = no split).
 template <Kind KIND, typename OutT>
-int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, int splits, bool* launched, cudaStream_t stream) {
-  *launched = false;
-  const int64_t tiles = ceil_div(p.M, kTileM) * ceil_div(p.N, 128);
-  const int k_stages = static_cast<int>(ceil_div(p.k_bytes, kStageKBytes));
+int choose_splits(int64_t M, int64_t N, int k_bytes, int* out) {
+  const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
+  const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
+  int splits = max_splits(M, N, k_bytes);
   for (; splits > 1; --splits) {
     int clusters = 0;
     if (int rc = split_clusters<KIND, 128, 2, 5, OutT, 1, false>(splits, &clusters)) return rc;
     if (clusters >= tiles) break;
   }
+  *out = static_cast<int>(ceil_div(k_stages, ceil_div(k_stages, splits)));  // none without a stage
+  return CK_OK;
+}
+
+template <Kind KIND, typename OutT>
+int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, bool* launched, cudaStream_t stream) {
+  *launched = false;
+  int splits = 1;
+  if (int rc = choose_splits<KIND, OutT>(p.M, p.N, p.k_bytes, &splits)) return rc;
   if (splits < 2) return CK_OK;
-  p.k_stages_per_split = static_cast<int>(ceil_div(k_stages, splits));
-  p.splits = static_cast<int>(ceil_div(k_stages, p.k_stages_per_split));
+  p.splits = splits;
+  p.k_stages_per_split = static_cast<int>(ceil_div(ceil_div(p.k_bytes, kStageKBytes), splits));
   *launched = true;
   return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1>(ops, p, os, stream);
+}
+
+template <Kind KIND>
+int tile_splits(int out_dtype, int64_t M, int64_t N, int k_bytes, int* splits) {
+  switch (out_dtype) {
+    case CK_DTYPE_BF16: return choose_splits<KIND, __nv_bfloat16>(M, N, k_bytes, splits);
+    case CK_DTYPE_F16: return choose_splits<KIND, __half>(M, N, k_bytes, splits);
+    default: return choose_splits<KIND, float>(M, N, k_bytes, splits);
+  }
 }
 
 struct FusedArgs {
@@ -182,13 +201,13 @@ int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, con
       return scaled_mm_small_m(KIND == Kind::kMxfp8, a, b, sfa, sfb, tsa, tsb, alpha, bias, bias_dtype, out, out_dtype, M, N, K, s);
     }
     // the rows of the result are written four columns at a time
-    if (const int splits = max_splits(M, N, p.k_bytes); splits > 1 && forced_config() == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+    if (max_splits(M, N, p.k_bytes) > 1 && forced_config() == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
       bool launched = false;
       int rc = CK_OK;
       switch (out_dtype) {
-        case CK_DTYPE_BF16: rc = launch_split<KIND, __nv_bfloat16>(ops, p, os, splits, &launched, s); break;
-        case CK_DTYPE_F16: rc = launch_split<KIND, __half>(ops, p, os, splits, &launched, s); break;
-        default: rc = launch_split<KIND, float>(ops, p, os, splits, &launched, s);
+        case CK_DTYPE_BF16: rc = launch_split<KIND, __nv_bfloat16>(ops, p, os, &launched, s); break;
+        case CK_DTYPE_F16: rc = launch_split<KIND, __half>(ops, p, os, &launched, s); break;
+        default: rc = launch_split<KIND, float>(ops, p, os, &launched, s);
       }
       if (rc != CK_OK || launched) return rc;
     }
@@ -255,6 +274,19 @@ extern "C" int64_t ck_scaled_mm_workspace_bytes(int is_mxfp8, int64_t M, int64_t
   const int k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
   const int splits = ck::small_m_applies(M, N, K) ? ck::small_m_max_splits(N, k_bytes) : ck::max_splits(M, N, k_bytes);
   return splits > 1 ? 256 : 0;
+}
+
+extern "C" int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K) {
+  using namespace ck;
+  if (M <= 0 || N <= 0 || K <= 0 || M >= (1ll << 30) || N >= (1ll << 30) || K >= (1ll << 30)) {
+    return -fail(CK_ERR_INVALID_ARGUMENT, "debug_gemm_splits: bad shape");
+  }
+  const int k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
+  int splits = 1;
+  int rc = small_m_applies(M, N, K) ? small_m_splits(is_mxfp8 != 0, out_dtype, M, N, k_bytes, &splits)
+           : is_mxfp8               ? tile_splits<Kind::kMxfp8>(out_dtype, M, N, k_bytes, &splits)
+                                    : tile_splits<Kind::kNvfp4>(out_dtype, M, N, k_bytes, &splits);
+  return rc == CK_OK ? splits : -rc;
 }
 
 extern "C" int ck_scaled_mm_nvfp4_ws(const void* a, const void* b, const void* sfa, const void* sfb,

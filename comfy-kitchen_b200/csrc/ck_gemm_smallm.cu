@@ -7,7 +7,8 @@
 // tensor-memory lanes, the activation rows are the MMA's N (32), the accumulator is 32 columns
 // wide and the epilogue writes 32 values per thread.  When the weight has few 128-row tiles and a
 // long K, every tile's K range is cut over a cluster of CTAs so that all SMs stream (two CTAs fit on
-// an SM); the cluster adds its partial tiles in split order through distributed shared memory.  Measured against the tile path: wins up to 32 rows, loses from 64 rows on.
+// an SM); the cluster adds its partial tiles in split order through distributed shared memory.
+// Measured against the tile path: wins up to 32 rows, loses from 64 rows on.
 #include "ck_gemm_kernel.cuh"
 
 namespace ck {
@@ -15,6 +16,31 @@ namespace {
 
 constexpr int kMaxSmallM = 32;
 constexpr int kSmallTileN = 32;  // the MMA's N: activation rows, padded
+
+// CTAs per tile (1 = no split).  The most whose clusters all run at once with one CTA on an SM; with two on an SM
+// when that leaves a CTA more than ten stages, or sixteen with up to four activation rows, whose exchange is
+// short.  (The occupancy query counts one for every kernel that allocates tensor memory; two of this
+// configuration share an SM.  A cluster that finds no room runs later: nobody waits for it.)  Measured, us, few
+// CTAs of many stages / twice as many: NVFP4 32 x 4096 x 12288 (12 stages) 9.11 / 8.60, MXFP8 32 x 6144 x 12288 (48)
+// 19.0 / 12.5, 1 x 4096 x 12288 (24) 11.6 / 10.2; but NVFP4 1 x 4096 x 8192 (8) 7.2 / 7.9, 1 x 6144 x 6144 (12) 7.8 / 8.4.
+template <Kind KIND, typename OutT>
+int choose_splits(int64_t M, int64_t N, int k_bytes, int* out) {
+  const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
+  const int64_t tiles = ceil_div(N, kTileM);
+  const int most = small_m_max_splits(N, k_bytes);
+  const int max_stages_alone = M <= 4 ? 16 : 10;
+  int splits = 1;
+  for (int per_sm = 1; per_sm <= 2; ++per_sm) {
+    for (splits = most; splits > 1; --splits) {
+      int clusters = 0;
+      if (int rc = split_clusters<KIND, kSmallTileN, 2, 4, OutT, 0, true>(splits, &clusters)) return rc;
+      if (clusters * per_sm >= tiles) break;
+    }
+    if (ceil_div(k_stages, splits) <= max_stages_alone) break;
+  }
+  *out = static_cast<int>(ceil_div(k_stages, ceil_div(k_stages, splits)));  // none without a stage
+  return CK_OK;
+}
 
 template <Kind KIND, typename OutT>
 int launch_small(const Operands& ops, GemmParams p, cudaStream_t stream) {
@@ -24,17 +50,13 @@ int launch_small(const Operands& ops, GemmParams p, cudaStream_t stream) {
   os.n = 1;
   os.pitch = p.N;
   os.col_offset = 0;
-  const int k_stages = static_cast<int>(ceil_div(p.k_bytes, kStageKBytes));
-  const int64_t tiles = ceil_div(p.M, kTileM);
-  int splits = small_m_max_splits(p.M, p.k_bytes);
-  for (; splits > 1; --splits) {
-    int clusters = 0;
-    if (int rc = split_clusters<KIND, kSmallTileN, 2, 4, OutT, 0, true>(splits, &clusters)) return rc;
-    if (clusters >= tiles) break;
+  if (int rc = choose_splits<KIND, OutT>(p.N, p.M, p.k_bytes, &p.splits)) return rc;
+  p.k_stages_per_split = static_cast<int>(ceil_div(ceil_div(p.k_bytes, kStageKBytes), p.splits));
+  // a quarter tile of one activation row per warp of the cluster, if there are warps enough for all of them
+  if (4 * p.N <= p.splits * epilogue_warps(false, kSmallTileN)) {
+    return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true>(ops, p, os, stream);
   }
-  p.k_stages_per_split = static_cast<int>(ceil_div(k_stages, splits));
-  p.splits = static_cast<int>(ceil_div(k_stages, p.k_stages_per_split));
-  return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true>(ops, p, os, stream);
+  return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true, true>(ops, p, os, stream);
 }
 
 }  // namespace
@@ -51,6 +73,21 @@ int small_m_max_splits(int64_t N, int k_bytes) {
   const int64_t by_sms = 2 * static_cast<int64_t>(sm_count()) / tiles;
   if (by_sms < splits) splits = static_cast<int>(by_sms);
   return max(splits, 1);
+}
+
+int small_m_splits(bool is_mxfp8, int out_dtype, int64_t M, int64_t N, int k_bytes, int* splits) {
+  if (is_mxfp8) {
+    switch (out_dtype) {
+      case CK_DTYPE_BF16: return choose_splits<Kind::kMxfp8, __nv_bfloat16>(M, N, k_bytes, splits);
+      case CK_DTYPE_F16: return choose_splits<Kind::kMxfp8, __half>(M, N, k_bytes, splits);
+      default: return choose_splits<Kind::kMxfp8, float>(M, N, k_bytes, splits);
+    }
+  }
+  switch (out_dtype) {
+    case CK_DTYPE_BF16: return choose_splits<Kind::kNvfp4, __nv_bfloat16>(M, N, k_bytes, splits);
+    case CK_DTYPE_F16: return choose_splits<Kind::kNvfp4, __half>(M, N, k_bytes, splits);
+    default: return choose_splits<Kind::kNvfp4, float>(M, N, k_bytes, splits);
+  }
 }
 
 // a: activation [M, K], b: weight [N, K] (the public argument order); shapes and pointers were validated by the caller.

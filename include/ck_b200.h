@@ -349,6 +349,11 @@ CK_API int ck_peer_status(int* status_out);
  */
 CK_API int ck_gemm_status(int* status_out);
 
+/* Validation aid with no counterpart in the reference: the number of CTAs that share a tile's K range when
+ * ck_scaled_mm_* computes this shape on the current device (1 = K is not split), or a negative error code.
+ * A result that does not start on a 16-byte boundary is not split beyond 32 rows. */
+CK_API int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K);
+
 /* Validation aid with no counterpart in the reference: writes `value` into the GEMM status
  * word of the current device from the host (synchronises first), so that a caller's handling
  * of a non-zero status can be tested without making any kernel fail. */
