@@ -49,7 +49,7 @@ _SIGNATURES = {
     "ck_abi_version": [],
     "ck_last_error": [],
     "ck_device_supported": [_I],
-    "ck_debug_gemm_splits": [_I, _I, _L, _L, _L],
+    "ck_debug_gemm_splits": [_I, _I, _L, _L, _L, _I],
     "ck_debug_set_exact_division": [_I],
     "ck_quantize_nvfp4": [_P, _I, _P, _P, _P, _L, _L, _L, _L, _I, _P],
     "ck_quantize_nvfp4_dynamic_scratch_bytes": [_L],
@@ -256,6 +256,7 @@ def nvfp4_tensor_scale(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
+_ON_CHIP = 256  # the workspace size of a GEMM that does not use one (ck_scaled_mm_workspace_bytes)
 _WHOLE_INPUT_BYTES = 64 << 10  # inputs up to here take no reduction kernel (ck_quantize_nvfp4_dynamic)
 
 
@@ -381,9 +382,11 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        _check(lib.ck_scaled_mm_nvfp4(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), _ptr(tsa), _ptr(tsb),
-                                      _ptr(alpha_t), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
-                                      _stream(dev)), "scaled_mm_nvfp4")
+        need = _workspace_bytes("ck_scaled_mm_workspace_bytes", 0, m, n, k)
+        ws = _call_workspace(need, dev) if need > _ON_CHIP else None
+        _check(lib.ck_scaled_mm_nvfp4_ws(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), _ptr(tsa), _ptr(tsb),
+                                         _ptr(alpha_t), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
+                                         _ptr(ws), need, _stream(dev)), "scaled_mm_nvfp4")
     del bias_keep
     return out
 
@@ -618,8 +621,11 @@ def scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tenso
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        _check(lib.ck_scaled_mm_mxfp8(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), bias_ptr, bias_code,
-                                      _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, _stream(dev)), "scaled_mm_mxfp8")
+        need = _workspace_bytes("ck_scaled_mm_workspace_bytes", 1, m, n, k)
+        ws = _call_workspace(need, dev) if need > _ON_CHIP else None
+        _check(lib.ck_scaled_mm_mxfp8_ws(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), bias_ptr, bias_code,
+                                         _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, _ptr(ws), need, _stream(dev)),
+               "scaled_mm_mxfp8")
     del bias_keep
     return out
 

@@ -64,9 +64,8 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
 // ---------------------------------------------------------------------------
 // split-K
 // ---------------------------------------------------------------------------
-// Few 128 x 128 tiles and a long K: the K range of a tile is spread over a cluster of CTAs that add
-// their partial tiles through distributed shared memory (ck_gemm_kernel.cuh).  At most as many CTAs
-// per tile as leave every CTA six pipeline stages and let all clusters run at once; 1 = no split.
+// Few 128 x 128 tiles and a long K: the K range of a tile is spread over several CTAs.  At most as many as fit the
+// chip and leave every CTA six pipeline stages; 1 = no split.
 int max_splits(int64_t M, int64_t N, int k_bytes) {
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
@@ -77,40 +76,120 @@ int max_splits(int64_t M, int64_t N, int k_bytes) {
   return max(splits, 1);
 }
 
-// CTAs per tile: the most whose clusters all run at once (1 = no split).
+struct SplitPlan {
+  int splits;            // CTAs per tile
+  int k_stages;          // of each
+  bool through_workspace;
+};
+
+int64_t split_workspace_bytes(int64_t M, int64_t N, const SplitPlan& plan) { return plan.splits * M * N * 4; }
+
+// A cluster of CTAs adds its partial tiles on chip (ck_gemm_kernel.cuh): the most CTAs per tile whose clusters all run
+// at once.  A cluster sits in one part of the chip, which can leave SMs idle that a split without clusters uses; its
+// CTAs store their partial tiles to a workspace and a second kernel adds them.  That exchange costs about one
+// pipeline stage per partial tile, so it is taken where it saves a CTA more stages than there are partial tiles.
+// Graph replays, us, clusters / workspace: 256 x 3072 x 12288 14.0 / 12.4 with NVFP4 (24 / 16 stages, 3 partial tiles), 20.4 / 16.5
+// with MXFP8 (48 / 32), x 6144 NVFP4 10.2 / 9.7 (12 / 8), 256 x 2176 x 16384 13.0 / 12.7 (22 / 16, 4); but 256 x 2176 x 12288 11.1 / 11.5
+// (16 / 12, 4), 256 x 1152 x 12288 MXFP8 11.1 / 11.9 (16 / 12, 8).
 template <Kind KIND, typename OutT>
-int choose_splits(int64_t M, int64_t N, int k_bytes, int* out) {
+int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitPlan* plan) {
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
-  int splits = max_splits(M, N, k_bytes);
+  const int most = max_splits(M, N, k_bytes);
+  int splits = most;
   for (; splits > 1; --splits) {
     int clusters = 0;
     if (int rc = split_clusters<KIND, 128, 2, 5, OutT, 1, false>(splits, &clusters)) return rc;
     if (clusters >= tiles) break;
   }
-  *out = static_cast<int>(ceil_div(k_stages, ceil_div(k_stages, splits)));  // none without a stage
+  plan->through_workspace = have_workspace && ceil_div(k_stages, splits) - ceil_div(k_stages, most) > most;
+  plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
+  plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage
   return CK_OK;
 }
 
+// out = cast(alpha * (partial_0 + partial_1 + ...) + bias), four consecutive columns per thread; the partials are
+// added in index order, so the result does not depend on scheduling.
+template <typename OutT>
+__global__ void __launch_bounds__(256)
+splitk_reduce_kernel(const float* partials, int splits, int64_t mn, int n_cols, const float* alpha_ptr, const float* tsa,
+                     const float* tsb, const void* bias, int bias_dtype, OutT* out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+  if (i >= mn) return;
+  float alpha = 1.0f;
+  if (alpha_ptr != nullptr) {
+    alpha = ld_f32_dependent(alpha_ptr);
+  } else if (tsa != nullptr && tsb != nullptr) {
+    alpha = ld_f32_dependent(tsa) * ld_f32_dependent(tsb);
+  }
+  float4 acc = *reinterpret_cast<const float4*>(partials + i);
+  for (int s = 1; s < splits; ++s) {
+    const float4 v = *reinterpret_cast<const float4*>(partials + s * mn + i);
+    acc.x += v.x;
+    acc.y += v.y;
+    acc.z += v.z;
+    acc.w += v.w;
+  }
+  const int n = static_cast<int>(i % n_cols);  // N % 8 == 0: a group of four never straddles two rows
+  float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = load_bias(bias, bias_dtype, n + j);
+  }
+  const float y[4] = {fmaf(acc.x, alpha, b[0]), fmaf(acc.y, alpha, b[1]), fmaf(acc.z, alpha, b[2]), fmaf(acc.w, alpha, b[3])};
+  store_four(out + i, y);
+}
+
 template <Kind KIND, typename OutT>
-int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, bool* launched, cudaStream_t stream) {
+int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, void* workspace, int64_t workspace_bytes, bool* launched,
+                 cudaStream_t stream) {
   *launched = false;
-  int splits = 1;
-  if (int rc = choose_splits<KIND, OutT>(p.M, p.N, p.k_bytes, &splits)) return rc;
-  if (splits < 2) return CK_OK;
-  p.splits = splits;
-  p.k_stages_per_split = static_cast<int>(ceil_div(ceil_div(p.k_bytes, kStageKBytes), splits));
+  SplitPlan plan = {};
+  if (int rc = choose_splits<KIND, OutT>(p.M, p.N, p.k_bytes, workspace != nullptr, &plan)) return rc;
+  if (plan.through_workspace && (workspace_bytes < split_workspace_bytes(p.M, p.N, plan) || reinterpret_cast<uintptr_t>(workspace) % 16 != 0)) {
+    if (int rc = choose_splits<KIND, OutT>(p.M, p.N, p.k_bytes, false, &plan)) return rc;
+  }
+  if (plan.splits < 2) return CK_OK;
   *launched = true;
-  return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1>(ops, p, os, stream);
+  const int64_t mn = static_cast<int64_t>(p.M) * p.N;
+  const GemmParams result = p;
+  p.splits = plan.splits;
+  p.k_stages_per_split = plan.k_stages;
+  if (!plan.through_workspace) return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1>(ops, p, os, stream);
+  p.split_outputs = 1;
+  p.tsa = p.tsb = p.alpha = nullptr;
+  p.bias = nullptr;
+  p.out = workspace;
+  p.out_dtype = CK_DTYPE_F32;
+  void* parts[kMaxOutputs] = {};
+  for (int i = 0; i < plan.splits; ++i) parts[i] = static_cast<float*>(workspace) + i * mn;
+  OutputSpec partials;
+  partials.ptrs = parts;
+  partials.n = plan.splits;
+  partials.pitch = p.N;
+  partials.col_offset = 0;
+  if (int rc = launch_config<KIND, 128, 2, 5, 1, float, false, 1>(ops, p, partials, stream)) return rc;
+  CK_CUDA(launch_pdl(splitk_reduce_kernel<OutT>, dim3(static_cast<unsigned>(ceil_div(mn / 4, 256))), dim3(256), 0, stream,
+                     static_cast<const float*>(workspace), plan.splits, mn, p.N, result.alpha, result.tsa, result.tsb, result.bias,
+                     result.bias_dtype, static_cast<OutT*>(result.out)));
+  return CK_OK;
 }
 
 template <Kind KIND>
-int tile_splits(int out_dtype, int64_t M, int64_t N, int k_bytes, int* splits) {
+int tile_plan(int out_dtype, int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitPlan* plan) {
   switch (out_dtype) {
-    case CK_DTYPE_BF16: return choose_splits<KIND, __nv_bfloat16>(M, N, k_bytes, splits);
-    case CK_DTYPE_F16: return choose_splits<KIND, __half>(M, N, k_bytes, splits);
-    default: return choose_splits<KIND, float>(M, N, k_bytes, splits);
+    case CK_DTYPE_BF16: return choose_splits<KIND, __nv_bfloat16>(M, N, k_bytes, have_workspace, plan);
+    case CK_DTYPE_F16: return choose_splits<KIND, __half>(M, N, k_bytes, have_workspace, plan);
+    default: return choose_splits<KIND, float>(M, N, k_bytes, have_workspace, plan);
   }
+}
+
+int tile_plan(bool is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K, bool have_workspace, SplitPlan* plan) {
+  const int k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
+  return is_mxfp8 ? tile_plan<Kind::kMxfp8>(out_dtype, M, N, k_bytes, have_workspace, plan)
+                  : tile_plan<Kind::kNvfp4>(out_dtype, M, N, k_bytes, have_workspace, plan);
 }
 
 struct FusedArgs {
@@ -125,7 +204,7 @@ template <Kind KIND>
 int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
               const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
               int64_t M, int64_t N, int64_t K, void* stream, const FusedArgs& fused = FusedArgs(),
-              const OutputSpec* out_spec = nullptr) {
+              const OutputSpec* out_spec = nullptr, void* workspace = nullptr, int64_t workspace_bytes = 0) {
   CK_REQUIRE(a && b && sfa && sfb, "%s: null pointer", op);
   CK_REQUIRE(out != nullptr || (fused.enabled && fused.rq_codes != nullptr), "%s: no output requested", op);
   if (fused.enabled) {
@@ -205,9 +284,9 @@ int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, con
       bool launched = false;
       int rc = CK_OK;
       switch (out_dtype) {
-        case CK_DTYPE_BF16: rc = launch_split<KIND, __nv_bfloat16>(ops, p, os, &launched, s); break;
-        case CK_DTYPE_F16: rc = launch_split<KIND, __half>(ops, p, os, &launched, s); break;
-        default: rc = launch_split<KIND, float>(ops, p, os, &launched, s);
+        case CK_DTYPE_BF16: rc = launch_split<KIND, __nv_bfloat16>(ops, p, os, workspace, workspace_bytes, &launched, s); break;
+        case CK_DTYPE_F16: rc = launch_split<KIND, __half>(ops, p, os, workspace, workspace_bytes, &launched, s); break;
+        default: rc = launch_split<KIND, float>(ops, p, os, workspace, workspace_bytes, &launched, s);
       }
       if (rc != CK_OK || launched) return rc;
     }
@@ -267,41 +346,47 @@ extern "C" int ck_linear_nvfp4_fused(const void* a, const void* b, const void* s
                                          bias_dtype, out, out_dtype, M, N, K, stream, f);
 }
 
-// The split-K clusters exchange their partial tiles on chip: the workspace of these entry points is
-// accepted and not used.  The size stays non-zero for the shapes whose K is split.
+// Non-zero for the shapes whose K may be split: kOnChip where the partial tiles stay on chip (or K is long, but not
+// long enough), which callers of this query have been given for those shapes before and which is not used.
 extern "C" int64_t ck_scaled_mm_workspace_bytes(int is_mxfp8, int64_t M, int64_t N, int64_t K) {
+  using namespace ck;
+  constexpr int64_t kOnChip = 256;
   if (M <= 0 || N <= 0 || K <= 0 || M >= (1ll << 30) || N >= (1ll << 30) || K >= (1ll << 30)) return 0;
   const int k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
-  const int splits = ck::small_m_applies(M, N, K) ? ck::small_m_max_splits(N, k_bytes) : ck::max_splits(M, N, k_bytes);
-  return splits > 1 ? 256 : 0;
+  if (small_m_applies(M, N, K)) return small_m_max_splits(N, k_bytes) > 1 ? kOnChip : 0;
+  if (ceil_div(M, kTileM) * ceil_div(N, 128) * 2 > sm_count() || ceil_div(k_bytes, kStageKBytes) < 16) return 0;
+  SplitPlan plan = {};
+  if (tile_plan(is_mxfp8 != 0, CK_DTYPE_BF16, M, N, K, true, &plan) != CK_OK || !plan.through_workspace) return kOnChip;
+  return split_workspace_bytes(M, N, plan);
 }
 
-extern "C" int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K) {
+extern "C" int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K, int with_workspace) {
   using namespace ck;
   if (M <= 0 || N <= 0 || K <= 0 || M >= (1ll << 30) || N >= (1ll << 30) || K >= (1ll << 30)) {
     return -fail(CK_ERR_INVALID_ARGUMENT, "debug_gemm_splits: bad shape");
   }
-  const int k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
-  int splits = 1;
-  int rc = small_m_applies(M, N, K) ? small_m_splits(is_mxfp8 != 0, out_dtype, M, N, k_bytes, &splits)
-           : is_mxfp8               ? tile_splits<Kind::kMxfp8>(out_dtype, M, N, k_bytes, &splits)
-                                    : tile_splits<Kind::kNvfp4>(out_dtype, M, N, k_bytes, &splits);
-  return rc == CK_OK ? splits : -rc;
+  SplitPlan plan = {};
+  const int rc = small_m_applies(M, N, K)
+                     ? small_m_splits(is_mxfp8 != 0, out_dtype, M, N, static_cast<int>(is_mxfp8 ? K : K / 2), &plan.splits)
+                     : tile_plan(is_mxfp8 != 0, out_dtype, M, N, K, with_workspace != 0, &plan);
+  return rc == CK_OK ? plan.splits : -rc;
 }
 
 extern "C" int ck_scaled_mm_nvfp4_ws(const void* a, const void* b, const void* sfa, const void* sfb,
                                      const float* tensor_scale_a, const float* tensor_scale_b, const float* alpha,
                                      const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M, int64_t N,
-                                     int64_t K, void* /*workspace*/, int64_t /*workspace_bytes*/, void* stream) {
+                                     int64_t K, void* workspace, int64_t workspace_bytes, void* stream) {
   return ck::scaled_mm<ck::Kind::kNvfp4>("scaled_mm_nvfp4", a, b, sfa, sfb, tensor_scale_a, tensor_scale_b, alpha, bias,
-                                         bias_dtype, out, out_dtype, M, N, K, stream);
+                                         bias_dtype, out, out_dtype, M, N, K, stream, ck::FusedArgs(), nullptr, workspace,
+                                         workspace_bytes);
 }
 
 extern "C" int ck_scaled_mm_mxfp8_ws(const void* a, const void* b, const void* sfa, const void* sfb, const void* bias,
                                      int bias_dtype, void* out, int out_dtype, int64_t M, int64_t N, int64_t K,
-                                     void* /*workspace*/, int64_t /*workspace_bytes*/, void* stream) {
+                                     void* workspace, int64_t workspace_bytes, void* stream) {
   return ck::scaled_mm<ck::Kind::kMxfp8>("scaled_mm_mxfp8", a, b, sfa, sfb, nullptr, nullptr, nullptr, bias, bias_dtype,
-                                         out, out_dtype, M, N, K, stream);
+                                         out, out_dtype, M, N, K, stream, ck::FusedArgs(), nullptr, workspace,
+                                         workspace_bytes);
 }
 
 extern "C" int ck_scaled_mm_nvfp4_allgather(const void* a, const void* b, const void* sfa, const void* sfb,

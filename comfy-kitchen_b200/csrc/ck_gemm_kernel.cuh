@@ -141,7 +141,8 @@ struct GemmParams {
   int out_tma;             // the output qualifies for TMA stores (16-byte aligned base and pitch)
   int n_out;               // destinations of every output tile (1, or one per GPU of an all-gather)
   int splits;              // split-K: CTAs per tile (1 = off), one thread-block cluster; CTA s of it covers pipeline stages
-  int k_stages_per_split;  //   [s * k_stages_per_split, ...) and the cluster adds the raw fp32 partial tiles in its shared memory
+  int k_stages_per_split;  //   [s * k_stages_per_split, ...) and the cluster adds the raw fp32 partial tiles in its shared memory,
+  int split_outputs;       //   or, set, no cluster: CTA s stores its raw fp32 partial tile to destination s
   int* status;             // device status word: set non-zero when a wait gave up
   int trace_launch;        // sequence number of the launch (timeline builds only)
   // fused epilogue (FUSED kernels only)
@@ -417,6 +418,8 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // configurations whose tiles may be split along K over the CTAs of a cluster
   constexpr bool kCanSplit = CTAS == 1 && !FUSED && (SWAP || TILE_N == 128);
   static_assert(!kCanSplit || kTileM * TILE_N * 4 <= Cfg::kRingBytes, "a partial tile fits in the operand ring");
+  // and the one whose CTAs may instead store their partial tiles each to a destination of its own
+  constexpr bool kCanSplitOutputs = kCanSplit && !SWAP && std::is_same<OutT, float>::value;
   // Everything the kernel does until a role's griddepcontrol.wait is independent of the kernel
   // before it in the stream, so the next kernel may be scheduled as early as resources allow.
   pdl_launch_dependents();
@@ -864,7 +867,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
       }
       if constexpr (kCanSplit) {
-        if (splits > 1) {
+        if (splits > 1 && !(kCanSplitOutputs && p.split_outputs)) {
           // Raw partial to the CTA's own shared memory: row r at r * TILE_N * 4 bytes, its 16-byte unit u
           // at position u ^ (r % 8) (the eight rows of a store phase meet eight different bank groups).
           const int r = quarter * 32 + lane;
@@ -948,8 +951,12 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 __syncwarp();
                 const int col = n0 + c0 + (c / kChunksPerBox) * kBoxCols;
                 if (lane == 0 && row0 < p.M && col < p.N) {
-                  // the same staged box goes to every destination (peer stores cross NVLink)
-                  for (int d = 0; d < p.n_out; ++d) tma_store_2d_addr(&maps_out.m[d], stage_box, col, row0);
+                  if (kCanSplitOutputs && p.split_outputs) {
+                    tma_store_2d_addr(&maps_out.m[item - tile * splits], stage_box, col, row0);  // this item's partial
+                  } else {
+                    // the same staged box goes to every destination (peer stores cross NVLink)
+                    for (int d = 0; d < p.n_out; ++d) tma_store_2d_addr(&maps_out.m[d], stage_box, col, row0);
+                  }
                 }
                 // (an empty group when nothing was stored keeps the ring's group count in step)
                 if (lane == 0) bulk_commit_group();
@@ -1104,10 +1111,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // against partial tiles through L2 (graph replays, us; linear = quantize + GEMM in one call, which
   // had no workspace and ran unsplit): MXFP8 1 x 3072 x 12288 linear 30.1 -> 12.5, 256 rows 33.0 -> 24.4;
   // NVFP4 1 x 1024 x 15360 GEMM 8.7 -> 6.3, linear 21.8 -> 8.1; 64 x 3072 x 12288 11.3 -> 9.6.  A cluster
-  // must find its SMs in one part of the chip: where three CTAs per tile no longer fit at once, two are
-  // used (256 x 3072 x 12288 GEMM: 13.0 -> 14.4 with NVFP4, 17.0 -> 20.8 with MXFP8).
+  // must find its SMs in one part of the chip: where that costs too many CTAs per tile, the GEMMs that have
+  // a workspace go through it (choose_splits in ck_gemm.cu).
   if constexpr (kCanSplit) {
-    if (splits > 1) {
+    if (splits > 1 && !(kCanSplitOutputs && p.split_outputs)) {
       __syncwarp();
       cluster_sync_all();
       if (warp >= 2) {
@@ -1405,7 +1412,8 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS == 1 ? p.splits : CTAS;  // split-K: the CTAs of one tile are a cluster
+  const bool cluster_split = CTAS == 1 && p.splits > 1 && p.split_outputs == 0;
+  attr[0].val.clusterDim.x = cluster_split ? p.splits : CTAS;  // split-K: the CTAs of one tile are a cluster
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1427,7 +1435,7 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
     if (dev >= 0 && dev < 64) max_workers[dev].store(resident, std::memory_order_release);
   }
   int workers = min(p.tiles_m * p.tiles_n * p.splits, resident);
-  if (p.splits > 1) workers = p.tiles_m * p.tiles_n * p.splits;  // one item per CTA
+  if (cluster_split) workers = p.tiles_m * p.tiles_n * p.splits;  // one item per CTA
 #ifdef CK_GEMM_TRACE
   if (const char* e = getenv("CK_GEMM_MAX_WORKERS")) workers = min(workers, atoi(e));
   static std::atomic<int> launch_seq{0};
@@ -1457,13 +1465,14 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
     // TMA stores need 16-byte aligned bases and row pitch.  A single dense [M, N] result whose rows
     // start on 32-byte boundaries is written straight from registers instead (256-bit stores, whole
     // sectors): measured 1-3 % faster than staging it for TMA stores, whose shared-memory traffic
-    // slows the next tile's main loop.  Multi-destination stores (all-gather) go through the staged path.
+    // slows the next tile's main loop.  Multi-destination stores (all-gather, partial tiles of a split) go
+    // through the staged path.
     bool ok = p.out != nullptr && (os.pitch * static_cast<int64_t>(sizeof(OutT))) % 16 == 0 &&
               (os.col_offset * static_cast<int64_t>(sizeof(OutT))) % 16 == 0;
     for (int d = 0; ok && d < os.n; ++d) ok = os.ptrs[d] != nullptr && reinterpret_cast<uintptr_t>(os.ptrs[d]) % 16 == 0;
     const bool direct = os.n == 1 && os.plain(p.N) && p.out != nullptr &&
                         (static_cast<int64_t>(p.N) * sizeof(OutT)) % 32 == 0 && reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
-    ok = ok && !direct && p.splits == 1;  // a split-K cluster writes its result itself
+    ok = ok && !direct && !cluster_split;  // a split-K cluster writes its result itself
     if (ok) {
       for (int d = 0; d < os.n; ++d) {
         void* base = static_cast<uint8_t*>(os.ptrs[d]) + os.col_offset * static_cast<int64_t>(sizeof(OutT));

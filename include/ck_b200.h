@@ -270,8 +270,11 @@ CK_API int ck_scaled_mm_mxfp8(const void* a, const void* b, const void* sfa, con
  * same way, comfy_kitchen/backends/cuda/__init__.py:117-124, ops/cublas_gemm_nvfp4.cu:297-311).
  * Problems with few output tiles and a long K are computed split-K by every GEMM entry point: a
  * cluster of CTAs per tile adds its fp32 partial tiles on chip, in a fixed order (deterministic).
- * The workspace is therefore accepted and not used, null included;
- * ck_scaled_mm_workspace_bytes is non-zero for the shapes that may be split.
+ * For some shapes beyond 32 rows a split over more CTAs, whose partial tiles go through a workspace, is
+ * faster: these entry points take it when they are handed 16-byte aligned device memory of at least
+ * ck_scaled_mm_workspace_bytes bytes, with no requirement on its contents (calls that can overlap on the
+ * GPU need separate workspaces).  Null, or fewer bytes: as the entry points above.  The size is
+ * non-zero for all shapes that may be split, and 256 for those that do not use the workspace.
  */
 CK_API int64_t ck_scaled_mm_workspace_bytes(int is_mxfp8, int64_t M, int64_t N, int64_t K);
 CK_API int ck_scaled_mm_nvfp4_ws(const void* a, const void* b, const void* block_scale_a,
@@ -350,9 +353,10 @@ CK_API int ck_peer_status(int* status_out);
 CK_API int ck_gemm_status(int* status_out);
 
 /* Validation aid with no counterpart in the reference: the number of CTAs that share a tile's K range when
- * ck_scaled_mm_* computes this shape on the current device (1 = K is not split), or a negative error code.
+ * ck_scaled_mm_* (with_workspace != 0: its variant with a workspace of the size that it asks for)
+ * computes this shape on the current device (1 = K is not split), or a negative error code.
  * A result that does not start on a 16-byte boundary is not split beyond 32 rows. */
-CK_API int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K);
+CK_API int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int64_t N, int64_t K, int with_workspace);
 
 /* Validation aid with no counterpart in the reference: writes `value` into the GEMM status
  * word of the current device from the host (synchronises first), so that a caller's handling
