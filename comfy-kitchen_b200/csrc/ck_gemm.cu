@@ -65,11 +65,12 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
 // split-K
 // ---------------------------------------------------------------------------
 // Few 128 x 128 tiles and a long K: the K range of a tile is spread over several CTAs.  At most as many as fit the
-// chip and leave every CTA six pipeline stages; 1 = no split.
+// chip and leave every CTA six pipeline stages; 1 = no split, also where only two CTAs would come of it (below 18
+// stages; graph replays, us, split in two / unsplit: NVFP4 128 x 3072 x 4096 8.7 / 7.4, 256 x 4096 x 4096 9.2 / 8.3).
 int max_splits(int64_t M, int64_t N, int k_bytes) {
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
-  if (tiles * 2 > sm_count() || k_stages < 16) return 1;
+  if (tiles * 2 > sm_count() || k_stages < 18) return 1;
   int splits = min(kMaxSplits, k_stages / 6);
   const int64_t by_sms = sm_count() / tiles;
   if (by_sms < splits) splits = static_cast<int>(by_sms);

@@ -36,6 +36,8 @@ def test_few_rows(splits, cuda_device, n, rows, mx, dtype):
 def test_not_split(splits, mx):
     assert splits(mx, 1, 6400, 12288) == 1      # more than a third of the SMs have a tile
     assert splits(mx, 32, 1024, 1024) == 1      # a short K
+    assert splits(mx, 128, 3072, 17 * (128 if mx else 256)) == 1  # tiles of which two CTAs would come
+    assert splits(mx, 128, 3072, 18 * (128 if mx else 256)) == 3
     assert splits(mx, 4096, 3072, 12288) == 1   # many tiles
     assert splits(mx, 0, 128, 4096) < 0
 
