@@ -782,7 +782,8 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
         if (warp == 2) CK_TRACE(13);
         if (a_row < p.M) {
-          OutT* dst = out + a_row;
+          // one address, moved from row to row: 32 of them at once cost the 16-bit results 40 registers and spills
+          OutT* dst = out + static_cast<int64_t>(n0 + c0) * p.M + a_row;
 #pragma unroll
           for (int c = 0; c < kChunks; ++c) {
 #pragma unroll
@@ -790,16 +791,8 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               const int b_row = n0 + c0 + c * 32 + i;  // activation row = output row
               if (c == 0 && i == 1 && warp == 2) CK_TRACE(14);
               if (c == 0 && i == 8 && warp == 2) CK_TRACE(15);
-              if (b_row < p.N) {
-                const float y = fmaf(__uint_as_float(buf[c][i]), alpha, bias_v);
-                if constexpr (std::is_same<OutT, __nv_bfloat16>::value) {
-                  dst[static_cast<int64_t>(b_row) * p.M] = __float2bfloat16_rn(y);
-                } else if constexpr (std::is_same<OutT, __half>::value) {
-                  dst[static_cast<int64_t>(b_row) * p.M] = __float2half_rn(y);
-                } else {
-                  dst[static_cast<int64_t>(b_row) * p.M] = y;
-                }
-              }
+              if (b_row < p.N) *dst = to_out<OutT>(fmaf(__uint_as_float(buf[c][i]), alpha, bias_v));
+              dst += p.M;
             }
           }
         }
