@@ -46,7 +46,7 @@ int launch_amax_partials(const void* x, int dtype, int64_t n_vecs, float* partia
 // GEMMs with few activation rows (ck_gemm_smallm.cu).
 bool small_m_applies(int64_t M, int64_t N, int64_t K);
 int small_m_max_splits(int64_t N, int k_bytes);
-int small_m_splits(bool is_mxfp8, int out_dtype, int64_t M, int64_t N, int k_bytes, int* splits);
+int small_m_splits(bool is_mxfp8, int out_dtype, int64_t N, int k_bytes, int* splits);
 int scaled_mm_small_m(bool is_mxfp8, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
                       const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
                       int64_t M, int64_t N, int64_t K, cudaStream_t stream);

@@ -66,7 +66,7 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
 // ---------------------------------------------------------------------------
 // Few 128 x 128 tiles and a long K: the K range of a tile is spread over several CTAs.  At most as many as fit the
 // chip and leave every CTA six pipeline stages; 1 = no split, also where only two CTAs would come of it (below 18
-// stages; graph replays, us, split in two / unsplit: NVFP4 128 x 3072 x 4096 8.7 / 7.4, 256 x 4096 x 4096 9.2 / 8.3).
+// stages; graph replays, us, split in two / unsplit: NVFP4 128 x 3072 x 4096 8.3 / 7.3, 256 x 4096 x 4096 8.7 / 7.9).
 int max_splits(int64_t M, int64_t N, int k_bytes) {
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
@@ -87,11 +87,11 @@ int64_t split_workspace_bytes(int64_t M, int64_t N, const SplitPlan& plan) { ret
 
 // A cluster of CTAs adds its partial tiles on chip (ck_gemm_kernel.cuh): the most CTAs per tile whose clusters all run
 // at once.  A cluster sits in one part of the chip, which can leave SMs idle that a split without clusters uses; its
-// CTAs store their partial tiles to a workspace and a second kernel adds them.  That exchange costs about one
-// pipeline stage per partial tile, so it is taken where it saves a CTA more stages than there are partial tiles.
-// Graph replays, us, clusters / workspace: 256 x 3072 x 12288 14.0 / 12.4 with NVFP4 (24 / 16 stages, 3 partial tiles), 20.4 / 16.5
-// with MXFP8 (48 / 32), x 6144 NVFP4 10.2 / 9.7 (12 / 8), 256 x 2176 x 16384 13.0 / 12.7 (22 / 16, 4); but 256 x 2176 x 12288 11.1 / 11.5
-// (16 / 12, 4), 256 x 1152 x 12288 MXFP8 11.1 / 11.9 (16 / 12, 8).
+// CTAs store their partial tiles to a workspace and a second kernel adds them.  That exchange costs about four
+// thirds of a pipeline stage per partial tile, so it is taken where it saves a CTA that many.  Graph replays, us,
+// clusters / workspace: 256 x 3072 x 12288 13.3 / 11.9 with NVFP4 (24 / 16 stages, 3 partial tiles), 19.5 / 15.8 with MXFP8
+// (48 / 32), x 6144 NVFP4 9.7 / 9.4 (12 / 8), 256 x 2176 x 12288 MXFP8 14.7 / 14.0 (32 / 24, 4); but 256 x 2176 x 12288 NVFP4
+// 10.6 / 11.0 (16 / 12, 4), 256 x 1152 x 12288 MXFP8 10.6 / 11.5 (16 / 12, 8), 128 x 3712 x 16384 MXFP8 14.8 / 14.9 (32 / 26, 5).
 template <Kind KIND, typename OutT>
 int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitPlan* plan) {
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);
@@ -103,7 +103,7 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
     if (int rc = split_clusters<KIND, 128, 2, 5, OutT, 1, false>(splits, &clusters)) return rc;
     if (clusters >= tiles) break;
   }
-  plan->through_workspace = have_workspace && ceil_div(k_stages, splits) - ceil_div(k_stages, most) > most;
+  plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
   plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
   plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage
   return CK_OK;
@@ -158,8 +158,7 @@ int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, void* 
   const GemmParams result = p;
   p.splits = plan.splits;
   p.k_stages_per_split = plan.k_stages;
-  if (!plan.through_workspace) return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1>(ops, p, os, stream);
-  p.split_outputs = 1;
+  if (!plan.through_workspace) return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1, false, Split::kCluster>(ops, p, os, stream);
   p.tsa = p.tsb = p.alpha = nullptr;
   p.bias = nullptr;
   p.out = workspace;
@@ -171,7 +170,7 @@ int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, void* 
   partials.n = plan.splits;
   partials.pitch = p.N;
   partials.col_offset = 0;
-  if (int rc = launch_config<KIND, 128, 2, 5, 1, float, false, 1>(ops, p, partials, stream)) return rc;
+  if (int rc = launch_config<KIND, 128, 2, 5, 1, float, false, 1, false, Split::kOutputs>(ops, p, partials, stream)) return rc;
   CK_CUDA(launch_pdl(splitk_reduce_kernel<OutT>, dim3(static_cast<unsigned>(ceil_div(mn / 4, 256))), dim3(256), 0, stream,
                      static_cast<const float*>(workspace), plan.splits, mn, p.N, result.alpha, result.tsa, result.tsb, result.bias,
                      result.bias_dtype, static_cast<OutT*>(result.out)));
@@ -368,7 +367,7 @@ extern "C" int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int6
   }
   SplitPlan plan = {};
   const int rc = small_m_applies(M, N, K)
-                     ? small_m_splits(is_mxfp8 != 0, out_dtype, M, N, static_cast<int>(is_mxfp8 ? K : K / 2), &plan.splits)
+                     ? small_m_splits(is_mxfp8 != 0, out_dtype, N, static_cast<int>(is_mxfp8 ? K : K / 2), &plan.splits)
                      : tile_plan(is_mxfp8 != 0, out_dtype, M, N, K, with_workspace != 0, &plan);
   return rc == CK_OK ? plan.splits : -rc;
 }

@@ -121,6 +121,15 @@ struct Config {
 
 constexpr int kMaxSplits = 8;       // CTAs of a split-K cluster (the portable cluster size)
 
+// Whether and how a tile's K range is split over CTAs.  A kernel of its own for each: code for a split costs the
+// calls that do not split 0.1 to 0.6 us (registers, and the tile's index by a division).
+enum class Split {
+  kNone,
+  kCluster,          // the cluster's CTAs add their partial tiles through distributed shared memory
+  kClusterManyRows,  // the same with swapped operands and more activation rows than a warp each would do for
+  kOutputs           // CTA s stores its raw fp32 partial tile to destination s
+};
+
 struct GemmParams {
   const uint8_t* sfa;      // A scales, tiled layout, [ceil(M/128)][sf_col_tiles] tiles of 512 bytes
   const uint8_t* sfb;      // B scales, same layout over N
@@ -140,9 +149,8 @@ struct GemmParams {
   int raster;              // order in which workers walk the tiles: 0 = down the rows first, 1 = along the columns first
   int out_tma;             // the output qualifies for TMA stores (16-byte aligned base and pitch)
   int n_out;               // destinations of every output tile (1, or one per GPU of an all-gather)
-  int splits;              // split-K: CTAs per tile (1 = off), one thread-block cluster; CTA s of it covers pipeline stages
-  int k_stages_per_split;  //   [s * k_stages_per_split, ...) and the cluster adds the raw fp32 partial tiles in its shared memory,
-  int split_outputs;       //   or, set, no cluster: CTA s stores its raw fp32 partial tile to destination s
+  int splits;              // split-K: CTAs per tile (1 = off); CTA s of a tile covers pipeline stages
+  int k_stages_per_split;  //   [s * k_stages_per_split, ...)
   int* status;             // device status word: set non-zero when a wait gave up
   int trace_launch;        // sequence number of the launch (timeline builds only)
   // fused epilogue (FUSED kernels only)
@@ -372,6 +380,13 @@ __device__ __forceinline__ void store_four(OutT* dst, const float (&y)[4]) {
   }
 }
 
+__device__ __forceinline__ void sums_scaled(float4 acc, float alpha, const float (&bias)[4], float (&y)[4]) {
+  y[0] = fmaf(acc.x, alpha, bias[0]);
+  y[1] = fmaf(acc.y, alpha, bias[1]);
+  y[2] = fmaf(acc.z, alpha, bias[2]);
+  y[3] = fmaf(acc.w, alpha, bias[3]);
+}
+
 // Four values at `offset` of every CTA's partial tile, added in split order (all loads before the first add).
 __device__ __forceinline__ float4 add_partials(const uint32_t (&base)[kMaxSplits], int splits, uint32_t offset) {
   float4 v[kMaxSplits];
@@ -400,11 +415,8 @@ __device__ __forceinline__ float4 add_partials(const uint32_t (&base)[kMaxSplits
 // with few activation rows fills the 128-row MMA dimension with weight rows and streams the weight
 // once.  p.M / p.N are then the weight's and the activation's row counts, the output is written
 // transposed (out[b_row][a_row]) and the bias runs along the A rows.
-//
-// MANY_ROWS (SWAP only): how the cluster's CTAs share the sums of a split tile.  A kernel of its own for each:
-// with both in one, the calls of few activation rows take 0.1 to 0.2 us longer.
 template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE, bool SWAP = false,
-          bool MANY_ROWS = false>
+          Split SPLIT = Split::kNone>
 __global__ void __launch_bounds__(num_threads(FUSED, TILE_N), (SWAP && TILE_N <= 128) ? 2 : 1)
 block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
@@ -415,11 +427,11 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   constexpr int kNumEpilogueWarps = epilogue_warps(FUSED, TILE_N);
   constexpr int kThreads = num_threads(FUSED, TILE_N);
   static_assert(TILE_N <= 32 * kNumEpilogueWarps, "one bias value per epilogue thread");
-  // configurations whose tiles may be split along K over the CTAs of a cluster
-  constexpr bool kCanSplit = CTAS == 1 && !FUSED && (SWAP || TILE_N == 128);
-  static_assert(!kCanSplit || kTileM * TILE_N * 4 <= Cfg::kRingBytes, "a partial tile fits in the operand ring");
-  // and the one whose CTAs may instead store their partial tiles each to a destination of its own
-  constexpr bool kCanSplitOutputs = kCanSplit && !SWAP && std::is_same<OutT, float>::value;
+  constexpr bool kCluster = SPLIT == Split::kCluster || SPLIT == Split::kClusterManyRows;
+  static_assert(SPLIT == Split::kNone || (CTAS == 1 && !FUSED), "only plain one-CTA tiles are split");
+  static_assert(SPLIT != Split::kClusterManyRows || SWAP, "rows of swapped operands");
+  static_assert(SPLIT != Split::kOutputs || (!SWAP && OUT_STAGE != 0 && std::is_same<OutT, float>::value), "raw partial tiles, staged");
+  static_assert(!kCluster || kTileM * TILE_N * 4 <= Cfg::kRingBytes, "a partial tile fits in the operand ring");
   // Everything the kernel does until a role's griddepcontrol.wait is independent of the kernel
   // before it in the stream, so the next kernel may be scheduled as early as resources allow.
   pdl_launch_dependents();
@@ -459,7 +471,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // wait itself (1-3 % of these 6-10 us kernels).  The tile configurations are slower with it
   // (config 2: 18.7 vs 18.5 us; the requests share the TMA unit with the first loads).
   if (SWAP && warp == 0 && elect_one()) {
-    const int pf_splits = p.splits;
+    const int pf_splits = SPLIT == Split::kNone ? 1 : p.splits;
     const int pf_k_stages = (p.k_bytes + kStageKBytes - 1) / kStageKBytes;
     if (worker < p.tiles_m * p.tiles_n * pf_splits) {
       const int tile0 = worker / pf_splits;
@@ -525,7 +537,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   CK_TRACE3(1);
 
   const int num_tiles = p.tiles_m * p.tiles_n;
-  const int splits = p.splits;
+  const int splits = SPLIT == Split::kNone ? 1 : p.splits;
+  // kCluster: what the exchange at the end will scale by and add; the epilogue warps fetch it ahead of their waits
+  [[maybe_unused]] float split_alpha = 1.0f;
+  [[maybe_unused]] float split_bias[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   const int num_items = num_tiles * splits;
   const int k_stages = (p.k_bytes + kStageKBytes - 1) / kStageKBytes;
   const int total_mma = (p.k_bytes + kMmaKBytes - 1) / kMmaKBytes;
@@ -733,6 +748,26 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     } else if (p.tsa != nullptr && p.tsb != nullptr) {
       alpha = ld_f32_dependent(p.tsa) * ld_f32_dependent(p.tsb);
     }
+    if constexpr (kCluster) {
+      split_alpha = alpha;
+      if (p.bias != nullptr) {
+        const int tile = worker / splits;
+        if constexpr (SWAP) {
+          const int first = SPLIT == Split::kClusterManyRows ? lane * 4 : ((static_cast<int>(cluster_cta_rank()) + splits * (warp - 2)) & 3) * 32 + lane;
+          const int a_row = tile_row_block(p, tile) * kTileM + first;
+#pragma unroll
+          for (int j = 0; j < (SPLIT == Split::kClusterManyRows ? 4 : 1); ++j) {
+            if (a_row + j < p.M) split_bias[j] = load_bias(p.bias, p.bias_dtype, a_row + j);
+          }
+        } else {
+          const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (col + j < p.N) split_bias[j] = load_bias(p.bias, p.bias_dtype, col + j);
+          }
+        }
+      }
+    }
     OutT* out = static_cast<OutT*>(p.out);
     const bool vec_ok = (static_cast<int64_t>(p.N) * sizeof(OutT)) % 32 == 0 &&
                         (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0 && (TILE_N * sizeof(OutT)) % 32 == 0;
@@ -767,7 +802,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
         if (warp == 2) CK_TRACE(8);
-        if (splits > 1) {
+        if constexpr (kCluster) {
           // Raw partial to the CTA's own shared memory, [column][128 rows]; added below by the cluster.
           float* part = reinterpret_cast<float*>(smem) + r_in_tile;
 #pragma unroll
@@ -859,22 +894,20 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           mbar_arrive(&acc_empty_bar[acc]);
         }
       }
-      if constexpr (kCanSplit) {
-        if (splits > 1 && !(kCanSplitOutputs && p.split_outputs)) {
-          // Raw partial to the CTA's own shared memory: row r at r * TILE_N * 4 bytes, its 16-byte unit u
-          // at position u ^ (r % 8) (the eight rows of a store phase meet eight different bank groups).
-          const int r = quarter * 32 + lane;
-          const uint32_t part_row = smem_u32(smem) + r * (TILE_N * 4);
+      if constexpr (kCluster) {
+        // Raw partial to the CTA's own shared memory: row r at r * TILE_N * 4 bytes, its 16-byte unit u
+        // at position u ^ (r % 8) (the eight rows of a store phase meet eight different bank groups).
+        const int r = quarter * 32 + lane;
+        const uint32_t part_row = smem_u32(smem) + r * (TILE_N * 4);
 #pragma unroll
-          for (int c = 0; c < kChunks; ++c) {
+        for (int c = 0; c < kChunks; ++c) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int u = (c0 + c * 32) / 4 + j;
-              st_shared_128(part_row + ((u ^ (r & 7)) << 4), buf[c][4 * j], buf[c][4 * j + 1], buf[c][4 * j + 2], buf[c][4 * j + 3]);
-            }
+          for (int j = 0; j < 8; ++j) {
+            const int u = (c0 + c * 32) / 4 + j;
+            st_shared_128(part_row + ((u ^ (r & 7)) << 4), buf[c][4 * j], buf[c][4 * j + 1], buf[c][4 * j + 2], buf[c][4 * j + 3]);
           }
-          continue;
         }
+        continue;
       }
       if (has_next) {
         if (et < TILE_N) smem_bias[((tile_it + 1) % 3) * TILE_N + et] = bias_prefetched;
@@ -944,7 +977,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 __syncwarp();
                 const int col = n0 + c0 + (c / kChunksPerBox) * kBoxCols;
                 if (lane == 0 && row0 < p.M && col < p.N) {
-                  if (kCanSplitOutputs && p.split_outputs) {
+                  if constexpr (SPLIT == Split::kOutputs) {
                     tma_store_2d_addr(&maps_out.m[item - tile * splits], stage_box, col, row0);  // this item's partial
                   } else {
                     // the same staged box goes to every destination (peer stores cross NVLink)
@@ -1106,91 +1139,75 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // NVFP4 1 x 1024 x 15360 GEMM 8.7 -> 6.3, linear 21.8 -> 8.1; 64 x 3072 x 12288 11.3 -> 9.6.  A cluster
   // must find its SMs in one part of the chip: where that costs too many CTAs per tile, the GEMMs that have
   // a workspace go through it (choose_splits in ck_gemm.cu).
-  if constexpr (kCanSplit) {
-    if (splits > 1 && !(kCanSplitOutputs && p.split_outputs)) {
-      __syncwarp();
-      cluster_sync_all();
-      if (warp >= 2) {
-        const int rank = static_cast<int>(cluster_cta_rank());
-        const int tile = worker / splits;
-        const uint32_t part = smem_u32(smem);
-        float alpha = 1.0f;
-        if (p.alpha != nullptr) {
-          alpha = ld_f32_dependent(p.alpha);
-        } else if (p.tsa != nullptr && p.tsb != nullptr) {
-          alpha = ld_f32_dependent(p.tsa) * ld_f32_dependent(p.tsb);
-        }
-        uint32_t base[kMaxSplits];
+  if constexpr (kCluster) {
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 2) {
+      const int rank = static_cast<int>(cluster_cta_rank());
+      const int tile = worker / splits;
+      const uint32_t part = smem_u32(smem);
+      uint32_t base[kMaxSplits];
 #pragma unroll
-        for (int i = 0; i < kMaxSplits; ++i) base[i] = map_to_cta(part, i < splits ? i : 0);
-        if constexpr (SWAP) {
-          OutT* out = static_cast<OutT*>(p.out);
-          const int a_row0 = tile_row_block(p, tile) * kTileM;
-          if constexpr (!MANY_ROWS) {
-            // a warp takes 32 of the weight rows (a coalesced run of the output) of one of them
-            for (int u = rank + splits * (warp - 2); u < 4 * p.N; u += splits * kNumEpilogueWarps) {
-              const int col = u >> 2;
-              const int r = (u & 3) * 32 + lane;
-              const int a_row = a_row0 + r;
-              const float bias_v = (p.bias != nullptr && a_row < p.M) ? load_bias(p.bias, p.bias_dtype, a_row) : 0.0f;
-              float v[kMaxSplits];
+      for (int i = 0; i < kMaxSplits; ++i) base[i] = map_to_cta(part, i < splits ? i : 0);
+      if constexpr (SWAP) {
+        OutT* out = static_cast<OutT*>(p.out);
+        const int a_row0 = tile_row_block(p, tile) * kTileM;
+        if constexpr (SPLIT == Split::kCluster) {
+          // a warp takes 32 of the weight rows (a coalesced run of the output) of one activation row; the host sees
+          // to it that there are warps enough
+          const int u = rank + splits * (warp - 2);
+          const int col = u >> 2;
+          const int r = (u & 3) * 32 + lane;
+          if (col < p.N) {
+            float v[kMaxSplits];
 #pragma unroll
-              for (int i = 0; i < kMaxSplits; ++i) {
-                if (i < splits) v[i] = ld_shared_cluster_f32(base[i] + (col * kTileM + r) * 4);
-              }
-              float acc = v[0];
-#pragma unroll
-              for (int i = 1; i < kMaxSplits; ++i) {
-                if (i < splits) acc += v[i];
-              }
-              if (a_row < p.M) out[static_cast<int64_t>(col) * p.M + a_row] = to_out<OutT>(fmaf(acc, alpha, bias_v));
+            for (int i = 0; i < kMaxSplits; ++i) {
+              if (i < splits) v[i] = ld_shared_cluster_f32(base[i] + (col * kTileM + r) * 4);
             }
-          } else {
-            // a warp takes all 128 weight rows of one activation row, a lane four of them: up to 32 activation rows in
-            // one to three rounds (NVFP4 32 x 1024 x 4096: 5.8 us, against 7.1 with 32 weight rows at a time)
-            const int a_row = a_row0 + lane * 4;
-            const bool in_rows = a_row < p.M;  // the output's row length is a multiple of 8: all four or none
-            const bool vec = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(OutT) - 1)) == 0;
-            float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (p.bias != nullptr && in_rows) {
+            float acc = v[0];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) b[j] = load_bias(p.bias, p.bias_dtype, a_row + j);
+            for (int i = 1; i < kMaxSplits; ++i) {
+              if (i < splits) acc += v[i];
             }
-            for (int col = rank + splits * (warp - 2); col < p.N; col += splits * kNumEpilogueWarps) {
-              const float4 acc = add_partials(base, splits, (col * kTileM + lane * 4) * 4);
-              if (in_rows) {
-                const float y[4] = {fmaf(acc.x, alpha, b[0]), fmaf(acc.y, alpha, b[1]), fmaf(acc.z, alpha, b[2]), fmaf(acc.w, alpha, b[3])};
-                OutT* dst = out + static_cast<int64_t>(col) * p.M + a_row;
-                if (vec) {
-                  store_four(dst, y);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) dst[j] = to_out<OutT>(y[j]);
-                }
-              }
-            }
+            if (a_row0 + r < p.M) out[static_cast<int64_t>(col) * p.M + a_row0 + r] = to_out<OutT>(fmaf(acc, split_alpha, split_bias[0]));
           }
         } else {
-          // a warp takes one row of the tile, a lane four neighbouring columns
-          const int row0 = tile_row_block(p, tile) * kTileM;
-          const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
-          const bool in_cols = col < p.N;  // N % 8 == 0: a group of four never straddles the edge
-          float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-          if (p.bias != nullptr && in_cols) {
+          // a warp takes all 128 weight rows of one activation row, a lane four of them: up to 32 activation rows in
+          // one to three rounds (NVFP4 32 x 1024 x 4096: 5.8 us, against 7.1 with 32 weight rows at a time)
+          const int a_row = a_row0 + lane * 4;
+          const bool in_rows = a_row < p.M;  // the output's row length is a multiple of 8: all four or none
+          const bool vec = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(OutT) - 1)) == 0;
+          for (int col = rank + splits * (warp - 2); col < p.N; col += splits * kNumEpilogueWarps) {
+            const float4 acc = add_partials(base, splits, (col * kTileM + lane * 4) * 4);
+            if (in_rows) {
+              float y[4];
+              sums_scaled(acc, split_alpha, split_bias, y);
+              OutT* dst = out + static_cast<int64_t>(col) * p.M + a_row;
+              if (vec) {
+                store_four(dst, y);
+              } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = load_bias(p.bias, p.bias_dtype, col + j);
-          }
-          const int rows = min(kTileM, p.M - row0);
-          for (int r = rank + splits * (warp - 2); r < rows; r += splits * kNumEpilogueWarps) {
-            const float4 acc = add_partials(base, splits, r * (TILE_N * 4) + ((lane ^ (r & 7)) << 4));
-            const float y[4] = {fmaf(acc.x, alpha, b[0]), fmaf(acc.y, alpha, b[1]), fmaf(acc.z, alpha, b[2]), fmaf(acc.w, alpha, b[3])};
-            if (in_cols) store_four(static_cast<OutT*>(p.out) + static_cast<int64_t>(row0 + r) * p.N + col, y);
+                for (int j = 0; j < 4; ++j) dst[j] = to_out<OutT>(y[j]);
+              }
+            }
           }
         }
+      } else {
+        // a warp takes one row of the tile, a lane four neighbouring columns
+        const int row0 = tile_row_block(p, tile) * kTileM;
+        const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
+        const bool in_cols = col < p.N;  // N % 8 == 0: a group of four never straddles the edge
+        const int rows = min(kTileM, p.M - row0);
+        for (int r = rank + splits * (warp - 2); r < rows; r += splits * kNumEpilogueWarps) {
+          const float4 acc = add_partials(base, splits, r * (TILE_N * 4) + ((lane ^ (r & 7)) << 4));
+          float y[4];
+          sums_scaled(acc, split_alpha, split_bias, y);
+          if (in_cols) store_four(static_cast<OutT*>(p.out) + static_cast<int64_t>(row0 + r) * p.N + col, y);
+        }
       }
-      __syncwarp();
-      cluster_sync_all();  // no CTA leaves while another may still read its partial
     }
+    __syncwarp();
+    cluster_sync_all();  // no CTA leaves while another may still read its partial
   }
 
   // ------------------------------------------------------------------ teardown
@@ -1359,7 +1376,7 @@ int split_clusters(int splits, int* out) {
   CK_CUDA(cudaGetDevice(&dev));
   int n = (dev >= 0 && dev < 64) ? cached[dev][splits].load(std::memory_order_relaxed) : 0;
   if (n == 0) {
-    auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, 1, OutT, false, OUT_STAGE, SWAP>;
+    auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, 1, OutT, false, OUT_STAGE, SWAP, Split::kCluster>;
     CK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(num_threads(false, TILE_N));
@@ -1381,10 +1398,10 @@ int split_clusters(int splits, int* out) {
 }
 
 template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE = 0, bool SWAP = false,
-          bool MANY_ROWS = false>
+          Split SPLIT = Split::kNone>
 int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaStream_t stream) {
   using Cfg = Config<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OUT_STAGE>;
-  auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OutT, FUSED, OUT_STAGE, SWAP, MANY_ROWS>;
+  auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OutT, FUSED, OUT_STAGE, SWAP, SPLIT>;
   // only the tensor maps this configuration uses are encoded (host time is visible for small problems)
   CUtensorMap map_a, map_b;
   if (int rc = make_operand_map(&map_a, ops.a, p.M, p.k_bytes, kTileM)) return rc;
@@ -1405,7 +1422,7 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  const bool cluster_split = CTAS == 1 && p.splits > 1 && p.split_outputs == 0;
+  constexpr bool cluster_split = SPLIT == Split::kCluster || SPLIT == Split::kClusterManyRows;
   attr[0].val.clusterDim.x = cluster_split ? p.splits : CTAS;  // split-K: the CTAs of one tile are a cluster
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;

@@ -18,17 +18,17 @@ constexpr int kMaxSmallM = 32;
 constexpr int kSmallTileN = 32;  // the MMA's N: activation rows, padded
 
 // CTAs per tile (1 = no split).  The most whose clusters all run at once with one CTA on an SM; with two on an SM
-// when that leaves a CTA more than ten stages, or sixteen with up to four activation rows, whose exchange is
-// short.  (The occupancy query counts one for every kernel that allocates tensor memory; two of this
-// configuration share an SM.  A cluster that finds no room runs later: nobody waits for it.)  Measured, us, few
-// CTAs of many stages / twice as many: NVFP4 32 x 4096 x 12288 (12 stages) 9.11 / 8.60, MXFP8 32 x 6144 x 12288 (48)
-// 19.0 / 12.5, 1 x 4096 x 12288 (24) 11.6 / 10.2; but NVFP4 1 x 4096 x 8192 (8) 7.2 / 7.9, 1 x 6144 x 6144 (12) 7.8 / 8.4.
+// when that leaves a CTA more than ten stages.  (The occupancy query counts one for every kernel that allocates
+// tensor memory; two of this configuration share an SM.  A cluster that finds no room runs later: nobody waits for
+// it.)  Graph replays, us, few CTAs of many stages / more: NVFP4 32 x 4096 x 12288 (12 stages / 8) 8.9 / 8.0,
+// 1 x 6144 x 8192 (16 / 7) 8.9 / 8.1, 1 x 6144 x 6144 (12 / 5) 7.6 / 7.6, MXFP8 32 x 6144 x 12288 (48 / 20) 18.3 / 11.7,
+// 1 x 4096 x 12288 (24 / 16) 10.9 / 9.6; but NVFP4 1 x 4096 x 8192 (8 / 6) 6.6 / 7.1, 1 x 6144 x 4096 (8 / 4) 6.2 / 6.4.
 template <Kind KIND, typename OutT>
-int choose_splits(int64_t M, int64_t N, int k_bytes, int* out) {
+int choose_splits(int64_t N, int k_bytes, int* out) {
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
   const int64_t tiles = ceil_div(N, kTileM);
   const int most = small_m_max_splits(N, k_bytes);
-  const int max_stages_alone = M <= 4 ? 16 : 10;
+  constexpr int kMaxStagesAlone = 10;
   int splits = 1;
   for (int per_sm = 1; per_sm <= 2; ++per_sm) {
     for (splits = most; splits > 1; --splits) {
@@ -36,7 +36,7 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, int* out) {
       if (int rc = split_clusters<KIND, kSmallTileN, 2, 4, OutT, 0, true>(splits, &clusters)) return rc;
       if (clusters * per_sm >= tiles) break;
     }
-    if (ceil_div(k_stages, splits) <= max_stages_alone) break;
+    if (ceil_div(k_stages, splits) <= kMaxStagesAlone) break;
   }
   *out = static_cast<int>(ceil_div(k_stages, ceil_div(k_stages, splits)));  // none without a stage
   return CK_OK;
@@ -50,13 +50,14 @@ int launch_small(const Operands& ops, GemmParams p, cudaStream_t stream) {
   os.n = 1;
   os.pitch = p.N;
   os.col_offset = 0;
-  if (int rc = choose_splits<KIND, OutT>(p.N, p.M, p.k_bytes, &p.splits)) return rc;
+  if (int rc = choose_splits<KIND, OutT>(p.M, p.k_bytes, &p.splits)) return rc;
   p.k_stages_per_split = static_cast<int>(ceil_div(ceil_div(p.k_bytes, kStageKBytes), p.splits));
+  if (p.splits == 1) return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true>(ops, p, os, stream);
   // a quarter tile of one activation row per warp of the cluster, if there are warps enough for all of them
   if (4 * p.N <= p.splits * epilogue_warps(false, kSmallTileN)) {
-    return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true>(ops, p, os, stream);
+    return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true, Split::kCluster>(ops, p, os, stream);
   }
-  return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true, true>(ops, p, os, stream);
+  return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true, Split::kClusterManyRows>(ops, p, os, stream);
 }
 
 }  // namespace
@@ -75,18 +76,18 @@ int small_m_max_splits(int64_t N, int k_bytes) {
   return max(splits, 1);
 }
 
-int small_m_splits(bool is_mxfp8, int out_dtype, int64_t M, int64_t N, int k_bytes, int* splits) {
+int small_m_splits(bool is_mxfp8, int out_dtype, int64_t N, int k_bytes, int* splits) {
   if (is_mxfp8) {
     switch (out_dtype) {
-      case CK_DTYPE_BF16: return choose_splits<Kind::kMxfp8, __nv_bfloat16>(M, N, k_bytes, splits);
-      case CK_DTYPE_F16: return choose_splits<Kind::kMxfp8, __half>(M, N, k_bytes, splits);
-      default: return choose_splits<Kind::kMxfp8, float>(M, N, k_bytes, splits);
+      case CK_DTYPE_BF16: return choose_splits<Kind::kMxfp8, __nv_bfloat16>(N, k_bytes, splits);
+      case CK_DTYPE_F16: return choose_splits<Kind::kMxfp8, __half>(N, k_bytes, splits);
+      default: return choose_splits<Kind::kMxfp8, float>(N, k_bytes, splits);
     }
   }
   switch (out_dtype) {
-    case CK_DTYPE_BF16: return choose_splits<Kind::kNvfp4, __nv_bfloat16>(M, N, k_bytes, splits);
-    case CK_DTYPE_F16: return choose_splits<Kind::kNvfp4, __half>(M, N, k_bytes, splits);
-    default: return choose_splits<Kind::kNvfp4, float>(M, N, k_bytes, splits);
+    case CK_DTYPE_BF16: return choose_splits<Kind::kNvfp4, __nv_bfloat16>(N, k_bytes, splits);
+    case CK_DTYPE_F16: return choose_splits<Kind::kNvfp4, __half>(N, k_bytes, splits);
+    default: return choose_splits<Kind::kNvfp4, float>(N, k_bytes, splits);
   }
 }
 
