@@ -12,6 +12,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+import threading
 
 import torch
 
@@ -135,6 +136,9 @@ def _stream(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", lambda: False)  # absent from builds without CUDA
+
+
 class _NoSwitch:
     def __enter__(self):
         return None
@@ -152,7 +156,7 @@ def _on_device(device):
     if type(device) is not torch.device:
         device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device)
     index = device.index
-    if index is None or index == torch.cuda.current_device():
+    if index is None or (torch._C._cuda_getDevice() if torch.cuda.is_initialized() else torch.cuda.current_device()) == index:
         return _NO_SWITCH
     return torch.cuda.device(device)
 
@@ -194,8 +198,8 @@ def quantize_nvfp4(x: torch.Tensor, per_tensor_scale: torch.Tensor, epsilon: flo
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
     sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)
     with _on_device(x.device):
-        _check(lib.ck_quantize_nvfp4(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(scale), _ptr(qx), _ptr(sx), rows, cols,
-                                     out_rows, out_cols, int(bool(hi_first)), _stream(x.device)), "quantize_nvfp4")
+        _check(lib.ck_quantize_nvfp4(x.data_ptr(), DTYPE_TO_CODE[x.dtype], scale.data_ptr(), qx.data_ptr(), sx.data_ptr(), rows,
+                                     cols, out_rows, out_cols, int(bool(hi_first)), _stream(x.device)), "quantize_nvfp4")
     return qx, sx
 
 
@@ -213,7 +217,7 @@ def quantize_mxfp8(x: torch.Tensor, pad_32x: bool = False) -> tuple[torch.Tensor
     qx = torch.empty((out_rows, out_cols), device=x.device, dtype=torch.float8_e4m3fn)
     sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 32, 4)), device=x.device, dtype=torch.float8_e8m0fnu)
     with _on_device(x.device):
-        _check(lib.ck_quantize_mxfp8(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(qx), _ptr(sx), rows, cols, out_rows,
+        _check(lib.ck_quantize_mxfp8(x.data_ptr(), DTYPE_TO_CODE[x.dtype], qx.data_ptr(), sx.data_ptr(), rows, cols, out_rows,
                                      out_cols, _stream(x.device)), "quantize_mxfp8")
     return qx, sx
 
@@ -260,11 +264,27 @@ _ON_CHIP = 256  # the workspace size of a GEMM that does not use one (ck_scaled_
 _WHOLE_INPUT_BYTES = 64 << 10  # inputs up to here take no reduction kernel (ck_quantize_nvfp4_dynamic)
 
 
-def _call_workspace(need: int, device) -> torch.Tensor:
-    """Device memory of this one call, from the caching allocator's pool of the current stream: the next
-    allocation that gets the same block is ordered behind this call's kernels, and a captured call's block
-    belongs to its graph.  (Never empty: the library reports an unsupported shape itself.)"""
-    return torch.empty(max(need, 1), dtype=torch.uint8, device=device)
+_workspaces = threading.local()
+
+
+def _workspace_for(need: int, device, stream: int) -> torch.Tensor:
+    """Device memory for what passes from one launch of a call to the next, at least ``need`` bytes (never
+    none: the library reports an unsupported shape itself).  Kept per thread, device and stream, so that
+    threads whose launches interleave on one stream do not share it, and freed with the thread; a captured
+    call has its own, which belongs to its graph.  An outgrown one goes back to the caching allocator's pool
+    of its stream, behind the kernels that use it."""
+    if _capturing():
+        return torch.empty(max(need, 1), dtype=torch.uint8, device=device)
+    try:
+        ws = _workspaces.of[device.index, stream]
+        if ws.numel() >= need:
+            return ws
+    except KeyError:
+        pass
+    except AttributeError:  # this thread's first
+        _workspaces.of = {}
+    ws = _workspaces.of[device.index, stream] = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
+    return ws
 
 
 def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
@@ -290,15 +310,13 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     if rows * cols * x.element_size() <= _WHOLE_INPUT_BYTES:
         scratch = _scale_scratch_for(x.device, stream, need)  # nothing is kept in it between two launches
     else:
-        # The partial maxima go from one launch to the next: a buffer that another thread of this stream (or
-        # another graph captured on it) also uses could be written by its reduction in between.
-        scratch = _call_workspace(need, x.device)
+        scratch = _workspace_for(need, x.device, stream)  # the partial maxima go from one launch to the next
     scale = torch.empty((), dtype=torch.float32, device=x.device)
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
     sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)
     with _on_device(x.device):
-        _check(lib.ck_quantize_nvfp4_dynamic(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(scale), _ptr(qx), _ptr(sx), rows, cols, out_rows,
-                                             out_cols, int(bool(hi_first)), _ptr(scratch), scratch.numel(), stream),
+        _check(lib.ck_quantize_nvfp4_dynamic(x.data_ptr(), DTYPE_TO_CODE[x.dtype], scale.data_ptr(), qx.data_ptr(), sx.data_ptr(),
+                                             rows, cols, out_rows, out_cols, int(bool(hi_first)), scratch.data_ptr(), scratch.numel(), stream),
                "quantize_nvfp4_dynamic")
     return qx, sx, scale
 
@@ -316,7 +334,8 @@ def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_sca
     scale = _scalar_f32(per_tensor_scale, qx.device, "per_tensor_scale")
     out = torch.empty((rows, cols), device=qx.device, dtype=output_type)
     with _on_device(qx.device):
-        _check(lib.ck_dequantize_nvfp4(_ptr(qx), _ptr(scale), _ptr(block_scales), _ptr(out), DTYPE_TO_CODE[output_type],
+        _check(lib.ck_dequantize_nvfp4(qx.data_ptr(), scale.data_ptr(), block_scales.data_ptr(), out.data_ptr(),
+                                       DTYPE_TO_CODE[output_type],
                                        rows, cols, int(bool(hi_first)), _stream(qx.device)), "dequantize_nvfp4")
     return out
 
@@ -332,7 +351,7 @@ def dequantize_mxfp8(qx: torch.Tensor, block_scales: torch.Tensor,
     assert block_scales.shape == (roundup(rows, 128), roundup(cols // 32, 4)), "Invalid scale shape"
     out = torch.empty((rows, cols), device=qx.device, dtype=output_type)
     with _on_device(qx.device):
-        _check(lib.ck_dequantize_mxfp8(_ptr(qx), _ptr(block_scales), _ptr(out), DTYPE_TO_CODE[output_type], rows, cols,
+        _check(lib.ck_dequantize_mxfp8(qx.data_ptr(), block_scales.data_ptr(), out.data_ptr(), DTYPE_TO_CODE[output_type], rows, cols,
                                        _stream(qx.device)), "dequantize_mxfp8")
     return out
 
@@ -382,11 +401,12 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
+        stream = _stream(dev)
         need = _workspace_bytes("ck_scaled_mm_workspace_bytes", 0, m, n, k)
-        ws = _call_workspace(need, dev) if need > _ON_CHIP else None
-        _check(lib.ck_scaled_mm_nvfp4_ws(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), _ptr(tsa), _ptr(tsb),
-                                         _ptr(alpha_t), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
-                                         _ptr(ws), need, _stream(dev)), "scaled_mm_nvfp4")
+        ws = _workspace_for(need, dev, stream) if need > _ON_CHIP else None
+        _check(lib.ck_scaled_mm_nvfp4_ws(a.data_ptr(), b.data_ptr(), block_scale_a.data_ptr(), block_scale_b.data_ptr(),
+                                         tsa.data_ptr(), tsb.data_ptr(), _ptr(alpha_t), bias_ptr, bias_code, out.data_ptr(), DTYPE_TO_CODE[out_dtype], m, n, k,
+                                         _ptr(ws), need, stream), "scaled_mm_nvfp4")
     del bias_keep
     return out
 
@@ -494,9 +514,8 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
 
     ``x`` [M, K] float; ``w_codes`` uint8 [N, K/2] with its tiled E4M3 ``w_block_scales`` and fp32
     ``w_scale``; ``x_scale`` a static per-tensor scale or None for ``amax(|x|)/2688``.  Same bits
-    as ``quantize_nvfp4`` followed by ``scaled_mm_nvfp4``.  The quantized activation goes to a
-    workspace of this call: it passes from one launch to the next, and threads that share a stream
-    may interleave their launches."""
+    as ``quantize_nvfp4`` followed by ``scaled_mm_nvfp4``.  The quantized activation passes
+    from one launch to the next in a workspace (:func:`_workspace_for`)."""
     lib = load_library()
     x, w_codes, w_block_scales = _plain(x), _plain(w_codes), _plain(w_block_scales)
     assert x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor"
@@ -514,11 +533,11 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     if sx is None and need and x.data_ptr() % 32:
         sx = nvfp4_tensor_scale(x)  # as in quantize_nvfp4_dynamic
     stream = _stream(dev)
-    ws = _call_workspace(need, dev)
+    ws = _workspace_for(need, dev, stream)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        _check(lib.ck_linear_nvfp4_from_float(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(sx), _ptr(w_codes), _ptr(w_block_scales),
-                                              _ptr(sw), bias_ptr, bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k,
+        _check(lib.ck_linear_nvfp4_from_float(x.data_ptr(), DTYPE_TO_CODE[x.dtype], _ptr(sx), w_codes.data_ptr(), w_block_scales.data_ptr(),
+                                              sw.data_ptr(), bias_ptr, bias_code, out.data_ptr(), DTYPE_TO_CODE[out_dtype], m, n, k,
                                               ws.data_ptr(), ws.numel(), stream), "linear_nvfp4_from_float")
     del bias_keep
     return out
@@ -528,8 +547,8 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
                             bias: torch.Tensor | None = None, out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """MXFP8 linear on a dense activation in one library call: quantize -> GEMM.  ``x`` [M, K] float;
     ``w_data`` float8_e4m3fn [N, K] with its tiled E8M0 ``w_block_scales``.  Same bits as
-    ``quantize_mxfp8`` followed by ``scaled_mm_mxfp8``; the quantized activation goes to a workspace
-    of this call, as in :func:`linear_nvfp4_from_float`."""
+    ``quantize_mxfp8`` followed by ``scaled_mm_mxfp8``; the quantized activation passes through a
+    workspace, as in :func:`linear_nvfp4_from_float`."""
     lib = load_library()
     x, w_data, w_block_scales = _plain(x), _plain(w_data), _plain(w_block_scales)
     assert x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor"
@@ -544,11 +563,11 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     need = _workspace_bytes("ck_linear_mxfp8_from_float_workspace_bytes", m, k)
     stream = _stream(dev)
-    ws = _call_workspace(need, dev)
+    ws = _workspace_for(need, dev, stream)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        _check(lib.ck_linear_mxfp8_from_float(_ptr(x), DTYPE_TO_CODE[x.dtype], _ptr(w_data), _ptr(w_block_scales), bias_ptr,
-                                              bias_code, _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, ws.data_ptr(),
+        _check(lib.ck_linear_mxfp8_from_float(x.data_ptr(), DTYPE_TO_CODE[x.dtype], w_data.data_ptr(), w_block_scales.data_ptr(), bias_ptr,
+                                              bias_code, out.data_ptr(), DTYPE_TO_CODE[out_dtype], m, n, k, ws.data_ptr(),
                                               ws.numel(), stream), "linear_mxfp8_from_float")
     del bias_keep
     return out
@@ -621,10 +640,11 @@ def scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tenso
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
+        stream = _stream(dev)
         need = _workspace_bytes("ck_scaled_mm_workspace_bytes", 1, m, n, k)
-        ws = _call_workspace(need, dev) if need > _ON_CHIP else None
-        _check(lib.ck_scaled_mm_mxfp8_ws(_ptr(a), _ptr(b), _ptr(block_scale_a), _ptr(block_scale_b), bias_ptr, bias_code,
-                                         _ptr(out), DTYPE_TO_CODE[out_dtype], m, n, k, _ptr(ws), need, _stream(dev)),
+        ws = _workspace_for(need, dev, stream) if need > _ON_CHIP else None
+        _check(lib.ck_scaled_mm_mxfp8_ws(a.data_ptr(), b.data_ptr(), block_scale_a.data_ptr(), block_scale_b.data_ptr(), bias_ptr, bias_code,
+                                         out.data_ptr(), DTYPE_TO_CODE[out_dtype], m, n, k, _ptr(ws), need, stream),
                "scaled_mm_mxfp8")
     del bias_keep
     return out

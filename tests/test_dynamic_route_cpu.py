@@ -27,6 +27,7 @@ def recorded(monkeypatch):
     monkeypatch.setattr(backend, "_lib", lib)
     monkeypatch.setattr(backend, "load_library", lambda: lib)
     monkeypatch.setattr(backend, "_stream", lambda device: 0)
+    monkeypatch.setattr(backend, "_capturing", lambda: False)
     monkeypatch.setattr(backend, "_on_device", lambda device: contextlib.nullcontext())
     monkeypatch.setattr(backend, "_scale_scratch", {})
     backend._workspace_bytes.cache_clear()

@@ -67,6 +67,7 @@ def test_threads_of_one_stream_keep_their_own_intermediates(entry, monkeypatch):
     monkeypatch.setattr(backend, "_lib", lib)
     monkeypatch.setattr(backend, "load_library", lambda: lib)
     monkeypatch.setattr(backend, "_stream", lambda device: 0)
+    monkeypatch.setattr(backend, "_capturing", lambda: False)
     monkeypatch.setattr(backend, "_on_device", lambda device: contextlib.nullcontext())
     backend._workspace_bytes.cache_clear()
     _call(backend, entry, torch.ones(128, 256))  # buffers that are kept from call to call exist now
