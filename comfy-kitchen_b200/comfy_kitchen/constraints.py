@@ -91,10 +91,17 @@ class ParamConstraint:
 
     def accepts(self, value, default_devices: frozenset[str]) -> bool:
         """All three checks (of a value that is not a tensor: its dtype alone)."""
-        if not self.check_dtype(value):
+        if not isinstance(value, torch.Tensor):
+            return self.dtypes is None or value in self.dtypes
+        if self.dtypes is not None and value.dtype not in self.dtypes:
             return False
-        return not isinstance(value, torch.Tensor) or (self.check_device(value, default_devices) and
-                                                       (not self.shape_rules or self.check_shape(value)))
+        allowed = default_devices if self.devices is None else self.devices
+        if not (value.is_cuda and "cuda" in allowed) and "*" not in allowed and value.device.type not in allowed:
+            return False
+        for rule in self.shape_rules:
+            if not rule.check(value):
+                return False
+        return True
 
 
 @dataclass(frozen=True)
@@ -147,7 +154,7 @@ def validate_function_call(constraints: FunctionConstraints, kwargs: Mapping, co
     if need is not None:
         if compute_capability is None:
             return ValidationResult.fail("__hardware__", "CUDA compute capability required but not available")
-        if tuple(compute_capability) < tuple(need):
+        if compute_capability != need and tuple(compute_capability) < tuple(need):
             return ValidationResult.fail(
                 "__hardware__",
                 f"compute capability {compute_capability[0]}.{compute_capability[1]} < required {need[0]}.{need[1]}")

@@ -25,6 +25,7 @@ DTYPE_TO_CODE = {v: k for k, v in DTYPE_CODE_TO_DTYPE.items()}
 
 
 _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+_MAY_BE_PENDING = (torch.float32, torch.bfloat16, torch.float16)  # parts of complex tensors, tangents: no codes or block scales
 
 
 def _impl(name: str, kwargs: dict):
@@ -73,7 +74,9 @@ def dispatcher_adds_nothing(tensors, optional=()) -> bool:
         return False
     grad = torch.is_grad_enabled()
     for t in tensors:
-        if type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad) or t.is_neg() or t._is_zerotensor():
+        if type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad):
+            return False
+        if t.dtype in _MAY_BE_PENDING and (t.is_neg() or t._is_zerotensor()):
             return False
     for t in optional:
         if t is not None and (type(t) not in _PLAIN_TYPES or not t.is_cuda or (grad and t.requires_grad) or t.is_neg() or

@@ -126,12 +126,13 @@ class BackendRegistry:
     def get_capable_backend(self, func_name: str, kwargs: Mapping[str, Any] | None = None) -> str:
         failures: dict[str, str] = {}
         override = getattr(self._tls, "override", None)
-        order = ([override] if override else []) + [n for n in self._priority if n != override]
+        order = [override] + [n for n in self._priority if n != override] if override else self._priority
         for name in order:
-            if name != override and name not in self._backends:
+            if name not in self._backends and name != override:
                 continue  # never-registered backends are not "failures", they just do not exist
             if self._try(name, func_name, kwargs, failures):
-                logger.debug("Backend %s selected for %s", name, func_name)
+                if logger.isEnabledFor(logging.DEBUG):
+                    logger.debug("Backend %s selected for %s", name, func_name)
                 return name
         for name, why in self._unavailable.items():
             failures.setdefault(name, why)
