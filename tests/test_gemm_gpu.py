@@ -210,9 +210,9 @@ def test_gemm_is_deterministic_and_row_independent(ck, cuda_device):
 
 @pytest.mark.parametrize("shape", [(16, 3072, 12288), (256, 3072, 12288), (1, 1024, 8192), (130, 640, 4096), (48, 136, 6144)])
 def test_split_k_for_small_m_long_k(ck, cuda_device, shape):
-    """Few output tiles and a long K: the public call computes split-K through its cached workspace
-    (the library reports a non-zero workspace size for these shapes) and still meets the GEMM
-    contract, deterministically."""
+    """Few output tiles and a long K, the forms whose K is split (the library reports a non-zero workspace size
+    for them; how many CTAs share a tile is asserted in test_split_choice_gpu): the public call meets the
+    GEMM contract, deterministically."""
     from comfy_kitchen.backends import cuda as backend
 
     m, n, k = shape

@@ -99,3 +99,35 @@ def test_workspace_and_clusters_agree(cuda_device, fmt, dtype):
     assert ((outs["full"].float() - ref).norm() / ref.norm()).item() <= bound
     status = ctypes.c_int(-1)
     assert lib.ck_gemm_status(ctypes.byref(status)) == 0 and status.value == 0
+
+
+# (rows, columns, stages) of every number of CTAs per tile, operands swapped (up to 32 rows) and not
+@pytest.mark.parametrize("m, n, stages, want", [
+    (9, 6144, 16, 2), (1, 5120, 16, 3), (32, 128, 16, 4), (3, 128, 20, 5), (31, 136, 24, 6), (1, 128, 28, 7), (17, 1024, 32, 8),
+    (40, 8192, 24, 2), (33, 128, 18, 3), (130, 264, 25, 4), (257, 128, 30, 5), (64, 520, 36, 6), (128, 128, 42, 7), (129, 384, 48, 8)])
+@pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
+def test_every_cluster_size(splits, cuda_device, monkeypatch, fmt, m, n, stages, want):
+    """Against the unsplit 128 x 128 tiles; the bound as in test_workspace_and_clusters_agree."""
+    from comfy_kitchen.backends import cuda as backend
+
+    mx = fmt == "mxfp8"
+    k = stages * (128 if mx else 256) - 32  # a short last stage
+    assert splits(mx, m, n, k, dtype=0) == want == splits(mx, m, n, k, dtype=0, workspace=1)
+    gen = torch.Generator(device=cuda_device).manual_seed(stages)
+    a, b = (torch.randn(r, k, generator=gen, device=cuda_device) for r in (m, n))
+    one, bias = torch.tensor(0.01, device=cuda_device), torch.linspace(-9, 9, n, device=cuda_device)
+    if mx:
+        (qa, sa), (qb, sb) = backend.quantize_mxfp8(a), backend.quantize_mxfp8(b)
+
+        def call():
+            return backend.scaled_mm_mxfp8(qa, qb, sa, sb, bias=bias, out_dtype=torch.float32)
+    else:
+        (qa, sa), (qb, sb) = backend.quantize_nvfp4(a, one), backend.quantize_nvfp4(b, one)
+
+        def call():
+            return backend.scaled_mm_nvfp4(qa, qb, one, one, sa, sb, bias=bias, out_dtype=torch.float32)
+    got = call()
+    monkeypatch.setenv("CK_GEMM_CONFIG", "1")
+    ref = call()
+    monkeypatch.delenv("CK_GEMM_CONFIG")
+    assert ((got - ref).norm() / ref.norm()).item() <= 1e-5
