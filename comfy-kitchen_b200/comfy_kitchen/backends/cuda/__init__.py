@@ -300,14 +300,16 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     else:
         out_rows, out_cols = rows, cols
         assert out_cols % 16 == 0, f"num_cols must be divisible by 16, got {out_cols}"
-    if out_cols != cols or cols % (64 // x.element_size()) or x.data_ptr() % 32:
+    size, x_ptr = x.element_size(), x.data_ptr()
+    if out_cols != cols or cols % (64 // size) or x_ptr % 32:
         # Not the streaming quantizer's form: the one-kernel scale, whose cached scratch is zero already.  (The
         # one call would clear its counter first: another launch in front of the other two.)
         scale = nvfp4_tensor_scale(x)
         return (*quantize_nvfp4(x, scale, pad_16x=pad_16x, hi_first=hi_first), scale)
     stream = _stream(x.device)
-    need = _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
-    if rows * cols * x.element_size() <= _WHOLE_INPUT_BYTES:
+    # the smallest workspace that is kept does up to 2^31 elements: no need to ask
+    need = 1 << 20 if rows * cols < 1 << 31 else _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
+    if rows * cols * size <= _WHOLE_INPUT_BYTES:
         scratch = _scale_scratch_for(x.device, stream, need)  # nothing is kept in it between two launches
     else:
         scratch = _workspace_for(need, x.device, stream)  # the partial maxima go from one launch to the next
@@ -315,7 +317,7 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
     sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)
     with _on_device(x.device):
-        _check(lib.ck_quantize_nvfp4_dynamic(x.data_ptr(), DTYPE_TO_CODE[x.dtype], scale.data_ptr(), qx.data_ptr(), sx.data_ptr(),
+        _check(lib.ck_quantize_nvfp4_dynamic(x_ptr, DTYPE_TO_CODE[x.dtype], scale.data_ptr(), qx.data_ptr(), sx.data_ptr(),
                                              rows, cols, out_rows, out_cols, int(bool(hi_first)), scratch.data_ptr(), scratch.numel(), stream),
                "quantize_nvfp4_dynamic")
     return qx, sx, scale
@@ -517,7 +519,8 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     as ``quantize_nvfp4`` followed by ``scaled_mm_nvfp4``.  The quantized activation passes
     from one launch to the next in a workspace (:func:`_workspace_for`)."""
     lib = load_library()
-    x, w_codes, w_block_scales = _plain(x), _plain(w_codes), _plain(w_block_scales)
+    if not (type(x) is type(w_codes) is type(w_block_scales) is torch.Tensor):
+        x, w_codes, w_block_scales = _plain(x), _plain(w_codes), _plain(w_block_scales)
     assert x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor"
     m, k = x.shape
     n, kb = w_codes.shape
@@ -530,13 +533,14 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     sx = None if x_scale is None else _scalar_f32(x_scale, dev, "x_scale")
     bias_ptr, bias_code, bias_keep = _bias_args(bias, n, dev)
     need = _workspace_bytes("ck_linear_nvfp4_from_float_workspace_bytes", m, k, int(sx is None))
-    if sx is None and need and x.data_ptr() % 32:
+    x_ptr = x.data_ptr()
+    if sx is None and need and x_ptr % 32:
         sx = nvfp4_tensor_scale(x)  # as in quantize_nvfp4_dynamic
     stream = _stream(dev)
     ws = _workspace_for(need, dev, stream)
     out = torch.empty((m, n), dtype=out_dtype, device=dev)
     with _on_device(dev):
-        _check(lib.ck_linear_nvfp4_from_float(x.data_ptr(), DTYPE_TO_CODE[x.dtype], _ptr(sx), w_codes.data_ptr(), w_block_scales.data_ptr(),
+        _check(lib.ck_linear_nvfp4_from_float(x_ptr, DTYPE_TO_CODE[x.dtype], _ptr(sx), w_codes.data_ptr(), w_block_scales.data_ptr(),
                                               sw.data_ptr(), bias_ptr, bias_code, out.data_ptr(), DTYPE_TO_CODE[out_dtype], m, n, k,
                                               ws.data_ptr(), ws.numel(), stream), "linear_nvfp4_from_float")
     del bias_keep
@@ -550,7 +554,8 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     ``quantize_mxfp8`` followed by ``scaled_mm_mxfp8``; the quantized activation passes through a
     workspace, as in :func:`linear_nvfp4_from_float`."""
     lib = load_library()
-    x, w_data, w_block_scales = _plain(x), _plain(w_data), _plain(w_block_scales)
+    if not (type(x) is type(w_data) is type(w_block_scales) is torch.Tensor):
+        x, w_data, w_block_scales = _plain(x), _plain(w_data), _plain(w_block_scales)
     assert x.dim() == 2 and x.is_contiguous(), "x must be a contiguous 2-D tensor"
     m, k = x.shape
     n, kb = w_data.shape

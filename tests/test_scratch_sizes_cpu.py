@@ -40,3 +40,8 @@ def test_linear_takes_up_to_2_30_elements_with_a_dynamic_scale(lib, m, k, suppor
     assert (lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, 1) > 0) == supported
     assert lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, 0) > 0
     assert lib.ck_linear_nvfp4_from_float_workspace_bytes(m, k, 0) % 256 == 0
+
+
+def test_one_mebibyte_does_all_but_huge_inputs(lib):
+    """The wrappers' smallest buffer, handed in without asking for the size."""
+    assert lib.ck_quantize_nvfp4_dynamic_scratch_bytes((1 << 31) - 1) <= 1 << 20
