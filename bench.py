@@ -815,8 +815,7 @@ def run_mlp_pair(args, torch, ck, backend, device, clocks_cls, local_rank) -> di
 
 def run_gemm_sweep(args, torch, ck, device) -> dict:
     """NVFP4 GEMM over the sweep on one GPU: M in {1, 16, 256, 4096, 16384} x (K, N) in {(3072, 3072),
-    (3072, 12288), (12288, 3072), (3072, 15360)}, bf16 output, through ``ck.scaled_mm_nvfp4`` (workspace
-    paths included).  Each shape: a CUDA graph of 20 launches that cycle through enough copies of the
+    (3072, 12288), (12288, 3072), (3072, 15360)}, bf16 output, through ``ck.scaled_mm_nvfp4``.  Each shape: a CUDA graph of 20 launches that cycle through enough copies of the
     weight to exceed the L2 cache, median of 11 replays.  Rows with M <= 256 are weight streaming: they
     are read against the HBM roofline (0.5625 (M K + N K) + 2 M N bytes), the others against the tensor peak."""
     peaks, peak_kind = load_peaks()

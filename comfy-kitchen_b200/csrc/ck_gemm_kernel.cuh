@@ -343,9 +343,9 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 }
 
 // The same for two values: the multiplies and adds as packed pairs (same roundings, same bits).  The fused
-// epilogue is bound by its instruction count (33 per element measured, 10.4 k cycles a tile against the
-// 6.3 k of its main loop); with the pairs here, in the drain and in the quantizer's products the MLP pair
-// 4608 x 12288 x 3072 goes from 188.7 to 177.2 us (163.0 to 154.5 on a cool chip).
+// epilogue was bound by its instruction count (33 per element, 10.4 k cycles a tile against the 6.3 k of its
+// main loop); with the pairs here, in the drain and in the quantizer's products it is 21 per element, and fc1 of
+// 4608 x 12288 x 3072 takes 99.7 us instead of 108.6 (graph replays), the MLP pair 181.3 instead of 189.9 (eager passes).
 __device__ __forceinline__ float2 gelu_tanh_x2(float2 x) {
   const float2 w = fma_x2(make_float2(-0.10294324f, -0.10294324f), mul_x2(x, x), make_float2(-2.3022082f, -2.3022082f));
   const float2 u = mul_x2(x, w);

@@ -475,7 +475,9 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
 }
 
 // Inputs of at most this many bytes: every block of the quantizer takes the maximum of the whole input
-// itself (a few 16 KiB passes out of L2) instead of waiting for a reduction kernel.
+// itself (a few 16 KiB passes out of L2) instead of waiting for a reduction kernel.  Scale and quantizer, us, whole
+// input / reduction kernel: at the line 8 x 4096 bf16 3.5 / 4.4, 1 x 32768 bf16 4.5 / 5.3; beyond it 128 KiB 3.9 / 4.5 still, 256 KiB
+// (fp32) 4.0 / 3.8, 384 KiB 6.3 / 5.2: the line could lie near 200 KiB.
 constexpr int64_t kWholeInputBytes = 64 * 1024;
 constexpr int64_t kDynamicScratchHead = 256;
 

@@ -78,7 +78,7 @@ def run(shape: str, ring: int, verbose: bool) -> None:
     out = [torch.empty(mp, n, dtype=torch.bfloat16, device=dev) for _ in range(ring)]
 
     need = int(lib.ck_scaled_mm_workspace_bytes(0, mp, n, k))
-    ws = torch.zeros(max(need, 16), dtype=torch.uint8, device=dev)
+    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=dev)
     small = m <= 32  # the weight-streaming path lives in its own translation unit, with its own buffers
     suffix = "_smallm" if small else ""
 
