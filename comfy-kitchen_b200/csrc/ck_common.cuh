@@ -43,10 +43,22 @@ int gemm_status_word(int** out);
 int64_t amax_partials(int64_t n_vecs);
 int launch_amax_partials(const void* x, int dtype, int64_t n_vecs, float* partials, int* n_partials, cudaStream_t s);
 
+// Validation hooks: the kernel configuration that CK_GEMM_CONFIG pins (0 = none; ck_gemm.cu), and whether the quantizers
+// divide every element (ck_quantize.cu).
+int forced_gemm_config();
+bool exact_division();
+
+// One-call linears with very few activation rows (ck_gemm_smallm.cu).
+bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const void* w, const void* w_scales, int bias_dtype, int out_dtype,
+                            int64_t M, int64_t N, int64_t K);
+int linear_small_m(bool is_mxfp8, const void* x, int x_dtype, const float* x_scale, const float* partials, int n_partials, const void* w,
+                   const void* w_scales, const float* w_scale, const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M,
+                   int64_t N, int64_t K, cudaStream_t stream);
+
 // GEMMs with few activation rows (ck_gemm_smallm.cu).
 bool small_m_applies(int64_t M, int64_t N, int64_t K);
 int small_m_max_splits(int64_t N, int k_bytes);
-int small_m_splits(bool is_mxfp8, int out_dtype, int64_t N, int k_bytes, int* splits);
+int small_m_splits(bool is_mxfp8, int64_t N, int k_bytes, int* splits);
 int scaled_mm_small_m(bool is_mxfp8, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
                       const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
                       int64_t M, int64_t N, int64_t K, cudaStream_t stream);

@@ -21,9 +21,7 @@ int gemm_status_word(int** out) {
   return CK_OK;
 }
 
-namespace {
-
-int forced_config() {
+int forced_gemm_config() {
   // CK_GEMM_CONFIG pins the kernel configuration (used by the tests to cover each one); unset =
   // choose by shape.
   //   1 = one CTA, 128 x 128 tiles (two accumulators)   3 = one CTA, 128 x 256 tiles
@@ -32,9 +30,11 @@ int forced_config() {
   return e ? atoi(e) : 0;
 }
 
+namespace {
+
 template <Kind KIND, typename OutT, bool FUSED>
 int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, cudaStream_t stream) {
-  int config = forced_config();
+  int config = forced_gemm_config();
   if (config == 0) {
     const int64_t pair_tiles = ceil_div(p.M, 256) * ceil_div(p.N, 256);
     if (pair_tiles * 4 >= sm_count()) {
@@ -100,7 +100,7 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
   int splits = most;
   for (; splits > 1; --splits) {
     int clusters = 0;
-    if (int rc = split_clusters<KIND, 128, 2, 5, OutT, 1, false>(splits, &clusters)) return rc;
+    if (int rc = split_clusters<KIND, 128, 2, 5, OutT, 1>(splits, &clusters)) return rc;
     if (clusters >= tiles) break;
   }
   plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
@@ -158,7 +158,7 @@ int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, void* 
   const GemmParams result = p;
   p.splits = plan.splits;
   p.k_stages_per_split = plan.k_stages;
-  if (!plan.through_workspace) return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1, false, Split::kCluster>(ops, p, os, stream);
+  if (!plan.through_workspace) return launch_config<KIND, 128, 2, 5, 1, OutT, false, 1, Split::kCluster>(ops, p, os, stream);
   p.tsa = p.tsb = p.alpha = nullptr;
   p.bias = nullptr;
   p.out = workspace;
@@ -170,7 +170,7 @@ int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, void* 
   partials.n = plan.splits;
   partials.pitch = p.N;
   partials.col_offset = 0;
-  if (int rc = launch_config<KIND, 128, 2, 5, 1, float, false, 1, false, Split::kOutputs>(ops, p, partials, stream)) return rc;
+  if (int rc = launch_config<KIND, 128, 2, 5, 1, float, false, 1, Split::kOutputs>(ops, p, partials, stream)) return rc;
   CK_CUDA(launch_pdl(splitk_reduce_kernel<OutT>, dim3(static_cast<unsigned>(ceil_div(mn / 4, 256))), dim3(256), 0, stream,
                      static_cast<const float*>(workspace), plan.splits, mn, p.N, result.alpha, result.tsa, result.tsb, result.bias,
                      result.bias_dtype, static_cast<OutT*>(result.out)));
@@ -276,11 +276,11 @@ int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, con
   if (!fused.enabled && out_spec == nullptr) {
     // Few activation rows: the weight-streaming path (operands swapped, K split over all SMs).
     // CK_GEMM_CONFIG=9 forces it, any other forced configuration keeps it off.
-    if (small_m_applies(M, N, K) && (forced_config() == 0 || forced_config() == 9)) {
+    if (small_m_applies(M, N, K) && (forced_gemm_config() == 0 || forced_gemm_config() == 9)) {
       return scaled_mm_small_m(KIND == Kind::kMxfp8, a, b, sfa, sfb, tsa, tsb, alpha, bias, bias_dtype, out, out_dtype, M, N, K, s);
     }
     // the rows of the result are written four columns at a time
-    if (max_splits(M, N, p.k_bytes) > 1 && forced_config() == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+    if (max_splits(M, N, p.k_bytes) > 1 && forced_gemm_config() == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
       bool launched = false;
       int rc = CK_OK;
       switch (out_dtype) {
@@ -367,7 +367,7 @@ extern "C" int ck_debug_gemm_splits(int is_mxfp8, int out_dtype, int64_t M, int6
   }
   SplitPlan plan = {};
   const int rc = small_m_applies(M, N, K)
-                     ? small_m_splits(is_mxfp8 != 0, out_dtype, N, static_cast<int>(is_mxfp8 ? K : K / 2), &plan.splits)
+                     ? small_m_splits(is_mxfp8 != 0, N, static_cast<int>(is_mxfp8 ? K : K / 2), &plan.splits)
                      : tile_plan(is_mxfp8 != 0, out_dtype, M, N, K, with_workspace != 0, &plan);
   return rc == CK_OK ? plan.splits : -rc;
 }

@@ -126,7 +126,6 @@ constexpr int kMaxSplits = 8;       // CTAs of a split-K cluster (the portable c
 enum class Split {
   kNone,
   kCluster,          // the cluster's CTAs add their partial tiles through distributed shared memory
-  kClusterManyRows,  // the same with swapped operands and more activation rows than a warp each would do for
   kOutputs           // CTA s stores its raw fp32 partial tile to destination s
 };
 
@@ -410,27 +409,19 @@ __device__ __forceinline__ float4 add_partials(const uint32_t (&base)[kMaxSplits
 // FUSED: the epilogue applies an activation to the output rounded to OutT (what an unfused
 // caller would see), optionally stores it, and optionally re-quantizes it to NVFP4 (codes +
 // tiled block scales against a static per-tensor scale) as the A operand of the next GEMM.
-// SWAP: the operands have changed places - "A" (128-row tiles, tensor-memory lanes) is the weight
-// [N, K] and "B" (the MMA's N dimension, TILE_N >= M) is the small activation [M, K] - so that a GEMM
-// with few activation rows fills the 128-row MMA dimension with weight rows and streams the weight
-// once.  p.M / p.N are then the weight's and the activation's row counts, the output is written
-// transposed (out[b_row][a_row]) and the bias runs along the A rows.
-template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE, bool SWAP = false,
-          Split SPLIT = Split::kNone>
-__global__ void __launch_bounds__(num_threads(FUSED, TILE_N), (SWAP && TILE_N <= 128) ? 2 : 1)
+template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE, Split SPLIT = Split::kNone>
+__global__ void __launch_bounds__(num_threads(FUSED, TILE_N), 1)
 block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
                          const __grid_constant__ OutputMaps maps_out, const GemmParams p) {
   using Cfg = Config<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OUT_STAGE>;
   static_assert(!(FUSED && OUT_STAGE != 0), "the fused epilogue stores from registers");
-  static_assert(!SWAP || (!FUSED && OUT_STAGE == 0 && CTAS == 1), "swapped operands: plain epilogue, one CTA");
   constexpr int kNumEpilogueWarps = epilogue_warps(FUSED, TILE_N);
   constexpr int kThreads = num_threads(FUSED, TILE_N);
   static_assert(TILE_N <= 32 * kNumEpilogueWarps, "one bias value per epilogue thread");
-  constexpr bool kCluster = SPLIT == Split::kCluster || SPLIT == Split::kClusterManyRows;
+  constexpr bool kCluster = SPLIT == Split::kCluster;
   static_assert(SPLIT == Split::kNone || (CTAS == 1 && !FUSED), "only plain one-CTA tiles are split");
-  static_assert(SPLIT != Split::kClusterManyRows || SWAP, "rows of swapped operands");
-  static_assert(SPLIT != Split::kOutputs || (!SWAP && OUT_STAGE != 0 && std::is_same<OutT, float>::value), "raw partial tiles, staged");
+  static_assert(SPLIT != Split::kOutputs || (OUT_STAGE != 0 && std::is_same<OutT, float>::value), "raw partial tiles, staged");
   static_assert(!kCluster || kTileM * TILE_N * 4 <= Cfg::kRingBytes, "a partial tile fits in the operand ring");
   // Everything the kernel does until a role's griddepcontrol.wait is independent of the kernel
   // before it in the stream, so the next kernel may be scheduled as early as resources allow.
@@ -463,28 +454,6 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   CK_TRACE3(0);
-
-  // Weight streaming (SWAP): first thing, ahead of the set-up and of the dependency wait, ask L2 for
-  // the operand boxes of this CTA's first stages.  A prefetch only warms the cache (L2 is the point
-  // of coherence: what the previous kernel still writes is seen by the loads after the wait); the
-  // DRAM latency of the first loads then overlaps barrier set-up, tensor-memory allocation and the
-  // wait itself (1-3 % of these 6-10 us kernels).  The tile configurations are slower with it
-  // (config 2: 18.7 vs 18.5 us; the requests share the TMA unit with the first loads).
-  if (SWAP && warp == 0 && elect_one()) {
-    const int pf_splits = SPLIT == Split::kNone ? 1 : p.splits;
-    const int pf_k_stages = (p.k_bytes + kStageKBytes - 1) / kStageKBytes;
-    if (worker < p.tiles_m * p.tiles_n * pf_splits) {
-      const int tile0 = worker / pf_splits;
-      const int ks0 = (worker - tile0 * pf_splits) * p.k_stages_per_split;
-      const int ks1 = min(min(pf_k_stages, ks0 + p.k_stages_per_split), ks0 + STAGES);
-      const int pm0 = tile_row_block(p, tile0) * Cfg::kTileRows + static_cast<int>(cta_rank) * kTileM;
-      const int pn0 = tile_col_block(p, tile0) * TILE_N + static_cast<int>(cta_rank) * Cfg::kBRows;
-      for (int ks = ks0; ks < ks1; ++ks) {
-        tma_prefetch_2d(&map_a, ks * kStageKBytes, pm0);
-        tma_prefetch_2d(&map_b, ks * kStageKBytes, pn0);
-      }
-    }
-  }
 
   // ------------------------------------------------------------------ set-up
   // The producer warp creates the barriers and goes straight to its loads; the other warps
@@ -752,19 +721,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       split_alpha = alpha;
       if (p.bias != nullptr) {
         const int tile = worker / splits;
-        if constexpr (SWAP) {
-          const int first = SPLIT == Split::kClusterManyRows ? lane * 4 : ((static_cast<int>(cluster_cta_rank()) + splits * (warp - 2)) & 3) * 32 + lane;
-          const int a_row = tile_row_block(p, tile) * kTileM + first;
+        const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
 #pragma unroll
-          for (int j = 0; j < (SPLIT == Split::kClusterManyRows ? 4 : 1); ++j) {
-            if (a_row + j < p.M) split_bias[j] = load_bias(p.bias, p.bias_dtype, a_row + j);
-          }
-        } else {
-          const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (col + j < p.N) split_bias[j] = load_bias(p.bias, p.bias_dtype, col + j);
-          }
+        for (int j = 0; j < 4; ++j) {
+          if (col + j < p.N) split_bias[j] = load_bias(p.bias, p.bias_dtype, col + j);
         }
       }
     }
@@ -782,58 +742,6 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int n0 = tile_n * TILE_N;
       const int acc = tile_it % NUM_ACC;
       const uint32_t acc_ph = (tile_it / NUM_ACC) & 1;
-      if constexpr (SWAP) {
-        // ---- swapped operands: lane = weight row (output column), accumulator columns = activation rows
-        const int r_in_tile = quarter * 32 + lane;
-        const int a_row = tile_m * kTileM + r_in_tile;  // weight row = output column
-        const int c0 = half * kColsPerWarp;
-        // fetched ahead of the accumulator wait, which hides the latency
-        const float bias_v = (p.bias != nullptr && a_row < p.M) ? load_bias(p.bias, p.bias_dtype, a_row) : 0.0f;
-        if (warp == 2) CK_TRACE(6);
-        mbar_wait(&acc_full_bar[acc], acc_ph, abort_flag);
-        if (warp == 2) CK_TRACE(7);
-        tc_fence_after_sync();
-        const uint32_t t_row = tmem_base + acc * Cfg::kAccCols + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
-        uint32_t buf[kChunks][32];
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) tmem_load_32x32(t_row + c * 32, buf[c]);
-        tmem_load_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
-        if (warp == 2) CK_TRACE(8);
-        if constexpr (kCluster) {
-          // Raw partial to the CTA's own shared memory, [column][128 rows]; added below by the cluster.
-          float* part = reinterpret_cast<float*>(smem) + r_in_tile;
-#pragma unroll
-          for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int col = c0 + c * 32 + i;
-              if (n0 + col < p.N) part[col * kTileM] = __uint_as_float(buf[c][i]);
-            }
-          }
-          continue;
-        }
-        if (warp == 2) CK_TRACE(13);
-        if (a_row < p.M) {
-          // one address, moved from row to row: 32 of them at once cost the 16-bit results 40 registers and spills
-          OutT* dst = out + static_cast<int64_t>(n0 + c0) * p.M + a_row;
-#pragma unroll
-          for (int c = 0; c < kChunks; ++c) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int b_row = n0 + c0 + c * 32 + i;  // activation row = output row
-              if (c == 0 && i == 1 && warp == 2) CK_TRACE(14);
-              if (c == 0 && i == 8 && warp == 2) CK_TRACE(15);
-              if (b_row < p.N) *dst = to_out<OutT>(fmaf(__uint_as_float(buf[c][i]), alpha, bias_v));
-              dst += p.M;
-            }
-          }
-        }
-        if (warp == 2) CK_TRACE(9);
-        continue;
-      }
       // Bias of a tile's columns as fp32 in shared memory, three buffers in rotation: the
       // buffer of tile t is filled while tile t - 1 is in its epilogue (right after the drain,
       // where the warps are aligned anyway), so no barrier stands between the end of one
@@ -1149,61 +1057,16 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       uint32_t base[kMaxSplits];
 #pragma unroll
       for (int i = 0; i < kMaxSplits; ++i) base[i] = map_to_cta(part, i < splits ? i : 0);
-      if constexpr (SWAP) {
-        OutT* out = static_cast<OutT*>(p.out);
-        const int a_row0 = tile_row_block(p, tile) * kTileM;
-        if constexpr (SPLIT == Split::kCluster) {
-          // a warp takes 32 of the weight rows (a coalesced run of the output) of one activation row; the host sees
-          // to it that there are warps enough
-          const int u = rank + splits * (warp - 2);
-          const int col = u >> 2;
-          const int r = (u & 3) * 32 + lane;
-          if (col < p.N) {
-            float v[kMaxSplits];
-#pragma unroll
-            for (int i = 0; i < kMaxSplits; ++i) {
-              if (i < splits) v[i] = ld_shared_cluster_f32(base[i] + (col * kTileM + r) * 4);
-            }
-            float acc = v[0];
-#pragma unroll
-            for (int i = 1; i < kMaxSplits; ++i) {
-              if (i < splits) acc += v[i];
-            }
-            if (a_row0 + r < p.M) out[static_cast<int64_t>(col) * p.M + a_row0 + r] = to_out<OutT>(fmaf(acc, split_alpha, split_bias[0]));
-          }
-        } else {
-          // a warp takes all 128 weight rows of one activation row, a lane four of them: up to 32 activation rows in
-          // one to three rounds (NVFP4 32 x 1024 x 4096: 5.8 us, against 7.1 with 32 weight rows at a time)
-          const int a_row = a_row0 + lane * 4;
-          const bool in_rows = a_row < p.M;  // the output's row length is a multiple of 8: all four or none
-          const bool vec = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(OutT) - 1)) == 0;
-          for (int col = rank + splits * (warp - 2); col < p.N; col += splits * kNumEpilogueWarps) {
-            const float4 acc = add_partials(base, splits, (col * kTileM + lane * 4) * 4);
-            if (in_rows) {
-              float y[4];
-              sums_scaled(acc, split_alpha, split_bias, y);
-              OutT* dst = out + static_cast<int64_t>(col) * p.M + a_row;
-              if (vec) {
-                store_four(dst, y);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dst[j] = to_out<OutT>(y[j]);
-              }
-            }
-          }
-        }
-      } else {
-        // a warp takes one row of the tile, a lane four neighbouring columns
-        const int row0 = tile_row_block(p, tile) * kTileM;
-        const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
-        const bool in_cols = col < p.N;  // N % 8 == 0: a group of four never straddles the edge
-        const int rows = min(kTileM, p.M - row0);
-        for (int r = rank + splits * (warp - 2); r < rows; r += splits * kNumEpilogueWarps) {
-          const float4 acc = add_partials(base, splits, r * (TILE_N * 4) + ((lane ^ (r & 7)) << 4));
-          float y[4];
-          sums_scaled(acc, split_alpha, split_bias, y);
-          if (in_cols) store_four(static_cast<OutT*>(p.out) + static_cast<int64_t>(row0 + r) * p.N + col, y);
-        }
+      // a warp takes one row of the tile, a lane four neighbouring columns
+      const int row0 = tile_row_block(p, tile) * kTileM;
+      const int col = tile_col_block(p, tile) * TILE_N + lane * 4;
+      const bool in_cols = col < p.N;  // N % 8 == 0: a group of four never straddles the edge
+      const int rows = min(kTileM, p.M - row0);
+      for (int r = rank + splits * (warp - 2); r < rows; r += splits * kNumEpilogueWarps) {
+        const float4 acc = add_partials(base, splits, r * (TILE_N * 4) + ((lane ^ (r & 7)) << 4));
+        float y[4];
+        sums_scaled(acc, split_alpha, split_bias, y);
+        if (in_cols) store_four(static_cast<OutT*>(p.out) + static_cast<int64_t>(row0 + r) * p.N + col, y);
       }
     }
     __syncwarp();
@@ -1368,7 +1231,7 @@ struct Operands {
 };
 
 // Clusters of `splits` CTAs of this configuration that can run at once on the current device, one CTA to an SM.
-template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, typename OutT, int OUT_STAGE, bool SWAP>
+template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, typename OutT, int OUT_STAGE>
 int split_clusters(int splits, int* out) {
   using Cfg = Config<KIND, TILE_N, NUM_ACC, STAGES, 1, OUT_STAGE>;
   static std::atomic<int> cached[64][kMaxSplits + 1];
@@ -1376,7 +1239,7 @@ int split_clusters(int splits, int* out) {
   CK_CUDA(cudaGetDevice(&dev));
   int n = (dev >= 0 && dev < 64) ? cached[dev][splits].load(std::memory_order_relaxed) : 0;
   if (n == 0) {
-    auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, 1, OutT, false, OUT_STAGE, SWAP, Split::kCluster>;
+    auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, 1, OutT, false, OUT_STAGE, Split::kCluster>;
     CK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(num_threads(false, TILE_N));
@@ -1397,11 +1260,10 @@ int split_clusters(int splits, int* out) {
   return CK_OK;
 }
 
-template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE = 0, bool SWAP = false,
-          Split SPLIT = Split::kNone>
+template <Kind KIND, int TILE_N, int NUM_ACC, int STAGES, int CTAS, typename OutT, bool FUSED, int OUT_STAGE = 0, Split SPLIT = Split::kNone>
 int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaStream_t stream) {
   using Cfg = Config<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OUT_STAGE>;
-  auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OutT, FUSED, OUT_STAGE, SWAP, SPLIT>;
+  auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OutT, FUSED, OUT_STAGE, SPLIT>;
   // only the tensor maps this configuration uses are encoded (host time is visible for small problems)
   CUtensorMap map_a, map_b;
   if (int rc = make_operand_map(&map_a, ops.a, p.M, p.k_bytes, kTileM)) return rc;
@@ -1422,7 +1284,7 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  constexpr bool cluster_split = SPLIT == Split::kCluster || SPLIT == Split::kClusterManyRows;
+  constexpr bool cluster_split = SPLIT == Split::kCluster;
   attr[0].val.clusterDim.x = cluster_split ? p.splits : CTAS;  // split-K: the CTAs of one tile are a cluster
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
@@ -1435,7 +1297,7 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   static std::atomic<int> max_workers[64];
   int resident = (dev >= 0 && dev < 64) ? max_workers[dev].load(std::memory_order_acquire) : 0;
   if (resident == 0) {
-    resident = sm_count() / CTAS * ((SWAP && TILE_N <= 128) ? 2 : 1);  // the small swapped configurations share an SM
+    resident = sm_count() / CTAS;
     if (CTAS > 1) {
       cfg.gridDim = dim3(sm_count() / CTAS * CTAS);
       int clusters = 0;
@@ -1461,13 +1323,11 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   // (A row blocks + B column blocks of one wave), so that a long operand is not pulled through L2
   // once per tile column (M = 16384, K = 12288: 100 MB of A per wave down the rows, 28 MB along the
   // columns).
-  if (!SWAP) {
-    const int64_t a_block = static_cast<int64_t>(Cfg::kTileRows) * p.k_bytes, b_block = static_cast<int64_t>(TILE_N) * p.k_bytes;
-    const int64_t w = workers, tm = p.tiles_m, tn = p.tiles_n;
-    const int64_t down = (w < tm ? w : tm) * a_block + ceil_div(w, tm) * b_block;
-    const int64_t along = ceil_div(w, tn) * a_block + (w < tn ? w : tn) * b_block;
-    p.raster = along < down ? 1 : 0;
-  }
+  const int64_t a_block = static_cast<int64_t>(Cfg::kTileRows) * p.k_bytes, b_block = static_cast<int64_t>(TILE_N) * p.k_bytes;
+  const int64_t w = workers, tm = p.tiles_m, tn = p.tiles_n;
+  const int64_t down = (w < tm ? w : tm) * a_block + ceil_div(w, tm) * b_block;
+  const int64_t along = ceil_div(w, tn) * a_block + (w < tn ? w : tn) * b_block;
+  p.raster = along < down ? 1 : 0;
   OutputMaps maps_out = {};
   p.out_tma = 0;
   p.n_out = 1;

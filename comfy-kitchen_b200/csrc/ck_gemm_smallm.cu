@@ -1,30 +1,518 @@
-// Block-scaled GEMMs with very few activation rows (M <= 32): weight streaming.
+// Block-scaled GEMMs with very few activation rows (M <= 32): weight streaming, and the one-call linears that quantize a
+// dense activation of up to 16 rows inside it.
 //
-// out[M, N] = x[M, K] . W[N, K]^T with M small reads the whole weight once and does almost no
-// arithmetic: it is bound by HBM (0.5625 bytes per NVFP4 weight element) and by fixed latencies.
-// The 128-row tile configurations spend their MMA rows, their operand loads and their epilogue on
-// padding.  Here the operands change places (ck_gemm_kernel.cuh, SWAP): weight rows fill the 128
-// tensor-memory lanes, the activation rows are the MMA's N (32), the accumulator is 32 columns
-// wide and the epilogue writes 32 values per thread.  When the weight has few 128-row tiles and a
-// long K, every tile's K range is cut over a cluster of CTAs so that all SMs stream (two CTAs fit on
-// an SM); the cluster adds its partial tiles in split order through distributed shared memory.
-// Measured against the tile path: wins up to 32 rows, loses from 64 rows on.
+// out[M, N] = x[M, K] . W[N, K]^T with M small reads the whole weight once and does almost no arithmetic: it is bound
+// by HBM (0.5625 bytes per NVFP4 weight element) and by fixed latencies.  The 128-row tile configurations spend their
+// MMA rows, their operand loads and their epilogue on padding.  Here the operands change places: weight rows fill the
+// 128 tensor-memory lanes, the activation rows are the MMA's N (32), the accumulator is 32 columns wide and the epilogue
+// writes the result transposed.  Measured against the tile path: wins up to 32 rows, loses from 64 rows on.
+//
+// A CTA has one item; the hardware queues what does not fit the chip.  How the weight is cut (choose_plan):
+//   * a 128-row tile to a CTA;
+//   * few tiles and a long K: every tile's K range over a cluster of CTAs, which add their partial tiles in split order
+//     through distributed shared memory.
+// (Half and quarter tiles to a CTA were measured: nothing gained.  An MMA of 128 weight rows takes the tensor pipe some 135 cycles
+// whatever N is, so that a CTA streams at most 4 KiB in that time; four accumulators in turn change nothing either.)
+//
+// Dense activations (XT): as two kernels, the quantizer of a few rows is one wave of load latency, arithmetic and store
+// latency before the GEMM's loads may begin.  Here every CTA quantizes the rows it multiplies by, stage by stage, straight
+// into the shared-memory ring the tensor cores read (codes in the 128-byte swizzle, scale bytes in the tiles
+// tcgen05.cp takes), while the weight's tiles come by TMA; the quantized activation never leaves the SM.  The same
+// operations in the same order as quantizer + GEMM: the same bits.
+//   warp 0      asks L2 for the first weight boxes ahead of the dependency wait, then TMA loads into the ring
+//   warp 1      scale copies and MMAs
+//   warps 2-9   dynamic tensor scale and quantizer of a dense activation (`stage_warps` of them do one stage, so that with few
+//               rows several stages are in the making at once), epilogue
 #include "ck_gemm_kernel.cuh"
 
 namespace ck {
 namespace {
 
 constexpr int kMaxSmallM = 32;
-constexpr int kSmallTileN = 32;  // the MMA's N: activation rows, padded
+constexpr int kMaxDenseM = 16;       // rows that are quantized here (which of them by format: linear_small_m_applies)
+constexpr int kMmaN = 32;            // of the MMA: activation rows; those past M are whatever the ring holds, their columns are not read
+constexpr int kQuantWarps = 8;
+constexpr int kSmallThreads = 64 + 32 * kQuantWarps;
+constexpr int kMaxSmemBytes = 224 * 1024;  // of a CTA alone on its SM
+
+struct SmallParams {
+  const void* x;             // dense activation [M, K], or null: quantized, and
+  const uint8_t* x_scales;   //   its tiled block scales
+  const float* x_scale;      // tensor scale of the activation (NVFP4); of a dense one the static scale, or null: from
+  const float* partials;     //   the maxima of a reduction pass, or without them
+  int n_partials;
+  int n_vecs;                //   from x itself, n_vecs 32-byte units that every CTA reads
+  const uint8_t* w_scales;   // tiled block scales of the weight
+  const float* w_scale;      // its tensor scale (NVFP4)
+  const float* alpha;        // replaces the product of the tensor scales when non-null
+  const void* bias;
+  void* out;                 // [M, N]
+  int bias_dtype, out_dtype;
+  int M, N, K;
+  int k_bytes, sf_col_tiles;
+  int splits, k_stages_per_split;
+  int ring;                  // stages of the ring
+  int x_rows;                // activation rows of a stage's slot: 16 or 32
+  int prefetch;              // weight boxes asked from L2 ahead of the dependency wait
+  int stage_warps;           // dense: quantizer warps to a stage, 2, 4 or 8
+  int* status;
+};
+
+template <Kind KIND>
+struct Small {
+  static constexpr int kSfTiles = KIND == Kind::kNvfp4 ? 4 : 1;
+  static constexpr int kSfBytes = kSfTiles * 512;
+  static constexpr int kMaxRing = 7;
+  static constexpr int kSfCols = 2 * kSfTiles * 4;  // tensor-memory columns of a stage's scales
+  static constexpr int kTmemCols = pow2_at_least(kMmaN + kMaxRing * kSfCols);
+  static constexpr int kStageElems = KIND == Kind::kNvfp4 ? 2 * kStageKBytes : kStageKBytes;
+  static constexpr int kRowThreads = kStageElems / 16;  // a thread takes 16 elements of a row
+  static constexpr uint32_t kIdesc = make_block_scaled_idesc(KIND == Kind::kNvfp4 ? 1u : 0u, KIND == Kind::kNvfp4 ? 0u : 1u, kTileM, kMmaN);
+  static_assert(kTmemCols <= 256, "two CTAs to an SM");
+  static_assert(kMaxDenseM * kRowThreads <= 32 * kQuantWarps, "a stage's rows in one go");
+  // The ring: weight [ring][128 rows x 128 bytes], activation codes [ring][x_rows x 128 bytes], scale tiles of both.  (An MMA
+  // reads 32 activation rows: with slots of 16 into what follows.)
+  static constexpr int smem_bytes(int ring, int x_rows) {
+    return ring * ((kTileM + x_rows) * kStageKBytes + 2 * kSfBytes) + 1024 /*alignment slack*/;
+  }
+  static_assert(2 * 4 * kSfBytes >= 16 * kStageKBytes, "what a slot of 16 rows lacks");
+  static_assert(kMaxSmallM * kTileM * 4 <= 4 * kTileM * kStageKBytes, "a partial tile fits in the weight's slots");
+};
+
+// 16 elements of the activation
+template <typename T>
+struct Sixteen {
+  Vec256 v[sizeof(T) / 2];
+};
+
+template <typename T>
+__device__ __forceinline__ Sixteen<T> load_sixteen(const T* p, bool valid) {
+  Sixteen<T> r = {};
+  if (valid) {
+    r.v[0] = ld_global_stream_256(p);
+    if constexpr (sizeof(T) == 4) r.v[1] = ld_global_stream_256(p + 8);
+  }
+  return r;
+}
+
+template <typename T>
+__device__ __forceinline__ void widen_sixteen(const Sixteen<T>& s, float (&v)[16]) {
+  if constexpr (sizeof(T) == 2) {
+    quant::widen16<T>(s.v[0].w, v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] = __uint_as_float(s.v[0].w[i]);
+      v[8 + i] = __uint_as_float(s.v[1].w[i]);
+    }
+  }
+}
+
+// amax(|x|) / 2688 by the quantizer warps (all of them return it)
+template <typename T>
+__device__ __forceinline__ float dynamic_scale(const SmallParams& p, int tid, float* warp_max) {
+  constexpr int kThreads = 32 * kQuantWarps;
+  constexpr int kInFlight = 8;
+  float m = 0.0f;
+  if (p.n_partials > 0) {
+    for (int i = tid; i < p.n_partials; i += kThreads) m = fmaxf(m, ld_f32_dependent(p.partials + i));
+  } else {
+    const T* x = static_cast<const T*>(p.x);
+    for (int i = tid; i < p.n_vecs; i += kInFlight * kThreads) {
+      Vec256 raw[kInFlight];
+#pragma unroll
+      for (int j = 0; j < kInFlight; ++j) {
+        raw[j] = i + j * kThreads < p.n_vecs ? ld_global_stream_256(x + (i + j * kThreads) * (32 / sizeof(T))) : Vec256{};
+      }
+#pragma unroll
+      for (int j = 0; j < kInFlight; ++j) m = fmaxf(m, quant::abs_max_of_vec<T>(raw[j]));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+  if ((tid & 31) == 0) warp_max[tid >> 5] = m;
+  named_barrier_sync(1, kThreads);
+#pragma unroll
+  for (int w = 0; w < kQuantWarps; ++w) m = fmaxf(m, warp_max[w]);
+  return quant::nvfp4_scale_of_amax<T>(m);
+}
+
+// Position in the ring: `step` moves on by up to a round.
+struct RingAt {
+  int slot;
+  uint32_t phase;
+  __device__ explicit RingAt(int first) : slot(first), phase(0) {}
+  __device__ __forceinline__ void step(int by, int ring) {
+    slot += by;
+    if (slot >= ring) {
+      slot -= ring;
+      phase ^= 1u;
+    }
+  }
+};
+
+template <typename OutT>
+__device__ __forceinline__ void store_columns(OutT* dst, int64_t pitch, const uint32_t (&acc)[16], float alpha, float bias, int count) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if (i < count) *dst = to_out<OutT>(fmaf(__uint_as_float(acc[i]), alpha, bias));
+    dst += pitch;
+  }
+}
+
+// The cluster's share of one weight tile: partial tiles lie in the CTAs' shared memory as [activation row][128].
+template <typename OutT>
+__device__ __forceinline__ void add_cluster_tile(const SmallParams& p, OutT* out, const uint32_t (&base)[kMaxSplits], int rank, int qw,
+                                                 int lane, int n0, float alpha) {
+  if (4 * p.M <= p.splits * kQuantWarps) {  // a warp to 32 weight rows of one activation row, if there are warps enough
+    const int u = rank + p.splits * qw, m = u >> 2, r = (u & 3) * 32 + lane, n = n0 + r;
+    if (m < p.M) {
+      float v[kMaxSplits];
+#pragma unroll
+      for (int i = 0; i < kMaxSplits; ++i) {
+        if (i < p.splits) v[i] = ld_shared_cluster_f32(base[i] + (m * kTileM + r) * 4);
+      }
+      float acc = v[0];
+#pragma unroll
+      for (int i = 1; i < kMaxSplits; ++i) {
+        if (i < p.splits) acc += v[i];
+      }
+      if (n < p.N) {
+        const float bias = p.bias != nullptr ? load_bias(p.bias, p.bias_dtype, n) : 0.0f;
+        out[static_cast<int64_t>(m) * p.N + n] = to_out<OutT>(fmaf(acc, alpha, bias));
+      }
+    }
+    return;
+  }
+  // else all 128 weight rows, a lane four of them (NVFP4 32 x 1024 x 4096: 5.8 us, against 7.1 with 32 weight rows at a time)
+  const int n = n0 + lane * 4;
+  const bool inside = n < p.N;  // N % 8 == 0: all four or none
+  const bool vec = (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(OutT) - 1)) == 0;
+  float bias[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (p.bias != nullptr && inside) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bias[j] = load_bias(p.bias, p.bias_dtype, n + j);
+  }
+  for (int m = rank + p.splits * qw; m < p.M; m += p.splits * kQuantWarps) {
+    const float4 acc = add_partials(base, p.splits, (m * kTileM + lane * 4) * 4);
+    if (inside) {
+      float y[4];
+      sums_scaled(acc, alpha, bias, y);
+      OutT* dst = out + static_cast<int64_t>(m) * p.N + n;
+      if (vec) {
+        store_four(dst, y);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dst[j] = to_out<OutT>(y[j]);
+      }
+    }
+  }
+}
+
+template <Kind KIND, typename XT, bool SPLIT>
+__global__ void __launch_bounds__(kSmallThreads, 2)
+small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SmallParams p) {
+  using C = Small<KIND>;
+  constexpr bool kDense = !std::is_void<XT>::value;
+  pdl_launch_dependents();
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int kABytes = kTileM * kStageKBytes;
+  const int b_bytes = p.x_rows * kStageKBytes;
+  uint8_t* smem_a = smem;
+  uint8_t* smem_b = smem_a + p.ring * kABytes;
+  uint8_t* smem_sfa = smem_b + p.ring * b_bytes;
+  uint8_t* smem_sfb = smem_sfa + p.ring * C::kSfBytes;
+  __shared__ uint64_t full_bar[C::kMaxRing];   // loads landed and rows quantized -> MMA
+  __shared__ uint64_t empty_bar[C::kMaxRing];  // MMA -> producer and quantizers
+  __shared__ uint64_t acc_bar[1];
+  __shared__ uint32_t tmem_base_slot[1];
+  __shared__ int abort_word;
+  __shared__ float warp_max[kQuantWarps];
+  volatile int* abort_flag = &abort_word;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = SPLIT ? blockIdx.x : 0;
+  const int n0 = blockIdx.y * kTileM;  // this tile's weight rows
+  const int k_stages = (p.k_bytes + kStageKBytes - 1) / kStageKBytes;
+  const int ks0 = rank * p.k_stages_per_split;
+  const int n_stages = min(k_stages - ks0, p.k_stages_per_split);
+  const uint8_t* w_scales = p.w_scales + (static_cast<int64_t>(blockIdx.y) * p.sf_col_tiles + ks0 * C::kSfTiles) * 512;
+  const int sf_tiles = min(p.sf_col_tiles - ks0 * C::kSfTiles, n_stages * C::kSfTiles);  // of this CTA's K range
+
+  uint32_t tmem_base = 0;
+  if (warp == 0) {
+    if (elect_one()) {
+      // A prefetch only warms L2 (the point of coherence): it may run ahead of the kernel before this one.
+      for (int i = 0; i < min(n_stages, p.prefetch); ++i) {
+        tma_prefetch_2d(&map_w, (ks0 + i) * kStageKBytes, n0);
+        if constexpr (!kDense) tma_prefetch_2d(&map_x, (ks0 + i) * kStageKBytes, 0);
+      }
+      if (p.prefetch > 0) bulk_prefetch_l2(w_scales, static_cast<uint32_t>(min(sf_tiles, p.prefetch * C::kSfTiles)) * 512u);
+      *abort_flag = 0;
+      for (int s = 0; s < p.ring; ++s) {
+        mbar_init(&full_bar[s], kDense ? 1 + p.stage_warps : 1);
+        mbar_init(&empty_bar[s], 1);
+      }
+      mbar_init(acc_bar, 1);
+      fence_barrier_init();
+      __threadfence_block();
+    }
+    __syncwarp();
+    named_barrier_arrive(2, kSmallThreads);
+  } else {
+    if (warp == 1) {
+      tmem_alloc<1>(tmem_base_slot, C::kTmemCols);
+    } else if constexpr (kDense) {
+      // the rows of this CTA's K range: one 128-byte line per thread and step
+      const int lines = (n_stages * C::kStageElems * static_cast<int>(sizeof(XT)) + 127) / 128;
+      const int pitch = p.K * static_cast<int>(sizeof(XT));
+      const int first = ks0 * C::kStageElems * static_cast<int>(sizeof(XT));
+      for (int m = warp - 2; m < p.M; m += kQuantWarps) {
+        for (int l = lane; l < lines; l += 32) {
+          if (first + l * 128 < pitch) prefetch_l2(static_cast<const uint8_t*>(p.x) + static_cast<int64_t>(m) * pitch + first + l * 128);
+        }
+      }
+    }
+    tc_fence_before_sync();
+    named_barrier_sync(2, kSmallThreads);
+    tc_fence_after_sync();
+    tmem_base = *tmem_base_slot;
+  }
+
+  float alpha = 1.0f;  // quantizer warps
+  if (warp == 0) {
+    // ------------------------------------------------------------------ weight loads
+    pdl_wait();
+    RingAt at(0);
+    for (int i = 0; i < n_stages; ++i, at.step(1, p.ring)) {
+      const int s = at.slot;
+      mbar_wait(&empty_bar[s], at.phase ^ 1, abort_flag);
+      if (elect_one()) {
+        const uint32_t sf_bytes = static_cast<uint32_t>(min(C::kSfTiles, sf_tiles - i * C::kSfTiles)) * 512u;
+        mbar_arrive_expect_tx(&full_bar[s], kDense ? kABytes + sf_bytes : kABytes + b_bytes + 2 * sf_bytes);
+        tma_load_2d(smem_a + s * kABytes, &map_w, &full_bar[s], (ks0 + i) * kStageKBytes, n0);
+        bulk_load_1d(smem_sfa + s * C::kSfBytes, w_scales + static_cast<int64_t>(i) * C::kSfTiles * 512, sf_bytes, &full_bar[s]);
+        if constexpr (!kDense) {
+          tma_load_2d(smem_b + s * b_bytes, &map_x, &full_bar[s], (ks0 + i) * kStageKBytes, 0);
+          bulk_load_1d(smem_sfb + s * C::kSfBytes, p.x_scales + static_cast<int64_t>(ks0 + i) * C::kSfTiles * 512, sf_bytes, &full_bar[s]);
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    pdl_wait();  // see ck_gemm_kernel.cuh: keeps the bounded waits from running out behind a long predecessor
+    const uint32_t a_lo0 = static_cast<uint32_t>(make_operand_desc_sw128(smem_u32(smem_a)));
+    const uint32_t b_lo0 = static_cast<uint32_t>(make_operand_desc_sw128(smem_u32(smem_b)));
+    const uint32_t op_hi = static_cast<uint32_t>(make_operand_desc_sw128(0) >> 32);
+    const uint32_t sfa_lo0 = static_cast<uint32_t>(make_scale_desc(smem_u32(smem_sfa)));
+    const uint32_t sfb_lo0 = static_cast<uint32_t>(make_scale_desc(smem_u32(smem_sfb)));
+    const uint32_t sf_hi = static_cast<uint32_t>(make_scale_desc(0) >> 32);
+    const int total_mma = (p.k_bytes + kMmaKBytes - 1) / kMmaKBytes - ks0 * kMmaPerStage;
+    RingAt at(0);
+    for (int i = 0; i < n_stages; ++i, at.step(1, p.ring)) {
+      const int s = at.slot;
+      mbar_wait(&full_bar[s], at.phase, abort_flag);
+      tc_fence_after_sync();
+      if (elect_one()) {
+        const uint32_t t_sfa = tmem_base + kMmaN + s * C::kSfCols, t_sfb = t_sfa + C::kSfTiles * 4;
+#pragma unroll
+        for (int t = 0; t < C::kSfTiles; ++t) {
+          tc_copy_scales_32x128b<1>(t_sfa + t * 4, desc64(sfa_lo0 + s * (C::kSfBytes >> 4) + t * 32, sf_hi));
+          tc_copy_scales_32x128b<1>(t_sfb + t * 4, desc64(sfb_lo0 + s * (C::kSfBytes >> 4) + t * 32, sf_hi));
+        }
+        const int n_mma = min(kMmaPerStage, total_mma - i * kMmaPerStage);
+#pragma unroll
+        for (int kb = 0; kb < kMmaPerStage; ++kb) {
+          if (kb < n_mma) {
+            const uint32_t accumulate = (i != 0 || kb != 0) ? 1u : 0u;
+            const uint64_t a_desc = desc64(a_lo0 + s * (kABytes >> 4) + kb * 2, op_hi);
+            const uint64_t b_desc = desc64(b_lo0 + s * (b_bytes >> 4) + kb * 2, op_hi);
+            if constexpr (KIND == Kind::kNvfp4) {
+              mma_nvfp4<1>(tmem_base, a_desc, b_desc, C::kIdesc, t_sfa + kb * 4, t_sfb + kb * 4, accumulate);
+            } else {
+              mma_mxfp8<1>(tmem_base, a_desc, b_desc, idesc_with_scale_ids(C::kIdesc, kb), t_sfa, t_sfb, accumulate);
+            }
+          }
+        }
+        tc_commit<1>(smem_u32(&empty_bar[s]));
+        if (i == n_stages - 1) tc_commit<1>(smem_u32(acc_bar));
+      }
+      __syncwarp();
+    }
+  } else {
+    // ------------------------------------------------------------------ quantizer, epilogue
+    pdl_wait();
+    const int qw = warp - 2, qt = threadIdx.x - 64;
+    if constexpr (kDense) {
+      float g = 1.0f;
+      if constexpr (KIND == Kind::kNvfp4) {
+        g = p.x_scale != nullptr ? ld_f32_dependent(p.x_scale) : dynamic_scale<XT>(p, qt, warp_max);
+        alpha = g * ld_f32_dependent(p.w_scale);
+      }
+      [[maybe_unused]] const quant::TensorScale ts = quant::make_tensor_scale(g);
+      // A group of stage_warps warps does every groups-th stage.  No more groups than slots: when a group comes to a stage, the
+      // one two rounds before it in its slot has then been used up (a wait by parity cannot tell a phase from the one two later).
+      const int groups = kQuantWarps / p.stage_warps;
+      const int group = qw / p.stage_warps, t_in_group = (qw % p.stage_warps) * 32 + lane;
+      const int unit = t_in_group % C::kRowThreads, row = t_in_group / C::kRowThreads;  // 16 elements of a row of the stage
+      const bool in_rows = row < p.M;
+      const XT* x = static_cast<const XT*>(p.x) + static_cast<int64_t>(in_rows ? row : 0) * p.K + static_cast<int64_t>(ks0) * C::kStageElems + unit * 16;
+      const int cols = p.K - ks0 * C::kStageElems - unit * 16;  // columns left from this thread's first element on
+      auto load_stage = [&](int i) { return load_sixteen<XT>(x + i * C::kStageElems, in_rows && i < n_stages && i * C::kStageElems < cols); };
+      const uint32_t data_at = row * kStageKBytes + (KIND == Kind::kNvfp4 ? (((unit >> 1) ^ (row & 7)) << 4) + (unit & 1) * 8 : (unit ^ (row & 7)) << 4);
+      const uint32_t scale_at = row * 16 + (KIND == Kind::kNvfp4 ? (unit >> 2) * 512 + (unit & 3) : unit >> 1);
+      Sixteen<XT> next = load_stage(group), after = load_stage(group + groups);  // the loads run two stages ahead
+      RingAt at(group);
+      for (int i = group; i < n_stages; i += groups, at.step(groups, p.ring)) {
+        const int s = at.slot;
+        const Sixteen<XT> now = next;
+        next = after;
+        after = load_stage(i + 2 * groups);
+        if constexpr (KIND == Kind::kNvfp4) {
+          uint32_t lo, hi, scale;
+          if constexpr (sizeof(XT) == 2) {
+            quant::nvfp4_block_packed<XT, true>(now.v[0].w, ts, lo, hi, scale);
+          } else {
+            float v[16];
+            widen_sixteen(now, v);
+            quant::nvfp4_block<true>(v, g, true, lo, hi, scale);
+          }
+          if (i * C::kStageElems >= cols) lo = hi = scale = 0;  // past K: the last MMA may reach there
+          mbar_wait(&empty_bar[s], at.phase ^ 1, abort_flag);
+          if (in_rows) {
+            *reinterpret_cast<uint2*>(smem_b + s * b_bytes + data_at) = make_uint2(lo, hi);
+            smem_sfb[s * C::kSfBytes + scale_at] = static_cast<uint8_t>(scale);
+          }
+        } else {
+          float v[16];
+          widen_sixteen(now, v);
+          float amax = quant::amax16(v);
+          amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));  // the block's other half
+          const quant::Mxfp8Scale sc = quant::mxfp8_scale(amax);
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) w[j] = quant::mxfp8_four(v + 4 * j, sc);
+          mbar_wait(&empty_bar[s], at.phase ^ 1, abort_flag);
+          if (in_rows) {
+            *reinterpret_cast<uint4*>(smem_b + s * b_bytes + data_at) = make_uint4(w[0], w[1], w[2], w[3]);
+            if ((unit & 1) == 0) smem_sfb[s * C::kSfBytes + scale_at] = static_cast<uint8_t>(sc.byte);
+          }
+        }
+        fence_proxy_async();  // what was written becomes visible to the tensor cores' reads
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_bar[s]);
+      }
+    } else {
+      if (p.alpha != nullptr) {
+        alpha = ld_f32_dependent(p.alpha);
+      } else if (p.x_scale != nullptr && p.w_scale != nullptr) {
+        alpha = ld_f32_dependent(p.x_scale) * ld_f32_dependent(p.w_scale);
+      }
+    }
+    // ---- epilogue: lane = weight row (output column), accumulator columns = activation rows, 16 to a warp
+    const int quarter = warp & 3, m0 = (qw >> 2) * 16;
+    const int r = quarter * 32 + lane, n = n0 + r;
+    if (m0 < p.M) {
+      float bias = 0.0f;
+      if (!SPLIT && p.bias != nullptr && n < p.N) bias = load_bias(p.bias, p.bias_dtype, n);
+      mbar_wait(acc_bar, 0, abort_flag);
+      tc_fence_after_sync();
+      uint32_t acc[16];
+      tmem_load_32x16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + m0, acc);
+      tmem_load_wait();
+      if constexpr (SPLIT) {
+        float* partial = reinterpret_cast<float*>(smem) + m0 * kTileM + r;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          if (m0 + c < p.M) partial[c * kTileM] = __uint_as_float(acc[c]);
+        }
+      } else if (n < p.N) {
+        const int64_t at = static_cast<int64_t>(m0) * p.N + n;
+        switch (p.out_dtype) {
+          case CK_DTYPE_BF16: store_columns(static_cast<__nv_bfloat16*>(p.out) + at, p.N, acc, alpha, bias, p.M - m0); break;
+          case CK_DTYPE_F16: store_columns(static_cast<__half*>(p.out) + at, p.N, acc, alpha, bias, p.M - m0); break;
+          default: store_columns(static_cast<float*>(p.out) + at, p.N, acc, alpha, bias, p.M - m0);
+        }
+      }
+    }
+  }
+
+  if constexpr (SPLIT) {
+    // the CTAs of the cluster add their partial tiles in split order (ck_gemm_kernel.cuh)
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 2) {
+      uint32_t base[kMaxSplits];
+#pragma unroll
+      for (int i = 0; i < kMaxSplits; ++i) base[i] = map_to_cta(smem_u32(smem), i < p.splits ? i : 0);
+      switch (p.out_dtype) {
+        case CK_DTYPE_BF16: add_cluster_tile(p, static_cast<__nv_bfloat16*>(p.out), base, rank, warp - 2, lane, n0, alpha); break;
+        case CK_DTYPE_F16: add_cluster_tile(p, static_cast<__half*>(p.out), base, rank, warp - 2, lane, n0, alpha); break;
+        default: add_cluster_tile(p, static_cast<float*>(p.out), base, rank, warp - 2, lane, n0, alpha);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // no CTA leaves while another may still read its partial
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {
+    if (threadIdx.x == 0) atomicExch(p.status, 1);
+    // give copies that may still be in flight time to land before the CTA's memory is released
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc<1>(tmem_base, C::kTmemCols);
+  }
+}
+
+struct SmallPlan {
+  int splits;        // CTAs that share a tile's K range
+  bool two_per_sm;   // some SMs get two CTAs at once
+};
+
+// Clusters of `splits` CTAs that run at once with one CTA on an SM (the request for shared memory sees to that).
+template <Kind KIND>
+int clusters_of(int splits, int* out) {
+  static std::atomic<int> cached[64][kMaxSplits + 1];
+  int dev = 0;
+  CK_CUDA(cudaGetDevice(&dev));
+  int n = (dev >= 0 && dev < 64) ? cached[dev][splits].load(std::memory_order_relaxed) : 0;
+  if (n == 0) {
+    constexpr int kMoreThanHalf = 128 * 1024;
+    auto kernel = small_m_kernel<KIND, void, true>;
+    CK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.gridDim = dim3(static_cast<unsigned>(splits), static_cast<unsigned>(sm_count() / splits));
+    cfg.dynamicSmemBytes = kMoreThanHalf;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CK_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+    if (n < 1) n = 1;
+    if (dev >= 0 && dev < 64) cached[dev][splits].store(n, std::memory_order_relaxed);
+  }
+  *out = n;
+  return CK_OK;
+}
 
 // CTAs per tile (1 = no split).  The most whose clusters all run at once with one CTA on an SM; with two on an SM
-// when that leaves a CTA more than ten stages.  (The occupancy query counts one for every kernel that allocates
-// tensor memory; two of this configuration share an SM.  A cluster that finds no room runs later: nobody waits for
+// when that leaves a CTA more than ten stages.  (A cluster that finds no room runs later: nobody waits for
 // it.)  Graph replays, us, few CTAs of many stages / more: NVFP4 32 x 4096 x 12288 (12 stages / 8) 8.9 / 8.0,
 // 1 x 6144 x 8192 (16 / 7) 8.9 / 8.1, 1 x 6144 x 6144 (12 / 5) 7.6 / 7.6, MXFP8 32 x 6144 x 12288 (48 / 20) 18.3 / 11.7,
 // 1 x 4096 x 12288 (24 / 16) 10.9 / 9.6; but NVFP4 1 x 4096 x 8192 (8 / 6) 6.6 / 7.1, 1 x 6144 x 4096 (8 / 4) 6.2 / 6.4.
-template <Kind KIND, typename OutT>
-int choose_splits(int64_t N, int k_bytes, int* out) {
+template <Kind KIND>
+int choose_plan(int64_t N, int k_bytes, SmallPlan* plan) {
   const int k_stages = static_cast<int>(ceil_div(k_bytes, kStageKBytes));
   const int64_t tiles = ceil_div(N, kTileM);
   const int most = small_m_max_splits(N, k_bytes);
@@ -33,36 +521,108 @@ int choose_splits(int64_t N, int k_bytes, int* out) {
   for (int per_sm = 1; per_sm <= 2; ++per_sm) {
     for (splits = most; splits > 1; --splits) {
       int clusters = 0;
-      if (int rc = split_clusters<KIND, kSmallTileN, 2, 4, OutT, 0, true>(splits, &clusters)) return rc;
+      if (int rc = clusters_of<KIND>(splits, &clusters)) return rc;
       if (clusters * per_sm >= tiles) break;
     }
     if (ceil_div(k_stages, splits) <= kMaxStagesAlone) break;
   }
-  *out = static_cast<int>(ceil_div(k_stages, ceil_div(k_stages, splits)));  // none without a stage
+  plan->splits = static_cast<int>(ceil_div(k_stages, ceil_div(k_stages, splits)));  // none without a stage
+  int alone = 0;
+  if (int rc = clusters_of<KIND>(plan->splits, &alone)) return rc;
+  plan->two_per_sm = tiles > alone;
   return CK_OK;
 }
 
-template <Kind KIND, typename OutT>
-int launch_small(const Operands& ops, GemmParams p, cudaStream_t stream) {
-  OutputSpec os;
-  void* const single[1] = {p.out};
-  os.ptrs = single;
-  os.n = 1;
-  os.pitch = p.N;
-  os.col_offset = 0;
-  if (int rc = choose_splits<KIND, OutT>(p.M, p.k_bytes, &p.splits)) return rc;
-  p.k_stages_per_split = static_cast<int>(ceil_div(ceil_div(p.k_bytes, kStageKBytes), p.splits));
-  if (p.splits == 1) return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true>(ops, p, os, stream);
-  // a quarter tile of one activation row per warp of the cluster, if there are warps enough for all of them
-  if (4 * p.N <= p.splits * epilogue_warps(false, kSmallTileN)) {
-    return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true, Split::kCluster>(ops, p, os, stream);
+template <Kind KIND, typename XT, bool SPLIT>
+int launch_as(const void* w, const void* codes, const SmallParams& p, cudaStream_t stream) {
+  using C = Small<KIND>;
+  auto kernel = small_m_kernel<KIND, XT, SPLIT>;
+  CUtensorMap map_w, map_x = {};
+  if (int rc = make_operand_map(&map_w, w, p.N, p.k_bytes, kTileM)) return rc;
+  if (std::is_void<XT>::value) {
+    if (int rc = make_operand_map(&map_x, codes, p.M, p.k_bytes, p.x_rows)) return rc;
   }
-  return launch_config<KIND, kSmallTileN, 2, 4, 1, OutT, false, 0, true, Split::kClusterManyRows>(ops, p, os, stream);
+  const int smem = C::smem_bytes(p.ring, p.x_rows);
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  CK_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+    CK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
+    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.splits), static_cast<unsigned>(ceil_div(p.N, kTileM)));
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n_attrs = 0;
+  if (SPLIT) {
+    attr[n_attrs].id = cudaLaunchAttributeClusterDimension;
+    attr[n_attrs].val.clusterDim.x = p.splits;
+    attr[n_attrs].val.clusterDim.y = 1;
+    attr[n_attrs++].val.clusterDim.z = 1;
+  }
+  if (pdl_enabled()) {
+    attr[n_attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n_attrs;
+  CK_CUDA(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p));
+  return CK_OK;
+}
+
+template <Kind KIND, typename XT>
+int launch(const void* w, const void* codes, SmallParams p, cudaStream_t stream) {
+  SmallPlan plan = {};
+  if (int rc = choose_plan<KIND>(p.N, p.k_bytes, &plan)) return rc;
+  p.splits = plan.splits;
+  p.k_stages_per_split = static_cast<int>(ceil_div(ceil_div(p.k_bytes, kStageKBytes), p.splits));
+  p.x_rows = p.M <= 16 ? 16 : 32;
+  constexpr int kTwoToAnSm = 228 * 1024 / 2 - 1024 /*reserved*/ - 512 /*barriers, maxima*/;
+  static_assert(Small<KIND>::smem_bytes(5, 16) <= kTwoToAnSm && Small<KIND>::smem_bytes(4, 32) <= kTwoToAnSm, "two CTAs to an SM");
+  static_assert(Small<KIND>::smem_bytes(7, 32) <= kMaxSmemBytes, "one CTA to an SM");
+  // Alone on its SM a CTA gets all the stages that tensor memory has columns for; where two share an SM, what leaves room for
+  // both (MXFP8 8 x 18432 x 6144, us: four stages 22.7, five 21.9, seven 20.5; NVFP4 16 x 18432 x 12288 24.1 / 23.5 / 22.0, 8 x 9216
+  // x 3072 6.40 / 6.13 / 5.92; but MXFP8 8 x 3072 x 12288, eight CTAs to a tile, 10.4 / 10.3 / 15.3).
+  p.ring = !plan.two_per_sm ? 7 : p.x_rows == 16 ? 5 : 4;
+  // Weight boxes asked from L2 ahead of the dependency wait.  Few: the requests queue in front of the loads in the TMA unit
+  // (NVFP4 8 x 18432 x 3072 from a dense activation: none 8.56 us, two 8.41, four 8.69, sixteen 9.44; lines asked by the idle
+  // quantizer threads instead, twelve boxes' worth, 9.81; quantized, sixteen instead of four 10.4 against 8.9).
+  p.prefetch = std::is_void<XT>::value ? 4 : 2;
+  // a thread takes 16 elements: 16 (NVFP4) or 8 (MXFP8) threads to a row of a stage
+  const int stage_warps = static_cast<int>(ceil_div(p.M * Small<KIND>::kRowThreads, 32));
+  p.stage_warps = stage_warps <= 2 ? 2 : stage_warps <= 4 ? 4 : 8;
+  if (int rc = gemm_status_word(&p.status)) return rc;
+  return p.splits > 1 ? launch_as<KIND, XT, true>(w, codes, p, stream) : launch_as<KIND, XT, false>(w, codes, p, stream);
+}
+
+template <typename XT>
+int launch(bool is_mxfp8, const void* w, const void* codes, const SmallParams& p, cudaStream_t s) {
+  return is_mxfp8 ? launch<Kind::kMxfp8, XT>(w, codes, p, s) : launch<Kind::kNvfp4, XT>(w, codes, p, s);
+}
+
+SmallParams params_of(bool is_mxfp8, const void* w_scales, const float* w_scale, const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M,
+                      int64_t N, int64_t K) {
+  SmallParams p{};
+  p.w_scales = static_cast<const uint8_t*>(w_scales);
+  p.w_scale = w_scale;
+  p.bias = bias;
+  p.out = out;
+  p.bias_dtype = bias_dtype;
+  p.out_dtype = out_dtype;
+  p.M = static_cast<int>(M);
+  p.N = static_cast<int>(N);
+  p.K = static_cast<int>(K);
+  p.k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
+  p.sf_col_tiles = static_cast<int>(ceil_div(K / (is_mxfp8 ? 32 : 16), 4));
+  return p;
 }
 
 }  // namespace
 
-bool small_m_applies(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= kMaxSmallM && N >= 1 && K >= 32; }
+bool small_m_applies(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= kMaxSmallM && N >= 1 && N <= 65535ll * kTileM && K >= 32; }
 
 // CTAs per 128-row weight tile (1 = no split): as many as let two CTAs run on every SM and leave each
 // of them four pipeline stages.
@@ -76,72 +636,53 @@ int small_m_max_splits(int64_t N, int k_bytes) {
   return max(splits, 1);
 }
 
-int small_m_splits(bool is_mxfp8, int out_dtype, int64_t N, int k_bytes, int* splits) {
-  if (is_mxfp8) {
-    switch (out_dtype) {
-      case CK_DTYPE_BF16: return choose_splits<Kind::kMxfp8, __nv_bfloat16>(N, k_bytes, splits);
-      case CK_DTYPE_F16: return choose_splits<Kind::kMxfp8, __half>(N, k_bytes, splits);
-      default: return choose_splits<Kind::kMxfp8, float>(N, k_bytes, splits);
-    }
-  }
-  switch (out_dtype) {
-    case CK_DTYPE_BF16: return choose_splits<Kind::kNvfp4, __nv_bfloat16>(N, k_bytes, splits);
-    case CK_DTYPE_F16: return choose_splits<Kind::kNvfp4, __half>(N, k_bytes, splits);
-    default: return choose_splits<Kind::kNvfp4, float>(N, k_bytes, splits);
-  }
+int small_m_splits(bool is_mxfp8, int64_t N, int k_bytes, int* splits) {
+  SmallPlan plan = {};
+  const int rc = is_mxfp8 ? choose_plan<Kind::kMxfp8>(N, k_bytes, &plan) : choose_plan<Kind::kNvfp4>(N, k_bytes, &plan);
+  *splits = plan.splits;
+  return rc;
 }
 
 // a: activation [M, K], b: weight [N, K] (the public argument order); shapes and pointers were validated by the caller.
 int scaled_mm_small_m(bool is_mxfp8, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
                       const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
                       int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
-  const int block = is_mxfp8 ? 32 : 16;
-  GemmParams p{};
-  // operands change places: the kernel's "A" is the weight
-  p.sfa = static_cast<const uint8_t*>(sfb);
-  p.sfb = static_cast<const uint8_t*>(sfa);
-  p.tsa = tsa;
-  p.tsb = tsb;
+  SmallParams p = params_of(is_mxfp8, sfb, tsb, bias, bias_dtype, out, out_dtype, M, N, K);
+  p.x_scales = static_cast<const uint8_t*>(sfa);
+  p.x_scale = tsa;
   p.alpha = alpha;
-  p.bias = bias;
-  p.out = out;
-  p.bias_dtype = bias_dtype;
-  p.out_dtype = out_dtype;
-  p.M = static_cast<int>(N);
-  p.N = static_cast<int>(M);
-  p.k_bytes = static_cast<int>(is_mxfp8 ? K : K / 2);
-  p.sf_col_tiles = static_cast<int>(ceil_div(K / block, 4));
-  p.n_row_blocks_a = static_cast<int>(ceil_div(N, 128));
-  p.n_row_blocks_b = static_cast<int>(ceil_div(M, 128));
-  if (int rc = gemm_status_word(&p.status)) return rc;
-  p.splits = 1;
-  const Operands ops = {b, a};
-  if (is_mxfp8) {
-    switch (out_dtype) {
-      case CK_DTYPE_BF16: return launch_small<Kind::kMxfp8, __nv_bfloat16>(ops, p, stream);
-      case CK_DTYPE_F16: return launch_small<Kind::kMxfp8, __half>(ops, p, stream);
-      default: return launch_small<Kind::kMxfp8, float>(ops, p, stream);
-    }
-  }
-  switch (out_dtype) {
-    case CK_DTYPE_BF16: return launch_small<Kind::kNvfp4, __nv_bfloat16>(ops, p, stream);
-    case CK_DTYPE_F16: return launch_small<Kind::kNvfp4, __half>(ops, p, stream);
-    default: return launch_small<Kind::kNvfp4, float>(ops, p, stream);
+  return launch<void>(is_mxfp8, b, a, p, stream);
+}
+
+// What is quantized inside the GEMM; everything else, wrong arguments among it, is left to the separate calls.
+bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const void* w, const void* w_scales, int bias_dtype, int out_dtype,
+                            int64_t M, int64_t N, int64_t K) {
+  auto aligned = [](const void* p, uintptr_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; };
+  auto is_float = [](int dtype) { return dtype == CK_DTYPE_F32 || dtype == CK_DTYPE_F16 || dtype == CK_DTYPE_BF16; };
+  // Up to 8 rows of NVFP4 and 16 of MXFP8, whose rows take half the threads, the quantizer's warps keep up with the stream.
+  // Quantizer + GEMM / one kernel, us: NVFP4 static scale 8 x 18432 x 3072 9.9 / 8.5, 8 x 3072 x 3072 8.0 / 6.6, but 10 x 3072 x 3072 8.7 / 9.2,
+  // 16 x 6144 x 3072 9.2 / 10.2; MXFP8 16 x 3072 x 3072 7.3 / 5.8, 16 x 18432 x 12288 42.8 / 41.9.
+  const int64_t limit = is_mxfp8 ? 16 : 8;
+  const int forced = forced_gemm_config();
+  return M <= limit && small_m_applies(M, N, K) && N % 8 == 0 && K % 32 == 0 && K <= (1 << 28) && is_float(x_dtype) && is_float(out_dtype) &&
+         is_float(bias_dtype) && aligned(x, 32) && aligned(w, 16) && aligned(w_scales, 16) && !exact_division() && (forced == 0 || forced == 9);
+}
+
+// `partials`: maxima of a reduction pass for a dynamic scale, or null (every CTA reads all of x).
+int linear_small_m(bool is_mxfp8, const void* x, int x_dtype, const float* x_scale, const float* partials, int n_partials, const void* w,
+                   const void* w_scales, const float* w_scale, const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M,
+                   int64_t N, int64_t K, cudaStream_t stream) {
+  SmallParams p = params_of(is_mxfp8, w_scales, w_scale, bias, bias_dtype, out, out_dtype, M, N, K);
+  p.x = x;
+  p.x_scale = x_scale;
+  p.partials = partials;
+  p.n_partials = n_partials;
+  p.n_vecs = static_cast<int>(M * K / (x_dtype == CK_DTYPE_F32 ? 8 : 16));
+  switch (x_dtype) {
+    case CK_DTYPE_BF16: return launch<__nv_bfloat16>(is_mxfp8, w, nullptr, p, stream);
+    case CK_DTYPE_F16: return launch<__half>(is_mxfp8, w, nullptr, p, stream);
+    default: return launch<float>(is_mxfp8, w, nullptr, p, stream);
   }
 }
 
 }  // namespace ck
-
-#ifdef CK_GEMM_TRACE
-// Timeline buffers of this translation unit's kernels (see gemm_timeline.py --small-m).
-extern "C" __attribute__((visibility("default"))) int ck_debug_trace_smallm(long long* host_out) {
-  CK_CUDA(cudaDeviceSynchronize());
-  CK_CUDA(cudaMemcpyFromSymbol(host_out, ck::g_trace, sizeof(long long) * 160 * ck::kTraceTiles * ck::kTraceSlots));
-  return CK_OK;
-}
-extern "C" __attribute__((visibility("default"))) int ck_debug_trace3_smallm(long long* host_out) {
-  CK_CUDA(cudaDeviceSynchronize());
-  CK_CUDA(cudaMemcpyFromSymbol(host_out, ck::g_trace3, sizeof(long long) * 8 * 160 * 8));
-  return CK_OK;
-}
-#endif

@@ -15,6 +15,9 @@ struct FromFloatLayout {
 };
 
 // Workspace layout: tensor-scale scratch | dynamic tensor scale | codes [M, K/2] | tiled block scales.
+// Few rows, quantized inside the GEMM: up to here every CTA takes the maximum of the whole activation itself (the quantizers' line
+// for the same choice, ck_quantize.cu); beyond it a reduction kernel leaves partial maxima.
+constexpr int64_t kSmallLinearWholeInputBytes = 64 * 1024;
 constexpr int64_t kScaleScratchBytes = 256 + 256 * 1024;  // 2^30 elements: 65536 partials behind the head
 
 FromFloatLayout from_float_layout(int64_t M, int64_t K) {
@@ -55,6 +58,17 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   uint8_t* codes = ws + l.codes_off;
   uint8_t* scales = ws + l.scales_off;
+  if (linear_small_m_applies(false, x, x_dtype, w_codes, w_block_scales, bias == nullptr ? out_dtype : bias_dtype, out_dtype, M, N, K)) {
+    const int64_t elem = x_dtype == CK_DTYPE_F32 ? 4 : 2;
+    float* partials = nullptr;
+    int n_partials = 0;
+    if (dynamic && M * K * elem > kSmallLinearWholeInputBytes) {
+      partials = reinterpret_cast<float*>(ws + l.scratch_off);
+      if (int rc = launch_amax_partials(x, x_dtype, M * K * elem / 32, partials, &n_partials, static_cast<cudaStream_t>(stream))) return rc;
+    }
+    return linear_small_m(false, x, x_dtype, x_scale, partials, n_partials, w_codes, w_block_scales, w_scale, bias, bias_dtype, out, out_dtype,
+                          M, N, K, static_cast<cudaStream_t>(stream));
+  }
   const float* scale = x_scale;
   if (dynamic) {
     float* dyn = reinterpret_cast<float*>(ws + l.scale_off);
@@ -88,6 +102,10 @@ extern "C" int ck_linear_mxfp8_from_float(const void* x, int x_dtype, const void
   const int64_t need = ck_linear_mxfp8_from_float_workspace_bytes(M, K);
   CK_REQUIRE(workspace_bytes >= need, "linear_mxfp8_from_float: workspace of %lld bytes, %lld needed",
              (long long)workspace_bytes, (long long)need);
+  if (linear_small_m_applies(true, x, x_dtype, w_data, w_block_scales, bias == nullptr ? out_dtype : bias_dtype, out_dtype, M, N, K)) {
+    return linear_small_m(true, x, x_dtype, nullptr, nullptr, 0, w_data, w_block_scales, nullptr, bias, bias_dtype, out, out_dtype, M, N, K,
+                          static_cast<cudaStream_t>(stream));
+  }
   uint8_t* data = static_cast<uint8_t*>(workspace);
   uint8_t* scales = data + round_up(M * K, 256);
   if (int rc = ck_quantize_mxfp8(x, x_dtype, data, scales, M, K, M, K, stream)) return rc;

@@ -327,6 +327,60 @@ __device__ __forceinline__ void nvfp4_block_packed(const uint32_t (&w)[8], const
 }
 
 // ---------------------------------------------------------------------------
+// MXFP8 (comfy_kitchen/backends/eager/quantization.py:292-318)
+// ---------------------------------------------------------------------------
+// clamp(ceil(log2(r)) + 127, 0, 254) for r >= 2^-127, from the bits of r
+// (comfy_kitchen/backends/eager/quantization.py:295-300).  r = amax/448 with amax an
+// f16/bf16 number is either an exact power of two or far enough from one that the
+// reference's float32 log2 cannot round across an integer, so this integer form is
+// bit-identical for those input types.
+__device__ __forceinline__ uint32_t e8m0_ceil_exponent(float r) {
+  const uint32_t bits = __float_as_uint(r);
+  const uint32_t e = bits >> 23;  // r > 0
+  const uint32_t frac = bits & 0x7FFFFFu;
+  uint32_t biased;
+  if (e == 0) {
+    biased = frac > 0x400000u ? 1u : 0u;  // [2^-127, 2^-126): exactly 2^-127 -> 0
+  } else {
+    biased = e + (frac != 0u);
+  }
+  return min(biased, 254u);
+}
+
+// What a block of 32 elements with the largest magnitude `amax` is multiplied by, and its scale byte.
+struct Mxfp8Scale {
+  float inv;
+  uint32_t byte;
+  bool dead;  // an all-zero block
+};
+__device__ __forceinline__ Mxfp8Scale mxfp8_scale(float amax) {
+  const float need = fmaxf(__fdiv_rn(amax, 448.0f), 0x1p-127f);  // :294-295
+  const uint32_t e = e8m0_ceil_exponent(need);                   // :298-302
+  Mxfp8Scale s;
+  s.dead = (amax == 0.0f);  // :306
+  // :303-310: divide by 2^(e-127).  For e in [1, 253] that is an exact multiplication by
+  // 2^(127-e); e == 254 needs the subnormal 2^-127; e == 0 decodes to a zero scale and
+  // the reference divides by zero (inputs below 448 * 2^-127, outside the pinned domain).
+  if (e == 0) {
+    s.inv = __int_as_float(0x7F800000);
+  } else if (e == 254) {
+    s.inv = 0x1p-127f;
+  } else {
+    s.inv = __uint_as_float((254u - e) << 23);
+  }
+  if (s.dead) s.inv = 0.0f;  // :307,311 -> all zeros (positive)
+  s.byte = s.dead ? 0u : e;  // :318
+  return s;
+}
+
+// Four elements -> four E4M3 bytes; :314-315 clamp to +-448 and round to E4M3: satfinite performs the clamp
+__device__ __forceinline__ uint32_t mxfp8_four(const float* v, const Mxfp8Scale& s) {
+  const uint32_t lo = f32x2_to_e4m3x2(s.dead ? 0.0f : v[1] * s.inv, s.dead ? 0.0f : v[0] * s.inv);
+  const uint32_t hi = f32x2_to_e4m3x2(s.dead ? 0.0f : v[3] * s.inv, s.dead ? 0.0f : v[2] * s.inv);
+  return lo | (hi << 16);
+}
+
+// ---------------------------------------------------------------------------
 // dynamic per-tensor scale
 // ---------------------------------------------------------------------------
 template <typename T>

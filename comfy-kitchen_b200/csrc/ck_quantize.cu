@@ -290,24 +290,6 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
 // ---------------------------------------------------------------------------
 // MXFP8
 // ---------------------------------------------------------------------------
-// clamp(ceil(log2(r)) + 127, 0, 254) for r >= 2^-127, from the bits of r
-// (comfy_kitchen/backends/eager/quantization.py:295-300).  r = amax/448 with amax an
-// f16/bf16 number is either an exact power of two or far enough from one that the
-// reference's float32 log2 cannot round across an integer, so this integer form is
-// bit-identical for those input types.
-__device__ __forceinline__ uint32_t e8m0_ceil_exponent(float r) {
-  const uint32_t bits = __float_as_uint(r);
-  const uint32_t e = bits >> 23;  // r > 0
-  const uint32_t frac = bits & 0x7FFFFFu;
-  uint32_t biased;
-  if (e == 0) {
-    biased = frac > 0x400000u ? 1u : 0u;  // [2^-127, 2^-126): exactly 2^-127 -> 0
-  } else {
-    biased = e + (frac != 0u);
-  }
-  return min(biased, 254u);
-}
-
 // kVec: whole aligned blocks, unpadded columns.  kPadRows: rows past orig_rows are zeros.
 template <typename T, bool kVec, bool kPadRows>
 __global__ void __launch_bounds__(kThreads)
@@ -340,41 +322,24 @@ quantize_mxfp8_kernel(const T* x, uint8_t* __restrict__ data, uint8_t* __restric
       load16_guarded(x, row, sc * 32 + 16, orig_rows, orig_cols, hi);
     }
     const float amax = fmaxf(amax16(lo), amax16(hi));          // :292
-    const float need = fmaxf(__fdiv_rn(amax, 448.0f), 0x1p-127f);  // :294-295
-    const uint32_t e = e8m0_ceil_exponent(need);               // :298-302
-    const bool dead = (amax == 0.0f);                          // :306
-    // :303-310: divide by 2^(e-127).  For e in [1, 253] that is an exact multiplication by
-    // 2^(127-e); e == 254 needs the subnormal 2^-127; e == 0 decodes to a zero scale and
-    // the reference divides by zero (inputs below 448 * 2^-127, outside the pinned domain).
-    float inv;
-    if (e == 0) {
-      inv = __int_as_float(0x7F800000);
-    } else if (e == 254) {
-      inv = 0x1p-127f;
-    } else {
-      inv = __uint_as_float((254u - e) << 23);
-    }
-    if (dead) inv = 0.0f;  // :307,311 -> all zeros (positive)
+    const Mxfp8Scale scale = mxfp8_scale(amax);
     Vec256 out;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      // :314-315 clamp to +-448 and round to E4M3: satfinite performs the clamp
-      const uint32_t p0 = f32x2_to_e4m3x2(dead ? 0.0f : lo[4 * i + 1] * inv, dead ? 0.0f : lo[4 * i] * inv);
-      const uint32_t p1 = f32x2_to_e4m3x2(dead ? 0.0f : lo[4 * i + 3] * inv, dead ? 0.0f : lo[4 * i + 2] * inv);
-      out.w[i] = p0 | (p1 << 16);
-      const uint32_t p2 = f32x2_to_e4m3x2(dead ? 0.0f : hi[4 * i + 1] * inv, dead ? 0.0f : hi[4 * i] * inv);
-      const uint32_t p3 = f32x2_to_e4m3x2(dead ? 0.0f : hi[4 * i + 3] * inv, dead ? 0.0f : hi[4 * i + 2] * inv);
-      out.w[4 + i] = p2 | (p3 << 16);
+      out.w[i] = mxfp8_four(lo + 4 * i, scale);
+      out.w[4 + i] = mxfp8_four(hi + 4 * i, scale);
     }
     st_global_256(data + row * num_cols + sc * 32, out);
-    scale_byte = dead ? 0u : e;  // :318
+    scale_byte = scale.byte;
   }
   store_scale_quad(scales, row, sc, sc_pad >> 2, scale_byte, sc < sc_pad);
 }
 
 std::atomic<int> g_exact_division{-1};  // -1: not set, follow CK_EXACT_DIV
 
-bool use_exact_division() {
+}  // namespace
+
+bool exact_division() {
   const int v = g_exact_division.load(std::memory_order_relaxed);
   if (v >= 0) return v != 0;
   // CK_EXACT_DIV=1 forces __fdiv_rn for every element (validation of the fast quotient).
@@ -385,13 +350,15 @@ bool use_exact_division() {
   return env;
 }
 
+namespace {
+
 // The streaming kernel takes rows of whole 64-byte units (rows may be padded, columns not), with
 // aligned input and codes.
 template <typename T>
 bool streaming_applies(const void* input, const void* codes, int64_t orig_rows, int64_t orig_cols, int64_t num_rows, int64_t num_cols) {
   return orig_cols == num_cols && orig_rows <= num_rows && num_cols % (64 / static_cast<int64_t>(sizeof(T))) == 0 &&
          reinterpret_cast<uintptr_t>(input) % 32 == 0 && reinterpret_cast<uintptr_t>(codes) % 16 == 0 &&
-         num_rows < (1 << 30) && num_cols < (1 << 30) && !use_exact_division();
+         num_rows < (1 << 30) && num_cols < (1 << 30) && !exact_division();
 }
 
 template <typename T, bool kDynamic, bool kMark>
@@ -460,7 +427,7 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
   // vector path: every 16-element run is inside the input and 32-byte aligned
   const bool vec = (orig_rows == num_rows) && (orig_cols == num_cols) &&
                    (reinterpret_cast<uintptr_t>(input) % 32 == 0);
-  const bool exact = use_exact_division();
+  const bool exact = exact_division();
 #define CK_LAUNCH(VEC, FAST)                                                                                  \
   CK_CUDA(launch_pdl(quantize_nvfp4_kernel<T, VEC, FAST>, grid, block, 0, stream, x, gs, c, s, orig_rows, orig_cols, \
                      num_rows, num_cols, sc_pad, hi_first))
@@ -563,7 +530,7 @@ int check_quant_shapes(const char* op, int64_t block, const void* input, const v
 }  // namespace ck
 
 extern "C" int ck_debug_set_exact_division(int on) {
-  const bool before = ck::use_exact_division();
+  const bool before = ck::exact_division();
   ck::g_exact_division.store(on != 0 ? 1 : 0, std::memory_order_relaxed);
   return before ? 1 : 0;
 }

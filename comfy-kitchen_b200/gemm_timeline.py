@@ -79,8 +79,7 @@ def run(shape: str, ring: int, verbose: bool) -> None:
 
     need = int(lib.ck_scaled_mm_workspace_bytes(0, mp, n, k))
     ws = torch.empty(max(need, 16), dtype=torch.uint8, device=dev)
-    small = m <= 32  # the weight-streaming path lives in its own translation unit, with its own buffers
-    suffix = "_smallm" if small else ""
+    assert m > 32, "the weight-streaming kernel of up to 32 rows keeps no timeline"
 
     def launch(i, st):
         j = i % ring
@@ -111,7 +110,7 @@ def run(shape: str, ring: int, verbose: bool) -> None:
 
     # ---- per launch and CTA: global timer and SM clock at entry / set-up done / dependency wait done / end
     stamps = np.zeros((8, 160, 4, 2), dtype=np.int64)
-    trace3 = getattr(lib, "ck_debug_trace3" + suffix)
+    trace3 = lib.ck_debug_trace3
     trace3.argtypes = [ctypes.c_void_p]
     assert trace3(stamps.ctypes.data) == 0
     ncta = int((stamps[0, :, 0, 0] != 0).sum())
@@ -135,7 +134,7 @@ def run(shape: str, ring: int, verbose: bool) -> None:
 
     # ---- per tile (SM clock, last launch)
     tiles = np.zeros((160, 40, 16), dtype=np.int64)
-    trace = getattr(lib, "ck_debug_trace" + suffix)
+    trace = lib.ck_debug_trace
     trace.argtypes = [ctypes.c_void_p]
     assert trace(tiles.ctypes.data) == 0
     slots = ["mma:acc_wait", "mma:acc_free", "mma:first_stage", "mma:last_stage", "tma:first", "tma:last", "epi:wait", "epi:acc_full",
@@ -154,7 +153,7 @@ def run(shape: str, ring: int, verbose: bool) -> None:
             if not row.any():
                 break
             print(f"  tile {t}: " + "  ".join(f"{nm}={(int(v) - int(base)) & 0xFFFFFFFF}" for nm, v in zip(slots, row) if v))
-    if verbose and not small:
+    if verbose:
         per_stage = np.zeros((160, 4, 64), dtype=np.int64)
         lib.ck_debug_trace2.argtypes = [ctypes.c_void_p]
         assert lib.ck_debug_trace2(per_stage.ctypes.data) == 0
