@@ -79,33 +79,18 @@ struct Small {
   static_assert(kMaxSmallM * kTileM * 4 <= 4 * kTileM * kStageKBytes, "a partial tile fits in the weight's slots");
 };
 
-// 16 elements of the activation
 template <typename T>
-struct Sixteen {
-  Vec256 v[sizeof(T) / 2];
-};
-
-template <typename T>
-__device__ __forceinline__ Sixteen<T> load_sixteen(const T* p, bool valid) {
-  Sixteen<T> r = {};
+__device__ __forceinline__ quant::Sixteen<T> load_sixteen(const T* p, bool valid) {
+  quant::Sixteen<T> r = {};
   if (valid) {
-    r.v[0] = ld_global_stream_256(p);
-    if constexpr (sizeof(T) == 4) r.v[1] = ld_global_stream_256(p + 8);
-  }
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ void widen_sixteen(const Sixteen<T>& s, float (&v)[16]) {
-  if constexpr (sizeof(T) == 2) {
-    quant::widen16<T>(s.v[0].w, v);
-  } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[i] = __uint_as_float(s.v[0].w[i]);
-      v[8 + i] = __uint_as_float(s.v[1].w[i]);
+    for (int h = 0; h < static_cast<int>(sizeof(T)) / 2; ++h) {
+      const Vec256 v = ld_global_stream_256(p + 8 * h);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r.w[8 * h + i] = v.w[i];
     }
   }
+  return r;
 }
 
 // amax(|x|) / 2688 by the quantizer warps (all of them return it)
@@ -358,27 +343,24 @@ small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int group = qw / p.stage_warps, t_in_group = (qw % p.stage_warps) * 32 + lane;
       const int unit = t_in_group % C::kRowThreads, row = t_in_group / C::kRowThreads;  // 16 elements of a row of the stage
       const bool in_rows = row < p.M;
+      // threads past the last row take the first one's elements (nothing slow like a division of zeros) and write nothing
       const XT* x = static_cast<const XT*>(p.x) + static_cast<int64_t>(in_rows ? row : 0) * p.K + static_cast<int64_t>(ks0) * C::kStageElems + unit * 16;
       const int cols = p.K - ks0 * C::kStageElems - unit * 16;  // columns left from this thread's first element on
-      auto load_stage = [&](int i) { return load_sixteen<XT>(x + i * C::kStageElems, in_rows && i < n_stages && i * C::kStageElems < cols); };
+      auto load_stage = [&](int i) { return load_sixteen<XT>(x + i * C::kStageElems, i < n_stages && i * C::kStageElems < cols); };
       const uint32_t data_at = row * kStageKBytes + (KIND == Kind::kNvfp4 ? (((unit >> 1) ^ (row & 7)) << 4) + (unit & 1) * 8 : (unit ^ (row & 7)) << 4);
       const uint32_t scale_at = row * 16 + (KIND == Kind::kNvfp4 ? (unit >> 2) * 512 + (unit & 3) : unit >> 1);
-      Sixteen<XT> next = load_stage(group), after = load_stage(group + groups);  // the loads run two stages ahead
+      quant::Sixteen<XT> next = load_stage(group), after = load_stage(group + groups);  // the loads run two stages ahead
       RingAt at(group);
       for (int i = group; i < n_stages; i += groups, at.step(groups, p.ring)) {
         const int s = at.slot;
-        const Sixteen<XT> now = next;
+        const quant::Sixteen<XT> now = next;
         next = after;
         after = load_stage(i + 2 * groups);
         if constexpr (KIND == Kind::kNvfp4) {
-          uint32_t lo, hi, scale;
-          if constexpr (sizeof(XT) == 2) {
-            quant::nvfp4_block_packed<XT, true>(now.v[0].w, ts, lo, hi, scale);
-          } else {
-            float v[16];
-            widen_sixteen(now, v);
-            quant::nvfp4_block<true>(v, g, true, lo, hi, scale);
-          }
+          const quant::Sixteen<XT> one[1] = {now};
+          uint32_t codes[1][2], byte[1];
+          quant::nvfp4_blocks<XT, true, 1>(one, ts, codes, byte);
+          uint32_t lo = codes[0][0], hi = codes[0][1], scale = byte[0];
           if (i * C::kStageElems >= cols) lo = hi = scale = 0;  // past K: the last MMA may reach there
           mbar_wait(&empty_bar[s], at.phase ^ 1, abort_flag);
           if (in_rows) {
@@ -387,7 +369,7 @@ small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           }
         } else {
           float v[16];
-          widen_sixteen(now, v);
+          now.widen(v);
           float amax = quant::amax16(v);
           amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));  // the block's other half
           const quant::Mxfp8Scale sc = quant::mxfp8_scale(amax);

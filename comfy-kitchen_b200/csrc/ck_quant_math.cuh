@@ -189,6 +189,7 @@ __device__ __forceinline__ float amax16_packed(const uint32_t (&w)[8]) {
 // range where the reciprocal-FMA quotients below are exact.
 struct TensorScale {
   float g, rcp;
+  float s_hi, s_lo;  // bracket 1 / (6 g) by 2^-21 (see nvfp4_blocks)
   bool in_window;
 };
 __device__ __forceinline__ TensorScale make_tensor_scale(float g) {
@@ -196,6 +197,9 @@ __device__ __forceinline__ TensorScale make_tensor_scale(float g) {
   t.g = g;
   t.in_window = (g >= 0x1p-40f) && (g <= 0x1p40f);
   t.rcp = __frcp_rn(t.in_window ? g : 1.0f);
+  const float sixth = __frcp_rn(__fmul_rn(6.0f, t.in_window ? g : 1.0f));
+  t.s_hi = __fmul_rn(sixth, 0x1.000008p0f);
+  t.s_lo = __fmul_rn(sixth, 0x1.fffffp-1f);
   return t;
 }
 
@@ -324,6 +328,99 @@ __device__ __forceinline__ void nvfp4_block_packed(const uint32_t (&w)[8], const
   lo_word = r.lo;
   hi_word = r.hi;
   scale_byte = r.scale_byte;
+}
+
+// ---------------------------------------------------------------------------
+// NVFP4 blocks of one thread without a branch in the common case
+// ---------------------------------------------------------------------------
+// The E4M3 scale is bracketed like the codes: s = RN(RN(amax / 6) / g) deviates from amax / (6 g) by at most 2^-23, and
+// amax * s_hi and amax * s_lo lie 2^-21 on either side of it less the 2^-22 of their own four roundings; when both
+// round to the same E4M3 byte, that is the byte of s.  The codes' reciprocal is the hardware's (one unit in the last
+// place, 2^-23): with the products' roundings and the quotient's own 1.25 * 2^-22, still inside the bracket.
+// Everything is computed for all of a thread's blocks before one test asks whether some bracket was split or some
+// operand lies outside the window; those blocks are done again, out of line.  Straight code lets the blocks' serial
+// chains (maximum, scale, conversion there and back, reciprocal) overlap, and has no Markstein chains in it.
+
+// Sixteen elements in registers: packed pairs of a 16-bit type, or floats.
+template <typename T>
+struct Sixteen {
+  uint32_t w[4 * sizeof(T)];
+  __device__ __forceinline__ void widen(float (&v)[16]) const {
+    if constexpr (sizeof(T) == 2) {
+      widen16<T>(w, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(w[i]);
+    }
+  }
+  __device__ __forceinline__ float amax() const {
+    if constexpr (sizeof(T) == 2) {
+      return amax16_packed<T>(w);
+    } else {
+      float v[16];
+      widen(v);
+      return amax16(v);
+    }
+  }
+};
+
+// A block that the straight code could not settle.  `total` is its scale times g where that much is certain, else negative.
+template <typename T, bool kHiFirst>
+__device__ __noinline__ BlockCodes nvfp4_block_exact(Sixteen<T> x, float g, float total) {
+  float v[16];
+  x.widen(v);
+  BlockCodes r;
+  r.scale_byte = 0;
+  if (total > 0.0f && x.amax() <= total * 0x1p20f) {  // residuals of the exact chain representable
+    const float y = __frcp_rn(total);
+    float q[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) q[i] = div_markstein(v[i], total, y);
+    r.lo = scaled_e2m1_word<kHiFirst>(q, 1.0f);
+    r.hi = scaled_e2m1_word<kHiFirst>(q + 8, 1.0f);
+    return r;
+  }
+  nvfp4_block<false>(v, g, kHiFirst, r.lo, r.hi, r.scale_byte);
+  return r;
+}
+
+template <typename T, bool kHiFirst, int kBlocks>
+__device__ __forceinline__ void nvfp4_blocks(const Sixteen<T> (&x)[kBlocks], const TensorScale& ts, uint32_t (&codes)[kBlocks][2],
+                                             uint32_t (&scale_byte)[kBlocks]) {
+  float total[kBlocks];
+  bool ok[kBlocks], sure[kBlocks];
+  bool all = true;
+#pragma unroll
+  for (int b = 0; b < kBlocks; ++b) {
+    const float amax = x[b].amax();
+    const uint32_t both = f32x2_to_e4m3x2(__fmul_rn(amax, ts.s_hi), __fmul_rn(amax, ts.s_lo));
+    scale_byte[b] = both & 0xFFu;
+    total[b] = __fmul_rn(ts.g, e4m3_byte_to_f32(scale_byte[b]));
+    const bool dead = total[b] == 0.0f;
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(dead ? 1.0f : total[b]));
+    const float y_hi = __fmul_rn(y, 0x1.000008p0f), y_lo = __fmul_rn(y, 0x1.fffffp-1f);
+    float v[16];
+    x[b].widen(v);
+    const uint32_t lo = scaled_e2m1_word<kHiFirst>(v, y_hi), hi = scaled_e2m1_word<kHiFirst>(v + 8, y_hi);
+    const uint32_t split = (lo ^ scaled_e2m1_word<kHiFirst>(v, y_lo)) | (hi ^ scaled_e2m1_word<kHiFirst>(v + 8, y_lo));
+    codes[b][0] = dead ? 0u : lo;  // zero scale: every code is +0
+    codes[b][1] = dead ? 0u : hi;
+    sure[b] = (both >> 8) == scale_byte[b] && ts.in_window && amax <= 0x1p60f && (amax >= 0x1p-60f || amax == 0.0f);
+    ok[b] = sure[b] && (split == 0u || dead);
+    all = all && ok[b];
+  }
+  if (!all) {
+#pragma unroll
+    for (int b = 0; b < kBlocks; ++b) {
+      if (!ok[b]) {
+        const BlockCodes r = nvfp4_block_exact<T, kHiFirst>(x[b], ts.g, sure[b] ? total[b] : -1.0f);
+        codes[b][0] = r.lo;
+        codes[b][1] = r.hi;
+        if (!sure[b]) scale_byte[b] = r.scale_byte;
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
