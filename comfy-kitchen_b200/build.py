@@ -1,4 +1,5 @@
-"""Build the C-ABI shared library (lib/libck_b200.so) from csrc/*.cu for sm_100a.
+"""Build the C-ABI shared library (lib/libck_b200.so) from csrc/*.cu for sm_100a, and the Python
+wrappers' native half (lib/_ck_host.so) from csrc/host against the installed torch's headers.
 
     python comfy-kitchen_b200/build.py [--force] [--verbose]
 
@@ -10,16 +11,20 @@ from __future__ import annotations
 
 import argparse
 import glob
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libck_b200.so")
 OBJ_DIR = os.path.join(HERE, "build")
+HOST_SRC = os.path.join(CSRC, "host", "ck_host.cpp")
+HOST_PATH = os.path.join(LIB_DIR, "_ck_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -46,6 +51,26 @@ def _stale(target: str, deps: list[str]) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def build_host(force: bool = False, verbose: bool = False) -> str:
+    """The extension module that backends/cuda calls for plain eager calls (torch is found, not imported)."""
+    os.makedirs(LIB_DIR, exist_ok=True)
+    torch_dir = list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+    if not force and not _stale(HOST_PATH, [HOST_SRC, os.path.join(torch_dir, "version.py")]):
+        return HOST_PATH
+    include, libs = os.path.join(torch_dir, "include"), os.path.join(torch_dir, "lib")
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    cmd = [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + include,
+           "-I" + os.path.join(include, "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"], "-I" + cuda_include,
+           HOST_SRC, "-o", HOST_PATH, "-L" + libs, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        print(r.stdout, flush=True)
+        raise RuntimeError("the host extension does not build")
+    return HOST_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -80,6 +105,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
+    build_host(force, verbose)
     return LIB_PATH
 
 

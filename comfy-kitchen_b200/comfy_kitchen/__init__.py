@@ -18,7 +18,7 @@ from .backends import eager as _eager_backend  # noqa: F401
 from .backends import triton as _triton_backend  # noqa: F401
 from .exceptions import BackendError, BackendNotFoundError, BackendNotImplementedError, NoCapableBackendError
 from .float_utils import from_blocked, swap_nibbles, to_blocked
-from .ops import DTYPE_TO_CODE, _impl, dispatcher_adds_nothing, replaced
+from .ops import DTYPE_TO_CODE, _impl, dispatcher_adds_nothing, host_operator, replaced
 from .registry import registry
 
 __version__ = "0.1.0"
@@ -55,6 +55,11 @@ def quantize_nvfp4(x: torch.Tensor, per_tensor_scale: torch.Tensor, epsilon: flo
     to multiples of 16.  ``hi_first`` puts the even-indexed element of each pair in the
     high nibble.  ``epsilon`` is unused (kept for signature compatibility).
     """
+    host = host_operator("quantize_nvfp4")
+    if host is not None and type(epsilon) is float:
+        out = host(x, per_tensor_scale, pad_16x, hi_first)
+        if out is not None:
+            return out
     if not replaced("quantize_nvfp4") and dispatcher_adds_nothing((x, per_tensor_scale)) and type(epsilon) is float and \
             type(pad_16x) is bool and type(hi_first) is bool:
         return _impl("quantize_nvfp4", {"x": x, "per_tensor_scale": per_tensor_scale, "epsilon": epsilon, "pad_16x": pad_16x,
@@ -66,6 +71,11 @@ def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_sca
                      output_type: torch.dtype = torch.bfloat16, hi_first: bool = True) -> torch.Tensor:
     """Inverse of :func:`quantize_nvfp4` into ``output_type`` (float32, float16 or bfloat16)."""
     code = DTYPE_TO_CODE[output_type]
+    host = host_operator("dequantize_nvfp4")
+    if host is not None:
+        out = host(qx, per_tensor_scale, block_scales, output_type, hi_first)
+        if out is not None:
+            return out
     if not replaced("dequantize_nvfp4") and dispatcher_adds_nothing((qx, per_tensor_scale, block_scales)) and type(hi_first) is bool:
         return _impl("dequantize_nvfp4", {"qx": qx, "per_tensor_scale": per_tensor_scale, "block_scales": block_scales,
                                           "output_type": output_type, "hi_first": hi_first})
@@ -79,6 +89,11 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
     if out_dtype is None:
         out_dtype = torch.bfloat16
     code = DTYPE_TO_CODE[out_dtype]
+    host = host_operator("scaled_mm_nvfp4")
+    if host is not None:
+        out = host(a, b, tensor_scale_a, tensor_scale_b, block_scale_a, block_scale_b, bias, out_dtype, alpha)
+        if out is not None:
+            return out
     if not replaced("scaled_mm_nvfp4") and \
             dispatcher_adds_nothing((a, b, tensor_scale_a, tensor_scale_b, block_scale_a, block_scale_b), (bias, alpha)):
         return _impl("scaled_mm_nvfp4", {
@@ -90,6 +105,11 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
 
 def quantize_mxfp8(x: torch.Tensor, pad_32x: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
     """Quantize a 2-D tensor to MXFP8: ``(float8_e4m3fn [M', K'], float8_e8m0fnu swizzled scales of 32-element blocks)``."""
+    host = host_operator("quantize_mxfp8")
+    if host is not None:
+        out = host(x, pad_32x)
+        if out is not None:
+            return out
     if not replaced("quantize_mxfp8") and dispatcher_adds_nothing((x,)) and type(pad_32x) is bool:
         return _impl("quantize_mxfp8", {"x": x, "pad_32x": pad_32x})
     return torch.ops.comfy_kitchen.quantize_mxfp8(x, pad_32x)
@@ -99,6 +119,11 @@ def dequantize_mxfp8(qx: torch.Tensor, block_scales: torch.Tensor,
                      output_type: torch.dtype = torch.bfloat16) -> torch.Tensor:
     """Inverse of :func:`quantize_mxfp8` into ``output_type``."""
     code = DTYPE_TO_CODE[output_type]
+    host = host_operator("dequantize_mxfp8")
+    if host is not None:
+        out = host(qx, block_scales, output_type)
+        if out is not None:
+            return out
     if not replaced("dequantize_mxfp8") and dispatcher_adds_nothing((qx, block_scales)):
         return _impl("dequantize_mxfp8", {"qx": qx, "block_scales": block_scales, "output_type": output_type})
     return torch.ops.comfy_kitchen.dequantize_mxfp8(qx, block_scales, code)
@@ -110,6 +135,11 @@ def scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tenso
     if out_dtype is None:
         out_dtype = torch.bfloat16
     code = DTYPE_TO_CODE[out_dtype]
+    host = host_operator("scaled_mm_mxfp8")
+    if host is not None:
+        out = host(a, b, block_scale_a, block_scale_b, bias, out_dtype)
+        if out is not None:
+            return out
     if not replaced("scaled_mm_mxfp8") and dispatcher_adds_nothing((a, b, block_scale_a, block_scale_b), (bias,)):
         return _impl("scaled_mm_mxfp8", {"a": a, "b": b, "block_scale_a": block_scale_a, "block_scale_b": block_scale_b,
                                          "bias": bias, "out_dtype": out_dtype})

@@ -11,7 +11,11 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import importlib.machinery
+import importlib.util
+import logging
 import os
+import sys
 import threading
 
 import torch
@@ -40,6 +44,8 @@ ABI_VERSION = 1
 
 _lib = None
 _lib_error: str | None = None
+_this_module = sys.modules[__name__]
+_host = None  # the wrappers' native half (csrc/host), bound to the loaded library: plain calls go through it
 
 _P = ctypes.c_void_p
 _I = ctypes.c_int
@@ -112,7 +118,31 @@ def load_library():
         _lib_error = f"cannot load {path}: {e}"
         raise RuntimeError(_lib_error) from e
     _lib = lib
+    _load_host(lib)
     return lib
+
+
+_HOST_NAMES = ("ck_quantize_nvfp4", "ck_quantize_nvfp4_dynamic_scratch_bytes", "ck_quantize_nvfp4_dynamic", "ck_quantize_mxfp8",
+               "ck_dequantize_nvfp4", "ck_dequantize_mxfp8", "ck_scaled_mm_workspace_bytes", "ck_scaled_mm_nvfp4_ws",
+               "ck_scaled_mm_mxfp8_ws", "ck_linear_nvfp4_from_float_workspace_bytes", "ck_linear_nvfp4_from_float",
+               "ck_linear_mxfp8_from_float_workspace_bytes", "ck_linear_mxfp8_from_float")
+
+
+def _load_host(lib) -> None:
+    """Each function of the extension does one wrapper's work for plain eager calls and returns None for any other, which the
+    wrapper then does in Python.  Without the extension (not built, built against another torch) every call does."""
+    global _host
+    path = os.path.join(_PKG_ROOT, "lib", "_ck_host.so")
+    if not os.path.exists(path):
+        return
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("_ck_host", path)
+        host = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ck_host", loader))
+        loader.exec_module(host)
+        host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _HOST_NAMES}, torch.nn.Parameter)
+        _host = host
+    except ImportError as e:
+        logging.getLogger("comfy_kitchen").warning("%s does not load (%s): calls go through the Python wrappers", path, e)
 
 
 def is_loaded() -> bool:
@@ -184,6 +214,10 @@ def quantize_nvfp4(x: torch.Tensor, per_tensor_scale: torch.Tensor, epsilon: flo
     ``epsilon`` is accepted for signature compatibility and unused, as in the reference.
     The scale tensor is allocated uninitialised: the kernel writes its padding as zeros.
     """
+    if _host is not None:
+        out = _host.quantize_nvfp4(x, per_tensor_scale, pad_16x, hi_first)
+        if out is not None:
+            return out
     lib = load_library()
     x = _plain(x)
     assert x.is_contiguous(), "Input tensor must be contiguous"
@@ -205,6 +239,10 @@ def quantize_nvfp4(x: torch.Tensor, per_tensor_scale: torch.Tensor, epsilon: flo
 
 def quantize_mxfp8(x: torch.Tensor, pad_32x: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
     """bf16/f16/f32 [M, K] -> (float8_e4m3fn [M', K'], float8_e8m0fnu swizzled block scales)."""
+    if _host is not None:
+        out = _host.quantize_mxfp8(x, pad_32x)
+        if out is not None:
+            return out
     lib = load_library()
     x = _plain(x)
     assert x.is_contiguous(), "Input tensor must be contiguous"
@@ -291,6 +329,13 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
                            hi_first: bool = True) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """``scale = nvfp4_tensor_scale(x)`` and ``quantize_nvfp4(x, scale)`` in one library call (same bits):
     ``(codes, block_scales, scale)``.  The reduction leaves partial maxima that the quantizer finishes."""
+    if _host is not None:
+        scratch = None
+        if type(x) is torch.Tensor and x.is_cuda and x.numel() * x.element_size() <= _WHOLE_INPUT_BYTES:
+            scratch = _scale_scratch_for(x.device, _stream(x.device), 1 << 20)  # nothing is kept in it between two launches
+        out = _host.quantize_nvfp4_dynamic(x, pad_16x, hi_first, scratch)
+        if out is not None:
+            return out
     lib = load_library()
     x = _plain(x)
     assert x.is_contiguous(), "Input tensor must be contiguous"
@@ -326,6 +371,10 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
 def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_scales: torch.Tensor,
                      output_type: torch.dtype = torch.bfloat16, hi_first: bool = True) -> torch.Tensor:
     """uint8 [M, K/2] codes + swizzled E4M3 scales + fp32 tensor scale -> [M, K] of ``output_type``."""
+    if _host is not None:
+        out = _host.dequantize_nvfp4(qx, per_tensor_scale, block_scales, output_type, hi_first)
+        if out is not None:
+            return out
     lib = load_library()
     qx, block_scales = _plain(qx), _plain(block_scales)
     assert qx.is_contiguous() and block_scales.is_contiguous(), "Input tensor must be contiguous"
@@ -345,6 +394,10 @@ def dequantize_nvfp4(qx: torch.Tensor, per_tensor_scale: torch.Tensor, block_sca
 def dequantize_mxfp8(qx: torch.Tensor, block_scales: torch.Tensor,
                      output_type: torch.dtype = torch.bfloat16) -> torch.Tensor:
     """float8_e4m3fn [M, K] + swizzled E8M0 scales -> [M, K] of ``output_type``."""
+    if _host is not None:
+        out = _host.dequantize_mxfp8(qx, block_scales, output_type)
+        if out is not None:
+            return out
     lib = load_library()
     qx, block_scales = _plain(qx), _plain(block_scales)
     assert qx.is_contiguous() and block_scales.is_contiguous(), "Input tensor must be contiguous"
@@ -382,6 +435,10 @@ def scaled_mm_nvfp4(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.Tens
     a: uint8 [M, K/2], b: uint8 [N, K/2]; block scales in the swizzled layout.  ``alpha``
     overrides the product of the tensor scales when given, as in the reference wrapper.
     """
+    if _host is not None:
+        out = _host.scaled_mm_nvfp4(a, b, tensor_scale_a, tensor_scale_b, block_scale_a, block_scale_b, bias, out_dtype, alpha)
+        if out is not None:
+            return out
     lib = load_library()
     a, b = _plain(a), _plain(b)
     block_scale_a, block_scale_b = _plain(block_scale_a), _plain(block_scale_b)
@@ -518,6 +575,10 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     ``w_scale``; ``x_scale`` a static per-tensor scale or None for ``amax(|x|)/2688``.  Same bits
     as ``quantize_nvfp4`` followed by ``scaled_mm_nvfp4``.  The quantized activation passes
     from one launch to the next in a workspace (:func:`_workspace_for`)."""
+    if _host is not None:
+        out = _host.linear_nvfp4_from_float(x, w_codes, w_scale, w_block_scales, bias, x_scale, out_dtype)
+        if out is not None:
+            return out
     lib = load_library()
     if not (type(x) is type(w_codes) is type(w_block_scales) is torch.Tensor):
         x, w_codes, w_block_scales = _plain(x), _plain(w_codes), _plain(w_block_scales)
@@ -553,6 +614,10 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     ``w_data`` float8_e4m3fn [N, K] with its tiled E8M0 ``w_block_scales``.  Same bits as
     ``quantize_mxfp8`` followed by ``scaled_mm_mxfp8``; the quantized activation passes through a
     workspace, as in :func:`linear_nvfp4_from_float`."""
+    if _host is not None:
+        out = _host.linear_mxfp8_from_float(x, w_data, w_block_scales, bias, out_dtype)
+        if out is not None:
+            return out
     lib = load_library()
     if not (type(x) is type(w_data) is type(w_block_scales) is torch.Tensor):
         x, w_data, w_block_scales = _plain(x), _plain(w_data), _plain(w_block_scales)
@@ -629,6 +694,10 @@ def linear_nvfp4_fused(a: torch.Tensor, b: torch.Tensor, tensor_scale_a: torch.T
 def scaled_mm_mxfp8(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tensor, block_scale_b: torch.Tensor,
                     bias: torch.Tensor | None = None, out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """out[M, N] = deq(a) @ deq(b).T + bias with E4M3 data [M, K] / [N, K] and E8M0 1x32 block scales."""
+    if _host is not None:
+        out = _host.scaled_mm_mxfp8(a, b, block_scale_a, block_scale_b, bias, out_dtype)
+        if out is not None:
+            return out
     lib = load_library()
     a, b = _plain(a), _plain(b)
     block_scale_a, block_scale_b = _plain(block_scale_a), _plain(block_scale_b)
@@ -703,8 +772,23 @@ def _build_constraints() -> dict:
     }
 
 
+_constraints: dict = {}  # as registered
+_stock = {name: globals()[name] for name in ("quantize_nvfp4", "quantize_mxfp8", "dequantize_nvfp4", "dequantize_mxfp8",
+                                             "scaled_mm_nvfp4", "scaled_mm_mxfp8")}
+
+
+def host_operator(name: str):
+    """The native half of operator ``name``, or None unless the registry would send every call that it takes to this
+    module's own function anyway."""
+    from comfy_kitchen.registry import registry
+
+    if _host is None or globals()[name] is not _stock[name] or \
+            not registry.leaves_no_choice(name, _this_module, _constraints.get(name)):
+        return None
+    return getattr(_host, name)
+
+
 def _register():
-    import sys
 
     from comfy_kitchen.registry import registry
 
@@ -716,7 +800,8 @@ def _register():
     if not torch.cuda.is_available():
         registry.mark_unavailable("cuda", "CUDA not available on this system")
         return
-    registry.register("cuda", sys.modules[__name__], _build_constraints())
+    _constraints.update(_build_constraints())
+    registry.register("cuda", _this_module, _constraints)
 
 
 _register()

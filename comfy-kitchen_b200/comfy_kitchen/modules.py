@@ -29,7 +29,7 @@ import torch
 import torch.nn as nn
 
 from .tensor import QuantizedTensor, TensorCoreMXFP8Layout, TensorCoreNVFP4Layout
-from .tensor.blockwise import direct_backend, quantized_linear, strict_mode, strict_status_check
+from .tensor.blockwise import direct_backend, host_half, quantized_linear, strict_mode, strict_status_check
 
 NVFP4 = "TensorCoreNVFP4Layout"
 MXFP8 = "TensorCoreMXFP8Layout"
@@ -188,6 +188,15 @@ class NVFP4Linear(_QuantizedLinearBase):
         """Dense CUDA activations take the one-call path (tensor scale, quantize and GEMM enqueued by a
         single library call: a third of the host time per layer of the layout path, same bits); quantized
         inputs, traced calls and anything the call refuses take the layout path."""
+        held = self._parameters
+        host, w = host_half(), held.get("weight")
+        if host is not None and w is not None and type(x) is torch.Tensor and not w._params.transposed:
+            # a plain eager call (None for any other): 9 us of host time instead of 18
+            params = w._params
+            y = host.linear_nvfp4_from_float(x, w._qdata, params.scale, params.block_scale, held.get("bias"),
+                                             held["input_scale"] if "input_scale" in held else self.input_scale, x.dtype)
+            if y is not None and y.shape[1] == self.out_features:
+                return y
         w = self.weight
         if not isinstance(x, QuantizedTensor) and w is not None and x.dim() >= 2 and x.shape[-1] % 32 == 0 and \
                 x.dtype in (torch.bfloat16, torch.float16, torch.float32) and not getattr(w._params, "transposed", False):
@@ -257,6 +266,12 @@ class MXFP8Linear(_QuantizedLinearBase):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """Dense CUDA activations take the one-call path (quantize and GEMM enqueued by a single library
         call, same bits); everything else the layout path."""
+        held = self._parameters
+        host, w = host_half(), held.get("weight")
+        if host is not None and w is not None and type(x) is torch.Tensor and not getattr(w._params, "transposed", False):
+            y = host.linear_mxfp8_from_float(x, w._qdata, w._params.scale, held.get("bias"), x.dtype)
+            if y is not None and y.shape[1] == self.out_features:
+                return y
         w = self.weight
         if not isinstance(x, QuantizedTensor) and w is not None and x.dim() >= 2 and x.shape[-1] % 32 == 0 and \
                 x.dtype in (torch.bfloat16, torch.float16, torch.float32) and not getattr(w._params, "transposed", False):

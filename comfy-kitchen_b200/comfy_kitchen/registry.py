@@ -38,6 +38,7 @@ class BackendRegistry:
         self._lock = threading.Lock()
         self._tls = threading.local()
         self._cc: tuple[int, int] | None | bool = False  # False = not probed yet
+        self._only: tuple[str, Any] | None = None  # the one backend, while no other is registered and it is in use
 
     # -- hardware ------------------------------------------------------------------------
     @property
@@ -61,6 +62,7 @@ class BackendRegistry:
             for fn, fc in capabilities.items():
                 self._constraints[(name, fn)] = fc
             self._unavailable.pop(name, None)
+            self._settle()
 
     def mark_unavailable(self, name: str, reason: str):
         with self._lock:
@@ -73,14 +75,31 @@ class BackendRegistry:
     def disable(self, backend_name: str):
         with self._lock:
             self._disabled.add(backend_name)
+            self._settle()
 
     def enable(self, backend_name: str):
         with self._lock:
             self._disabled.discard(backend_name)
+            self._settle()
 
     def set_priority(self, priority_list: list[str]):
         with self._lock:
             self._priority = list(priority_list)
+            self._settle()
+
+    def _settle(self) -> None:
+        name = next(iter(self._backends), None)
+        alone = len(self._backends) == 1 and name not in self._disabled and name in self._priority
+        self._only = (name, self._backends[name]) if alone else None
+
+    def leaves_no_choice(self, func_name: str, module, constraints: FunctionConstraints | None) -> bool:
+        """True when every call of ``func_name`` on this thread that meets ``constraints`` goes to ``module``: nothing else is
+        registered, it is enabled and nobody overrides it, and the device is one that it runs on."""
+        only = self._only
+        if only is None or only[1] is not module or constraints is None or getattr(self._tls, "override", None) is not None:
+            return False
+        cc = self._compute_capability
+        return self._constraints.get((only[0], func_name)) is constraints and cc is not None and cc >= constraints.min_compute_capability
 
     def is_available(self, backend_name: str) -> bool:
         return backend_name in self._backends and backend_name not in self._disabled

@@ -58,6 +58,16 @@ def direct_backend(*tensors):
     return _backend if _backend.is_loaded() else None
 
 
+def host_half():
+    """The native half of the CUDA backend's wrappers for a call outside of any tracing, or None."""
+    if torch.compiler.is_compiling():
+        return None
+    global _backend
+    if _backend is None:
+        from comfy_kitchen.backends import cuda as _backend
+    return _backend._host
+
+
 def crop(result: torch.Tensor, rows: int, cols: int) -> torch.Tensor:
     """Cut a padded matmul result back to the logical output shape."""
     if result.shape[0] != rows or result.shape[1] != cols:
