@@ -146,6 +146,18 @@ __device__ __forceinline__ Vec256 ld_global_stream_256(const void* p) {
   return r;
 }
 
+__device__ __forceinline__ uint2 ld_global_stream_64(const void* p) {
+  uint2 r;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t ld_global_u8(const void* p) {
+  uint32_t r;
+  asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(r) : "l"(p));
+  return r;
+}
+
 // The same load for data that this library will not read again: its lines are the first to leave L2.
 __device__ __forceinline__ Vec256 ld_global_last_use_256(const void* p) {
   Vec256 r;

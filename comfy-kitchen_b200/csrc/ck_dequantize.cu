@@ -73,61 +73,99 @@ __device__ __forceinline__ void e2m1x8_to_f16x2(uint32_t word, uint32_t (&h)[4])
       : "r"(word));
 }
 
-// one thread = one 16-element block of one row
-template <typename OutT, bool kHiFirst>
+// Bound by HBM (the result's write) for large tensors, by launch and latency for small ones.  A thread takes the same 16-
+// (NVFP4) or 32-element (MXFP8) block of kRows rows, four rows apart.  Two rows in flight pay where a thread's traffic is
+// small, for NVFP4 to a 16-bit type, and where the tensor fills the chip several times; launched like the other streaming
+// kernels, as a dependent of the kernel before it.  Graph replays, us, one row launched plainly / one row / two / four:
+// NVFP4 to bf16 12288 x 3072 18.3 / 17.8 / 17.0 / 17.5 (whole calls 20.4 -> 16.9), 36864 x 3072 49.8 / 49.2 / 47.2 / 48.0, 256 x 1024
+// 1.63 / 1.25 / 1.46 / 1.85; to fp32 4096 x 3072 11.2 / 10.7 / 10.6 / 11.7; MXFP8 to bf16 12288 x 3072 19.5 / 18.8 / 19.2 / 20.2.
+template <typename OutT, bool kHiFirst, int kRows>
 __global__ void __launch_bounds__(kThreads)
-dequantize_nvfp4_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ global_scale,
-                        const uint8_t* __restrict__ scales, OutT* __restrict__ out, int64_t rows, int64_t cols) {
+dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols) {
+  pdl_launch_dependents();
   const int64_t n_sc = cols >> 4;
   const int64_t sc = static_cast<int64_t>(blockIdx.y) * 64 + threadIdx.x;
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + threadIdx.y;
-  if (row >= rows || sc >= n_sc) return;
-  const uint2 packed = *reinterpret_cast<const uint2*>(codes + row * (cols >> 1) + sc * 8);
-  const uint32_t sbyte = scales[swizzled_scale_offset(row, sc, ceil_div(n_sc, 4))];
-  // :211 total scale in the output dtype
-  const float ts = round_to<OutT>(__ldg(global_scale));
-  const float bs = e4m3_byte_to_f32(sbyte);  // exact in every output dtype
-  const float total = round_to<OutT>(ts * bs);
-  float v[16];
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * (4 * kRows) + threadIdx.y;
+  const int64_t col_tiles = ceil_div(n_sc, 4);
+  if constexpr (kRows == 1) {
+    // ahead of the dependency wait: ask L2 for the 128-byte line of sixteen threads (warms the cache only)
+    if (sc < n_sc && row0 < rows && (threadIdx.x & 15) == 0) prefetch_l2(codes + row0 * (cols >> 1) + sc * 8);
+  }
+  pdl_wait();
+  if (sc >= n_sc) return;
+  uint2 packed[kRows];
+  uint32_t sbyte[kRows];
 #pragma unroll
-  for (int w = 0; w < 2; ++w) {
-    uint32_t h[4];
-    e2m1x8_to_f16x2(w == 0 ? packed.x : packed.y, h);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[i]));  // (low nibble, high nibble)
-      // :214, rounded by the store; the product of two OutT numbers is exact in float32
-      v[8 * w + 2 * i] = (kHiFirst ? f.y : f.x) * total;
-      v[8 * w + 2 * i + 1] = (kHiFirst ? f.x : f.y) * total;
+  for (int i = 0; i < kRows; ++i) {
+    const int64_t row = row0 + 4 * i;
+    if (row < rows) {
+      packed[i] = ld_global_stream_64(codes + row * (cols >> 1) + sc * 8);
+      sbyte[i] = ld_global_u8(scales + swizzled_scale_offset(row, sc, col_tiles));
     }
   }
-  store16<OutT>(out + row * cols + sc * 16, v);
-}
-
-// one thread = one 32-element block of one row
-template <typename OutT>
-__global__ void __launch_bounds__(kThreads)
-dequantize_mxfp8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ scales,
-                        OutT* __restrict__ out, int64_t rows, int64_t cols) {
-  const int64_t n_sc = cols >> 5;
-  const int64_t sc = static_cast<int64_t>(blockIdx.y) * 64 + threadIdx.x;
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + threadIdx.y;
-  if (row >= rows || sc >= n_sc) return;
-  const Vec256 raw = ld_global_stream_256(data + row * cols + sc * 32);
-  const uint32_t e = scales[swizzled_scale_offset(row, sc, ceil_div(n_sc, 4))];
-  const float scale = __uint_as_float(e << 23);  // byte 0 -> 0.0 (float_utils.py:376-382)
+  // :211 total scale in the output dtype
+  const float ts = round_to<OutT>(ld_f32_dependent(global_scale));
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int i = 0; i < kRows; ++i) {
+    const int64_t row = row0 + 4 * i;
+    if (row >= rows) break;
+    const float bs = e4m3_byte_to_f32(sbyte[i]);  // exact in every output dtype
+    const float total = round_to<OutT>(ts * bs);
     float v[16];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t w = raw.w[h * 4 + i];
-      v[4 * i + 0] = e4m3_byte_to_f32(w & 0xFFu) * scale;
-      v[4 * i + 1] = e4m3_byte_to_f32((w >> 8) & 0xFFu) * scale;
-      v[4 * i + 2] = e4m3_byte_to_f32((w >> 16) & 0xFFu) * scale;
-      v[4 * i + 3] = e4m3_byte_to_f32(w >> 24) * scale;
+    for (int w = 0; w < 2; ++w) {
+      uint32_t h[4];
+      e2m1x8_to_f16x2(w == 0 ? packed[i].x : packed[i].y, h);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[j]));  // (low nibble, high nibble)
+        // :214, rounded by the store; the product of two OutT numbers is exact in float32
+        v[8 * w + 2 * j] = (kHiFirst ? f.y : f.x) * total;
+        v[8 * w + 2 * j + 1] = (kHiFirst ? f.x : f.y) * total;
+      }
     }
-    store16<OutT>(out + row * cols + sc * 32 + h * 16, v);
+    store16<OutT>(out + row * cols + sc * 16, v);
+  }
+}
+
+template <typename OutT, int kRows>
+__global__ void __launch_bounds__(kThreads)
+dequantize_mxfp8_kernel(const uint8_t* data, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols) {
+  pdl_launch_dependents();
+  const int64_t n_sc = cols >> 5;
+  const int64_t sc = static_cast<int64_t>(blockIdx.y) * 64 + threadIdx.x;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * (4 * kRows) + threadIdx.y;
+  const int64_t col_tiles = ceil_div(n_sc, 4);
+  pdl_wait();
+  if (sc >= n_sc) return;
+  Vec256 raw[kRows];
+  uint32_t e[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int64_t row = row0 + 4 * i;
+    if (row < rows) {
+      raw[i] = ld_global_stream_256(data + row * cols + sc * 32);
+      e[i] = ld_global_u8(scales + swizzled_scale_offset(row, sc, col_tiles));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int64_t row = row0 + 4 * i;
+    if (row >= rows) break;
+    const float scale = __uint_as_float(e[i] << 23);  // byte 0 -> 0.0 (float_utils.py:376-382)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t w = raw[i].w[h * 4 + j];
+        v[4 * j + 0] = e4m3_byte_to_f32(w & 0xFFu) * scale;
+        v[4 * j + 1] = e4m3_byte_to_f32((w >> 8) & 0xFFu) * scale;
+        v[4 * j + 2] = e4m3_byte_to_f32((w >> 16) & 0xFFu) * scale;
+        v[4 * j + 3] = e4m3_byte_to_f32(w >> 24) * scale;
+      }
+      store16<OutT>(out + row * cols + sc * 32 + h * 16, v);
+    }
   }
 }
 
@@ -143,6 +181,30 @@ int check_common(const char* op, const void* in, const void* scales, const void*
   return CK_OK;
 }
 
+template <typename OutT, int kRows>
+int launch_nvfp4_rows(const uint8_t* codes, const float* global_scale, const uint8_t* scales, void* out, int64_t rows, int64_t cols, int hi_first,
+                      cudaStream_t stream) {
+  const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4 * kRows)), static_cast<unsigned>(ceil_div(cols / 16, 64))), block(64, 4);
+  auto kernel = hi_first ? dequantize_nvfp4_kernel<OutT, true, kRows> : dequantize_nvfp4_kernel<OutT, false, kRows>;
+  CK_CUDA(launch_pdl(kernel, grid, block, 0, stream, codes, global_scale, scales, static_cast<OutT*>(out), rows, cols));
+  return CK_OK;
+}
+
+template <typename OutT>
+int launch_nvfp4(const uint8_t* codes, const float* global_scale, const uint8_t* scales, void* out, int64_t rows, int64_t cols, int hi_first,
+                 cudaStream_t stream) {
+  constexpr int64_t kTwoRowsElements = 4 << 20;  // seven waves of one row to a thread
+  if (sizeof(OutT) == 2 && rows * cols >= kTwoRowsElements) return launch_nvfp4_rows<OutT, 2>(codes, global_scale, scales, out, rows, cols, hi_first, stream);
+  return launch_nvfp4_rows<OutT, 1>(codes, global_scale, scales, out, rows, cols, hi_first, stream);
+}
+
+template <typename OutT>
+int launch_mxfp8(const uint8_t* data, const uint8_t* scales, void* out, int64_t rows, int64_t cols, cudaStream_t stream) {
+  const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4)), static_cast<unsigned>(ceil_div(cols / 32, 64))), block(64, 4);
+  CK_CUDA(launch_pdl(dequantize_mxfp8_kernel<OutT, 1>, grid, block, 0, stream, data, scales, static_cast<OutT*>(out), rows, cols));
+  return CK_OK;
+}
+
 }  // namespace
 }  // namespace ck
 
@@ -152,22 +214,14 @@ extern "C" int ck_dequantize_nvfp4(const void* codes, const float* global_scale,
   if (int rc = check_common("dequantize_nvfp4", codes, block_scales, out, out_dtype, rows, cols, 16)) return rc;
   CK_REQUIRE(global_scale != nullptr, "dequantize_nvfp4: null global_scale");
   CK_REQUIRE(reinterpret_cast<uintptr_t>(codes) % 8 == 0, "dequantize_nvfp4: codes must be 8-byte aligned");
-  const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4)), static_cast<unsigned>(ceil_div(cols / 16, 64))), block(64, 4);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const uint8_t* c = static_cast<const uint8_t*>(codes);
   const uint8_t* sc = static_cast<const uint8_t*>(block_scales);
-  if (out_dtype == CK_DTYPE_BF16) {
-    if (hi_first) dequantize_nvfp4_kernel<__nv_bfloat16, true><<<grid, block, 0, s>>>(c, global_scale, sc, static_cast<__nv_bfloat16*>(out), rows, cols);
-    else dequantize_nvfp4_kernel<__nv_bfloat16, false><<<grid, block, 0, s>>>(c, global_scale, sc, static_cast<__nv_bfloat16*>(out), rows, cols);
-  } else if (out_dtype == CK_DTYPE_F16) {
-    if (hi_first) dequantize_nvfp4_kernel<__half, true><<<grid, block, 0, s>>>(c, global_scale, sc, static_cast<__half*>(out), rows, cols);
-    else dequantize_nvfp4_kernel<__half, false><<<grid, block, 0, s>>>(c, global_scale, sc, static_cast<__half*>(out), rows, cols);
-  } else {
-    if (hi_first) dequantize_nvfp4_kernel<float, true><<<grid, block, 0, s>>>(c, global_scale, sc, static_cast<float*>(out), rows, cols);
-    else dequantize_nvfp4_kernel<float, false><<<grid, block, 0, s>>>(c, global_scale, sc, static_cast<float*>(out), rows, cols);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (out_dtype) {
+    case CK_DTYPE_BF16: return launch_nvfp4<__nv_bfloat16>(c, global_scale, sc, out, rows, cols, hi_first, s);
+    case CK_DTYPE_F16: return launch_nvfp4<__half>(c, global_scale, sc, out, rows, cols, hi_first, s);
+    default: return launch_nvfp4<float>(c, global_scale, sc, out, rows, cols, hi_first, s);
   }
-  CK_CUDA(cudaGetLastError());
-  return CK_OK;
 }
 
 extern "C" int ck_dequantize_mxfp8(const void* data, const void* block_scales, void* out, int out_dtype, int64_t rows,
@@ -175,17 +229,12 @@ extern "C" int ck_dequantize_mxfp8(const void* data, const void* block_scales, v
   using namespace ck;
   if (int rc = check_common("dequantize_mxfp8", data, block_scales, out, out_dtype, rows, cols, 32)) return rc;
   CK_REQUIRE(reinterpret_cast<uintptr_t>(data) % 32 == 0, "dequantize_mxfp8: data must be 32-byte aligned");
-  const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4)), static_cast<unsigned>(ceil_div(cols / 32, 64))), block(64, 4);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const uint8_t* d = static_cast<const uint8_t*>(data);
   const uint8_t* sc = static_cast<const uint8_t*>(block_scales);
-  if (out_dtype == CK_DTYPE_BF16) {
-    dequantize_mxfp8_kernel<<<grid, block, 0, s>>>(d, sc, static_cast<__nv_bfloat16*>(out), rows, cols);
-  } else if (out_dtype == CK_DTYPE_F16) {
-    dequantize_mxfp8_kernel<<<grid, block, 0, s>>>(d, sc, static_cast<__half*>(out), rows, cols);
-  } else {
-    dequantize_mxfp8_kernel<<<grid, block, 0, s>>>(d, sc, static_cast<float*>(out), rows, cols);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (out_dtype) {
+    case CK_DTYPE_BF16: return launch_mxfp8<__nv_bfloat16>(d, sc, out, rows, cols, s);
+    case CK_DTYPE_F16: return launch_mxfp8<__half>(d, sc, out, rows, cols, s);
+    default: return launch_mxfp8<float>(d, sc, out, rows, cols, s);
   }
-  CK_CUDA(cudaGetLastError());
-  return CK_OK;
 }

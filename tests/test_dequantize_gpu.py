@@ -73,3 +73,19 @@ def test_round_trip_full_size(ck, cuda_device, dtype, kind, key):
     err = (out.float() - x.float()).norm() / x.float().norm()
     err8 = (out8.float() - x.float()).norm() / x.float().norm()
     assert err < 0.15 and err8 < 0.05
+
+
+@pytest.mark.parametrize("hi_first", [True, False])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_nvfp4_two_rows_to_a_thread(cuda_device, dtype, hi_first):
+    """From 2^22 elements on a thread of the 16-bit kernels takes two rows (here the last ones have no second): the values of
+    row blocks taken by themselves, which are smaller than that."""
+    from comfy_kitchen.backends import cuda as backend
+
+    gen = torch.Generator(device=cuda_device).manual_seed(11)
+    rows, cols, g = 1373, 3088, torch.tensor(0.0123, device=cuda_device)
+    x = torch.randn(rows, cols, generator=gen, device=cuda_device)
+    q, s = backend.quantize_nvfp4(x, g, hi_first=hi_first)
+    got = backend.dequantize_nvfp4(q, g, s, dtype, hi_first=hi_first)
+    parts = [backend.dequantize_nvfp4(q[r:r + 128], g, s[r:r + 128], dtype, hi_first=hi_first) for r in range(0, rows, 128)]
+    assert rows * cols > 1 << 22 and torch.equal(got, torch.cat(parts))
