@@ -191,7 +191,7 @@ __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSour
 // Measured, whole calls: 8 x 3072 dynamic linear 39.5 -> 34.8 us; 1003 padded rows through the tensor
 // subclass 86.3 -> 70.5 (padded rows took scalar loads before: 6.4 us for 6 MB); an fp32 weight of
 // 12288 x 3072 with its dynamic scale 56.8 -> 52.4.
-constexpr int kPairRows = 16;  // rows per thread block
+// kPairRows: rows of a thread block, two blocks of 16 to an SM or eight of 4 (launch_streaming_as says when).
 
 template <bool kMark>
 __device__ __forceinline__ Vec256 ld_stream_unit(const void* p) {
@@ -199,8 +199,8 @@ __device__ __forceinline__ Vec256 ld_stream_unit(const void* p) {
   return ld_global_stream_256(p);
 }
 
-template <typename T, bool kHiFirst, bool kDynamic, bool kMark>
-__global__ void __launch_bounds__(32 * kPairRows, 2)
+template <typename T, bool kHiFirst, bool kDynamic, bool kMark, int kPairRows>
+__global__ void __launch_bounds__(32 * kPairRows, 32 / kPairRows)
 quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
                              int data_rows, int rows, int cols, int rows_pad, int sc_pad, int row_groups) {
   constexpr int kElems = 64 / sizeof(T);  // elements of a thread's unit
@@ -364,17 +364,31 @@ bool streaming_applies(const void* input, const void* codes, int64_t orig_rows, 
          num_rows < (1 << 30) && num_cols < (1 << 30) && !exact_division();
 }
 
-template <typename T, bool kDynamic, bool kMark>
+// How many passes over the grid a streaming launch makes with all its blocks of 16 rows resident at once.
+template <typename T>
+int64_t resident_passes(int64_t num_rows, int64_t num_cols) {
+  const int64_t col_chunks = ceil_div(round_up(num_cols / 16, 4), 32 * (4 / static_cast<int64_t>(sizeof(T))));
+  return ceil_div(round_up(num_rows, 128) / 16 * col_chunks, 2ll * sm_count());
+}
+
+// Many passes: blocks of 4 rows that make two each, so that finished blocks make room for the loads of the next.  Graph replays,
+// us, resident blocks of 16 rows / so: bf16 8192 x 3072 (6 passes) 13.7 / 14.1, 16384 x 3072 (11) 28.4 / 26.9, 36864 x 3072
+// 57.3 / 50.2, fp16 8192 x 15360 54.7 / 51.7, bf16 16384 x 12288 98.8 / 95.5; fp32 12288 x 3072 (16) 25.8 / 27.2, 36864 x 3072
+// (47) 90.9 / 78.1.
+template <typename T>
+bool many_passes(int64_t num_rows, int64_t num_cols) { return resident_passes<T>(num_rows, num_cols) >= (sizeof(T) == 2 ? 8 : 32); }
+
+template <typename T, bool kDynamic, bool kMark, int kPairRows>
 int launch_streaming_as(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
-                        int64_t num_cols, int hi_first, cudaStream_t stream) {
+                        int64_t num_cols, int hi_first, int most_passes, cudaStream_t stream) {
   const int64_t sc_pad = round_up(num_cols / 16, 4);
   const int rows_pad = static_cast<int>(round_up(num_rows, 128));
   const int row_groups = rows_pad / kPairRows;
   const int col_chunks = static_cast<int>(ceil_div(sc_pad, 32 * (4 / static_cast<int>(sizeof(T)))));
   CK_REQUIRE(col_chunks <= 65535, "quantize_nvfp4: tensor too large for one launch");
-  auto kernel = hi_first ? quantize_nvfp4_stream_kernel<T, true, kDynamic, kMark> : quantize_nvfp4_stream_kernel<T, false, kDynamic, kMark>;
+  auto kernel = hi_first ? quantize_nvfp4_stream_kernel<T, true, kDynamic, kMark, kPairRows> : quantize_nvfp4_stream_kernel<T, false, kDynamic, kMark, kPairRows>;
   // All blocks resident at once and all of the same length: the grid is the number of
-  // row groups divided into the fewest equal passes that fit the device.
+  // row groups divided into the fewest equal passes that fit the device (or into most_passes).
   static std::atomic<int> blocks_per_sm[2] = {{0}, {0}};
   std::atomic<int>& known = blocks_per_sm[hi_first ? 1 : 0];
   int per_sm = known.load(std::memory_order_relaxed);
@@ -384,12 +398,33 @@ int launch_streaming_as(const T* x, const ScaleSource& src, uint8_t* codes, uint
     known.store(per_sm, std::memory_order_relaxed);
   }
   const int per_wave = max(1, sm_count() * per_sm / col_chunks);
-  const int waves = static_cast<int>(ceil_div(row_groups, per_wave));
+  const int waves = min(static_cast<int>(ceil_div(row_groups, per_wave)), most_passes);
   const int grid_x = static_cast<int>(ceil_div(row_groups, waves));
   const dim3 grid(static_cast<unsigned>(grid_x), static_cast<unsigned>(col_chunks)), block(32, kPairRows);
   CK_CUDA(launch_pdl(kernel, grid, block, 0, stream, x, src, codes, scales, static_cast<int>(orig_rows), static_cast<int>(num_rows),
                      static_cast<int>(num_cols), rows_pad, static_cast<int>(sc_pad), row_groups));
   return CK_OK;
+}
+
+template <typename T, bool kMark>
+int launch_streaming_marked(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
+                            int64_t num_cols, int hi_first, cudaStream_t stream) {
+  constexpr int kAll = 1 << 30;
+  if (src.given == nullptr) {
+    // Every block finishes the scale: few of them.  (One block that finishes it for all, then the launch for many passes:
+    // bf16 36864 x 3072 with its reduction 91.0 us instead of 87.9, whose quantizer begins in what the reduction left in L2.)
+    return launch_streaming_as<T, true, kMark, 16>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, kAll, stream);
+  }
+  if (many_passes<T>(num_rows, num_cols)) {
+    return launch_streaming_as<T, false, kMark, 4>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, 2, stream);
+  }
+  // Fewer blocks of 16 rows than SMs: four times as many of 4.  bf16 16 x 3072 2.26 / 1.79 us, 256 x 3072 2.78 / 2.28, 512 x 3072
+  // 3.38 / 2.80, 32 x 15360 3.22 / 2.41; with more, 1024 x 3072 3.73 / 3.85, 512 x 15360 6.05 / 6.16.
+  const int64_t col_chunks = ceil_div(round_up(num_cols / 16, 4), 32 * (4 / static_cast<int64_t>(sizeof(T))));
+  if (round_up(num_rows, 128) / 16 * col_chunks <= sm_count()) {
+    return launch_streaming_as<T, false, kMark, 4>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, kAll, stream);
+  }
+  return launch_streaming_as<T, false, kMark, 16>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, kAll, stream);
 }
 
 // Inputs of more than a quarter of L2 are marked as long as their codes and scales fit in half of it (64 MiB:
@@ -401,9 +436,8 @@ int launch_streaming(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t
                      int64_t num_cols, int hi_first, cudaStream_t stream) {
   const int64_t bytes = orig_rows * num_cols * static_cast<int64_t>(sizeof(T)), written = num_rows * num_cols / 16 * 9;
   const bool mark = bytes > (32ll << 20) && written <= (64ll << 20);
-  auto launch = src.given == nullptr ? (mark ? launch_streaming_as<T, true, true> : launch_streaming_as<T, true, false>)
-                                     : (mark ? launch_streaming_as<T, false, true> : launch_streaming_as<T, false, false>);
-  return launch(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream);
+  return mark ? launch_streaming_marked<T, true>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream)
+              : launch_streaming_marked<T, false>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream);
 }
 
 template <typename T>

@@ -42,3 +42,26 @@ def test_fp32_kernels_agree(cuda_device, rows, cols):
     padded, padded_scales = backend.quantize_nvfp4(x, scale, pad_16x=True)
     assert torch.equal(padded[:rows], codes) and not padded[rows:].any()
     assert torch.equal(padded_scales.view(torch.uint8), block_scales.view(torch.uint8))
+
+
+# on both sides of the lines between blocks of 4 and 16 rows, resident or two passes each, with rows and columns that end inside a block
+@pytest.mark.parametrize("rows, cols, dtype", [(128, 3072, torch.bfloat16), (777, 3072, torch.float16), (896, 3072, torch.bfloat16), (1, 64, torch.bfloat16),
+                                               (6145, 6208, torch.bfloat16), (6143, 6208, torch.float16), (12288, 3104, torch.bfloat16),
+                                               (3100, 6400, torch.float32), (25000, 3088, torch.float32), (18000, 3072, torch.float32)])
+@pytest.mark.parametrize("hi_first", [True, False])
+def test_block_shapes_of_the_static_quantizer(cuda_device, rows, cols, dtype, hi_first):
+    """Against the build of the quantizer that divides every element, whose kernel has one block shape."""
+    from comfy_kitchen.backends import cuda as backend
+
+    lib = backend.load_library()
+    gen = torch.Generator(device=cuda_device).manual_seed(rows)
+    x = torch.randn(rows, cols, generator=gen, device=cuda_device, dtype=torch.float32).to(dtype)
+    g = torch.tensor(0.0021, device=cuda_device)
+    got = backend.quantize_nvfp4(x, g, hi_first=hi_first)
+    before = lib.ck_debug_set_exact_division(1)
+    try:
+        want = backend.quantize_nvfp4(x, g, hi_first=hi_first)
+    finally:
+        lib.ck_debug_set_exact_division(before)
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
