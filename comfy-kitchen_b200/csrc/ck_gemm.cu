@@ -32,15 +32,27 @@ int forced_gemm_config() {
 
 namespace {
 
+// 128 x 64 tiles that find an SM each: half the columns to an epilogue, and more CTAs that load (us, 128 x 128 / 128 x 64: NVFP4 256 x 3072
+// x 3072 7.2 / 6.8, 128 x 9216 x 3072 7.8 / 7.4, 1003 x 1024 x 3072 7.2 / 6.8, 384 x 3072 x 2048 6.1 / 5.7, MXFP8 128 x 9216 x 1536 7.4 / 7.0).
+// With up to 64 rows, half of a tile, only where there are few tiles altogether (NVFP4 64 x 9216 x 3072 7.6 / 8.0).
+bool one_wave_of_half_tiles(int64_t M, int64_t N) { return M > 64 && ceil_div(M, kTileM) * ceil_div(N, 64) <= sm_count(); }
+
 template <Kind KIND, typename OutT, bool FUSED>
 int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, cudaStream_t stream) {
   int config = forced_gemm_config();
   if (config == 0) {
-    const int64_t pair_tiles = ceil_div(p.M, 256) * ceil_div(p.N, 256);
-    if (pair_tiles * 4 >= sm_count()) {
-      config = 4;  // measured: from about a quarter of the SM count in pair tiles the pair wins
-    } else if (ceil_div(p.M, kTileM) * ceil_div(p.N, 128) * 4 <= sm_count()) {
-      config = 7;  // so few 128 x 128 tiles that halving them still leaves SMs idle: more, smaller CTAs
+    const int64_t row_blocks = ceil_div(p.M, kTileM), tiles = row_blocks * ceil_div(p.N, 128);
+    const int k_stages = static_cast<int>(ceil_div(p.k_bytes, kStageKBytes));
+    // The pair, from about a quarter of the SM count in pair tiles on: not where its second CTA would have no rows (us, pair / 128 x 128,
+    // NVFP4 128 x 18432 x 1024 8.0 / 6.0, x 3072 11.4 / 9.4, x 8192 20.1 / 18.3, 128 x 36864 x 3072 17.1 / 15.1, MXFP8 128 x 18432 x 3072
+    // 16.4 / 14.2, the fused epilogue 128 x 12288 x 3072 12.8 / 9.8), and not for up to four stages while a CTA has at most
+    // two of the small tiles (NVFP4 512 x 9216 x 1024 7.4 / 6.7, 256 x 18432 x 1024 8.1 / 7.2, fused 512 x 8192 x 1024 9.7 / 9.4; with six
+    // stages 512 x 9216 x 1536 8.3 / 8.1 and 1003 x 3072 x 1536 7.5 / 7.6, with twelve 512 x 9216 x 3072 10.6 / 11.9).
+    const bool pair = ceil_div(p.M, 256) * ceil_div(p.N, 256) * 4 >= sm_count() && row_blocks > 1 && !(k_stages <= 4 && tiles <= 2 * sm_count());
+    if (pair) {
+      config = 4;
+    } else if (tiles * 4 <= sm_count() || one_wave_of_half_tiles(p.M, p.N)) {
+      config = 7;
     } else {
       config = 1;
     }
@@ -104,6 +116,9 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
     if (clusters >= tiles) break;
   }
   plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
+  // Two CTAs to a tile and up to 32 stages: half tiles instead (us, two CTAs / half tiles: MXFP8 128 x 9216 x 3072 11.8 / 10.4, NVFP4 128 x
+  // 9216 x 8192 14.5 / 13.6; MXFP8 128 x 9216 x 8192, 64 stages, 19.9 / 21.3).
+  if (splits == 2 && !plan->through_workspace && k_stages <= 32 && one_wave_of_half_tiles(M, N)) splits = 1;
   plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
   plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage
   return CK_OK;
