@@ -467,6 +467,14 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int lane = threadIdx.x & 31;
   CK_TRACE3(0);
 
+  // Unsplit one-CTA tiles: ahead of the dependency wait, ask L2 for the first box of B, which is the weight (a prefetch only
+  // warms the cache, L2 being the point of coherence).  One: the requests queue in front of the loads in the TMA unit (NVFP4 us, none
+  // / one / two / four boxes: 512 x 3072 x 3072 7.58 / 7.47 / 7.53 / 7.56, 128 x 18432 x 3072 9.42 / 9.26 / 9.22 / 9.33, 256 x 3072 x 3072
+  // 6.83 / 6.75 / 6.80 / 6.88; split tiles lose, 64 x 3072 x 8192 8.24 / 8.40, and so did pairs).
+  if constexpr (CTAS == 1 && SPLIT == Split::kNone) {
+    if (warp == 0 && worker < p.tiles_m * p.tiles_n && elect_one()) tma_prefetch_2d(&map_b, 0, tile_col_block(p, worker) * TILE_N);
+  }
+
   // ------------------------------------------------------------------ set-up
   // The producer warp creates the barriers and goes straight to its loads; the other warps
   // meet it at a named barrier it only arrives on (tensor memory is allocated meanwhile).
