@@ -637,8 +637,8 @@ int scaled_mm_small_m(bool is_mxfp8, const void* a, const void* b, const void* s
 }
 
 // What is quantized inside the GEMM; everything else, wrong arguments among it, is left to the separate calls.
-bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const void* w, const void* w_scales, int bias_dtype, int out_dtype,
-                            int64_t M, int64_t N, int64_t K) {
+bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const void* w, const void* w_scales, int bias_dtype, const void* out,
+                            int out_dtype, int64_t M, int64_t N, int64_t K) {
   auto aligned = [](const void* p, uintptr_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; };
   auto is_float = [](int dtype) { return dtype == CK_DTYPE_F32 || dtype == CK_DTYPE_F16 || dtype == CK_DTYPE_BF16; };
   // Up to 8 rows of NVFP4 and 16 of MXFP8, whose rows take half the threads, the quantizer's warps keep up with the stream.
@@ -646,7 +646,11 @@ bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const voi
   // 16 x 6144 x 3072 9.2 / 10.2; MXFP8 16 x 3072 x 3072 7.3 / 5.8, 16 x 18432 x 12288 42.8 / 41.9.
   const int64_t limit = is_mxfp8 ? 16 : 8;
   const int forced = forced_gemm_config();
-  return M <= limit && small_m_applies(M, N, K) && N % 8 == 0 && K % 32 == 0 && K <= (1 << 28) && is_float(x_dtype) && is_float(out_dtype) &&
+  // A result written over its own activation is for the separate kernels: here every CTA reads all of x until it ends.
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), out0 = reinterpret_cast<uintptr_t>(out);
+  auto bytes = [](int dtype, int64_t n) { return static_cast<uintptr_t>(n) * (dtype == CK_DTYPE_F32 ? 4 : 2); };
+  const bool apart = x0 + bytes(x_dtype, M * K) <= out0 || out0 + bytes(out_dtype, M * N) <= x0;
+  return apart && M <= limit && small_m_applies(M, N, K) && N % 8 == 0 && K % 32 == 0 && K <= (1 << 28) && is_float(x_dtype) && is_float(out_dtype) &&
          is_float(bias_dtype) && aligned(x, 32) && aligned(w, 16) && aligned(w_scales, 16) && !exact_division() && (forced == 0 || forced == 9);
 }
 

@@ -58,7 +58,7 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   uint8_t* codes = ws + l.codes_off;
   uint8_t* scales = ws + l.scales_off;
-  if (linear_small_m_applies(false, x, x_dtype, w_codes, w_block_scales, bias == nullptr ? out_dtype : bias_dtype, out_dtype, M, N, K)) {
+  if (linear_small_m_applies(false, x, x_dtype, w_codes, w_block_scales, bias == nullptr ? out_dtype : bias_dtype, out, out_dtype, M, N, K)) {
     const int64_t elem = x_dtype == CK_DTYPE_F32 ? 4 : 2;
     float* partials = nullptr;
     int n_partials = 0;
@@ -102,7 +102,7 @@ extern "C" int ck_linear_mxfp8_from_float(const void* x, int x_dtype, const void
   const int64_t need = ck_linear_mxfp8_from_float_workspace_bytes(M, K);
   CK_REQUIRE(workspace_bytes >= need, "linear_mxfp8_from_float: workspace of %lld bytes, %lld needed",
              (long long)workspace_bytes, (long long)need);
-  if (linear_small_m_applies(true, x, x_dtype, w_data, w_block_scales, bias == nullptr ? out_dtype : bias_dtype, out_dtype, M, N, K)) {
+  if (linear_small_m_applies(true, x, x_dtype, w_data, w_block_scales, bias == nullptr ? out_dtype : bias_dtype, out, out_dtype, M, N, K)) {
     return linear_small_m(true, x, x_dtype, nullptr, nullptr, 0, w_data, w_block_scales, nullptr, bias, bias_dtype, out, out_dtype, M, N, K,
                           static_cast<cudaStream_t>(stream));
   }
