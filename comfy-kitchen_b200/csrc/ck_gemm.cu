@@ -289,7 +289,7 @@ int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, con
     os.col_offset = 0;
   }
   if (!fused.enabled && out_spec == nullptr) {
-    // Few activation rows: the weight-streaming path (operands swapped, K split over all SMs).
+    // Few activation rows: the weight-streaming path (weight rows in the MMA's M, K split over clusters).
     // CK_GEMM_CONFIG=9 forces it, any other forced configuration keeps it off.
     if (small_m_applies(M, N, K) && (forced_gemm_config() == 0 || forced_gemm_config() == 9)) {
       return scaled_mm_small_m(KIND == Kind::kMxfp8, a, b, sfa, sfb, tsa, tsb, alpha, bias, bias_dtype, out, out_dtype, M, N, K, s);
