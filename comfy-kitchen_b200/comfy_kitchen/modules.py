@@ -193,7 +193,7 @@ class NVFP4Linear(_QuantizedLinearBase):
         if host is not None and w is not None and type(x) is torch.Tensor and not w._params.transposed:
             # a plain eager call (None for any other): 9 us of host time instead of 18
             params = w._params
-            y = host.linear_nvfp4_from_float(x, w._qdata, params.scale, params.block_scale, held.get("bias"),
+            y = host.linear_nvfp4_from_float(x, w._qdata, params.scale, params.block_scale, held["bias"] if "bias" in held else self.bias,
                                              held["input_scale"] if "input_scale" in held else self.input_scale, x.dtype)
             if y is not None and y.shape[1] == self.out_features:
                 return y
@@ -269,7 +269,7 @@ class MXFP8Linear(_QuantizedLinearBase):
         held = self._parameters
         host, w = host_half(), held.get("weight")
         if host is not None and w is not None and type(x) is torch.Tensor and not getattr(w._params, "transposed", False):
-            y = host.linear_mxfp8_from_float(x, w._qdata, w._params.scale, held.get("bias"), x.dtype)
+            y = host.linear_mxfp8_from_float(x, w._qdata, w._params.scale, held["bias"] if "bias" in held else self.bias, x.dtype)
             if y is not None and y.shape[1] == self.out_features:
                 return y
         w = self.weight
