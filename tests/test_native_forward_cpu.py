@@ -69,3 +69,12 @@ def test_bias_wherever_the_layer_holds_it(host, layout, held):
     layer(torch.zeros(4, 64, dtype=torch.bfloat16))
     (got,) = host.calls
     assert got is None if held == "none" else torch.equal(got, layer.bias)
+
+
+@pytest.mark.parametrize("out_features", [32, 40])  # 40: the weight has 48 or 64 rows
+@pytest.mark.parametrize("layout", ["nvfp4", "mxfp8"])
+def test_padded_weight_rows_are_cut_from_the_native_result(host, layout, out_features):
+    """One native call, whose result is the layer's."""
+    y = _layer(layout, out_features, bias=False)(torch.zeros(4, 64, dtype=torch.bfloat16))
+    assert len(host.calls) == 1
+    assert y.shape == (4, out_features) and torch.equal(y[3], torch.arange(float(out_features)).bfloat16())

@@ -47,3 +47,34 @@ def test_bias_wherever_the_layer_holds_it(cuda_device, layout, m, held):
         layer.parametrizations.bias.original.data.div_(2)  # a power of two: the same bias
     with torch.inference_mode():
         assert torch.equal(layer(x), plain)
+
+
+@pytest.mark.parametrize("m, n", [(1, 1000), (8, 200), (40, 1000), (300, 1000)])
+@pytest.mark.parametrize("layout", ["nvfp4", "mxfp8"])
+def test_padded_out_features(cuda_device, monkeypatch, layout, m, n):
+    """out_features that are no whole blocks, without a bias: the layout path's bits from one native call."""
+    from comfy_kitchen.backends import cuda as backend
+    from comfy_kitchen.modules import _QuantizedLinearBase
+
+    layer, x = _layer(layout, 512, n, False, cuda_device), _x(m, 512, cuda_device)
+    name = f"linear_{layout}_from_float"
+    native, taken = backend._host, []
+
+    class Counting:
+        def __getattr__(self, attribute):
+            fn = getattr(native, attribute)
+            if attribute != name:
+                return fn
+
+            def call(*args):
+                out = fn(*args)
+                taken.append(out is not None)
+                return out
+            return call
+
+    with torch.inference_mode():
+        want = _QuantizedLinearBase.forward(layer, x)
+        monkeypatch.setattr(backend, "_host", Counting())
+        got = layer(x)
+    assert got.shape == (m, n) and torch.equal(got, want)
+    assert taken == [True]
