@@ -793,6 +793,8 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       if (warp == 2) CK_TRACE(6);
       mbar_wait(&acc_full_bar[acc], acc_ph, abort_flag);  // in a pair: committed from the leader CTA
       if (warp == 2) CK_TRACE(7);
+      // the aligned loads below want the whole warp, of which the last tile's epilogue may have sent the rows past M another way
+      if constexpr (FUSED) __syncwarp();
       tc_fence_after_sync();
       const int c0 = half * kColsPerWarp;
       const uint32_t t_row = tmem_base + acc * Cfg::kAccCols + (static_cast<uint32_t>(quarter * 32) << 16) + c0;

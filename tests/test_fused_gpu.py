@@ -75,6 +75,26 @@ def test_fused_requant_equals_quantizer_on_its_own_output(env, cuda_device, shap
         assert torch.equal(codes_only, codes) and torch.equal(scales_only.view(torch.uint8), scales.view(torch.uint8))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m", [257, 1003])  # the last warp has rows on both sides of m
+@pytest.mark.parametrize("config", [0, 1, 3, 4])
+def test_ragged_rows_with_several_tiles_to_a_cta(env, cuda_device, monkeypatch, config, m, dtype):
+    """Codes alone (rows and padding rows of a warp part there) are the codes that come with the dense output."""
+    ck, backend = env
+    n, k = 12288, 256  # at least 96 pairs of tiles and 288 small ones: more than fit 148 SMs
+    monkeypatch.setenv("CK_GEMM_CONFIG", str(config))
+    rq_scale = torch.tensor(0.0045, device=cuda_device)
+    for seed in (1, 2, 3):
+        qx, bsx, sx, qw, bsw, sw, bias = _setup(ck, cuda_device, m, n, k, seed)
+        args = dict(bias=bias, activation="gelu_tanh", out_dtype=dtype, requant_scale=rq_scale)
+        h, codes, scales = backend.linear_nvfp4_fused(qx, qw, sx, sw, bsx, bsw, **args)
+        none, codes_only, scales_only = backend.linear_nvfp4_fused(qx, qw, sx, sw, bsx, bsw, return_dense=False, **args)
+        assert none is None and torch.equal(codes_only, codes) and torch.equal(scales_only.view(torch.uint8), scales.view(torch.uint8))
+        q, s = ck.quantize_nvfp4(h, rq_scale, pad_16x=True)
+        assert torch.equal(q[:m], codes) and torch.equal(s.view(torch.uint8), scales.view(torch.uint8))
+    backend.check_device_status("ragged rows, several tiles")
+
+
 def test_mlp_pair_fused_matches_unfused(env, cuda_device):
     """fc1 -> GELU -> re-quantize (fused) -> fc2 equals the unfused chain that quantizes the dense hidden."""
     ck, backend = env
