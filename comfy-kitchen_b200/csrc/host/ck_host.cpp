@@ -76,68 +76,57 @@ bool quiet() {
   return strict == nullptr || strict[0] != '1' || strict[1] != 0;
 }
 
-struct NotPlain {};  // thrown to leave a call to the Python wrapper
+// What follows refuses a call by a null pointer or false, never by an exception: the Python wrapper, whose call it then is, should not
+// pay for having asked (0.2 us; 1.3 to 1.7 with a C++ exception).
 
-void require(bool ok) {
-  if (!ok) throw NotPlain{};
-}
-
-// A plain dense CUDA tensor on the current device, of no autograd graph.
-const Tensor& plain(PyObject* o, int device) {
-  require(Py_TYPE(o) == reinterpret_cast<PyTypeObject*>(THPVariableClass) || Py_TYPE(o) == parameter_type);
+// A plain dense CUDA tensor on the current device, of no autograd graph; null for anything else.
+const Tensor* plain(PyObject* o, int device) {
+  if (Py_TYPE(o) != reinterpret_cast<PyTypeObject*>(THPVariableClass) && Py_TYPE(o) != parameter_type) return nullptr;
   const Tensor& t = THPVariable_Unpack(o);
   static const c10::DispatchKeySet usual = c10::DispatchKeySet(c10::DispatchKey::CUDA) | c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA) |
                                            c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) |
                                            c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA);
-  require(usual.has_all(t.key_set()) && t.is_cuda() && t.get_device() == device && t.is_contiguous() && !(t.requires_grad() && c10::GradMode::is_enabled()));
-  return t;
+  const bool ok = usual.has_all(t.key_set()) && t.is_cuda() && t.get_device() == device && t.is_contiguous() &&
+                  !(t.requires_grad() && c10::GradMode::is_enabled());
+  return ok ? &t : nullptr;
 }
 
-const Tensor& matrix(PyObject* o, int device) {
-  const Tensor& t = plain(o, device);
-  require(t.dim() == 2 && t.size(0) > 0 && t.size(1) > 0);
-  return t;
+const Tensor* matrix(PyObject* o, int device) {
+  const Tensor* t = plain(o, device);
+  return t != nullptr && t->dim() == 2 && t->size(0) > 0 && t->size(1) > 0 ? t : nullptr;
 }
 
-const Tensor& matrix(PyObject* o, int device, ScalarType type) {
-  const Tensor& t = matrix(o, device);
-  require(t.scalar_type() == type);
-  return t;
+const Tensor* matrix(PyObject* o, int device, ScalarType type) {
+  const Tensor* t = matrix(o, device);
+  return t != nullptr && t->scalar_type() == type ? t : nullptr;
 }
 
 const float* scalar(PyObject* o, int device) {
-  const Tensor& t = plain(o, device);
-  require(t.scalar_type() == ScalarType::Float && t.numel() == 1);
-  return static_cast<const float*>(t.const_data_ptr());
+  const Tensor* t = plain(o, device);
+  return t != nullptr && t->scalar_type() == ScalarType::Float && t->numel() == 1 ? static_cast<const float*>(t->const_data_ptr()) : nullptr;
 }
 
 struct Bias {
   const void* ptr = nullptr;
   int code = 0;
 };
-Bias bias_of(PyObject* o, int device, int64_t n) {
-  Bias b;
-  if (o == Py_None) return b;
-  const Tensor& t = plain(o, device);
-  b.code = code_of(t.scalar_type());
-  require(b.code >= 0 && t.numel() == n);
-  b.ptr = t.const_data_ptr();
-  return b;
+bool bias_of(PyObject* o, int device, int64_t n, Bias* b) {
+  if (o == Py_None) return true;
+  const Tensor* t = plain(o, device);
+  if (t == nullptr || code_of(t->scalar_type()) < 0 || t->numel() != n) return false;
+  b->code = code_of(t->scalar_type());
+  b->ptr = t->const_data_ptr();
+  return true;
 }
 
-void scales_fit(const Tensor& s, int64_t rows, int64_t columns) { require(s.size(0) == round_up(rows, 128) && s.size(1) == round_up(columns, 4)); }
+bool scales_fit(const Tensor& s, int64_t rows, int64_t columns) { return s.size(0) == round_up(rows, 128) && s.size(1) == round_up(columns, 4); }
 
-ScalarType dtype_of(PyObject* o, ScalarType otherwise) {
-  if (o == Py_None) return otherwise;
-  require(THPDtype_Check(o));
-  const ScalarType t = reinterpret_cast<THPDtype*>(o)->scalar_type;
-  require(code_of(t) >= 0);
-  return t;
-}
-
-bool flag(PyObject* o) {
-  require(PyBool_Check(o));
-  return o == Py_True;
+// A dense type that the caller names; `*type` stays what it is for None.
+bool dtype_of(PyObject* o, ScalarType* type) {
+  if (o == Py_None) return true;
+  if (!THPDtype_Check(o)) return false;
+  *type = reinterpret_cast<THPDtype*>(o)->scalar_type;
+  return code_of(*type) >= 0;
 }
 
 Tensor result(at::IntArrayRef sizes, ScalarType type, int device) {
@@ -161,13 +150,16 @@ struct Call {
   Call() : device(c10::cuda::current_device()), stream(c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream()) {}
 };
 
-template <typename Launch>
-void launched(Launch&& launch) {
-  int rc;
-  Py_BEGIN_ALLOW_THREADS;
-  rc = launch();
-  Py_END_ALLOW_THREADS;
-  require(rc == 0);
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
+// A call of the library without the GIL (its arguments were evaluated with it); false: refused.
+template <typename... P, typename... A>
+bool launched(int (*fn)(P...), A... args) {
+  const WithoutGil released;
+  return fn(args...) == 0;
 }
 
 PyObject* pair(Tensor a, Tensor b) {
@@ -178,12 +170,14 @@ PyObject* pair(Tensor a, Tensor b) {
   return t;
 }
 
-// Runs `body`; anything that it does not take, or that goes wrong in it, is the Python wrapper's.
+// What `body` returns; None when that is null (refused) or something goes wrong in it: the call is the Python wrapper's then.
 template <typename Body>
 PyObject* or_none(PyObject* const* args, Py_ssize_t got, Py_ssize_t wanted, Body&& body) {
   try {
-    if (got == wanted && THPVariable_Check(args[0]) && THPVariable_Unpack(args[0]).is_cuda() && quiet()) return body();
-  } catch (const NotPlain&) {
+    if (got == wanted && THPVariable_Check(args[0]) && THPVariable_Unpack(args[0]).is_cuda() && quiet()) {
+      PyObject* r = body();
+      if (r != nullptr || PyErr_Occurred() != nullptr) return r;
+    }
   } catch (const std::exception&) {
   }
   Py_RETURN_NONE;
@@ -195,18 +189,19 @@ using Args = PyObject* const*;
 PyObject* quantize_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // x, per_tensor_scale, pad_16x, hi_first
   return or_none(a, n_args, 4, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device);
-    const int code = code_of(x.scalar_type());
+    const Tensor* x = matrix(a[0], c.device);
     const float* scale = scalar(a[1], c.device);
-    const bool pad = flag(a[2]), hi_first = flag(a[3]);
-    const int64_t rows = x.size(0), cols = x.size(1), out_rows = pad ? round_up(rows, 16) : rows, out_cols = pad ? round_up(cols, 16) : cols;
-    require(code >= 0 && out_cols % 16 == 0);
+    if (x == nullptr || scale == nullptr || !PyBool_Check(a[2]) || !PyBool_Check(a[3])) return nullptr;
+    const int code = code_of(x->scalar_type());
+    const bool pad = a[2] == Py_True, hi_first = a[3] == Py_True;
+    const int64_t rows = x->size(0), cols = x->size(1), out_rows = pad ? round_up(rows, 16) : rows, out_cols = pad ? round_up(cols, 16) : cols;
+    if (code < 0 || out_cols % 16 != 0) return nullptr;
     Tensor q = result({out_rows, out_cols / 2}, ScalarType::Byte, c.device);
     Tensor s = result({round_up(out_rows, 128), round_up(out_cols / 16, 4)}, ScalarType::Float8_e4m3fn, c.device);
-    launched([&] {
-      return lib.quantize_nvfp4(x.const_data_ptr(), code, scale, q.mutable_data_ptr(), s.mutable_data_ptr(), rows, cols, out_rows, out_cols, hi_first,
-                                c.stream);
-    });
+    if (!launched(lib.quantize_nvfp4, x->const_data_ptr(), code, scale, q.mutable_data_ptr(), s.mutable_data_ptr(), rows, cols, out_rows, out_cols,
+                  hi_first, c.stream)) {
+      return nullptr;
+    }
     return pair(std::move(q), std::move(s));
   });
 }
@@ -214,27 +209,29 @@ PyObject* quantize_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // x, per_tens
 PyObject* quantize_nvfp4_dynamic(PyObject*, Args a, Py_ssize_t n_args) {  // x, pad_16x, hi_first, scratch or None
   return or_none(a, n_args, 4, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device);
-    const int code = code_of(x.scalar_type());
-    const bool pad = flag(a[1]), hi_first = flag(a[2]);
-    const int64_t rows = x.size(0), cols = x.size(1), out_rows = pad ? round_up(rows, 16) : rows, out_cols = pad ? round_up(cols, 16) : cols;
+    const Tensor* x = matrix(a[0], c.device);
+    if (x == nullptr || !PyBool_Check(a[1]) || !PyBool_Check(a[2])) return nullptr;
+    const int code = code_of(x->scalar_type());
+    const bool pad = a[1] == Py_True, hi_first = a[2] == Py_True;
+    const int64_t rows = x->size(0), cols = x->size(1), out_rows = pad ? round_up(rows, 16) : rows, out_cols = pad ? round_up(cols, 16) : cols;
     // the streaming quantizer's form; the one-kernel scale's scratch is the Python wrapper's
-    require(code >= 0 && out_cols == cols && cols % (64 / x.element_size()) == 0 && reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 32 == 0);
+    if (code < 0 || out_cols != cols || cols % (64 / x->element_size()) != 0 || reinterpret_cast<uintptr_t>(x->const_data_ptr()) % 32 != 0) return nullptr;
+    const int64_t need = lib.quantize_nvfp4_dynamic_scratch_bytes(rows * cols);
+    void* scratch = nullptr;
+    if (a[3] != Py_None) {
+      const Tensor* given = plain(a[3], c.device);
+      if (given == nullptr || given->scalar_type() != ScalarType::Byte || given->numel() < need) return nullptr;
+      scratch = given->mutable_data_ptr();
+    }
+    Workspace ws(scratch == nullptr ? need : 0);
+    if (scratch == nullptr) scratch = ws.ptr();
     Tensor q = result({out_rows, out_cols / 2}, ScalarType::Byte, c.device);
     Tensor s = result({round_up(out_rows, 128), round_up(out_cols / 16, 4)}, ScalarType::Float8_e4m3fn, c.device);
     Tensor scale = result({}, ScalarType::Float, c.device);
-    const int64_t need = lib.quantize_nvfp4_dynamic_scratch_bytes(rows * cols);
-    Workspace ws(a[3] == Py_None ? need : 0);
-    void* scratch = ws.ptr();
-    if (a[3] != Py_None) {
-      const Tensor& given = plain(a[3], c.device);
-      require(given.scalar_type() == ScalarType::Byte && given.numel() >= need);
-      scratch = given.mutable_data_ptr();
+    if (!launched(lib.quantize_nvfp4_dynamic, x->const_data_ptr(), code, static_cast<float*>(scale.mutable_data_ptr()), q.mutable_data_ptr(),
+                  s.mutable_data_ptr(), rows, cols, out_rows, out_cols, hi_first, scratch, need, c.stream)) {
+      return nullptr;
     }
-    launched([&] {
-      return lib.quantize_nvfp4_dynamic(x.const_data_ptr(), code, static_cast<float*>(scale.mutable_data_ptr()), q.mutable_data_ptr(), s.mutable_data_ptr(),
-                                        rows, cols, out_rows, out_cols, hi_first, scratch, need, c.stream);
-    });
     PyObject* t = PyTuple_New(3);
     if (t == nullptr) return nullptr;
     PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(q)));
@@ -247,16 +244,17 @@ PyObject* quantize_nvfp4_dynamic(PyObject*, Args a, Py_ssize_t n_args) {  // x, 
 PyObject* quantize_mxfp8(PyObject*, Args a, Py_ssize_t n_args) {  // x, pad_32x
   return or_none(a, n_args, 2, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device);
-    const int code = code_of(x.scalar_type());
-    const bool pad = flag(a[1]);
-    const int64_t rows = x.size(0), cols = x.size(1), out_rows = pad ? round_up(rows, 32) : rows, out_cols = pad ? round_up(cols, 32) : cols;
-    require(code >= 0 && out_cols % 32 == 0);
+    const Tensor* x = matrix(a[0], c.device);
+    if (x == nullptr || !PyBool_Check(a[1])) return nullptr;
+    const int code = code_of(x->scalar_type());
+    const bool pad = a[1] == Py_True;
+    const int64_t rows = x->size(0), cols = x->size(1), out_rows = pad ? round_up(rows, 32) : rows, out_cols = pad ? round_up(cols, 32) : cols;
+    if (code < 0 || out_cols % 32 != 0) return nullptr;
     Tensor q = result({out_rows, out_cols}, ScalarType::Float8_e4m3fn, c.device);
     Tensor s = result({round_up(out_rows, 128), round_up(out_cols / 32, 4)}, ScalarType::Float8_e8m0fnu, c.device);
-    launched([&] {
-      return lib.quantize_mxfp8(x.const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), rows, cols, out_rows, out_cols, c.stream);
-    });
+    if (!launched(lib.quantize_mxfp8, x->const_data_ptr(), code, q.mutable_data_ptr(), s.mutable_data_ptr(), rows, cols, out_rows, out_cols, c.stream)) {
+      return nullptr;
+    }
     return pair(std::move(q), std::move(s));
   });
 }
@@ -264,19 +262,19 @@ PyObject* quantize_mxfp8(PyObject*, Args a, Py_ssize_t n_args) {  // x, pad_32x
 PyObject* dequantize_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // qx, per_tensor_scale, block_scales, output_type, hi_first
   return or_none(a, n_args, 5, [&]() -> PyObject* {
     const Call c;
-    const Tensor& q = matrix(a[0], c.device, ScalarType::Byte);
+    const Tensor* q = matrix(a[0], c.device, ScalarType::Byte);
     const float* scale = scalar(a[1], c.device);
-    const Tensor& s = matrix(a[2], c.device, ScalarType::Float8_e4m3fn);
-    require(a[3] != Py_None);
-    const ScalarType type = dtype_of(a[3], ScalarType::BFloat16);
-    const bool hi_first = flag(a[4]);
-    const int64_t rows = q.size(0), cols = 2 * q.size(1);
-    require(cols % 16 == 0);
-    scales_fit(s, rows, cols / 16);
+    const Tensor* s = matrix(a[2], c.device, ScalarType::Float8_e4m3fn);
+    ScalarType type = ScalarType::BFloat16;
+    if (q == nullptr || scale == nullptr || s == nullptr || a[3] == Py_None || !dtype_of(a[3], &type) || !PyBool_Check(a[4])) return nullptr;
+    const bool hi_first = a[4] == Py_True;
+    const int64_t rows = q->size(0), cols = 2 * q->size(1);
+    if (cols % 16 != 0 || !scales_fit(*s, rows, cols / 16)) return nullptr;
     Tensor out = result({rows, cols}, type, c.device);
-    launched([&] {
-      return lib.dequantize_nvfp4(q.const_data_ptr(), scale, s.const_data_ptr(), out.mutable_data_ptr(), code_of(type), rows, cols, hi_first, c.stream);
-    });
+    if (!launched(lib.dequantize_nvfp4, q->const_data_ptr(), scale, s->const_data_ptr(), out.mutable_data_ptr(), code_of(type), rows, cols, hi_first,
+                  c.stream)) {
+      return nullptr;
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -284,17 +282,14 @@ PyObject* dequantize_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // qx, per_t
 PyObject* dequantize_mxfp8(PyObject*, Args a, Py_ssize_t n_args) {  // qx, block_scales, output_type
   return or_none(a, n_args, 3, [&]() -> PyObject* {
     const Call c;
-    const Tensor& q = matrix(a[0], c.device, ScalarType::Float8_e4m3fn);
-    const Tensor& s = matrix(a[1], c.device, ScalarType::Float8_e8m0fnu);
-    require(a[2] != Py_None);
-    const ScalarType type = dtype_of(a[2], ScalarType::BFloat16);
-    const int64_t rows = q.size(0), cols = q.size(1);
-    require(cols % 32 == 0);
-    scales_fit(s, rows, cols / 32);
+    const Tensor* q = matrix(a[0], c.device, ScalarType::Float8_e4m3fn);
+    const Tensor* s = matrix(a[1], c.device, ScalarType::Float8_e8m0fnu);
+    ScalarType type = ScalarType::BFloat16;
+    if (q == nullptr || s == nullptr || a[2] == Py_None || !dtype_of(a[2], &type)) return nullptr;
+    const int64_t rows = q->size(0), cols = q->size(1);
+    if (cols % 32 != 0 || !scales_fit(*s, rows, cols / 32)) return nullptr;
     Tensor out = result({rows, cols}, type, c.device);
-    launched([&] {
-      return lib.dequantize_mxfp8(q.const_data_ptr(), s.const_data_ptr(), out.mutable_data_ptr(), code_of(type), rows, cols, c.stream);
-    });
+    if (!launched(lib.dequantize_mxfp8, q->const_data_ptr(), s->const_data_ptr(), out.mutable_data_ptr(), code_of(type), rows, cols, c.stream)) return nullptr;
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -303,26 +298,30 @@ PyObject* dequantize_mxfp8(PyObject*, Args a, Py_ssize_t n_args) {  // qx, block
 PyObject* scaled_mm_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // a, b, scales of tensors and blocks (a, b each), bias, out_dtype, alpha
   return or_none(a, n_args, 9, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device, ScalarType::Byte);
-    const Tensor& w = matrix(a[1], c.device, ScalarType::Byte);
+    const Tensor* x = matrix(a[0], c.device, ScalarType::Byte);
+    const Tensor* w = matrix(a[1], c.device, ScalarType::Byte);
     const float* tsa = scalar(a[2], c.device);
     const float* tsb = scalar(a[3], c.device);
-    const Tensor& sa = matrix(a[4], c.device, ScalarType::Float8_e4m3fn);
-    const Tensor& sb = matrix(a[5], c.device, ScalarType::Float8_e4m3fn);
-    const int64_t m = x.size(0), n = w.size(0), k = 2 * x.size(1);
-    require(w.size(1) == x.size(1) && k % 32 == 0 && n % 8 == 0);
-    scales_fit(sa, m, k / 16);
-    scales_fit(sb, n, k / 16);
-    const Bias bias = bias_of(a[6], c.device, n);
-    const ScalarType type = dtype_of(a[7], ScalarType::BFloat16);
+    const Tensor* sa = matrix(a[4], c.device, ScalarType::Float8_e4m3fn);
+    const Tensor* sb = matrix(a[5], c.device, ScalarType::Float8_e4m3fn);
     const float* alpha = a[8] == Py_None ? nullptr : scalar(a[8], c.device);
+    if (x == nullptr || w == nullptr || tsa == nullptr || tsb == nullptr || sa == nullptr || sb == nullptr || (alpha == nullptr && a[8] != Py_None)) {
+      return nullptr;
+    }
+    const int64_t m = x->size(0), n = w->size(0), k = 2 * x->size(1);
+    Bias bias;
+    ScalarType type = ScalarType::BFloat16;
+    if (w->size(1) != x->size(1) || k % 32 != 0 || n % 8 != 0 || !scales_fit(*sa, m, k / 16) || !scales_fit(*sb, n, k / 16) ||
+        !bias_of(a[6], c.device, n, &bias) || !dtype_of(a[7], &type)) {
+      return nullptr;
+    }
     Tensor out = result({m, n}, type, c.device);
     const int64_t need = lib.scaled_mm_workspace_bytes(0, m, n, k);
     Workspace ws(need > kOnChip ? need : 0);
-    launched([&] {
-      return lib.scaled_mm_nvfp4_ws(x.const_data_ptr(), w.const_data_ptr(), sa.const_data_ptr(), sb.const_data_ptr(), tsa, tsb, alpha, bias.ptr, bias.code,
-                                    out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream);
-    });
+    if (!launched(lib.scaled_mm_nvfp4_ws, x->const_data_ptr(), w->const_data_ptr(), sa->const_data_ptr(), sb->const_data_ptr(), tsa, tsb, alpha, bias.ptr,
+                  bias.code, out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream)) {
+      return nullptr;
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -330,55 +329,58 @@ PyObject* scaled_mm_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // a, b, scal
 PyObject* scaled_mm_mxfp8(PyObject*, Args a, Py_ssize_t n_args) {  // a, b, block scales of a, of b, bias, out_dtype
   return or_none(a, n_args, 6, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device, ScalarType::Float8_e4m3fn);
-    const Tensor& w = matrix(a[1], c.device, ScalarType::Float8_e4m3fn);
-    const Tensor& sa = matrix(a[2], c.device, ScalarType::Float8_e8m0fnu);
-    const Tensor& sb = matrix(a[3], c.device, ScalarType::Float8_e8m0fnu);
-    const int64_t m = x.size(0), n = w.size(0), k = x.size(1);
-    require(w.size(1) == k && k % 32 == 0 && n % 8 == 0);
-    scales_fit(sa, m, k / 32);
-    scales_fit(sb, n, k / 32);
-    const Bias bias = bias_of(a[4], c.device, n);
-    const ScalarType type = dtype_of(a[5], ScalarType::BFloat16);
+    const Tensor* x = matrix(a[0], c.device, ScalarType::Float8_e4m3fn);
+    const Tensor* w = matrix(a[1], c.device, ScalarType::Float8_e4m3fn);
+    const Tensor* sa = matrix(a[2], c.device, ScalarType::Float8_e8m0fnu);
+    const Tensor* sb = matrix(a[3], c.device, ScalarType::Float8_e8m0fnu);
+    if (x == nullptr || w == nullptr || sa == nullptr || sb == nullptr) return nullptr;
+    const int64_t m = x->size(0), n = w->size(0), k = x->size(1);
+    Bias bias;
+    ScalarType type = ScalarType::BFloat16;
+    if (w->size(1) != k || k % 32 != 0 || n % 8 != 0 || !scales_fit(*sa, m, k / 32) || !scales_fit(*sb, n, k / 32) ||
+        !bias_of(a[4], c.device, n, &bias) || !dtype_of(a[5], &type)) {
+      return nullptr;
+    }
     Tensor out = result({m, n}, type, c.device);
     const int64_t need = lib.scaled_mm_workspace_bytes(1, m, n, k);
     Workspace ws(need > kOnChip ? need : 0);
-    launched([&] {
-      return lib.scaled_mm_mxfp8_ws(x.const_data_ptr(), w.const_data_ptr(), sa.const_data_ptr(), sb.const_data_ptr(), bias.ptr, bias.code,
-                                    out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream);
-    });
+    if (!launched(lib.scaled_mm_mxfp8_ws, x->const_data_ptr(), w->const_data_ptr(), sa->const_data_ptr(), sb->const_data_ptr(), bias.ptr, bias.code,
+                  out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream)) {
+      return nullptr;
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
 
 // ---- one-call linears -------------------------------------------------------------------------
-ScalarType linear_type(PyObject* o, ScalarType x) {
-  return dtype_of(o, x == ScalarType::Half || x == ScalarType::BFloat16 ? x : ScalarType::BFloat16);
-}
+ScalarType linear_type(ScalarType x) { return x == ScalarType::Half ? x : ScalarType::BFloat16; }  // of a result whose type nobody names
 
 PyObject* linear_nvfp4_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x, w_codes, w_scale, w_block_scales, bias, x_scale, out_dtype
   return or_none(a, n_args, 7, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device);
-    const int code = code_of(x.scalar_type());
-    const Tensor& w = matrix(a[1], c.device, ScalarType::Byte);
+    const Tensor* x = matrix(a[0], c.device);
+    const Tensor* w = matrix(a[1], c.device, ScalarType::Byte);
     const float* w_scale = scalar(a[2], c.device);
-    const Tensor& sw = matrix(a[3], c.device, ScalarType::Float8_e4m3fn);
-    const int64_t m = x.size(0), k = x.size(1), n = w.size(0);
-    require(code >= 0 && 2 * w.size(1) == k && k % 32 == 0 && n % 8 == 0);
-    scales_fit(sw, n, k / 16);
-    const Bias bias = bias_of(a[4], c.device, n);
+    const Tensor* sw = matrix(a[3], c.device, ScalarType::Float8_e4m3fn);
     const float* x_scale = a[5] == Py_None ? nullptr : scalar(a[5], c.device);
-    require(x_scale != nullptr || reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 32 == 0);  // else the one-kernel scale comes first
-    const ScalarType type = linear_type(a[6], x.scalar_type());
+    if (x == nullptr || w == nullptr || w_scale == nullptr || sw == nullptr || (x_scale == nullptr && a[5] != Py_None)) return nullptr;
+    const int code = code_of(x->scalar_type());
+    const int64_t m = x->size(0), k = x->size(1), n = w->size(0);
+    Bias bias;
+    ScalarType type = linear_type(x->scalar_type());
+    if (code < 0 || 2 * w->size(1) != k || k % 32 != 0 || n % 8 != 0 || !scales_fit(*sw, n, k / 16) || !bias_of(a[4], c.device, n, &bias) ||
+        !dtype_of(a[6], &type)) {
+      return nullptr;
+    }
+    if (x_scale == nullptr && reinterpret_cast<uintptr_t>(x->const_data_ptr()) % 32 != 0) return nullptr;  // the one-kernel scale comes first
     const int64_t need = lib.linear_nvfp4_from_float_workspace_bytes(m, k, x_scale == nullptr);
-    require(need > 0);
+    if (need <= 0) return nullptr;
     Workspace ws(need);
     Tensor out = result({m, n}, type, c.device);
-    launched([&] {
-      return lib.linear_nvfp4_from_float(x.const_data_ptr(), code, x_scale, w.const_data_ptr(), sw.const_data_ptr(), w_scale, bias.ptr, bias.code,
-                                         out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream);
-    });
+    if (!launched(lib.linear_nvfp4_from_float, x->const_data_ptr(), code, x_scale, w->const_data_ptr(), sw->const_data_ptr(), w_scale, bias.ptr, bias.code,
+                  out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream)) {
+      return nullptr;
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -386,23 +388,26 @@ PyObject* linear_nvfp4_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x,
 PyObject* linear_mxfp8_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x, w_data, w_block_scales, bias, out_dtype
   return or_none(a, n_args, 5, [&]() -> PyObject* {
     const Call c;
-    const Tensor& x = matrix(a[0], c.device);
-    const int code = code_of(x.scalar_type());
-    const Tensor& w = matrix(a[1], c.device, ScalarType::Float8_e4m3fn);
-    const Tensor& sw = matrix(a[2], c.device, ScalarType::Float8_e8m0fnu);
-    const int64_t m = x.size(0), k = x.size(1), n = w.size(0);
-    require(code >= 0 && w.size(1) == k && k % 32 == 0 && n % 8 == 0);
-    scales_fit(sw, n, k / 32);
-    const Bias bias = bias_of(a[3], c.device, n);
-    const ScalarType type = linear_type(a[4], x.scalar_type());
+    const Tensor* x = matrix(a[0], c.device);
+    const Tensor* w = matrix(a[1], c.device, ScalarType::Float8_e4m3fn);
+    const Tensor* sw = matrix(a[2], c.device, ScalarType::Float8_e8m0fnu);
+    if (x == nullptr || w == nullptr || sw == nullptr) return nullptr;
+    const int code = code_of(x->scalar_type());
+    const int64_t m = x->size(0), k = x->size(1), n = w->size(0);
+    Bias bias;
+    ScalarType type = linear_type(x->scalar_type());
+    if (code < 0 || w->size(1) != k || k % 32 != 0 || n % 8 != 0 || !scales_fit(*sw, n, k / 32) || !bias_of(a[3], c.device, n, &bias) ||
+        !dtype_of(a[4], &type)) {
+      return nullptr;
+    }
     const int64_t need = lib.linear_mxfp8_from_float_workspace_bytes(m, k);
-    require(need > 0);
+    if (need <= 0) return nullptr;
     Workspace ws(need);
     Tensor out = result({m, n}, type, c.device);
-    launched([&] {
-      return lib.linear_mxfp8_from_float(x.const_data_ptr(), code, w.const_data_ptr(), sw.const_data_ptr(), bias.ptr, bias.code, out.mutable_data_ptr(),
-                                         code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream);
-    });
+    if (!launched(lib.linear_mxfp8_from_float, x->const_data_ptr(), code, w->const_data_ptr(), sw->const_data_ptr(), bias.ptr, bias.code,
+                  out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream)) {
+      return nullptr;
+    }
     return THPVariable_Wrap(std::move(out));
   });
 }
