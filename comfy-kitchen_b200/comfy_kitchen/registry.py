@@ -93,10 +93,11 @@ class BackendRegistry:
         self._only = (name, self._backends[name]) if alone else None
 
     def leaves_no_choice(self, func_name: str, module, constraints: FunctionConstraints | None) -> bool:
-        """True when every call of ``func_name`` on this thread that meets ``constraints`` goes to ``module``: nothing else is
-        registered, it is enabled and nobody overrides it, and the device is one that it runs on."""
+        """True when every call of ``func_name`` on this thread that meets ``constraints`` goes to ``module`` without a word: nothing
+        else is registered, it is enabled and nobody overrides it, the device is one that it runs on, and the choice is not logged."""
         only = self._only
-        if only is None or only[1] is not module or constraints is None or getattr(self._tls, "override", None) is not None:
+        if only is None or only[1] is not module or constraints is None or getattr(self._tls, "override", None) is not None or \
+                logger.isEnabledFor(logging.DEBUG):
             return False
         cc = self._compute_capability
         return self._constraints.get((only[0], func_name)) is constraints and cc is not None and cc >= constraints.min_compute_capability

@@ -90,6 +90,14 @@ def test_registry_still_decides(cuda_device):
         ck.enable_backend("cuda")
 
 
+def test_the_registry_s_log_is_complete(cuda_device, caplog):
+    x, g = torch.randn(32, 64, device=cuda_device), torch.tensor(0.01, device=cuda_device)
+    with caplog.at_level("DEBUG", logger="comfy_kitchen.dispatch"):
+        codes, scales = ck.quantize_nvfp4(x, g)
+        ck.dequantize_nvfp4(codes, g, scales)
+    assert caplog.messages == ["Backend cuda selected for quantize_nvfp4", "Backend cuda selected for dequantize_nvfp4"]
+
+
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
 def test_deterministic_mode_fills_the_outputs(cuda_device, fmt):
     x, _, g, _ = _operands(cuda_device)

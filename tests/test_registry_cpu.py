@@ -195,3 +195,18 @@ def test_the_real_registry_has_one_backend_and_no_cpu_path():
     with pytest.raises(BackendNotFoundError):
         with ck.use_backend("eager"):
             pass
+
+
+def test_a_log_of_the_choices_is_asked_for(caplog):
+    """leaves_no_choice() lets a call pass the registry by: not while its choices are logged."""
+    r, module = BackendRegistry(), types.SimpleNamespace()
+    fc = FunctionConstraints(params={}, default_devices=CPU_AND_CUDA, min_compute_capability=(10, 0))
+    r.register("cuda", module, {"f": fc})
+    r._cc = (10, 0)
+    with caplog.at_level("INFO", logger="comfy_kitchen.dispatch"):
+        assert r.leaves_no_choice("f", module, fc)
+    with caplog.at_level("DEBUG", logger="comfy_kitchen.dispatch"):
+        assert not r.leaves_no_choice("f", module, fc)
+        assert r.get_capable_backend("f") == "cuda" and caplog.messages == ["Backend cuda selected for f"]
+    with caplog.at_level("INFO", logger="comfy_kitchen.dispatch"):
+        assert r.leaves_no_choice("f", module, fc)
