@@ -130,7 +130,8 @@ _HOST_NAMES = ("ck_quantize_nvfp4", "ck_quantize_nvfp4_dynamic_scratch_bytes", "
 
 def _load_host(lib) -> None:
     """Each function of the extension does one wrapper's work for plain eager calls and returns None for any other, which the
-    wrapper then does in Python.  Without the extension (not built, built against another torch) every call does."""
+    wrapper then does in Python.  Without the extension (not built, built against another torch or another library) every call
+    does."""
     global _host
     path = os.path.join(_PKG_ROOT, "lib", "_ck_host.so")
     if not os.path.exists(path):
@@ -141,7 +142,7 @@ def _load_host(lib) -> None:
         loader.exec_module(host)
         host.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _HOST_NAMES}, torch.nn.Parameter)
         _host = host
-    except ImportError as e:
+    except Exception as e:  # noqa: BLE001 - whatever is wrong with it, the library is complete without it
         logging.getLogger("comfy_kitchen").warning("%s does not load (%s): calls go through the Python wrappers", path, e)
 
 
