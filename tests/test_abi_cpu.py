@@ -71,3 +71,25 @@ def test_python_package_reports_backends_without_gpu(lib_path):
         assert not info["cuda"]["available"]
         with pytest.raises(ck.NoCapableBackendError):
             ck.quantize_nvfp4(torch.zeros(16, 16, dtype=torch.bfloat16), torch.ones((), dtype=torch.float32))
+
+
+@pytest.mark.parametrize("lacking", ["torch", "compiler", "headers"])
+def test_the_library_builds_without_what_only_the_host_extension_needs(monkeypatch, tmp_path, capfd, lacking):
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("ck_build", os.path.join(PKG_DIR, "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    path = mod.build()
+    host = tmp_path / "_ck_host.so"
+    host.write_bytes(b"built from older sources")
+    os.utime(host, (0, 0))
+    monkeypatch.setattr(mod, "HOST_PATH", str(host))
+    if lacking == "torch":
+        find = importlib.util.find_spec
+        monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
+    else:
+        monkeypatch.setenv("CXX", "false" if lacking == "headers" else str(tmp_path / "no-compiler"))
+    assert mod.build() == path and os.path.exists(path)
+    assert not host.exists()  # an old one might not fit the new library
+    assert "host extension" in capfd.readouterr().err
