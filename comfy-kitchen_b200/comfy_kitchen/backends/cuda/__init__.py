@@ -576,7 +576,7 @@ def linear_nvfp4_from_float(x: torch.Tensor, w_codes: torch.Tensor, w_scale: tor
     ``w_scale``; ``x_scale`` a static per-tensor scale or None for ``amax(|x|)/2688``.  Same bits
     as ``quantize_nvfp4`` followed by ``scaled_mm_nvfp4``.  The quantized activation passes
     from one launch to the next in a workspace (:func:`_workspace_for`)."""
-    if _host is not None:
+    if _host is not None and x.dim() == 2:
         out = _host.linear_nvfp4_from_float(x, w_codes, w_scale, w_block_scales, bias, x_scale, out_dtype)
         if out is not None:
             return out
@@ -615,7 +615,7 @@ def linear_mxfp8_from_float(x: torch.Tensor, w_data: torch.Tensor, w_block_scale
     ``w_data`` float8_e4m3fn [N, K] with its tiled E8M0 ``w_block_scales``.  Same bits as
     ``quantize_mxfp8`` followed by ``scaled_mm_mxfp8``; the quantized activation passes through a
     workspace, as in :func:`linear_nvfp4_from_float`."""
-    if _host is not None:
+    if _host is not None and x.dim() == 2:
         out = _host.linear_mxfp8_from_float(x, w_data, w_block_scales, bias, out_dtype)
         if out is not None:
             return out

@@ -196,7 +196,7 @@ class NVFP4Linear(_QuantizedLinearBase):
             y = host.linear_nvfp4_from_float(x, w._qdata, params.scale, params.block_scale, held["bias"] if "bias" in held else self.bias,
                                              held["input_scale"] if "input_scale" in held else self.input_scale, x.dtype)
             if y is not None:  # weight rows may be padded to the block size
-                return y if y.shape[1] == self.out_features else y[:, :self.out_features]
+                return y if y.shape[-1] == self.out_features else y[..., :self.out_features]
         w = self.weight
         if not isinstance(x, QuantizedTensor) and w is not None and x.dim() >= 2 and x.shape[-1] % 32 == 0 and \
                 x.dtype in (torch.bfloat16, torch.float16, torch.float32) and not getattr(w._params, "transposed", False):
@@ -271,7 +271,7 @@ class MXFP8Linear(_QuantizedLinearBase):
         if host is not None and w is not None and type(x) is torch.Tensor and not getattr(w._params, "transposed", False):
             y = host.linear_mxfp8_from_float(x, w._qdata, w._params.scale, held["bias"] if "bias" in held else self.bias, x.dtype)
             if y is not None:  # weight rows may be padded to the block size
-                return y if y.shape[1] == self.out_features else y[:, :self.out_features]
+                return y if y.shape[-1] == self.out_features else y[..., :self.out_features]
         w = self.weight
         if not isinstance(x, QuantizedTensor) and w is not None and x.dim() >= 2 and x.shape[-1] % 32 == 0 and \
                 x.dtype in (torch.bfloat16, torch.float16, torch.float32) and not getattr(w._params, "transposed", False):

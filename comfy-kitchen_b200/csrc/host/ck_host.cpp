@@ -8,6 +8,7 @@
 #include <Python.h>
 
 #include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/core/DimVector.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/record_function.h>
@@ -96,6 +97,12 @@ const Tensor* matrix(PyObject* o, int device) {
   return t != nullptr && t->dim() == 2 && t->size(0) > 0 && t->size(1) > 0 ? t : nullptr;
 }
 
+// Rows of any rank from two on.
+const Tensor* rows_of(PyObject* o, int device) {
+  const Tensor* t = plain(o, device);
+  return t != nullptr && t->dim() >= 2 && t->numel() > 0 ? t : nullptr;
+}
+
 const Tensor* matrix(PyObject* o, int device, ScalarType type) {
   const Tensor* t = matrix(o, device);
   return t != nullptr && t->scalar_type() == type ? t : nullptr;
@@ -143,6 +150,14 @@ struct Workspace {
   }
   void* ptr() { return block.get(); }
 };
+
+// Rows of `columns` values in the shape of x.
+Tensor rows_like(const Tensor& x, int64_t columns, ScalarType type, int device) {
+  if (x.dim() == 2) return result({x.size(0), columns}, type, device);
+  at::DimVector sizes(x.sizes());
+  sizes.back() = columns;
+  return result(sizes, type, device);
+}
 
 struct Call {
   int device;
@@ -353,30 +368,31 @@ PyObject* scaled_mm_mxfp8(PyObject*, Args a, Py_ssize_t n_args) {  // a, b, bloc
 }
 
 // ---- one-call linears -------------------------------------------------------------------------
+// The activation has any rank from two on, and the result its shape (the layers' callers pass [batch, tokens, features]).
 ScalarType linear_type(ScalarType x) { return x == ScalarType::Half ? x : ScalarType::BFloat16; }  // of a result whose type nobody names
 
 PyObject* linear_nvfp4_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x, w_codes, w_scale, w_block_scales, bias, x_scale, out_dtype
   return or_none(a, n_args, 7, [&]() -> PyObject* {
     const Call c;
-    const Tensor* x = matrix(a[0], c.device);
+    const Tensor* x = rows_of(a[0], c.device);
+    if (x == nullptr || (a[5] == Py_None && reinterpret_cast<uintptr_t>(x->const_data_ptr()) % 32 != 0)) return nullptr;  // the one-kernel scale comes first
     const Tensor* w = matrix(a[1], c.device, ScalarType::Byte);
     const float* w_scale = scalar(a[2], c.device);
     const Tensor* sw = matrix(a[3], c.device, ScalarType::Float8_e4m3fn);
     const float* x_scale = a[5] == Py_None ? nullptr : scalar(a[5], c.device);
-    if (x == nullptr || w == nullptr || w_scale == nullptr || sw == nullptr || (x_scale == nullptr && a[5] != Py_None)) return nullptr;
+    if (w == nullptr || w_scale == nullptr || sw == nullptr || (x_scale == nullptr && a[5] != Py_None)) return nullptr;
     const int code = code_of(x->scalar_type());
-    const int64_t m = x->size(0), k = x->size(1), n = w->size(0);
+    const int64_t k = x->size(-1), m = x->numel() / k, n = w->size(0);
     Bias bias;
     ScalarType type = linear_type(x->scalar_type());
     if (code < 0 || 2 * w->size(1) != k || k % 32 != 0 || n % 8 != 0 || !scales_fit(*sw, n, k / 16) || !bias_of(a[4], c.device, n, &bias) ||
         !dtype_of(a[6], &type)) {
       return nullptr;
     }
-    if (x_scale == nullptr && reinterpret_cast<uintptr_t>(x->const_data_ptr()) % 32 != 0) return nullptr;  // the one-kernel scale comes first
     const int64_t need = lib.linear_nvfp4_from_float_workspace_bytes(m, k, x_scale == nullptr);
     if (need <= 0) return nullptr;
     Workspace ws(need);
-    Tensor out = result({m, n}, type, c.device);
+    Tensor out = rows_like(*x, n, type, c.device);
     if (!launched(lib.linear_nvfp4_from_float, x->const_data_ptr(), code, x_scale, w->const_data_ptr(), sw->const_data_ptr(), w_scale, bias.ptr, bias.code,
                   out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream)) {
       return nullptr;
@@ -388,12 +404,12 @@ PyObject* linear_nvfp4_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x,
 PyObject* linear_mxfp8_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x, w_data, w_block_scales, bias, out_dtype
   return or_none(a, n_args, 5, [&]() -> PyObject* {
     const Call c;
-    const Tensor* x = matrix(a[0], c.device);
+    const Tensor* x = rows_of(a[0], c.device);
     const Tensor* w = matrix(a[1], c.device, ScalarType::Float8_e4m3fn);
     const Tensor* sw = matrix(a[2], c.device, ScalarType::Float8_e8m0fnu);
     if (x == nullptr || w == nullptr || sw == nullptr) return nullptr;
     const int code = code_of(x->scalar_type());
-    const int64_t m = x->size(0), k = x->size(1), n = w->size(0);
+    const int64_t k = x->size(-1), m = x->numel() / k, n = w->size(0);
     Bias bias;
     ScalarType type = linear_type(x->scalar_type());
     if (code < 0 || w->size(1) != k || k % 32 != 0 || n % 8 != 0 || !scales_fit(*sw, n, k / 32) || !bias_of(a[3], c.device, n, &bias) ||
@@ -403,7 +419,7 @@ PyObject* linear_mxfp8_from_float(PyObject*, Args a, Py_ssize_t n_args) {  // x,
     const int64_t need = lib.linear_mxfp8_from_float_workspace_bytes(m, k);
     if (need <= 0) return nullptr;
     Workspace ws(need);
-    Tensor out = result({m, n}, type, c.device);
+    Tensor out = rows_like(*x, n, type, c.device);
     if (!launched(lib.linear_mxfp8_from_float, x->const_data_ptr(), code, w->const_data_ptr(), sw->const_data_ptr(), bias.ptr, bias.code,
                   out.mutable_data_ptr(), code_of(type), m, n, k, ws.ptr(), ws.bytes, c.stream)) {
       return nullptr;

@@ -78,3 +78,40 @@ def test_padded_out_features(cuda_device, monkeypatch, layout, m, n):
         got = layer(x)
     assert got.shape == (m, n) and torch.equal(got, want)
     assert taken == [True]
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 512), (1, 40, 512), (3, 100, 512), (2, 1, 2, 4, 512), (1, 1, 512)])
+@pytest.mark.parametrize("n", [256, 200])
+@pytest.mark.parametrize("layout", ["nvfp4", "mxfp8"])
+def test_activations_of_any_rank(cuda_device, layout, n, shape):
+    """The rows' bits in the activation's shape, strides as the 2-D result has them, natively and through the Python route."""
+    from comfy_kitchen.backends import cuda as backend
+    from comfy_kitchen.modules import _QuantizedLinearBase
+
+    layer, flat = _layer(layout, 512, n, n == 256, cuda_device), _x(torch.Size(shape).numel() // 512, 512, cuda_device)
+    x = flat.view(shape)
+    with torch.inference_mode():
+        want = layer(flat)
+        got = layer(x)
+        assert got.shape == (*shape[:-1], n) and torch.equal(got.reshape(-1, n), want)
+        strides = [t.stride()[i] for t in (got, want.view(got.shape)) for i in range(len(shape)) if shape[i] > 1]
+        assert strides[: len(strides) // 2] == strides[len(strides) // 2 :]
+        assert torch.equal(got, _QuantizedLinearBase.forward(layer, x))
+        apart = torch.stack([x, x], dim=-1)[..., 0]  # not contiguous: the Python route
+        assert not apart.is_contiguous() and torch.equal(layer(apart), got)
+    w = layer.weight
+    args = (w._params.scale, w._params.block_scale) if layout == "nvfp4" else (w._params.scale,)
+    with pytest.raises(AssertionError):  # the wrapper itself takes a matrix
+        getattr(backend, f"linear_{layout}_from_float")(x, w._qdata, *args)
+
+
+@pytest.mark.parametrize("layout", ["nvfp4", "mxfp8"])
+def test_native_for_tokens_in_batches(cuda_device, layout):
+    from comfy_kitchen.backends import cuda as backend
+
+    layer, x = _layer(layout, 512, 256, True, cuda_device), _x(6, 512, cuda_device)
+    w, bias = layer.weight, layer.bias
+    native = getattr(backend._host, f"linear_{layout}_from_float")
+    args = (w._params.scale, w._params.block_scale, bias, None, x.dtype) if layout == "nvfp4" else (w._params.scale, bias, x.dtype)
+    assert native(x.view(2, 3, 512), w._qdata, *args).shape == (2, 3, 256)
+    assert native(x[0], w._qdata, *args) is None and native(x.view(2, 3, 512)[:0], w._qdata, *args) is None
