@@ -73,16 +73,26 @@ __device__ __forceinline__ void e2m1x8_to_f16x2(uint32_t word, uint32_t (&h)[4])
       : "r"(word));
 }
 
-// Bound by HBM (the result's write) for large tensors, by launch and latency for small ones.  A thread takes the same 16-
-// (NVFP4) or 32-element (MXFP8) block of kRows rows, four rows apart.  Two rows in flight pay where a thread's traffic is
-// small, for NVFP4 to a 16-bit type, and where the tensor fills the chip several times; launched like the other streaming
-// kernels, as a dependent of the kernel before it.  Graph replays, us, one row launched plainly / one row / two / four:
-// NVFP4 to bf16 12288 x 3072 18.3 / 17.8 / 17.0 / 17.5 (whole calls 20.4 -> 16.9), 36864 x 3072 49.8 / 49.2 / 47.2 / 48.0, 256 x 1024
-// 1.63 / 1.25 / 1.46 / 1.85; to fp32 4096 x 3072 11.2 / 10.7 / 10.6 / 11.7; MXFP8 to bf16 12288 x 3072 19.5 / 18.8 / 19.2 / 20.2.
+// Bound by HBM (the result's write) for large tensors, by launch and latency for small ones.  A thread takes a 16- (NVFP4) or
+// 32-element (MXFP8) block of one row, or of kRows rows, four apart.  Launched like the other streaming kernels, as a dependent of
+// the kernel before it.
+//
+// `early`: whether the next kernel's blocks may come once this block's loads are under way (else with its end).  Up to there a block
+// waits for the kernel before it, so that no third kernel gets in: blocks of several launches that wait together leave the next
+// launch a few SMs, where they bunch.  Triggered first thing, the back-to-back calls that now take 2.9 us (MXFP8 to fp32, 500 x 2816) took
+// 6.4, launched plainly 3.1.  Not where fp32 results of one to six (MXFP8: ten) blocks an SM keep the memory busy by themselves.  Graph replays,
+// us, launched plainly / triggered first thing / early / not: NVFP4 to bf16 300 x 768 1.65 / 1.33 / 1.11 / 1.30, 1200 x 2816 3.34 / 2.67 / 2.62 / 3.02, MXFP8 to
+// bf16 500 x 2816 2.59 / 3.08 / 2.21 / 2.48, 800 x 4480 3.49 / 3.67 / 3.00 / 3.37; to fp32, up to 148 blocks: NVFP4 300 x 768 2.13 / 1.71 / 1.56 / 2.02,
+// MXFP8 128 x 4480 3.00 / 4.97 / 2.59 / 2.83; more: NVFP4 800 x 2816 2.94 / 3.26 / 3.46 / 2.74, MXFP8 300 x 12288 6.43 / 9.00 / 7.63 / 5.94, 1658 x 4480
+// 10.04 / 10.74 / 10.48 / 9.63; beyond: NVFP4 800 x 4480 4.11 / 3.98 / 3.98 / 4.10, 2400 x 2816 6.93 / 6.37 / 6.34 / 6.67, MXFP8 6000 x 768 7.20 / 7.05 / 6.59 / 7.04.
+//
+// Two rows in flight pay where a thread's traffic is small, for NVFP4 to a 16-bit type, and where the tensor fills the chip several
+// times.  One row / two / four, us: NVFP4 to bf16 12288 x 3072 17.8 / 17.0 / 17.5 (whole calls 20.4 -> 16.9), 36864 x 3072 49.2 / 47.2 / 48.0, 256 x 1024
+// 1.25 / 1.46 / 1.85; to fp32 4096 x 3072 10.7 / 10.6 / 11.7; MXFP8 to bf16 12288 x 3072 18.8 / 19.2 / 20.2.
 template <typename OutT, bool kHiFirst, int kRows>
 __global__ void __launch_bounds__(kThreads)
-dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols) {
-  pdl_launch_dependents();
+dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols,
+                        bool early) {
   const int64_t n_sc = cols >> 4;
   const int64_t sc = static_cast<int64_t>(blockIdx.y) * 64 + threadIdx.x;
   const int64_t row0 = static_cast<int64_t>(blockIdx.x) * (4 * kRows) + threadIdx.y;
@@ -103,6 +113,7 @@ dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const u
       sbyte[i] = ld_global_u8(scales + swizzled_scale_offset(row, sc, col_tiles));
     }
   }
+  if (early) pdl_launch_dependents();
   // :211 total scale in the output dtype
   const float ts = round_to<OutT>(ld_f32_dependent(global_scale));
 #pragma unroll
@@ -130,8 +141,7 @@ dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const u
 
 template <typename OutT, int kRows>
 __global__ void __launch_bounds__(kThreads)
-dequantize_mxfp8_kernel(const uint8_t* data, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols) {
-  pdl_launch_dependents();
+dequantize_mxfp8_kernel(const uint8_t* data, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols, bool early) {
   const int64_t n_sc = cols >> 5;
   const int64_t sc = static_cast<int64_t>(blockIdx.y) * 64 + threadIdx.x;
   const int64_t row0 = static_cast<int64_t>(blockIdx.x) * (4 * kRows) + threadIdx.y;
@@ -148,6 +158,7 @@ dequantize_mxfp8_kernel(const uint8_t* data, const uint8_t* scales, OutT* __rest
       e[i] = ld_global_u8(scales + swizzled_scale_offset(row, sc, col_tiles));
     }
   }
+  if (early) pdl_launch_dependents();
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
     const int64_t row = row0 + 4 * i;
@@ -181,12 +192,20 @@ int check_common(const char* op, const void* in, const void* scales, const void*
   return CK_OK;
 }
 
+// See above the kernels.
+template <typename OutT>
+bool triggers_early(const dim3& grid, int many_to_an_sm) {
+  const int64_t blocks = static_cast<int64_t>(grid.x) * grid.y;
+  return sizeof(OutT) == 2 || blocks <= sm_count() || blocks > static_cast<int64_t>(many_to_an_sm) * sm_count();
+}
+
 template <typename OutT, int kRows>
 int launch_nvfp4_rows(const uint8_t* codes, const float* global_scale, const uint8_t* scales, void* out, int64_t rows, int64_t cols, int hi_first,
                       cudaStream_t stream) {
   const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4 * kRows)), static_cast<unsigned>(ceil_div(cols / 16, 64))), block(64, 4);
   auto kernel = hi_first ? dequantize_nvfp4_kernel<OutT, true, kRows> : dequantize_nvfp4_kernel<OutT, false, kRows>;
-  CK_CUDA(launch_pdl(kernel, grid, block, 0, stream, codes, global_scale, scales, static_cast<OutT*>(out), rows, cols));
+  CK_CUDA(launch_pdl(kernel, grid, block, 0, stream, codes, global_scale, scales, static_cast<OutT*>(out), rows, cols,
+                     triggers_early<OutT>(grid, 6)));
   return CK_OK;
 }
 
@@ -201,7 +220,8 @@ int launch_nvfp4(const uint8_t* codes, const float* global_scale, const uint8_t*
 template <typename OutT>
 int launch_mxfp8(const uint8_t* data, const uint8_t* scales, void* out, int64_t rows, int64_t cols, cudaStream_t stream) {
   const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4)), static_cast<unsigned>(ceil_div(cols / 32, 64))), block(64, 4);
-  CK_CUDA(launch_pdl(dequantize_mxfp8_kernel<OutT, 1>, grid, block, 0, stream, data, scales, static_cast<OutT*>(out), rows, cols));
+  CK_CUDA(launch_pdl(dequantize_mxfp8_kernel<OutT, 1>, grid, block, 0, stream, data, scales, static_cast<OutT*>(out), rows, cols,
+                     triggers_early<OutT>(grid, 10)));
   return CK_OK;
 }
 

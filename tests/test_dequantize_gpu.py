@@ -89,3 +89,31 @@ def test_nvfp4_two_rows_to_a_thread(cuda_device, dtype, hi_first):
     got = backend.dequantize_nvfp4(q, g, s, dtype, hi_first=hi_first)
     parts = [backend.dequantize_nvfp4(q[r:r + 128], g, s[r:r + 128], dtype, hi_first=hi_first) for r in range(0, rows, 128)]
     assert rows * cols > 1 << 22 and torch.equal(got, torch.cat(parts))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows, cols", [(592, 1024), (596, 1024), (3552, 1024), (3556, 1024), (5920, 1024), (5924, 1024)])  # 1, 6, 10 blocks an SM, and more
+@pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
+def test_back_to_back_with_a_reader(cuda_device, fmt, rows, cols, dtype):
+    """However early a dequantizer lets the next kernel's blocks in, that kernel reads what it wrote: chains on changing data."""
+    from comfy_kitchen.backends import cuda as backend
+
+    if fmt == "mxfp8":
+        cols *= 2  # the same number of blocks
+    gen = torch.Generator(device=cuda_device).manual_seed(rows)
+    xs = [torch.randn(rows, cols, generator=gen, device=cuda_device).bfloat16() * s for s in (1, 30, 0.1)]
+    if fmt == "mxfp8":
+        qs = [backend.quantize_mxfp8(x) for x in xs]
+        deq = [lambda q=q: backend.dequantize_mxfp8(*q, dtype) for q in qs]
+    else:
+        qs = [backend.quantize_nvfp4_dynamic(x) for x in xs]
+        deq = [lambda q=q: backend.dequantize_nvfp4(q[0], q[2], q[1], dtype) for q in qs]
+    want = []
+    for d in deq:
+        y = d()
+        torch.cuda.synchronize()
+        want.append(tuple(t.view(torch.uint8).clone() for t in backend.quantize_mxfp8(y)))
+        torch.cuda.synchronize()
+    for _ in range(15):
+        got = [backend.quantize_mxfp8(d()) for d in deq]
+        assert all(torch.equal(g.view(torch.uint8), w) for pair, ref in zip(got, want) for g, w in zip(pair, ref))
