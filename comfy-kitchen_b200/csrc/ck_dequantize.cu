@@ -74,7 +74,7 @@ __device__ __forceinline__ void e2m1x8_to_f16x2(uint32_t word, uint32_t (&h)[4])
 }
 
 // Bound by HBM (the result's write) for large tensors, by launch and latency for small ones.  A thread takes a 16- (NVFP4) or
-// 32-element (MXFP8) block of one row, or of kRows rows, four apart.  Launched like the other streaming kernels, as a dependent of
+// 32-element (MXFP8) block of one row, or of two, four apart (kRows, NVFP4).  Launched like the other streaming kernels, as a dependent of
 // the kernel before it.
 //
 // `early`: whether the next kernel's blocks may come once this block's loads are under way (else with its end).  Up to there a block
@@ -86,9 +86,10 @@ __device__ __forceinline__ void e2m1x8_to_f16x2(uint32_t word, uint32_t (&h)[4])
 // MXFP8 128 x 4480 3.00 / 4.97 / 2.59 / 2.83; more: NVFP4 800 x 2816 2.94 / 3.26 / 3.46 / 2.74, MXFP8 300 x 12288 6.43 / 9.00 / 7.63 / 5.94, 1658 x 4480
 // 10.04 / 10.74 / 10.48 / 9.63; beyond: NVFP4 800 x 4480 4.11 / 3.98 / 3.98 / 4.10, 2400 x 2816 6.93 / 6.37 / 6.34 / 6.67, MXFP8 6000 x 768 7.20 / 7.05 / 6.59 / 7.04.
 //
-// Two rows in flight pay where a thread's traffic is small, for NVFP4 to a 16-bit type, and where the tensor fills the chip several
-// times.  One row / two / four, us: NVFP4 to bf16 12288 x 3072 17.8 / 17.0 / 17.5 (whole calls 20.4 -> 16.9), 36864 x 3072 49.2 / 47.2 / 48.0, 256 x 1024
-// 1.25 / 1.46 / 1.85; to fp32 4096 x 3072 10.7 / 10.6 / 11.7; MXFP8 to bf16 12288 x 3072 18.8 / 19.2 / 20.2.
+// Two rows in flight pay where a thread's traffic is small, for NVFP4 to a 16-bit type, and where the blocks of one row do not all fit
+// at once (eight to an SM, 1184: 4.85 million elements).  One row / two, us, bf16: 1365 x 3072 (1026 blocks) 2.88 / 3.38, 4736 x 1024 (1184)
+// 3.03 / 3.55, 5000 x 1024 (1250) 3.94 / 3.68, 1600 x 3072 (1200) 3.86 / 3.68, 12288 x 3072 17.98 / 16.87; four 17.5.  To fp32 4096 x 3072 10.7 / 10.6 / 11.7;
+// MXFP8 to bf16 12288 x 3072 18.8 / 19.2 / 20.2.
 template <typename OutT, bool kHiFirst, int kRows>
 __global__ void __launch_bounds__(kThreads)
 dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols,
@@ -139,44 +140,30 @@ dequantize_nvfp4_kernel(const uint8_t* codes, const float* global_scale, const u
   }
 }
 
-template <typename OutT, int kRows>
+template <typename OutT>
 __global__ void __launch_bounds__(kThreads)
 dequantize_mxfp8_kernel(const uint8_t* data, const uint8_t* scales, OutT* __restrict__ out, int64_t rows, int64_t cols, bool early) {
   const int64_t n_sc = cols >> 5;
   const int64_t sc = static_cast<int64_t>(blockIdx.y) * 64 + threadIdx.x;
-  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * (4 * kRows) + threadIdx.y;
-  const int64_t col_tiles = ceil_div(n_sc, 4);
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + threadIdx.y;
   pdl_wait();
-  if (sc >= n_sc) return;
-  Vec256 raw[kRows];
-  uint32_t e[kRows];
-#pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    const int64_t row = row0 + 4 * i;
-    if (row < rows) {
-      raw[i] = ld_global_stream_256(data + row * cols + sc * 32);
-      e[i] = ld_global_u8(scales + swizzled_scale_offset(row, sc, col_tiles));
-    }
-  }
+  if (row >= rows || sc >= n_sc) return;
+  const Vec256 raw = ld_global_stream_256(data + row * cols + sc * 32);
+  const uint32_t e = ld_global_u8(scales + swizzled_scale_offset(row, sc, ceil_div(n_sc, 4)));
   if (early) pdl_launch_dependents();
+  const float scale = __uint_as_float(e << 23);  // byte 0 -> 0.0 (float_utils.py:376-382)
 #pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    const int64_t row = row0 + 4 * i;
-    if (row >= rows) break;
-    const float scale = __uint_as_float(e[i] << 23);  // byte 0 -> 0.0 (float_utils.py:376-382)
+  for (int h = 0; h < 2; ++h) {
+    float v[16];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float v[16];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t w = raw[i].w[h * 4 + j];
-        v[4 * j + 0] = e4m3_byte_to_f32(w & 0xFFu) * scale;
-        v[4 * j + 1] = e4m3_byte_to_f32((w >> 8) & 0xFFu) * scale;
-        v[4 * j + 2] = e4m3_byte_to_f32((w >> 16) & 0xFFu) * scale;
-        v[4 * j + 3] = e4m3_byte_to_f32(w >> 24) * scale;
-      }
-      store16<OutT>(out + row * cols + sc * 32 + h * 16, v);
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = raw.w[h * 4 + j];
+      v[4 * j + 0] = e4m3_byte_to_f32(w & 0xFFu) * scale;
+      v[4 * j + 1] = e4m3_byte_to_f32((w >> 8) & 0xFFu) * scale;
+      v[4 * j + 2] = e4m3_byte_to_f32((w >> 16) & 0xFFu) * scale;
+      v[4 * j + 3] = e4m3_byte_to_f32(w >> 24) * scale;
     }
+    store16<OutT>(out + row * cols + sc * 32 + h * 16, v);
   }
 }
 
@@ -212,15 +199,19 @@ int launch_nvfp4_rows(const uint8_t* codes, const float* global_scale, const uin
 template <typename OutT>
 int launch_nvfp4(const uint8_t* codes, const float* global_scale, const uint8_t* scales, void* out, int64_t rows, int64_t cols, int hi_first,
                  cudaStream_t stream) {
-  constexpr int64_t kTwoRowsElements = 4 << 20;  // seven waves of one row to a thread
-  if (sizeof(OutT) == 2 && rows * cols >= kTwoRowsElements) return launch_nvfp4_rows<OutT, 2>(codes, global_scale, scales, out, rows, cols, hi_first, stream);
+  if constexpr (sizeof(OutT) == 2) {
+    constexpr int64_t kBlocksPerSm = 2048 / kThreads;
+    if (ceil_div(rows, 4) * ceil_div(cols / 16, 64) > kBlocksPerSm * sm_count()) {
+      return launch_nvfp4_rows<OutT, 2>(codes, global_scale, scales, out, rows, cols, hi_first, stream);
+    }
+  }
   return launch_nvfp4_rows<OutT, 1>(codes, global_scale, scales, out, rows, cols, hi_first, stream);
 }
 
 template <typename OutT>
 int launch_mxfp8(const uint8_t* data, const uint8_t* scales, void* out, int64_t rows, int64_t cols, cudaStream_t stream) {
   const dim3 grid(static_cast<unsigned>(ceil_div(rows, 4)), static_cast<unsigned>(ceil_div(cols / 32, 64))), block(64, 4);
-  CK_CUDA(launch_pdl(dequantize_mxfp8_kernel<OutT, 1>, grid, block, 0, stream, data, scales, static_cast<OutT*>(out), rows, cols,
+  CK_CUDA(launch_pdl(dequantize_mxfp8_kernel<OutT>, grid, block, 0, stream, data, scales, static_cast<OutT*>(out), rows, cols,
                      triggers_early<OutT>(grid, 10)));
   return CK_OK;
 }

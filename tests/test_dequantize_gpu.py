@@ -78,8 +78,8 @@ def test_round_trip_full_size(ck, cuda_device, dtype, kind, key):
 @pytest.mark.parametrize("hi_first", [True, False])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_nvfp4_two_rows_to_a_thread(cuda_device, dtype, hi_first):
-    """From 2^22 elements on a thread of the 16-bit kernels takes two rows (here the last ones have no second): the values of
-    row blocks taken by themselves, which are smaller than that."""
+    """From 1185 blocks of one row on (here 1376) a thread of the 16-bit kernels takes two (here the last ones have no second): the
+    values of row blocks taken by themselves, which are smaller than that."""
     from comfy_kitchen.backends import cuda as backend
 
     gen = torch.Generator(device=cuda_device).manual_seed(11)
@@ -89,6 +89,18 @@ def test_nvfp4_two_rows_to_a_thread(cuda_device, dtype, hi_first):
     got = backend.dequantize_nvfp4(q, g, s, dtype, hi_first=hi_first)
     parts = [backend.dequantize_nvfp4(q[r:r + 128], g, s[r:r + 128], dtype, hi_first=hi_first) for r in range(0, rows, 128)]
     assert rows * cols > 1 << 22 and torch.equal(got, torch.cat(parts))
+
+
+@pytest.mark.parametrize("rows, cols", [(4736, 1024), (4737, 1024), (4741, 1008)])  # the last size of one row to a thread, the first of two
+def test_nvfp4_edge_of_two_rows_to_a_thread(cuda_device, rows, cols):
+    from comfy_kitchen.backends import cuda as backend
+
+    gen = torch.Generator(device=cuda_device).manual_seed(rows)
+    g = torch.tensor(0.0123, device=cuda_device)
+    q, s = backend.quantize_nvfp4(torch.randn(rows, cols, generator=gen, device=cuda_device), g)
+    got = backend.dequantize_nvfp4(q, g, s, torch.bfloat16)
+    parts = [backend.dequantize_nvfp4(q[r:r + 128], g, s[r:r + 128], torch.bfloat16) for r in range(0, rows, 128)]
+    assert torch.equal(got, torch.cat(parts))
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
