@@ -34,8 +34,17 @@ namespace {
 
 // 128 x 64 tiles that find an SM each: half the columns to an epilogue, and more CTAs that load (us, 128 x 128 / 128 x 64: NVFP4 256 x 3072
 // x 3072 7.2 / 6.8, 128 x 9216 x 3072 7.8 / 7.4, 1003 x 1024 x 3072 7.2 / 6.8, 384 x 3072 x 2048 6.1 / 5.7, MXFP8 128 x 9216 x 1536 7.4 / 7.0).
-// With up to 64 rows, half of a tile, only where there are few tiles altogether (NVFP4 64 x 9216 x 3072 7.6 / 8.0).
 bool one_wave_of_half_tiles(int64_t M, int64_t N) { return M > 64 && ceil_div(M, kTileM) * ceil_div(N, 64) <= sm_count(); }
+
+// Whether they pay.  Twice the CTAs ask for the same rows of the activation at once.  Rows that straddle the 128-byte lines cost each
+// of them two: with one or two row blocks that is dearer (NVFP4 68 x 6304 x 2976 7.7 / 9.6, 128 x 8512 x 3808 10.1 / 10.8, 256 x 4640 x 3296 8.8 / 9.4).
+// So are activations of less than 128 KiB, slow to load, up to 80 rows and from eight stages on (NVFP4 65 x 9216, K of 1792 5.95 / 5.99, 2048
+// 6.33 / 6.39, 2816 7.25 / 7.62, 3840 8.52 / 9.57; of 4096, 130 KiB, 8.80 / 8.36; 88 x 9216 x 2816 7.26 / 7.23, 96 x 9216 x 3072 7.59 / 7.16).
+bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
+  if (!one_wave_of_half_tiles(M, N)) return false;
+  if (k_bytes % kStageKBytes != 0) return M > 2 * kTileM;
+  return M > 80 || M * k_bytes >= (128 << 10) || k_bytes < 8 * kStageKBytes;
+}
 
 template <Kind KIND, typename OutT, bool FUSED>
 int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, cudaStream_t stream) {
@@ -51,7 +60,7 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
     const bool pair = ceil_div(p.M, 256) * ceil_div(p.N, 256) * 4 >= sm_count() && row_blocks > 1 && !(k_stages <= 4 && tiles <= 2 * sm_count());
     if (pair) {
       config = 4;
-    } else if (tiles * 4 <= sm_count() || one_wave_of_half_tiles(p.M, p.N)) {
+    } else if (tiles * 4 <= sm_count() || half_tiles_pay(p.M, p.N, p.k_bytes)) {
       config = 7;
     } else {
       config = 1;
@@ -90,7 +99,8 @@ int max_splits(int64_t M, int64_t N, int k_bytes) {
 }
 
 struct SplitPlan {
-  int splits;            // CTAs per tile
+  int splits;            // CTAs per tile; 1:
+  bool half_tiles;       //   tiles of half the columns instead of two CTAs to one
   int k_stages;          // of each
   bool through_workspace;
 };
@@ -118,7 +128,8 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
   plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
   // Two CTAs to a tile and up to 32 stages: half tiles instead (us, two CTAs / half tiles: MXFP8 128 x 9216 x 3072 11.8 / 10.4, NVFP4 128 x
   // 9216 x 8192 14.5 / 13.6; MXFP8 128 x 9216 x 8192, 64 stages, 19.9 / 21.3).
-  if (splits == 2 && !plan->through_workspace && k_stages <= 32 && one_wave_of_half_tiles(M, N)) splits = 1;
+  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= 32 && one_wave_of_half_tiles(M, N);
+  if (plan->half_tiles) splits = 1;
   plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
   plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage
   return CK_OK;
@@ -167,8 +178,9 @@ int launch_split(const Operands& ops, GemmParams p, const OutputSpec& os, void* 
   if (plan.through_workspace && (workspace_bytes < split_workspace_bytes(p.M, p.N, plan) || reinterpret_cast<uintptr_t>(workspace) % 16 != 0)) {
     if (int rc = choose_splits<KIND, OutT>(p.M, p.N, p.k_bytes, false, &plan)) return rc;
   }
+  *launched = plan.splits > 1 || plan.half_tiles;
+  if (plan.half_tiles) return launch_config<KIND, 64, 2, 6, 1, OutT, false, 1>(ops, p, os, stream);
   if (plan.splits < 2) return CK_OK;
-  *launched = true;
   const int64_t mn = static_cast<int64_t>(p.M) * p.N;
   const GemmParams result = p;
   p.splits = plan.splits;

@@ -7,9 +7,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # one row block and two, half tiles that just fit 148 SMs and do not, four stages (K of NVFP4 1024, MXFP8 512) and five, a split in two
-# that half tiles replace (24 stages) and one that they do not (40)
+# that half tiles replace (24 stages) and one that they do not (40); 80 rows and 81 of eight stages, 80 of seven, rows of K that are no whole
+# 128-byte lines in one to three row blocks
 SHAPES = [(128, 18440, 96), (129, 18440, 96), (33, 24584, 32), (65, 9216, 288), (64, 9216, 288), (66, 9536, 288), (1003, 1160, 544), (512, 9224, 1024),
-          (512, 9224, 1056), (700, 3080, 512), (700, 3080, 544), (100, 9216, 24 * 128), (100, 9216, 40 * 256)]
+          (512, 9224, 1056), (700, 3080, 512), (700, 3080, 544), (100, 9216, 24 * 128), (100, 9216, 40 * 256),
+          (80, 9216, 2048), (81, 9216, 2048), (80, 9216, 1792), (68, 6304, 2976), (256, 4640, 1696), (257, 2080, 1696)]
 
 
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
