@@ -126,9 +126,14 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
     if (clusters >= tiles) break;
   }
   plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
-  // Two CTAs to a tile and up to 32 stages: half tiles instead (us, two CTAs / half tiles: MXFP8 128 x 9216 x 3072 11.8 / 10.4, NVFP4 128 x
-  // 9216 x 8192 14.5 / 13.6; MXFP8 128 x 9216 x 8192, 64 stages, 19.9 / 21.3).
-  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= 32 && one_wave_of_half_tiles(M, N);
+  // Two CTAs to a tile: half tiles instead, while their longer K costs less than the exchange.  They end in TMA stores, which want
+  // rows of whole 64-byte units (N of 16 bits off by 16: MXFP8 512 x 1648 x 2784 10.0 / 10.7, NVFP4 517 x 1584 x 4800 9.7 / 10.7).  With one row block and
+  // nearly all SMs the weight's stream gains too.  us, two CTAs / half tiles: MXFP8 128 x 9216, 24 stages, 11.9 / 10.3, 32 14.1 / 12.6, 64 19.9 / 21.3;
+  // 512 x 2304, 28 stages, 11.2 / 10.9, 32 11.9 / 12.1; NVFP4 128 x 9216, 32 stages, 14.7 / 13.6, 128 x 6400 11.1 / 10.7 with 24, 12.8 / 13.0 with 32;
+  // 512 x 2304, 20 stages, 10.0 / 9.4, 24 10.6 / 10.7, 32 12.0 / 13.1.
+  const bool streams = M <= kTileM && 8 * ceil_div(N, 64) >= 7 * sm_count() && k_bytes % kStageKBytes == 0;
+  const int most_stages = streams ? 32 : KIND == Kind::kNvfp4 ? 23 : 28;
+  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= most_stages && N % 32 == 0 && one_wave_of_half_tiles(M, N);
   if (plan->half_tiles) splits = 1;
   plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
   plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage

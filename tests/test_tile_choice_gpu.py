@@ -8,10 +8,11 @@ pytestmark = pytest.mark.gpu
 
 # one row block and two, half tiles that just fit 148 SMs and do not, four stages (K of NVFP4 1024, MXFP8 512) and five, a split in two
 # that half tiles replace (24 stages) and one that they do not (40); 80 rows and 81 of eight stages, 80 of seven, rows of K that are no whole
-# 128-byte lines in one to three row blocks
+# 128-byte lines in one to three row blocks; 23 stages and a split in two, columns that are no 64-byte units, 32 stages of one row block
 SHAPES = [(128, 18440, 96), (129, 18440, 96), (33, 24584, 32), (65, 9216, 288), (64, 9216, 288), (66, 9536, 288), (1003, 1160, 544), (512, 9224, 1024),
           (512, 9224, 1056), (700, 3080, 512), (700, 3080, 544), (100, 9216, 24 * 128), (100, 9216, 40 * 256),
-          (80, 9216, 2048), (81, 9216, 2048), (80, 9216, 1792), (68, 6304, 2976), (256, 4640, 1696), (257, 2080, 1696)]
+          (80, 9216, 2048), (81, 9216, 2048), (80, 9216, 1792), (68, 6304, 2976), (256, 4640, 1696), (257, 2080, 1696),
+          (500, 1632, 23 * 128), (500, 1632, 23 * 256), (500, 1648, 20 * 128), (500, 1648, 20 * 256), (90, 8448, 32 * 128), (90, 8448, 32 * 256)]
 
 
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
