@@ -55,6 +55,10 @@ int linear_small_m(bool is_mxfp8, const void* x, int x_dtype, const float* x_sca
                    const void* w_scales, const float* w_scale, const void* bias, int bias_dtype, void* out, int out_dtype, int64_t M,
                    int64_t N, int64_t K, cudaStream_t stream);
 
+// ck_scaled_mm_nvfp4 behind a reduction and its quantizer (ck_gemm.cu).
+int scaled_mm_of_dynamic_linear(const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa, const float* tsb, const void* bias,
+                                int bias_dtype, void* out, int out_dtype, int64_t M, int64_t N, int64_t K, void* stream);
+
 // GEMMs with few activation rows (ck_gemm_smallm.cu).
 bool small_m_applies(int64_t M, int64_t N, int64_t K);
 int small_m_max_splits(int64_t N, int k_bytes);

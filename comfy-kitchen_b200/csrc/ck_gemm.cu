@@ -46,8 +46,19 @@ bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
   return M > 80 || M * k_bytes >= (128 << 10) || k_bytes < 8 * kStageKBytes;
 }
 
+// In a linear with a dynamic scale.  Such calls in a row are a chain of reduction, quantizer and GEMM whose launches overlap, and the quantizer's
+// few large blocks find room beside the GEMM before them only on SMs that it leaves free.  A GEMM of more, smaller CTAs gains less than
+// the quantizer then loses, unless a quarter of the SMs stays free (whole linears, us, 128 x 128 / half tiles: 200 x 4544 x 768 9.2 / 10.1, 65 x 9216 x 3072
+// 12.2 / 13.8, 1003 x 1024 x 768 9.5 / 9.9; 128 x 6848 x 3072, 107 half tiles, 13.3 / 11.8, 1003 x 576 x 352 9.3 / 8.2; pair / 128 x 128: 512 x 6848 x 768, 54 pairs,
+// 11.3 / 12.4, 1003 x 3072 x 512 11.4 / 11.8; 640 x 6848 x 768, 81 pairs on 74, 14.8 / 12.8).
+struct Room {
+  bool wanted;
+  bool left_by_half_tiles(int64_t M, int64_t N) const { return !wanted || ceil_div(M, kTileM) * ceil_div(N, 64) * 4 <= 3 * sm_count(); }
+  bool left_by_pairs(int64_t pairs) const { return wanted && pairs * 2 <= sm_count(); }
+};
+
 template <Kind KIND, typename OutT, bool FUSED>
-int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, cudaStream_t stream) {
+int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, const Room& room, cudaStream_t stream) {
   int config = forced_gemm_config();
   if (config == 0) {
     const int64_t row_blocks = ceil_div(p.M, kTileM), tiles = row_blocks * ceil_div(p.N, 128);
@@ -57,10 +68,11 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
     // 16.4 / 14.2, the fused epilogue 128 x 12288 x 3072 12.8 / 9.8), and not for up to four stages while a CTA has at most
     // two of the small tiles (NVFP4 512 x 9216 x 1024 7.4 / 6.7, 256 x 18432 x 1024 8.1 / 7.2, fused 512 x 8192 x 1024 9.7 / 9.4; with six
     // stages 512 x 9216 x 1536 8.3 / 8.1 and 1003 x 3072 x 1536 7.5 / 7.6, with twelve 512 x 9216 x 3072 10.6 / 11.9).
-    const bool pair = ceil_div(p.M, 256) * ceil_div(p.N, 256) * 4 >= sm_count() && row_blocks > 1 && !(k_stages <= 4 && tiles <= 2 * sm_count());
+    const int64_t pairs = ceil_div(p.M, 256) * ceil_div(p.N, 256);
+    const bool pair = pairs * 4 >= sm_count() && row_blocks > 1 && (!(k_stages <= 4 && tiles <= 2 * sm_count()) || room.left_by_pairs(pairs));
     if (pair) {
       config = 4;
-    } else if (tiles * 4 <= sm_count() || half_tiles_pay(p.M, p.N, p.k_bytes)) {
+    } else if (tiles * 4 <= sm_count() || (half_tiles_pay(p.M, p.N, p.k_bytes) && room.left_by_half_tiles(p.M, p.N))) {
       config = 7;
     } else {
       config = 1;
@@ -236,7 +248,7 @@ template <Kind KIND>
 int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa,
               const float* tsb, const float* alpha, const void* bias, int bias_dtype, void* out, int out_dtype,
               int64_t M, int64_t N, int64_t K, void* stream, const FusedArgs& fused = FusedArgs(),
-              const OutputSpec* out_spec = nullptr, void* workspace = nullptr, int64_t workspace_bytes = 0) {
+              const OutputSpec* out_spec = nullptr, void* workspace = nullptr, int64_t workspace_bytes = 0, const Room& room = Room{false}) {
   CK_REQUIRE(a && b && sfa && sfb, "%s: null pointer", op);
   CK_REQUIRE(out != nullptr || (fused.enabled && fused.rq_codes != nullptr), "%s: no output requested", op);
   if (fused.enabled) {
@@ -327,25 +339,32 @@ int scaled_mm(const char* op, const void* a, const void* b, const void* sfa, con
     if (fused.enabled) {
       switch (out_dtype) {
         case CK_DTYPE_BF16:
-          return launch_for_shape<KIND, __nv_bfloat16, true>(ops, p, os, s);
+          return launch_for_shape<KIND, __nv_bfloat16, true>(ops, p, os, room, s);
         case CK_DTYPE_F16:
-          return launch_for_shape<KIND, __half, true>(ops, p, os, s);
+          return launch_for_shape<KIND, __half, true>(ops, p, os, room, s);
         default:
-          return launch_for_shape<KIND, float, true>(ops, p, os, s);
+          return launch_for_shape<KIND, float, true>(ops, p, os, room, s);
       }
     }
   }
   switch (out_dtype) {
     case CK_DTYPE_BF16:
-      return launch_for_shape<KIND, __nv_bfloat16, false>(ops, p, os, s);
+      return launch_for_shape<KIND, __nv_bfloat16, false>(ops, p, os, room, s);
     case CK_DTYPE_F16:
-      return launch_for_shape<KIND, __half, false>(ops, p, os, s);
+      return launch_for_shape<KIND, __half, false>(ops, p, os, room, s);
     default:
-      return launch_for_shape<KIND, float, false>(ops, p, os, s);
+      return launch_for_shape<KIND, float, false>(ops, p, os, room, s);
   }
 }
 
 }  // namespace
+
+int scaled_mm_of_dynamic_linear(const void* a, const void* b, const void* sfa, const void* sfb, const float* tsa, const float* tsb, const void* bias,
+                                int bias_dtype, void* out, int out_dtype, int64_t M, int64_t N, int64_t K, void* stream) {
+  return scaled_mm<Kind::kNvfp4>("scaled_mm_nvfp4", a, b, sfa, sfb, tsa, tsb, nullptr, bias, bias_dtype, out, out_dtype, M, N, K, stream, FusedArgs(),
+                                 nullptr, nullptr, 0, Room{true});
+}
+
 }  // namespace ck
 
 extern "C" int ck_scaled_mm_nvfp4(const void* a, const void* b, const void* sfa, const void* sfb,

@@ -69,17 +69,15 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
     return linear_small_m(false, x, x_dtype, x_scale, partials, n_partials, w_codes, w_block_scales, w_scale, bias, bias_dtype, out, out_dtype,
                           M, N, K, static_cast<cudaStream_t>(stream));
   }
-  const float* scale = x_scale;
   if (dynamic) {
     float* dyn = reinterpret_cast<float*>(ws + l.scale_off);
     if (int rc = ck_quantize_nvfp4_dynamic(x, x_dtype, dyn, codes, scales, M, K, M, K, /*hi_first=*/1, ws + l.scratch_off,
                                            kScaleScratchBytes, stream))
       return rc;
-    scale = dyn;
-  } else if (int rc = ck_quantize_nvfp4(x, x_dtype, scale, codes, scales, M, K, M, K, /*hi_first=*/1, stream)) {
-    return rc;
+    return scaled_mm_of_dynamic_linear(codes, w_codes, scales, w_block_scales, dyn, w_scale, bias, bias_dtype, out, out_dtype, M, N, K, stream);
   }
-  return ck_scaled_mm_nvfp4(codes, w_codes, scales, w_block_scales, scale, w_scale, nullptr, bias, bias_dtype, out,
+  if (int rc = ck_quantize_nvfp4(x, x_dtype, x_scale, codes, scales, M, K, M, K, /*hi_first=*/1, stream)) return rc;
+  return ck_scaled_mm_nvfp4(codes, w_codes, scales, w_block_scales, x_scale, w_scale, nullptr, bias, bias_dtype, out,
                             out_dtype, M, N, K, stream);
 }
 

@@ -48,3 +48,20 @@ def test_same_bits(cuda_device, monkeypatch, fmt, m, n, k):
         want = fused()
         assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(got, want))
     backend.check_device_status("tile choice")
+
+
+@pytest.mark.parametrize("m, n, k", [(512, 6848, 768), (640, 6848, 288), (200, 4544, 768), (128, 6848, 544), (128, 7168, 544)])
+def test_dynamic_linears(cuda_device, m, n, k):
+    """A linear with a dynamic scale leaves SMs to the next one (54 pairs; 81, too many; half tiles on 142, 107 and 112 SMs): the bits of
+    the separate calls, several in a row."""
+    from comfy_kitchen.backends import cuda as backend
+
+    gen = torch.Generator(device=cuda_device).manual_seed(m + n)
+    w, bias = torch.randn(n, k, generator=gen, device=cuda_device).bfloat16(), torch.linspace(-1, 1, n, device=cuda_device)
+    qw = backend.quantize_nvfp4_dynamic(w)
+    xs = [torch.randn(m, k, generator=gen, device=cuda_device).bfloat16() * s for s in (1, 20, 0.3)]
+    got = [backend.linear_nvfp4_from_float(x, qw[0], qw[2], qw[1], bias=bias) for x in xs]
+    for x, y in zip(xs, got):
+        q, s, g = backend.quantize_nvfp4_dynamic(x)
+        assert torch.equal(y, backend.scaled_mm_nvfp4(q, qw[0], g, qw[2], s, qw[1], bias=bias))
+    backend.check_device_status("dynamic linears")
