@@ -14,10 +14,10 @@ struct FromFloatLayout {
   int64_t scratch_off, scale_off, codes_off, scales_off, total;
 };
 
-// Workspace layout: tensor-scale scratch | dynamic tensor scale | codes [M, K/2] | tiled block scales.
 // Few rows, quantized inside the GEMM: up to here every CTA takes the maximum of the whole activation itself (the quantizers' line
 // for the same choice, ck_quantize.cu); beyond it a reduction kernel leaves partial maxima.
 constexpr int64_t kSmallLinearWholeInputBytes = 64 * 1024;
+// Workspace layout: tensor-scale scratch | dynamic tensor scale | codes [M, K/2] | tiled block scales.
 constexpr int64_t kScaleScratchBytes = 256 + 256 * 1024;  // 2^30 elements: 65536 partials behind the head
 
 FromFloatLayout from_float_layout(int64_t M, int64_t K) {
