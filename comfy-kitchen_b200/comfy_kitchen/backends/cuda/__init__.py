@@ -265,12 +265,16 @@ _scale_scratch: dict = {}
 _retired_workspaces: list = []  # outgrown buffers stay alive: a captured CUDA graph may still point at them
 
 
-def _scale_scratch_for(device, stream: int, need: int) -> torch.Tensor:
+def _scale_scratch_for(device, stream: int, need: int, zeros: bool = True) -> torch.Tensor:
     """The zeroed scratch buffer of the tensor-scale kernel for this device and stream, at least
-    ``need`` bytes.  An outgrown buffer is kept alive: a captured CUDA graph may still point at it."""
+    ``need`` bytes.  An outgrown buffer is kept alive: a captured CUDA graph may still point at it.
+    A captured call that finds none has its own, which belongs to its graph: its zeros, if it wants
+    any, are only written when that graph runs."""
     key = (device, stream)
     scratch = _scale_scratch.get(key)
     if scratch is None or scratch.numel() < need:
+        if _capturing():
+            return (torch.zeros if zeros else torch.empty)(need, dtype=torch.uint8, device=device)
         if scratch is not None:
             _retired_workspaces.append(scratch)
         # 1 MiB covers 2^33 elements: growth (an allocation and a memset) is a first-call event
@@ -333,7 +337,7 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     if _host is not None:
         scratch = None
         if type(x) is torch.Tensor and x.is_cuda and x.numel() * x.element_size() <= _WHOLE_INPUT_BYTES:
-            scratch = _scale_scratch_for(x.device, _stream(x.device), 1 << 20)  # nothing is kept in it between two launches
+            scratch = _scale_scratch_for(x.device, _stream(x.device), 1 << 20, zeros=False)  # nothing is kept in it between two launches
         out = _host.quantize_nvfp4_dynamic(x, pad_16x, hi_first, scratch)
         if out is not None:
             return out
@@ -356,7 +360,7 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     # the smallest workspace that is kept does up to 2^31 elements: no need to ask
     need = 1 << 20 if rows * cols < 1 << 31 else _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
     if rows * cols * size <= _WHOLE_INPUT_BYTES:
-        scratch = _scale_scratch_for(x.device, stream, need)  # nothing is kept in it between two launches
+        scratch = _scale_scratch_for(x.device, stream, need, zeros=False)  # nothing is kept in it between two launches
     else:
         scratch = _workspace_for(need, x.device, stream)  # the partial maxima go from one launch to the next
     scale = torch.empty((), dtype=torch.float32, device=x.device)
