@@ -22,6 +22,7 @@ import torch
 
 from comfy_kitchen.float_utils import roundup
 from comfy_kitchen.ops import DTYPE_TO_CODE
+from comfy_kitchen.registry import registry
 
 __all__ = [
     "quantize_nvfp4",
@@ -785,8 +786,6 @@ _stock = {name: globals()[name] for name in ("quantize_nvfp4", "quantize_mxfp8",
 def host_operator(name: str):
     """The native half of operator ``name``, or None unless the registry would send every call that it takes to this
     module's own function anyway."""
-    from comfy_kitchen.registry import registry
-
     if _host is None or globals()[name] is not _stock[name] or \
             not registry.leaves_no_choice(name, _this_module, _constraints.get(name)):
         return None
@@ -794,9 +793,6 @@ def host_operator(name: str):
 
 
 def _register():
-
-    from comfy_kitchen.registry import registry
-
     try:
         load_library()
     except RuntimeError as e:
