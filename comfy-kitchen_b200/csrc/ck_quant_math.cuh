@@ -236,28 +236,6 @@ __device__ __noinline__ BlockCodes nvfp4_block_packed_ieee(uint32_t w0, uint32_t
   return r;
 }
 
-// Codes of 16 exact quotients x / safe by the reciprocal-FMA chain (see div_markstein), out of
-// line: the streaming path below needs it only for blocks in which some quotient lies within
-// 2^-21 (relative) of an E2M1 rounding boundary.
-template <typename T, bool kHiFirst>
-__device__ __noinline__ uint2 nvfp4_codes_exact(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t w4,
-                                                uint32_t w5, uint32_t w6, uint32_t w7, float safe, float y) {
-  const uint32_t w[8] = {w0, w1, w2, w3, w4, w5, w6, w7};
-  float v[16], q[16];
-  widen16<T>(w, v);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) q[i] = div_markstein(v[i], safe, y);
-  uint2 r;
-  if constexpr (kHiFirst) {
-    r.x = f32x8_to_e2m1_word(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-    r.y = f32x8_to_e2m1_word(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
-  } else {
-    r.x = f32x8_to_e2m1_word(q[1], q[0], q[3], q[2], q[5], q[4], q[7], q[6]);
-    r.y = f32x8_to_e2m1_word(q[9], q[8], q[11], q[10], q[13], q[12], q[15], q[14]);
-  }
-  return r;
-}
-
 // 8 products v[i] * y -> one word of codes (nibble order as requested)
 template <bool kHiFirst>
 __device__ __forceinline__ uint32_t scaled_e2m1_word(const float* v, float y) {
@@ -275,50 +253,76 @@ __device__ __forceinline__ uint32_t scaled_e2m1_word(const float* v, float y) {
   }
 }
 
-// The element quotients are not computed at all in the common case.  The code of x / total is
-// a monotone step function of the quotient, and RN(x / total) lies strictly between
-// x * y_lo and x * y_hi with y_lo = y (1 - 2^-21), y_hi = y (1 + 2^-21), y = RN(1 / total)
-// (the three roundings involved are below 2^-23 each, the quotient's own below 2^-24).  So
-// when both bracketing products convert to the same codes for a whole block - two multiplies
-// and one convert per element - those are the codes of the exact quotients; only a block in
-// which some product straddles a rounding boundary is redone with exact quotients.  A zero
-// keeps its sign through the multiplication, as the reference's cast keeps it.
+// 1 / t for a positive normal t, one unit in the last place at most off.
+__device__ __forceinline__ float approximate_reciprocal(float t) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(t));
+  return y;
+}
+
+// Codes of sixteen 16-bit values divided by t: p = x y, then one correction by the residual, q = p - (t p - x) y.  For an x of
+// at most eleven significant bits the code of q is the code of RN(x / t): q is off by less than 2^-45 beside its own rounding, so the two
+// can only part where x / t lies that close to the middle between a rounding boundary and its neighbour, and x and the boundary
+// times t are then integers a few units apart; the cases there are have been gone through one by one (test_corrected_quotient_cpu),
+// with reciprocals up to two units in the last place off.  Only a significand of all ones fails, which the caller sends elsewhere.
+// The residual carries the sign opposite to x, so that the sum keeps a negative zero.  Per element one and a half packed
+// multiply-adds and half a conversion; two bracketing products took one multiply and one conversion, and the conversions' bytes twice.
+template <typename T, bool kHiFirst>
+__device__ __forceinline__ void nvfp4_codes_corrected(const uint32_t (&w)[8], float t, float y, uint32_t& lo_word, uint32_t& hi_word) {
+  const float2 t2 = make_float2(t, t), minus_y = make_float2(-y, -y);
+  float q[16];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float2 minus_x;
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      minus_x.x = __uint_as_float(w[i] * 0x10000u + 0x80000000u);
+      minus_x.y = __uint_as_float((w[i] & 0xFFFF0000u) ^ 0x80000000u);
+    } else {
+      minus_x = __half22float2(__hneg2(*reinterpret_cast<const __half2*>(&w[i])));
+    }
+    const float2 p = mul_x2(minus_x, minus_y);
+    const float2 r = fma_x2(t2, p, minus_x);
+    const float2 c = fma_x2(r, minus_y, p);
+    q[2 * i] = c.x;
+    q[2 * i + 1] = c.y;
+  }
+  if constexpr (kHiFirst) {
+    lo_word = f32x8_to_e2m1_word(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
+    hi_word = f32x8_to_e2m1_word(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
+  } else {
+    lo_word = f32x8_to_e2m1_word(q[1], q[0], q[3], q[2], q[5], q[4], q[7], q[6]);
+    hi_word = f32x8_to_e2m1_word(q[9], q[8], q[11], q[10], q[13], q[12], q[15], q[14]);
+  }
+}
+
+// Whether the significand of t is all ones (see nvfp4_codes_corrected).
+__device__ __forceinline__ bool all_ones(float t) { return (__float_as_uint(t) << 9) == 0xFFFFFE00u; }
+
+// Window: tensor scale within 2^+-40, amax zero or within 2^+-60; total = g * scale is then a normal number within 2^+-50 and no
+// residual matters that underflows (its quotient encodes as a signed zero).  Everything else takes the IEEE divisions.  The E4M3 scale
+// comes from two products that bracket amax / (6 g) by 2^-21 (see nvfp4_blocks) and, when those round apart, from the quotients themselves.
+//
+// The quantizer of 16-bit inputs was bound by its instructions (issue slots 77 % busy at 24576 x 3072): with bracketing products
+// and Markstein's scale / so, static scale, us: bf16 1024 x 3072 3.65 / 3.26, 4096 x 3072 7.90 / 7.35, 16384 x 3072 26.9 / 23.8, 24576 x 3072
+// 46.7 / 33.7 (0.88 of the copy rate), 36864 x 3072 50.0 / 49.2, 16384 x 12288 96.0 / 82; behind its reduction 16384 x 3072 44.8 / 39.5.
 template <typename T, bool kHiFirst>
 __device__ __forceinline__ void nvfp4_block_packed(const uint32_t (&w)[8], const TensorScale& ts, uint32_t& lo_word,
                                                    uint32_t& hi_word, uint32_t& scale_byte) {
   static_assert(sizeof(T) == 2, "packed 16-bit inputs");
   const float amax = amax16_packed<T>(w);
-  // Exactness window of the reciprocal-FMA quotients amax/6/g (all residuals representable):
-  // tensor scale within 2^+-40, amax zero or within 2^+-60; then total = g * scale is a normal
-  // number within 2^+-50 and its reciprocal is too.  Anything else takes the IEEE-division path.
-  const bool fast_s = ts.in_window && (amax <= 0x1p60f) && (amax >= 0x1p-60f || amax == 0.0f);
-  if (fast_s) {
-    float s = div_markstein_nonneg(div_markstein_nonneg(amax, 6.0f, 0x1.555556p-3f /* RN(1/6) */), ts.g, ts.rcp);
-    s = fminf(s, 448.0f);
-    scale_byte = f32_to_e4m3_byte(s);
-    const float total = __fmul_rn(ts.g, e4m3_byte_to_f32(scale_byte));
-    const bool dead = (total == 0.0f);
-    const float safe = dead ? 1.0f : total;
-    const float y = __frcp_rn(safe);
-    const float y_hi = __fmul_rn(y, 0x1.000008p0f), y_lo = __fmul_rn(y, 0x1.fffffp-1f);
-    float v[16];
-    widen16<T>(w, v);
-    lo_word = scaled_e2m1_word<kHiFirst>(v, y_hi);
-    hi_word = scaled_e2m1_word<kHiFirst>(v + 8, y_hi);
-    const uint32_t lo_b = scaled_e2m1_word<kHiFirst>(v, y_lo);
-    const uint32_t hi_b = scaled_e2m1_word<kHiFirst>(v + 8, y_lo);
-    if (((lo_word ^ lo_b) | (hi_word ^ hi_b)) != 0u) {
-      if (amax <= total * 0x1p20f) {  // residuals of the exact chain representable
-        const uint2 r = nvfp4_codes_exact<T, kHiFirst>(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], safe, y);
-        lo_word = r.x;
-        hi_word = r.y;
-      } else {
-        const BlockCodes r = nvfp4_block_packed_ieee<T, kHiFirst>(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], ts.g);
-        lo_word = r.lo;
-        hi_word = r.hi;
-      }
-    }
-    if (dead) {  // zero scale: every code is +0
+  const uint32_t both = f32x2_to_e4m3x2(__fmul_rn(amax, ts.s_hi), __fmul_rn(amax, ts.s_lo));
+  scale_byte = both & 0xFFu;
+  const bool in_window = ts.in_window && (amax <= 0x1p60f) && (amax >= 0x1p-60f || amax == 0.0f);
+  if ((both >> 8) != scale_byte && in_window) {
+    const float s = div_markstein_nonneg(div_markstein_nonneg(amax, 6.0f, 0x1.555556p-3f /* RN(1/6) */), ts.g, ts.rcp);
+    scale_byte = f32_to_e4m3_byte(fminf(s, 448.0f));
+  }
+  const float total = __fmul_rn(ts.g, e4m3_byte_to_f32(scale_byte));
+  if (in_window && !all_ones(total)) {
+    const bool dead = (total == 0.0f);  // zero scale: every code is +0
+    const float t = dead ? 1.0f : total;
+    nvfp4_codes_corrected<T, kHiFirst>(w, t, approximate_reciprocal(t), lo_word, hi_word);
+    if (dead) {
       lo_word = 0;
       hi_word = 0;
     }
@@ -328,6 +332,16 @@ __device__ __forceinline__ void nvfp4_block_packed(const uint32_t (&w)[8], const
   lo_word = r.lo;
   hi_word = r.hi;
   scale_byte = r.scale_byte;
+}
+
+// The same out of line, for callers whose registers are needed elsewhere.
+template <typename T, bool kHiFirst>
+__device__ __noinline__ BlockCodes nvfp4_block_packed_call(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t w4, uint32_t w5,
+                                                           uint32_t w6, uint32_t w7, TensorScale ts) {
+  const uint32_t w[8] = {w0, w1, w2, w3, w4, w5, w6, w7};
+  BlockCodes r;
+  nvfp4_block_packed<T, kHiFirst>(w, ts, r.lo, r.hi, r.scale_byte);
+  return r;
 }
 
 // ---------------------------------------------------------------------------
@@ -340,6 +354,9 @@ __device__ __forceinline__ void nvfp4_block_packed(const uint32_t (&w)[8], const
 // Everything is computed for all of a thread's blocks before one test asks whether some bracket was split or some
 // operand lies outside the window; those blocks are done again, out of line.  Straight code lets the blocks' serial
 // chains (maximum, scale, conversion there and back, reciprocal) overlap, and has no Markstein chains in it.
+// kCorrected: 16-bit codes by nvfp4_codes_corrected, which no bracket can split.  The few-row linear gains by it (8 x 3072 x 3072 6.56 us
+// against 6.12, 8 x 18432 x 3072 with a dynamic scale 9.23 / 9.03); the fused epilogue, which waits for a thread's chains, does not: bf16 4608 x
+// 12288 x 3072 79.7 us with brackets, 80.7 with the correction.
 
 // Sixteen elements in registers: packed pairs of a 16-bit type, or floats.
 template <typename T>
@@ -384,7 +401,7 @@ __device__ __noinline__ BlockCodes nvfp4_block_exact(Sixteen<T> x, float g, floa
   return r;
 }
 
-template <typename T, bool kHiFirst, int kBlocks>
+template <typename T, bool kHiFirst, int kBlocks, bool kCorrected = sizeof(T) == 2>
 __device__ __forceinline__ void nvfp4_blocks(const Sixteen<T> (&x)[kBlocks], const TensorScale& ts, uint32_t (&codes)[kBlocks][2],
                                              uint32_t (&scale_byte)[kBlocks]) {
   float total[kBlocks];
@@ -397,17 +414,24 @@ __device__ __forceinline__ void nvfp4_blocks(const Sixteen<T> (&x)[kBlocks], con
     scale_byte[b] = both & 0xFFu;
     total[b] = __fmul_rn(ts.g, e4m3_byte_to_f32(scale_byte[b]));
     const bool dead = total[b] == 0.0f;
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(dead ? 1.0f : total[b]));
-    const float y_hi = __fmul_rn(y, 0x1.000008p0f), y_lo = __fmul_rn(y, 0x1.fffffp-1f);
-    float v[16];
-    x[b].widen(v);
-    const uint32_t lo = scaled_e2m1_word<kHiFirst>(v, y_hi), hi = scaled_e2m1_word<kHiFirst>(v + 8, y_hi);
-    const uint32_t split = (lo ^ scaled_e2m1_word<kHiFirst>(v, y_lo)) | (hi ^ scaled_e2m1_word<kHiFirst>(v + 8, y_lo));
+    const float t = dead ? 1.0f : total[b], y = approximate_reciprocal(t);
+    sure[b] = (both >> 8) == scale_byte[b] && ts.in_window && amax <= 0x1p60f && (amax >= 0x1p-60f || amax == 0.0f);
+    uint32_t lo, hi;
+    if constexpr (kCorrected) {
+      nvfp4_codes_corrected<T, kHiFirst>(x[b].w, t, y, lo, hi);
+      sure[b] = sure[b] && !all_ones(total[b]);
+      ok[b] = sure[b];
+    } else {
+      const float y_hi = __fmul_rn(y, 0x1.000008p0f), y_lo = __fmul_rn(y, 0x1.fffffp-1f);
+      float v[16];
+      x[b].widen(v);
+      lo = scaled_e2m1_word<kHiFirst>(v, y_hi);
+      hi = scaled_e2m1_word<kHiFirst>(v + 8, y_hi);
+      const uint32_t split = (lo ^ scaled_e2m1_word<kHiFirst>(v, y_lo)) | (hi ^ scaled_e2m1_word<kHiFirst>(v + 8, y_lo));
+      ok[b] = sure[b] && (split == 0u || dead);
+    }
     codes[b][0] = dead ? 0u : lo;  // zero scale: every code is +0
     codes[b][1] = dead ? 0u : hi;
-    sure[b] = (both >> 8) == scale_byte[b] && ts.in_window && amax <= 0x1p60f && (amax >= 0x1p-60f || amax == 0.0f);
-    ok[b] = sure[b] && (split == 0u || dead);
     all = all && ok[b];
   }
   if (!all) {

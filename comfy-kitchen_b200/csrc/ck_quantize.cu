@@ -258,8 +258,8 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
     if (has_data && row < rows) {
       uint8_t* const dst = codes + static_cast<int64_t>(row) * code_pitch + pc * (kElems / 2);
       if constexpr (kBlocks == 2) {
-        // one block at a time, with the Markstein scale: the straight pair of nvfp4_blocks is slower here (bf16 4096 x 3072
-        // 7.9 us against 8.5, 512 x 3072 3.4 against 3.7), where the loads of the next row group are in flight meanwhile
+        // one block after the other: the straight pair of nvfp4_blocks is slower here (bf16 4096 x 3072 7.3 us against 7.5,
+        // 512 x 3072 2.72 against 2.84), where the loads of the next row group are in flight meanwhile
         uint32_t w0, w1, w2, w3, s0, s1;
         nvfp4_block_packed<T, kHiFirst>(a.w, ts, w0, w1, s0);
         nvfp4_block_packed<T, kHiFirst>(b.w, ts, w2, w3, s1);
