@@ -799,23 +799,28 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       tc_fence_after_sync();
       const int c0 = half * kColsPerWarp;
       const uint32_t t_row = tmem_base + acc * Cfg::kAccCols + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
-      // The fused 16-bit epilogue never holds the raw accumulator: it drains 32 columns at a
+      // The fused 16-bit epilogue never holds the raw accumulator: it drains 16 columns at a
       // time and keeps alpha * acc + bias rounded to OutT as packed pairs (a quarter of the
       // registers); the others pull their whole share with back-to-back loads.
       constexpr bool kPackedDrain = FUSED && sizeof(OutT) == 2;
-      uint32_t buf[kPackedDrain ? 1 : kChunks][32];
+      [[maybe_unused]] uint32_t buf[kPackedDrain ? 1 : kChunks][32];
       [[maybe_unused]] uint32_t pk[kPackedDrain ? kChunks : 1][16];
       if constexpr (kPackedDrain) {
+        // 16 columns at a time, the next ones on their way while these are scaled: the tensor pipe idles until the drain ends.
+        // 32 at a time and one after the other / so, us: bf16 4608 x 12288 x 3072 80.5 / 79.9, 1024 x 12288 x 3072 23.8 / 23.6, fp16 4608 x
+        // 12288 x 3072 87.2 / 81.7, 1000 x 8192 x 2048 16.2 / 15.7.
+        uint32_t part[2][16];
+        tmem_load_32x16(t_row, part[0]);
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-          tmem_load_32x32(t_row + c * 32, buf[0]);
+        for (int h = 0; h < 2 * kChunks; ++h) {
           tmem_load_wait();
-          const float2* b2 = reinterpret_cast<const float2*>(bias_s + c0 + c * 32);
+          if (h + 1 < 2 * kChunks) tmem_load_32x16(t_row + (h + 1) * 16, part[(h + 1) % 2]);
+          const float2* b2 = reinterpret_cast<const float2*>(bias_s + c0 + h * 16);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float2 y = fma_x2(make_float2(__uint_as_float(buf[0][2 * i]), __uint_as_float(buf[0][2 * i + 1])),
+          for (int i = 0; i < 8; ++i) {
+            const float2 y = fma_x2(make_float2(__uint_as_float(part[h % 2][2 * i]), __uint_as_float(part[h % 2][2 * i + 1])),
                                     make_float2(alpha, alpha), b2[i]);
-            pk[c][i] = pack_pair<OutT>(y.x, y.y);
+            pk[h / 2][8 * (h % 2) + i] = pack_pair<OutT>(y.x, y.y);
           }
         }
       } else {
@@ -960,7 +965,8 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           // GELU and re-quantization alone of a row's whole share of columns, the usual call: two blocks at a time in one
           // straight piece of code, in which their serial chains and the activation's overlap.  A tile took its epilogue 9.2 k
           // cycles (1.5 k more waiting for the next tile's bias behind its conversion) beside a main loop of 6.5 k.  fc1 in graph
-          // replays, before / one / two / four blocks at a time: 4608 x 12288 x 3072 85.4 / 85.6 / 81.5 / 89.7 us (four spill), 16384 x 8192
+          // replays, before / one / two / four blocks at a time: 4608 x 12288 x 3072 85.4 / 85.6 / 81.5 / 89.7 us (four spill; with the drain and the
+          // blocks' arithmetic as they are now two take 79.9, one at a time beside the next one's GELU 81.1 to 83.8), 16384 x 8192
           // x 2048 175.8 / 166.9 / 158.7 / 180.2.
           if (p.activation == CK_ACT_GELU_TANH && p.out == nullptr && row < p.M && n0 + c0 + kColsPerWarp <= p.N) {
 #pragma unroll
