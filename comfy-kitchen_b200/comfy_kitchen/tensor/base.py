@@ -241,9 +241,12 @@ class QuantizedTensor(torch.Tensor):
         generic = _DISPATCH_TABLE.get(func)
         if generic is not None:
             return generic(first, args, kwargs)
-        layout = _get_layout_from_args(args)
+        layout = LAYOUTS[first._layout_cls] if type(first) is QuantizedTensor else _get_layout_from_args(args)
         per_layout = _LAYOUT_DISPATCH_TABLE.get(func)
         if layout is not None and per_layout:
+            handler = per_layout.get(layout)
+            if handler is not None:
+                return handler(first, args, kwargs)
             for klass in layout.__mro__:
                 handler = per_layout.get(klass)
                 if handler is not None:
