@@ -433,6 +433,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   constexpr int kThreads = num_threads(FUSED, TILE_N);
   static_assert(TILE_N <= 32 * kNumEpilogueWarps, "one bias value per epilogue thread");
   constexpr bool kCluster = SPLIT == Split::kCluster;
+  constexpr bool kOneLane = CTAS == 1, kIssuerLane = CTAS == 1 || FUSED;
   static_assert(SPLIT == Split::kNone || (CTAS == 1 && !FUSED), "only plain one-CTA tiles are split");
   static_assert(SPLIT != Split::kOutputs || (OUT_STAGE != 0 && std::is_same<OutT, float>::value), "raw partial tiles, staged");
   static_assert(!kCluster || kTileM * TILE_N * 4 <= Cfg::kRingBytes, "a partial tile fits in the operand ring");
@@ -535,84 +536,81 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int k_stages = (p.k_bytes + kStageKBytes - 1) / kStageKBytes;
   const int total_mma = (p.k_bytes + kMmaKBytes - 1) / kMmaKBytes;
 
-  // The role loops below are executed by whole warps with warp-uniform control flow; the
-  // asynchronous instructions themselves are issued by one elected lane.
+  // Who walks a role's loop.  One CTA: one elected lane all of it.  As whole warps that elect a lane and meet again per stage the
+  // issuer took 600 cycles a stage and the producer 480 (128 x 128 tiles; the tensor pipe needs 320 with NVFP4's eight scale copies, 284
+  // with MXFP8's two), so, about 400 and 370.  us, whole warps / one lane: NVFP4 64 x 3072 x 3072 6.37 / 5.86, 256 x 3072 x 3072 6.64 / 6.06, 512 x
+  // 3072 x 3072 7.36 / 6.85, 256 x 3072 x 12288 13.5 / 13.1, MXFP8 512 x 3072 x 3072 10.8 / 9.8, 128 x 9216 x 3072 10.2 / 9.65.  Pairs are bound by the
+  // tensor pipe at 512 cycles, and whole warps serve them better (NVFP4 4096 x 3072 x 3072 18.8 / 19.2, 16384 x 9216 x 3072 180 / 184), except the issuer beside the
+  // fused epilogue's sixteen warps (1024 x 12288 x 3072 23.6 / 23.1).  Asking for the next stage's barrier ahead of a stage's MMAs gains nothing.
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     pdl_wait();  // operands and scales may come from the kernel before this one
     CK_TRACE3(2);
-    int ring_s = 0;
-    uint32_t ring_ph = 0;
-    [[maybe_unused]] uint32_t tile_it = 0;
-    for (int item = worker; item < num_items; item += num_workers, ++tile_it) {
-      const int tile = item / splits;
-      const int ks_begin = (item - tile * splits) * p.k_stages_per_split;
-      const int ks_end = min(k_stages, ks_begin + p.k_stages_per_split);
-      // consecutive workers take neighbouring tiles in the walking order the launch chose (p.raster)
-      const int tile_m = tile_row_block(p, tile);
-      const int tile_n = tile_col_block(p, tile);
-      const int m0 = tile_m * Cfg::kTileRows + static_cast<int>(cta_rank) * kTileM;  // this CTA's rows of A
-      const int n0 = tile_n * TILE_N;
-      const int rb_b0 = n0 / 128;
-      int rb_b_count = 0;
+    if (!kOneLane || elect_one()) {
+      const uint32_t full_addr = smem_u32(full_bar), empty_addr = smem_u32(empty_bar);
+      const uint32_t a_addr = smem_u32(smem_a), b_addr = smem_u32(smem_b), sfa_addr = smem_u32(smem_sfa), sfb_addr = smem_u32(smem_sfb);
+      int s = 0;  // ring position and phase as running counters (STAGES is not a power of two)
+      uint32_t ph = 0;
+      [[maybe_unused]] uint32_t tile_it = 0;
+      for (int item = worker; item < num_items; item += num_workers, ++tile_it) {
+        const int tile = item / splits;
+        const int ks_begin = (item - tile * splits) * p.k_stages_per_split;
+        const int ks_end = min(k_stages, ks_begin + p.k_stages_per_split);
+        // consecutive workers take neighbouring tiles in the walking order the launch chose (p.raster)
+        const int tile_m = tile_row_block(p, tile);
+        const int tile_n = tile_col_block(p, tile);
+        const int m0 = tile_m * Cfg::kTileRows + static_cast<int>(cta_rank) * kTileM;  // this CTA's rows of A
+        const int n0 = tile_n * TILE_N;
+        const int b_row = n0 + static_cast<int>(cta_rank) * Cfg::kBRows;
+        const int rb_a = m0 / kTileM, rb_b0 = n0 / 128;
+        [[maybe_unused]] int rb_b_count = 0;
 #pragma unroll
-      for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) rb_b_count += (rb_b0 + r < p.n_row_blocks_b) ? 1 : 0;
-      // the second CTA of a pair may own rows past M: it then has no scale row block to load
-      const bool have_sfa = (m0 / kTileM) < p.n_row_blocks_a;
-      const uint8_t* sfa_src = p.sfa + static_cast<int64_t>(m0 / kTileM) * p.sf_col_tiles * 512;
-      const uint8_t* sfb_src = p.sfb + static_cast<int64_t>(rb_b0) * p.sf_col_tiles * 512;
-      for (int ks = ks_begin; ks < ks_end; ++ks) {
-        // ring position and phase as running counters (STAGES is not a power of two)
-        const int s = ring_s;
-        const uint32_t ph = ring_ph;
-        if (++ring_s == STAGES) {
-          ring_s = 0;
-          ring_ph ^= 1u;
-        }
-        mbar_wait(&empty_bar[s], ph ^ 1, abort_flag);  // in a pair: signalled from the leader CTA
-        if (ks == ks_begin) CK_TRACE(4);
-        if (ks == ks_end - 1) CK_TRACE(5);
-        if constexpr (CTAS == 2) {
-          // Every load of both CTAs reports its bytes to the leader's barrier; scale tiles
-          // come through 3-D tensor maps {512 B, column tile, row block} so that tiles past
-          // the end read as zeros and every stage has the same byte count.
-          if (elect_one()) {
-            if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * Cfg::kStageBytes);
-            const int sf_tile0 = ks * Cfg::kSfTilesPerStage;
-            tma_load_2d_pair(smem_a + s * Cfg::kABytes, &map_a, &full_bar[s], ks * kStageKBytes, m0);
-            tma_load_2d_pair(smem_b + s * Cfg::kBBytes, &map_b, &full_bar[s], ks * kStageKBytes,
-                             n0 + static_cast<int>(cta_rank) * Cfg::kBRows);
-            tma_load_3d_pair(smem_sfa + s * Cfg::kSfaBytes, &map_sfa, &full_bar[s], 0, sf_tile0, m0 / kTileM);
+        for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) rb_b_count += (rb_b0 + r < p.n_row_blocks_b) ? 1 : 0;
+        // a CTA may own rows past M: it then has no scale row block to load
+        [[maybe_unused]] const bool have_sfa = rb_a < p.n_row_blocks_a;
+        [[maybe_unused]] const uint8_t* sfa_src = p.sfa + (static_cast<int64_t>(rb_a) * p.sf_col_tiles + ks_begin * Cfg::kSfTilesPerStage) * 512;
+        [[maybe_unused]] const uint8_t* sfb_src = p.sfb + (static_cast<int64_t>(rb_b0) * p.sf_col_tiles + ks_begin * Cfg::kSfTilesPerStage) * 512;
+        for (int ks = ks_begin; ks < ks_end; ++ks) {
+          mbar_wait(empty_addr + s * 8, ph ^ 1, abort_flag);  // in a pair: signalled from the leader CTA
+          if (ks == ks_begin) CK_TRACE_ELECTED(4);
+          if (ks == ks_end - 1) CK_TRACE_ELECTED(5);
+          if (kOneLane || elect_one()) {
+            const uint32_t bar = full_addr + s * 8;
+            if constexpr (CTAS == 2) {
+              // Every load of both CTAs reports its bytes to the leader's barrier; scale tiles
+              // come through 3-D tensor maps {512 B, column tile, row block} so that tiles past
+              // the end read as zeros and every stage has the same byte count.
+              if (cta_rank == 0) mbar_arrive_expect_tx(bar, 2 * Cfg::kStageBytes);
+              tma_load_2d_pair(a_addr + s * Cfg::kABytes, &map_a, bar, ks * kStageKBytes, m0);
+              tma_load_2d_pair(b_addr + s * Cfg::kBBytes, &map_b, bar, ks * kStageKBytes, b_row);
+              tma_load_3d_pair(sfa_addr + s * Cfg::kSfaBytes, &map_sfa, bar, 0, ks * Cfg::kSfTilesPerStage, rb_a);
+              tma_load_3d_pair(sfb_addr + s * Cfg::kSfbBytes, &map_sfb, bar, 0, ks * Cfg::kSfTilesPerStage, rb_b0);
+            } else {
+              const uint32_t sf_bytes = static_cast<uint32_t>(min(Cfg::kSfTilesPerStage, p.sf_col_tiles - ks * Cfg::kSfTilesPerStage)) * 512u;
+              mbar_arrive_expect_tx(bar, Cfg::kABytes + Cfg::kBBytes + sf_bytes * ((have_sfa ? 1 : 0) + rb_b_count));
+              tma_load_2d(a_addr + s * Cfg::kABytes, &map_a, bar, ks * kStageKBytes, m0);
+              tma_load_2d(b_addr + s * Cfg::kBBytes, &map_b, bar, ks * kStageKBytes, b_row);
+              if (have_sfa) bulk_load_1d(sfa_addr + s * Cfg::kSfaBytes, sfa_src, sf_bytes, bar);
 #pragma unroll
-            for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) {
-              tma_load_3d_pair(smem_sfb + s * Cfg::kSfbBytes + r * Cfg::kSfTilesPerStage * 512, &map_sfb, &full_bar[s],
-                               0, sf_tile0, rb_b0 + r);
+              for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) {
+                if (r < rb_b_count) {
+                  bulk_load_1d(sfb_addr + s * Cfg::kSfbBytes + r * Cfg::kSfTilesPerStage * 512, sfb_src + static_cast<int64_t>(r) * p.sf_col_tiles * 512,
+                               sf_bytes, bar);
+                }
+              }
+              sfa_src += Cfg::kSfTilesPerStage * 512;
+              sfb_src += Cfg::kSfTilesPerStage * 512;
             }
           }
-          __syncwarp();
-          continue;
-        }
-        if (elect_one()) {
-          const int sf_tile0 = ks * Cfg::kSfTilesPerStage;
-          const uint32_t sf_bytes = static_cast<uint32_t>(min(Cfg::kSfTilesPerStage, p.sf_col_tiles - sf_tile0)) * 512u;
-          mbar_arrive_expect_tx(&full_bar[s],
-                                Cfg::kABytes + Cfg::kBBytes + sf_bytes * ((have_sfa ? 1 : 0) + rb_b_count));
-          tma_load_2d(smem_a + s * Cfg::kABytes, &map_a, &full_bar[s], ks * kStageKBytes, m0);
-          tma_load_2d(smem_b + s * Cfg::kBBytes, &map_b, &full_bar[s], ks * kStageKBytes,
-                      n0 + static_cast<int>(cta_rank) * Cfg::kBRows);
-          if (have_sfa) bulk_load_1d(smem_sfa + s * Cfg::kSfaBytes, sfa_src + sf_tile0 * 512, sf_bytes, &full_bar[s]);
-#pragma unroll
-          for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) {
-            if (r < rb_b_count) {
-              bulk_load_1d(smem_sfb + s * Cfg::kSfbBytes + r * Cfg::kSfTilesPerStage * 512,
-                           sfb_src + (static_cast<int64_t>(r) * p.sf_col_tiles + sf_tile0) * 512, sf_bytes,
-                           &full_bar[s]);
-            }
+          if constexpr (!kOneLane) __syncwarp();
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
           }
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp == 1 && cta_rank != 0) {
     // second CTA of a pair: the leader issues the MMAs and the scale copies for both
   } else if (warp == 1) {
@@ -631,94 +629,98 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const uint32_t sf_hi = static_cast<uint32_t>(make_scale_desc(0) >> 32);
     const uint32_t t_sfa0 = tmem_base + Cfg::kSfaCol;
     const uint32_t t_sfb0 = tmem_base + Cfg::kSfbCol;
-    const uint32_t empty_addr = smem_u32(empty_bar);
+    const uint32_t full_addr = smem_u32(full_bar), empty_addr = smem_u32(empty_bar);
     const uint32_t acc_full_addr = smem_u32(acc_full_bar);
     const uint32_t empty_addr_peer = (CTAS == 2) ? map_to_cta(empty_addr, 1) : 0u;
     const uint32_t acc_full_addr_peer = (CTAS == 2) ? map_to_cta(acc_full_addr, 1) : 0u;
-    [[maybe_unused]] uint32_t it = 0;
-    int ring_s = 0;
-    uint32_t ring_ph = 0;
-    uint32_t tile_it = 0;
-    for (int item = worker; item < num_items; item += num_workers, ++tile_it) {
-      const int tile = item / splits;
-      const int ks_begin = (item - tile * splits) * p.k_stages_per_split;
-      const int ks_end = min(k_stages, ks_begin + p.k_stages_per_split);
-      const int n0 = tile_col_block(p, tile) * TILE_N;
-      const int acc = tile_it % NUM_ACC;
-      const uint32_t acc_ph = (tile_it / NUM_ACC) & 1;
-      const uint32_t d_tmem = tmem_base + acc * Cfg::kAccCols;
-      // B scale words of this tile start (n0 % 128) / 32 columns into the first row block
-      const uint32_t sfb_shift = (n0 % 128) / 32;
-      for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
-        const int s = ring_s;
-        const uint32_t ph = ring_ph;
-        if (++ring_s == STAGES) {
-          ring_s = 0;
-          ring_ph ^= 1u;
-        }
-        CK_TRACE2(1, it);
-        mbar_wait(&full_bar[s], ph, abort_flag);
-        if (ks == ks_begin) CK_TRACE(2);
-        if (ks == ks_end - 1) CK_TRACE(3);
-        CK_TRACE2(2, it);
-        tc_fence_after_sync();
-        if (elect_one()) {
-          const uint32_t a_lo = a_lo0 + s * (Cfg::kABytes >> 4);
-          const uint32_t b_lo = b_lo0 + s * (Cfg::kBBytes >> 4);
-          const int n_mma = min(kMmaPerStage, total_mma - ks * kMmaPerStage);
-          const uint32_t t_sfa = t_sfa0 + s * Cfg::kSfColsPerBuf;
-          const uint32_t t_sfb_tile = t_sfb0 + s * Cfg::kSfColsPerBuf + sfb_shift;
-          // scale tiles of this stage: shared -> tensor memory (512 bytes = 32 descriptor units);
-          // the tensor pipe runs them in order ahead of the MMAs that read them
-          const uint32_t sfa_lo = sfa_lo0 + s * (Cfg::kSfaBytes >> 4);
-          const uint32_t sfb_lo = sfb_lo0 + s * (Cfg::kSfbBytes >> 4);
-          const uint32_t t_sfb = t_sfb0 + s * Cfg::kSfColsPerBuf;
+    if (!kIssuerLane || elect_one()) {
+      [[maybe_unused]] uint32_t it = 0;
+      int ring_s = 0;
+      uint32_t ring_ph = 0;
+      uint32_t tile_it = 0;
+      for (int item = worker; item < num_items; item += num_workers, ++tile_it) {
+        const int tile = item / splits;
+        const int ks_begin = (item - tile * splits) * p.k_stages_per_split;
+        const int ks_end = min(k_stages, ks_begin + p.k_stages_per_split);
+        const int n0 = tile_col_block(p, tile) * TILE_N;
+        const int acc = tile_it % NUM_ACC;
+        const uint32_t acc_ph = (tile_it / NUM_ACC) & 1;
+        const uint32_t d_tmem = tmem_base + acc * Cfg::kAccCols;
+        // B scale words of this tile start (n0 % 128) / 32 columns into the first row block
+        const uint32_t sfb_shift = (n0 % 128) / 32;
+        for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
+          const int s = ring_s;
+          const uint32_t ph = ring_ph;
+          if (++ring_s == STAGES) {
+            ring_s = 0;
+            ring_ph ^= 1u;
+          }
+          CK_TRACE2(1, it);
+          mbar_wait(full_addr + s * 8, ph, abort_flag);
+          if (ks == ks_begin) CK_TRACE_ELECTED(2);
+          if (ks == ks_end - 1) CK_TRACE_ELECTED(3);
+          CK_TRACE2(2, it);
+          tc_fence_after_sync();
+          if (kIssuerLane || elect_one()) {
+            const uint32_t a_lo = a_lo0 + s * (Cfg::kABytes >> 4);
+            const uint32_t b_lo = b_lo0 + s * (Cfg::kBBytes >> 4);
+            const int n_mma = total_mma - ks * kMmaPerStage;  // left from here on
+            const uint32_t t_sfa = t_sfa0 + s * Cfg::kSfColsPerBuf;
+            const uint32_t t_sfb_tile = t_sfb0 + s * Cfg::kSfColsPerBuf + sfb_shift;
+            // scale tiles of this stage: shared -> tensor memory (512 bytes = 32 descriptor units);
+            // the tensor pipe runs them in order ahead of the MMAs that read them
+            const uint32_t sfa_lo = sfa_lo0 + s * (Cfg::kSfaBytes >> 4);
+            const uint32_t sfb_lo = sfb_lo0 + s * (Cfg::kSfbBytes >> 4);
+            const uint32_t t_sfb = t_sfb0 + s * Cfg::kSfColsPerBuf;
 #pragma unroll
-          for (int t = 0; t < Cfg::kSfTilesPerStage; ++t) {
-            tc_copy_scales_32x128b<CTAS>(t_sfa + t * 4, desc64(sfa_lo + t * 32, sf_hi));
+            for (int t = 0; t < Cfg::kSfTilesPerStage; ++t) {
+              tc_copy_scales_32x128b<CTAS>(t_sfa + t * 4, desc64(sfa_lo + t * 32, sf_hi));
 #pragma unroll
-            for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) {
-              tc_copy_scales_32x128b<CTAS>(t_sfb + t * Cfg::kSfbColsPerTile + r * 4,
-                                           desc64(sfb_lo + (r * Cfg::kSfTilesPerStage + t) * 32, sf_hi));
+              for (int r = 0; r < Cfg::kSfbRowBlocks; ++r) {
+                tc_copy_scales_32x128b<CTAS>(t_sfb + t * Cfg::kSfbColsPerTile + r * 4,
+                                             desc64(sfb_lo + (r * Cfg::kSfTilesPerStage + t) * 32, sf_hi));
+              }
             }
-          }
-          if (ks == ks_begin) {
-            // Only now does the tile need its accumulator: the wait for the epilogue to have
-            // drained it comes after the first stage has landed.
-            CK_TRACE_ELECTED(0);
-            mbar_wait(&acc_empty_bar[acc], acc_ph ^ 1, abort_flag);
-            CK_TRACE_ELECTED(1);
-            tc_fence_after_sync();
-          }
-#pragma unroll
-          for (int kb = 0; kb < kMmaPerStage; ++kb) {
-            if (kb < n_mma) {
+            if (ks == ks_begin) {
+              // Only now does the tile need its accumulator: the wait for the epilogue to have
+              // drained it comes after the first stage has landed.
+              CK_TRACE_ELECTED(0);
+              mbar_wait(&acc_empty_bar[acc], acc_ph ^ 1, abort_flag);
+              CK_TRACE_ELECTED(1);
+              tc_fence_after_sync();
+            }
+            auto mma = [&](int kb) {
               const uint32_t accumulate = (ks != ks_begin || kb != 0) ? 1u : 0u;
               // advancing K inside the swizzle atom = advancing the start address (32 B = 2 units)
               const uint64_t a_desc = desc64(a_lo + kb * 2, op_hi);
               const uint64_t b_desc = desc64(b_lo + kb * 2, op_hi);
               if constexpr (KIND == Kind::kNvfp4) {
-                mma_nvfp4<CTAS>(d_tmem, a_desc, b_desc, Cfg::kIdesc, t_sfa + kb * 4,
-                                t_sfb_tile + kb * Cfg::kSfbColsPerTile, accumulate);
+                mma_nvfp4<CTAS>(d_tmem, a_desc, b_desc, Cfg::kIdesc, t_sfa + kb * 4, t_sfb_tile + kb * Cfg::kSfbColsPerTile, accumulate);
               } else {
                 // one scale tile serves the four MMAs of the stage: byte kb of each scale word
-                mma_mxfp8<CTAS>(d_tmem, a_desc, b_desc, idesc_with_scale_ids(Cfg::kIdesc, kb), t_sfa, t_sfb_tile,
-                                accumulate);
+                mma_mxfp8<CTAS>(d_tmem, a_desc, b_desc, idesc_with_scale_ids(Cfg::kIdesc, kb), t_sfa, t_sfb_tile, accumulate);
               }
+            };
+            if (n_mma >= kMmaPerStage) {
+#pragma unroll
+              for (int kb = 0; kb < kMmaPerStage; ++kb) mma(kb);
+            } else {
+              for (int kb = 0; kb < n_mma; ++kb) mma(kb);
+            }
+            // stage (and its scale columns) reusable once these MMAs retire; in a pair both CTAs are told
+            tc_commit<CTAS>(empty_addr + s * 8);
+            if constexpr (CTAS == 2) tc_commit<CTAS>(empty_addr_peer + s * 8);
+            if (ks == ks_end - 1) {
+              tc_commit<CTAS>(acc_full_addr + acc * 8);
+              if constexpr (CTAS == 2) tc_commit<CTAS>(acc_full_addr_peer + acc * 8);
             }
           }
-          // stage (and its scale columns) reusable once these MMAs retire; in a pair both CTAs are told
-          tc_commit<CTAS>(empty_addr + s * 8);
-          if constexpr (CTAS == 2) tc_commit<CTAS>(empty_addr_peer + s * 8);
-          if (ks == ks_end - 1) {
-            tc_commit<CTAS>(acc_full_addr + acc * 8);
-            if constexpr (CTAS == 2) tc_commit<CTAS>(acc_full_addr_peer + acc * 8);
-          }
+          if constexpr (!kIssuerLane) __syncwarp();
+          CK_TRACE2(3, it);
         }
-        __syncwarp();
-        CK_TRACE2(3, it);
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2 ..)
     // Two warps share each 32-lane quarter of tensor memory and split the tile's columns.
@@ -1242,13 +1244,13 @@ int encode_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t
 }
 
 // Scale tensor in the tiled layout as a 3-D array {128 x uint32 (one 512-byte tile), column
-// tile, row block}; a box is `tiles` consecutive column tiles of one row block.
-int encode_scale_map(CUtensorMap* map, const void* base, int64_t row_blocks, int64_t col_tiles, int tiles) {
+// tile, row block}; a box is `tiles` consecutive column tiles of `box_row_blocks` row blocks.
+int encode_scale_map(CUtensorMap* map, const void* base, int64_t row_blocks, int64_t col_tiles, int tiles, int box_row_blocks) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return fail(CK_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(col_tiles), static_cast<cuuint64_t>(row_blocks)};
   const cuuint64_t strides[2] = {512, static_cast<cuuint64_t>(col_tiles) * 512};
-  const cuuint32_t box[3] = {128, static_cast<cuuint32_t>(tiles), 1};
+  const cuuint32_t box[3] = {128, static_cast<cuuint32_t>(tiles), static_cast<cuuint32_t>(box_row_blocks)};
   const cuuint32_t elem_strides[3] = {1, 1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(base), dims, strides, box,
                         elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -1278,9 +1280,9 @@ int make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t r
                     [&](CUtensorMap* m) { return encode_operand_map(m, base, rows, row_bytes, box_rows); });
 }
 
-int make_scale_map(CUtensorMap* map, const void* base, int64_t row_blocks, int64_t col_tiles, int tiles) {
-  return cached_map(map, MapKey{1, base, row_blocks, col_tiles, tiles, 0},
-                    [&](CUtensorMap* m) { return encode_scale_map(m, base, row_blocks, col_tiles, tiles); });
+int make_scale_map(CUtensorMap* map, const void* base, int64_t row_blocks, int64_t col_tiles, int tiles, int box_row_blocks) {
+  return cached_map(map, MapKey{1, base, row_blocks, col_tiles, tiles, box_row_blocks},
+                    [&](CUtensorMap* m) { return encode_scale_map(m, base, row_blocks, col_tiles, tiles, box_row_blocks); });
 }
 
 int make_output_map(CUtensorMap* map, void* base, int64_t rows, int64_t cols, int elem_bytes, int64_t pitch_elems) {
@@ -1390,8 +1392,8 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   cfg.gridDim = dim3(workers * CTAS);
   CUtensorMap map_sfa = {}, map_sfb = {};
   if (CTAS == 2) {
-    if (int rc = make_scale_map(&map_sfa, p.sfa, p.n_row_blocks_a, p.sf_col_tiles, Cfg::kSfTilesPerStage)) return rc;
-    if (int rc = make_scale_map(&map_sfb, p.sfb, p.n_row_blocks_b, p.sf_col_tiles, Cfg::kSfTilesPerStage)) return rc;
+    if (int rc = make_scale_map(&map_sfa, p.sfa, p.n_row_blocks_a, p.sf_col_tiles, Cfg::kSfTilesPerStage, 1)) return rc;
+    if (int rc = make_scale_map(&map_sfb, p.sfb, p.n_row_blocks_b, p.sf_col_tiles, Cfg::kSfTilesPerStage, Cfg::kSfbRowBlocks)) return rc;
   }
   // Walking order of the tiles: the one whose concurrently running tiles touch fewer operand bytes
   // (A row blocks + B column blocks of one wave), so that a long operand is not pulled through L2

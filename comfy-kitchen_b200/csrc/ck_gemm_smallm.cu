@@ -269,63 +269,71 @@ small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------------ weight loads
     pdl_wait();
-    RingAt at(0);
-    for (int i = 0; i < n_stages; ++i, at.step(1, p.ring)) {
-      const int s = at.slot;
-      mbar_wait(&empty_bar[s], at.phase ^ 1, abort_flag);
-      if (elect_one()) {
+    if (elect_one()) {  // for the whole loop: see ck_gemm_kernel.cuh
+      const uint32_t full_addr = smem_u32(full_bar), empty_addr = smem_u32(empty_bar);
+      const uint32_t a_addr = smem_u32(smem_a), b_addr = smem_u32(smem_b), sfa_addr = smem_u32(smem_sfa), sfb_addr = smem_u32(smem_sfb);
+      const uint8_t* x_scales = p.x_scales + static_cast<int64_t>(ks0) * C::kSfTiles * 512;
+      RingAt at(0);
+      for (int i = 0; i < n_stages; ++i, at.step(1, p.ring)) {
+        const int s = at.slot;
+        const uint32_t bar = full_addr + s * 8;
+        mbar_wait(empty_addr + s * 8, at.phase ^ 1, abort_flag);
         const uint32_t sf_bytes = static_cast<uint32_t>(min(C::kSfTiles, sf_tiles - i * C::kSfTiles)) * 512u;
-        mbar_arrive_expect_tx(&full_bar[s], kDense ? kABytes + sf_bytes : kABytes + b_bytes + 2 * sf_bytes);
-        tma_load_2d(smem_a + s * kABytes, &map_w, &full_bar[s], (ks0 + i) * kStageKBytes, n0);
-        bulk_load_1d(smem_sfa + s * C::kSfBytes, w_scales + static_cast<int64_t>(i) * C::kSfTiles * 512, sf_bytes, &full_bar[s]);
+        mbar_arrive_expect_tx(bar, kDense ? kABytes + sf_bytes : kABytes + b_bytes + 2 * sf_bytes);
+        tma_load_2d(a_addr + s * kABytes, &map_w, bar, (ks0 + i) * kStageKBytes, n0);
+        bulk_load_1d(sfa_addr + s * C::kSfBytes, w_scales + static_cast<int64_t>(i) * C::kSfTiles * 512, sf_bytes, bar);
         if constexpr (!kDense) {
-          tma_load_2d(smem_b + s * b_bytes, &map_x, &full_bar[s], (ks0 + i) * kStageKBytes, 0);
-          bulk_load_1d(smem_sfb + s * C::kSfBytes, p.x_scales + static_cast<int64_t>(ks0 + i) * C::kSfTiles * 512, sf_bytes, &full_bar[s]);
+          tma_load_2d(b_addr + s * b_bytes, &map_x, bar, (ks0 + i) * kStageKBytes, 0);
+          bulk_load_1d(sfb_addr + s * C::kSfBytes, x_scales + static_cast<int64_t>(i) * C::kSfTiles * 512, sf_bytes, bar);
         }
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     pdl_wait();  // see ck_gemm_kernel.cuh: keeps the bounded waits from running out behind a long predecessor
-    const uint32_t a_lo0 = static_cast<uint32_t>(make_operand_desc_sw128(smem_u32(smem_a)));
-    const uint32_t b_lo0 = static_cast<uint32_t>(make_operand_desc_sw128(smem_u32(smem_b)));
-    const uint32_t op_hi = static_cast<uint32_t>(make_operand_desc_sw128(0) >> 32);
-    const uint32_t sfa_lo0 = static_cast<uint32_t>(make_scale_desc(smem_u32(smem_sfa)));
-    const uint32_t sfb_lo0 = static_cast<uint32_t>(make_scale_desc(smem_u32(smem_sfb)));
-    const uint32_t sf_hi = static_cast<uint32_t>(make_scale_desc(0) >> 32);
-    const int total_mma = (p.k_bytes + kMmaKBytes - 1) / kMmaKBytes - ks0 * kMmaPerStage;
-    RingAt at(0);
-    for (int i = 0; i < n_stages; ++i, at.step(1, p.ring)) {
-      const int s = at.slot;
-      mbar_wait(&full_bar[s], at.phase, abort_flag);
-      tc_fence_after_sync();
-      if (elect_one()) {
+    if (elect_one()) {
+      const uint32_t full_addr = smem_u32(full_bar), empty_addr = smem_u32(empty_bar);
+      const uint32_t a_lo0 = static_cast<uint32_t>(make_operand_desc_sw128(smem_u32(smem_a)));
+      const uint32_t b_lo0 = static_cast<uint32_t>(make_operand_desc_sw128(smem_u32(smem_b)));
+      const uint32_t op_hi = static_cast<uint32_t>(make_operand_desc_sw128(0) >> 32);
+      const uint32_t sfa_lo0 = static_cast<uint32_t>(make_scale_desc(smem_u32(smem_sfa)));
+      const uint32_t sfb_lo0 = static_cast<uint32_t>(make_scale_desc(smem_u32(smem_sfb)));
+      const uint32_t sf_hi = static_cast<uint32_t>(make_scale_desc(0) >> 32);
+      const int total_mma = (p.k_bytes + kMmaKBytes - 1) / kMmaKBytes - ks0 * kMmaPerStage;
+      RingAt at(0);
+      for (int i = 0; i < n_stages; ++i, at.step(1, p.ring)) {
+        const int s = at.slot;
+        mbar_wait(full_addr + s * 8, at.phase, abort_flag);
+        tc_fence_after_sync();
         const uint32_t t_sfa = tmem_base + kMmaN + s * C::kSfCols, t_sfb = t_sfa + C::kSfTiles * 4;
 #pragma unroll
         for (int t = 0; t < C::kSfTiles; ++t) {
           tc_copy_scales_32x128b<1>(t_sfa + t * 4, desc64(sfa_lo0 + s * (C::kSfBytes >> 4) + t * 32, sf_hi));
           tc_copy_scales_32x128b<1>(t_sfb + t * 4, desc64(sfb_lo0 + s * (C::kSfBytes >> 4) + t * 32, sf_hi));
         }
-        const int n_mma = min(kMmaPerStage, total_mma - i * kMmaPerStage);
-#pragma unroll
-        for (int kb = 0; kb < kMmaPerStage; ++kb) {
-          if (kb < n_mma) {
-            const uint32_t accumulate = (i != 0 || kb != 0) ? 1u : 0u;
-            const uint64_t a_desc = desc64(a_lo0 + s * (kABytes >> 4) + kb * 2, op_hi);
-            const uint64_t b_desc = desc64(b_lo0 + s * (b_bytes >> 4) + kb * 2, op_hi);
-            if constexpr (KIND == Kind::kNvfp4) {
-              mma_nvfp4<1>(tmem_base, a_desc, b_desc, C::kIdesc, t_sfa + kb * 4, t_sfb + kb * 4, accumulate);
-            } else {
-              mma_mxfp8<1>(tmem_base, a_desc, b_desc, idesc_with_scale_ids(C::kIdesc, kb), t_sfa, t_sfb, accumulate);
-            }
+        auto mma = [&](int kb) {
+          const uint32_t accumulate = (i != 0 || kb != 0) ? 1u : 0u;
+          const uint64_t a_desc = desc64(a_lo0 + s * (kABytes >> 4) + kb * 2, op_hi);
+          const uint64_t b_desc = desc64(b_lo0 + s * (b_bytes >> 4) + kb * 2, op_hi);
+          if constexpr (KIND == Kind::kNvfp4) {
+            mma_nvfp4<1>(tmem_base, a_desc, b_desc, C::kIdesc, t_sfa + kb * 4, t_sfb + kb * 4, accumulate);
+          } else {
+            mma_mxfp8<1>(tmem_base, a_desc, b_desc, idesc_with_scale_ids(C::kIdesc, kb), t_sfa, t_sfb, accumulate);
           }
+        };
+        const int n_mma = total_mma - i * kMmaPerStage;  // left from here on
+        if (n_mma >= kMmaPerStage) {
+#pragma unroll
+          for (int kb = 0; kb < kMmaPerStage; ++kb) mma(kb);
+        } else {
+          for (int kb = 0; kb < n_mma; ++kb) mma(kb);
         }
-        tc_commit<1>(smem_u32(&empty_bar[s]));
+        tc_commit<1>(empty_addr + s * 8);
         if (i == n_stages - 1) tc_commit<1>(smem_u32(acc_bar));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ quantizer, epilogue
     pdl_wait();
