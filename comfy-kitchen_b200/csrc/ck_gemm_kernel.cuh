@@ -194,7 +194,7 @@ __device__ __forceinline__ long long global_timer_ns() {
 }
 #define CK_TRACE3(slot)                                                                              \
   do {                                                                                               \
-    if (threadIdx.x == 0 && blockIdx.x < 160) {                                                      \
+    if (((slot) == 2 || threadIdx.x == 0) && blockIdx.x < 160) {                                     \
       long long* t3 = g_trace3 + ((p.trace_launch & 7) * 160 + blockIdx.x) * 8 + 2 * (slot);         \
       t3[0] = global_timer_ns();                                                                     \
       t3[1] = clock64();                                                                             \
@@ -544,8 +544,6 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // fused epilogue's sixteen warps (1024 x 12288 x 3072 23.6 / 23.1).  Asking for the next stage's barrier ahead of a stage's MMAs gains nothing.
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    pdl_wait();  // operands and scales may come from the kernel before this one
-    CK_TRACE3(2);
     if (!kOneLane || elect_one()) {
       const uint32_t full_addr = smem_u32(full_bar), empty_addr = smem_u32(empty_bar);
       const uint32_t a_addr = smem_u32(smem_a), b_addr = smem_u32(smem_b), sfa_addr = smem_u32(smem_sfa), sfb_addr = smem_u32(smem_sfb);
@@ -570,6 +568,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         [[maybe_unused]] const bool have_sfa = rb_a < p.n_row_blocks_a;
         [[maybe_unused]] const uint8_t* sfa_src = p.sfa + (static_cast<int64_t>(rb_a) * p.sf_col_tiles + ks_begin * Cfg::kSfTilesPerStage) * 512;
         [[maybe_unused]] const uint8_t* sfb_src = p.sfb + (static_cast<int64_t>(rb_b0) * p.sf_col_tiles + ks_begin * Cfg::kSfTilesPerStage) * 512;
+        // Operands and scales may come from the kernel before this one.  Its end is waited for only when the first load is all that is
+        // left to do: the tile's place, its divisions and the reads of the kernel's arguments took 400 to 800 cycles behind that wait (us,
+        // before / so: NVFP4 128 x 1024 x 1024 3.89 / 3.46, 64 x 3072 x 3072 5.86 / 5.45, 512 x 3072 x 3072 6.84 / 6.59, 4096 x 3072 x 3072 18.9 / 18.6).
+        bool first = item == worker;
         for (int ks = ks_begin; ks < ks_end; ++ks) {
           mbar_wait(empty_addr + s * 8, ph ^ 1, abort_flag);  // in a pair: signalled from the leader CTA
           if (ks == ks_begin) CK_TRACE_ELECTED(4);
@@ -581,6 +583,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               // come through 3-D tensor maps {512 B, column tile, row block} so that tiles past
               // the end read as zeros and every stage has the same byte count.
               if (cta_rank == 0) mbar_arrive_expect_tx(bar, 2 * Cfg::kStageBytes);
+              if (first) {
+                pdl_wait();
+                CK_TRACE3(2);
+              }
               tma_load_2d_pair(a_addr + s * Cfg::kABytes, &map_a, bar, ks * kStageKBytes, m0);
               tma_load_2d_pair(b_addr + s * Cfg::kBBytes, &map_b, bar, ks * kStageKBytes, b_row);
               tma_load_3d_pair(sfa_addr + s * Cfg::kSfaBytes, &map_sfa, bar, 0, ks * Cfg::kSfTilesPerStage, rb_a);
@@ -588,6 +594,10 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             } else {
               const uint32_t sf_bytes = static_cast<uint32_t>(min(Cfg::kSfTilesPerStage, p.sf_col_tiles - ks * Cfg::kSfTilesPerStage)) * 512u;
               mbar_arrive_expect_tx(bar, Cfg::kABytes + Cfg::kBBytes + sf_bytes * ((have_sfa ? 1 : 0) + rb_b_count));
+              if (first) {
+                pdl_wait();
+                CK_TRACE3(2);
+              }
               tma_load_2d(a_addr + s * Cfg::kABytes, &map_a, bar, ks * kStageKBytes, m0);
               tma_load_2d(b_addr + s * Cfg::kBBytes, &map_b, bar, ks * kStageKBytes, b_row);
               if (have_sfa) bulk_load_1d(sfa_addr + s * Cfg::kSfaBytes, sfa_src, sf_bytes, bar);
@@ -603,6 +613,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
           }
           if constexpr (!kOneLane) __syncwarp();
+          first = false;
           if (++s == STAGES) {
             s = 0;
             ph ^= 1u;

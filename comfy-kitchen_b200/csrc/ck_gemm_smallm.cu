@@ -268,7 +268,6 @@ small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   float alpha = 1.0f;  // quantizer warps
   if (warp == 0) {
     // ------------------------------------------------------------------ weight loads
-    pdl_wait();
     if (elect_one()) {  // for the whole loop: see ck_gemm_kernel.cuh
       const uint32_t full_addr = smem_u32(full_bar), empty_addr = smem_u32(empty_bar);
       const uint32_t a_addr = smem_u32(smem_a), b_addr = smem_u32(smem_b), sfa_addr = smem_u32(smem_sfa), sfb_addr = smem_u32(smem_sfb);
@@ -280,6 +279,7 @@ small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         mbar_wait(empty_addr + s * 8, at.phase ^ 1, abort_flag);
         const uint32_t sf_bytes = static_cast<uint32_t>(min(C::kSfTiles, sf_tiles - i * C::kSfTiles)) * 512u;
         mbar_arrive_expect_tx(bar, kDense ? kABytes + sf_bytes : kABytes + b_bytes + 2 * sf_bytes);
+        if (i == 0) pdl_wait();
         tma_load_2d(a_addr + s * kABytes, &map_w, bar, (ks0 + i) * kStageKBytes, n0);
         bulk_load_1d(sfa_addr + s * C::kSfBytes, w_scales + static_cast<int64_t>(i) * C::kSfTiles * 512, sf_bytes, bar);
         if constexpr (!kDense) {
