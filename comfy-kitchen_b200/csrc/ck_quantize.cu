@@ -133,6 +133,7 @@ struct ScaleSource {
   int n_partials;          //   the whole (small) input, which every block then reads for itself
   int64_t n_vecs;          // 32-byte units of the input
   float* out;              // the dynamic scale for whoever needs it next
+  bool backward;           // begin with the last rows (large fp32 inputs behind their reduction)
 };
 
 // amax(|x|) / (448 * 6) of the whole input, by every block for itself (all threads return it).  NaNs
@@ -180,7 +181,8 @@ __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSour
 //
 // The row groups are walked in order, which is also the order of the reduction pass: walked backwards (for
 // what the reduction pass left in L2) a static scale pays 0.3 us at 1024 x 3072 (4.72 against 4.43, inputs
-// not in L2) and three layers on one 4096 x 3072 input 85.0 against 83.9; a dynamic one gains nothing.
+// not in L2) and three layers on one 4096 x 3072 input 85.0 against 83.9.  Behind a reduction it pays for fp32 inputs that are larger than
+// L2 (kBackwardBytes); 16-bit inputs, bound by their arithmetic, gain nothing (36864 x 3072 83.2 / 83.8).
 //
 // kMark: the input's lines are marked first to leave L2 (evict_first), so that they make room for each other
 // and not push out the codes, which the GEMM reads next.  By the rule in launch_streaming: not for inputs that
@@ -213,12 +215,14 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
   // warms the cache (L2 is the point of coherence: what the previous kernel still writes is seen
   // by the loads after the wait), and it takes the DRAM latency of the first loads off the
   // critical path of a kernel that only runs for a few microseconds.
-  const int first = static_cast<int>(blockIdx.x);
+  const bool backward = kDynamic && kMark && sizeof(T) == 4 && src.backward;
+  const int first = backward ? row_groups - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
+  const int step = backward ? -static_cast<int>(gridDim.x) : static_cast<int>(gridDim.x);
   if (has_data && (threadIdx.x & 1) == 0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int row = (first + i * static_cast<int>(gridDim.x)) * kPairRows + static_cast<int>(threadIdx.y);
-      if (row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
+      const int row = (first + i * step) * kPairRows + static_cast<int>(threadIdx.y);
+      if (row >= 0 && row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
     }
   }
   pdl_wait();  // the tensor scale and x may come from the kernel before this one
@@ -245,11 +249,11 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
   }
   if constexpr (!kDynamic) g = ld_f32_dependent(src.given);
   const TensorScale ts = make_tensor_scale(g);
-  for (int rg = first; rg < row_groups; rg += gridDim.x) {
+  for (int rg = first; rg >= 0 && rg < row_groups; rg += step) {
     const int row = rg * kPairRows + threadIdx.y;
-    const int next_row = row + static_cast<int>(gridDim.x) * kPairRows;
+    const int next_row = row + step * kPairRows;
     Vec256 an = {}, bn = {};
-    if (has_data && next_row < data_rows) {
+    if (has_data && next_row >= 0 && next_row < data_rows) {
       const T* at = x + static_cast<int64_t>(next_row) * cols + pc * kElems;
       an = ld_stream_unit<kMark>(at);
       bn = ld_stream_unit<kMark>(at + kElems / 2);
@@ -484,6 +488,10 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
 // (fp32) 4.0 / 3.8, 384 KiB 6.3 / 5.2: the line could lie near 200 KiB.
 constexpr int64_t kWholeInputBytes = 64 * 1024;
 constexpr int64_t kDynamicScratchHead = 256;
+// fp32 inputs from here on are quantized from their last rows on, which the reduction has just read.  Forwards / backwards, us: 6144 x 3072
+// (72 MiB) 24.1 / 24.3, 8192 x 3072 (96 MiB) 31.4 / 31.6, 12288 x 3072 (144 MiB) 48.0 / 46.4, 24576 x 3072 97.6 / 94.7, 36864 x 3072 147 / 143.
+// Marking what the reduction reads first evict_first, so that the last 64 to 96 MiB stay, gains less (47.0 to 47.5 at 144 MiB).
+constexpr int64_t kBackwardBytes = 120ll << 20;
 
 __global__ void clear_word_kernel(unsigned int* word) {
   pdl_launch_dependents();
@@ -506,6 +514,7 @@ int launch_nvfp4_dynamic(const void* input, int dtype, float* scale_out, void* c
       float* partials = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kDynamicScratchHead);
       if (int rc = launch_amax_partials(x, dtype, src.n_vecs, partials, &src.n_partials, stream)) return rc;
       src.partials = partials;
+      src.backward = sizeof(T) == 4 && n * 4 > kBackwardBytes;
     }
     return launch_streaming<T>(x, src, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), orig_rows, num_rows, num_cols,
                                hi_first, stream);
