@@ -57,6 +57,17 @@ struct Room {
   bool left_by_pairs(int64_t pairs) const { return wanted && pairs * 2 <= sm_count(); }
 };
 
+// 128 x 128 tiles that take no more waves than pair tiles: a wave of them is shorter, with half the output of an SM behind its main loop.
+// That is where the pairs' last rows or columns are padding, with 257 to 384 rows above all, or their last wave is nearly empty.  us, pair / 128 x 128:
+// NVFP4 300 x 6144 x 3072 (48 pairs, 144 tiles) 9.1 / 7.1, 300 x 12288 x 3072 13.7 / 11.1, 384 x 12288 x 6144 22.3 / 18.9, MXFP8 384 x 6144 x 3072
+// 13.4 / 10.5, fused 384 x 9600 x 3072 14.8 / 11.8, 1152 x 4096 x 3072 15.7 / 12.1; with one wave more 768 x 9216 x 3072 14.0 / 15.1.  In front of the next dynamic
+// linear (Room) a full wave of small tiles is not worth it, 144 x 9472 x 1792 (37 pairs, 148 tiles) 12.0 / 12.9, 832 x 2560 x 3136 (40, 140) 15.1 / 15.7, unless
+// a sixth of the pairs' tiles is padding: 282 x 5696 x 3136 (46, 135) 15.1 / 13.6.
+bool tiles_in_as_few_waves(int64_t tiles, int64_t pairs, const Room& room) {
+  const int64_t tile_waves = ceil_div(tiles, sm_count()), pair_waves = ceil_div(pairs, sm_count() / 2);
+  return tile_waves <= pair_waves && tile_waves <= 3 && (!room.wanted || tile_waves > 1 || 10 * pairs >= 3 * tiles);
+}
+
 template <Kind KIND, typename OutT, bool FUSED>
 int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, const Room& room, cudaStream_t stream) {
   int config = forced_gemm_config();
@@ -69,7 +80,8 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
     // two of the small tiles (NVFP4 512 x 9216 x 1024 7.4 / 6.7, 256 x 18432 x 1024 8.1 / 7.2, fused 512 x 8192 x 1024 9.7 / 9.4; with six
     // stages 512 x 9216 x 1536 8.3 / 8.1 and 1003 x 3072 x 1536 7.5 / 7.6, with twelve 512 x 9216 x 3072 10.6 / 11.9).
     const int64_t pairs = ceil_div(p.M, 256) * ceil_div(p.N, 256);
-    const bool pair = pairs * 4 >= sm_count() && row_blocks > 1 && (!(k_stages <= 4 && tiles <= 2 * sm_count()) || room.left_by_pairs(pairs));
+    const bool pair = pairs * 4 >= sm_count() && row_blocks > 1 && !tiles_in_as_few_waves(tiles, pairs, room) &&
+                      (!(k_stages <= 4 && tiles <= 2 * sm_count()) || room.left_by_pairs(pairs));
     if (pair) {
       config = 4;
     } else if (tiles * 4 <= sm_count() || (half_tiles_pay(p.M, p.N, p.k_bytes) && room.left_by_half_tiles(p.M, p.N))) {
@@ -139,13 +151,11 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
   }
   plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
   // Two CTAs to a tile: half tiles instead, while their longer K costs less than the exchange.  They end in TMA stores, which want
-  // rows of whole 64-byte units (N of 16 bits off by 16: MXFP8 512 x 1648 x 2784 10.0 / 10.7, NVFP4 517 x 1584 x 4800 9.7 / 10.7).  With one row block and
-  // nearly all SMs the weight's stream gains too.  us, two CTAs / half tiles: MXFP8 128 x 9216, 24 stages, 11.9 / 10.3, 32 14.1 / 12.6, 64 19.9 / 21.3;
-  // 512 x 2304, 28 stages, 11.2 / 10.9, 32 11.9 / 12.1; NVFP4 128 x 9216, 32 stages, 14.7 / 13.6, 128 x 6400 11.1 / 10.7 with 24, 12.8 / 13.0 with 32;
-  // 512 x 2304, 20 stages, 10.0 / 9.4, 24 10.6 / 10.7, 32 12.0 / 13.1.
-  const bool streams = M <= kTileM && 8 * ceil_div(N, 64) >= 7 * sm_count() && k_bytes % kStageKBytes == 0;
-  const int most_stages = streams ? 32 : KIND == Kind::kNvfp4 ? 23 : 28;
-  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= most_stages && N % 32 == 0 && one_wave_of_half_tiles(M, N);
+  // rows of whole 64-byte units (N of 16 bits off by 16: MXFP8 512 x 1648 x 2784 10.0 / 10.7, NVFP4 517 x 1584 x 4800 9.7 / 10.7).  us, two CTAs /
+  // half tiles: linears NVFP4 256 x 4608, 24 stages, 12.9 / 11.5, 300 x 2048, 24 stages, 12.3 / 11.4, MXFP8 256 x 4608, 30 stages, 12.9 / 12.0.  Over drawn sizes of
+  // both formats half tiles take 0.91 to 1.0 of the time from 24 to 35 stages, 1.0 from 36 to 41 and 1.05 from 42 on.
+  constexpr int kMostStages = 36;
+  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= kMostStages && N % 32 == 0 && one_wave_of_half_tiles(M, N);
   if (plan->half_tiles) splits = 1;
   plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
   plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage
