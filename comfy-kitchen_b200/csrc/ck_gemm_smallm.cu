@@ -11,8 +11,9 @@
 //   * a 128-row tile to a CTA;
 //   * few tiles and a long K: every tile's K range over a cluster of CTAs, which add their partial tiles in split order
 //     through distributed shared memory.
-// (Half and quarter tiles to a CTA were measured: nothing gained.  An MMA of 128 weight rows takes the tensor pipe some 135 cycles
-// whatever N is, so that a CTA streams at most 4 KiB in that time; four accumulators in turn change nothing either.)
+// (Half and quarter tiles to a CTA were measured: nothing gained.  A stage, 16 KiB of weight, takes the tensor pipe some 160 cycles for its
+// four MMAs, 315 with NVFP4's eight scale copies, 105 and 50 bytes a cycle: more than an SM's 24 of what HBM gives.  Four accumulators in turn
+// change nothing either.)
 //
 // Dense activations (XT): as two kernels, the quantizer of a few rows is one wave of load latency, arithmetic and store
 // latency before the GEMM's loads may begin.  Here every CTA quantizes the rows it multiplies by, stage by stage, straight
