@@ -771,6 +771,13 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const bool vec_ok = (static_cast<int64_t>(p.N) * sizeof(OutT)) % 32 == 0 &&
                         (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0 && (TILE_N * sizeof(OutT)) % 32 == 0;
     const uint32_t acc_empty_leader = (CTAS == 2) ? map_to_cta(smem_u32(acc_empty_bar), 0) : 0u;
+    // The fused 16-bit epilogue never holds the raw accumulator: it drains 16 columns at a
+    // time and keeps alpha * acc + bias rounded to OutT as packed pairs (a quarter of the
+    // registers); the others pull their whole share with back-to-back loads.
+    constexpr bool kPackedDrain = FUSED && sizeof(OutT) == 2;
+    constexpr bool kWarpBias = kPackedDrain;  // each warp its own columns' bias (below)
+    constexpr int kBiasPerThread = kWarpBias ? kColsPerWarp / 32 : 1;
+    const int bias_col = kWarpBias ? half * kColsPerWarp + lane : et;
     [[maybe_unused]] uint32_t out_box = 0;  // boxes this warp has staged so far (ring index)
     uint32_t tile_it = 0;
     for (int item = worker; item < num_items; item += num_workers, ++tile_it) {
@@ -781,27 +788,41 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int n0 = tile_n * TILE_N;
       const int acc = tile_it % NUM_ACC;
       const uint32_t acc_ph = (tile_it / NUM_ACC) & 1;
-      // Bias of a tile's columns as fp32 in shared memory, three buffers in rotation: the
-      // buffer of tile t is filled while tile t - 1 is in its epilogue (right after the drain,
-      // where the warps are aligned anyway), so no barrier stands between the end of one
-      // epilogue and the wait for the next accumulator.  A warp can run at most one tile ahead
-      // of the slowest one (the barrier below), hence the third buffer.  Each epilogue thread
-      // fetches one value of the next tile before it waits for the accumulator, so the load's
-      // latency hides behind that wait.
+      // Bias of a tile's columns as fp32 in shared memory, three buffers in rotation: the buffer of tile t is filled
+      // while tile t - 1 is in its epilogue, right after the drain, with values fetched ahead of the wait for the
+      // accumulator, whose latency that wait hides.
+      // Plain tiles and fp32: every thread fetches one value, and the warps meet at a barrier after the drain, where they
+      // are aligned anyway; a warp then runs at most one tile ahead of the slowest, hence the third buffer.  Fused 16-bit tiles: every warp fetches the columns it reads itself (the four warps of the same columns
+      // write the same values; tile t + 3's come behind the accumulator of t + 2, which waits for all warps' drains of t, where the bias of t is
+      // read), since a barrier a tile made each of sixteen warps wait for the one with the longest chains: bf16 4608 x
+      // 8192 x 2048 47.8 / 44.8 us, 4608 x 12288 x 3072 79.7 / 77.2, fp16 80.7 / 78.4, 128 x 12288 x 3072 9.0 / 9.0.  With fp32 it lost (77.6 / 78.3),
+      // and so did plain pairs (36864 x 9216 x 3072 407 / 416).
       float* bias_s = smem_bias + (tile_it % 3) * TILE_N;
       const bool with_bias = p.bias != nullptr;
       if (tile_it == 0) {
-        if (et < TILE_N) bias_s[et] = (with_bias && n0 + et < p.N) ? load_bias(p.bias, p.bias_dtype, n0 + et) : 0.0f;
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * kNumEpilogueWarps) : "memory");  // epilogue warps only
+        if constexpr (kWarpBias) {
+#pragma unroll
+          for (int i = 0; i < kBiasPerThread; ++i) {
+            const int n = n0 + bias_col + 32 * i;
+            bias_s[bias_col + 32 * i] = (with_bias && n < p.N) ? load_bias(p.bias, p.bias_dtype, n) : 0.0f;
+          }
+          __syncwarp();
+        } else {
+          if (et < TILE_N) bias_s[et] = (with_bias && n0 + et < p.N) ? load_bias(p.bias, p.bias_dtype, n0 + et) : 0.0f;
+          asm volatile("bar.sync 1, %0;" ::"n"(32 * kNumEpilogueWarps) : "memory");  // epilogue warps only
+        }
       }
       const int next_item = item + num_workers;
       const bool has_next = next_item < num_items;
-      std::conditional_t<FUSED, uint32_t, float> bias_prefetched = 0;  // bits or value: zero is 0.0 in every type
-      if (has_next && et < TILE_N) {
-        const int n = tile_col_block(p, next_item / splits) * TILE_N + et;
-        if (with_bias && n < p.N) {
-          if constexpr (FUSED) bias_prefetched = load_bias_bits(p.bias, p.bias_dtype, n);
-          else bias_prefetched = load_bias(p.bias, p.bias_dtype, n);
+      std::conditional_t<FUSED, uint32_t, float> bias_prefetched[kBiasPerThread] = {};  // bits or value: zero is 0.0 in every type
+      if (has_next && (kWarpBias || et < TILE_N)) {
+#pragma unroll
+        for (int i = 0; i < kBiasPerThread; ++i) {
+          const int n = tile_col_block(p, next_item / splits) * TILE_N + bias_col + 32 * i;
+          if (with_bias && n < p.N) {
+            if constexpr (FUSED) bias_prefetched[i] = load_bias_bits(p.bias, p.bias_dtype, n);
+            else bias_prefetched[i] = load_bias(p.bias, p.bias_dtype, n);
+          }
         }
       }
       if (warp == 2) CK_TRACE(6);
@@ -812,10 +833,6 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       tc_fence_after_sync();
       const int c0 = half * kColsPerWarp;
       const uint32_t t_row = tmem_base + acc * Cfg::kAccCols + (static_cast<uint32_t>(quarter * 32) << 16) + c0;
-      // The fused 16-bit epilogue never holds the raw accumulator: it drains 16 columns at a
-      // time and keeps alpha * acc + bias rounded to OutT as packed pairs (a quarter of the
-      // registers); the others pull their whole share with back-to-back loads.
-      constexpr bool kPackedDrain = FUSED && sizeof(OutT) == 2;
       [[maybe_unused]] uint32_t buf[kPackedDrain ? 1 : kChunks][32];
       [[maybe_unused]] uint32_t pk[kPackedDrain ? kChunks : 1][16];
       if constexpr (kPackedDrain) {
@@ -867,13 +884,20 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         continue;
       }
       if (has_next) {
-        if (et < TILE_N) {
-          float b;
-          if constexpr (FUSED) b = bias_of_bits(bias_prefetched, p.bias_dtype);
-          else b = bias_prefetched;
-          smem_bias[((tile_it + 1) % 3) * TILE_N + et] = b;
+        if (kWarpBias || et < TILE_N) {
+#pragma unroll
+          for (int i = 0; i < kBiasPerThread; ++i) {
+            float b;
+            if constexpr (FUSED) b = bias_of_bits(bias_prefetched[i], p.bias_dtype);
+            else b = bias_prefetched[i];
+            smem_bias[((tile_it + 1) % 3) * TILE_N + bias_col + 32 * i] = b;
+          }
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * kNumEpilogueWarps) : "memory");  // epilogue warps only
+        if constexpr (kWarpBias) {
+          __syncwarp();
+        } else {
+          asm volatile("bar.sync 1, %0;" ::"n"(32 * kNumEpilogueWarps) : "memory");  // epilogue warps only
+        }
       }
       OutT* out_row = out + static_cast<int64_t>(row) * p.N + n0 + c0;
       if constexpr (!FUSED) {
