@@ -33,13 +33,13 @@ int forced_gemm_config() {
 namespace {
 
 // 128 x 64 tiles that find an SM each: half the columns to an epilogue, and more CTAs that load (us, 128 x 128 / 128 x 64: NVFP4 256 x 3072
-// x 3072 7.2 / 6.8, 128 x 9216 x 3072 7.8 / 7.4, 1003 x 1024 x 3072 7.2 / 6.8, 384 x 3072 x 2048 6.1 / 5.7, MXFP8 128 x 9216 x 1536 7.4 / 7.0).
+// x 3072 6.5 / 6.0, 128 x 9216 x 3072 7.2 / 6.8, 1003 x 1024 x 3072 6.2 / 6.1, 384 x 3072 x 2048 5.5 / 5.4, MXFP8 128 x 9216 x 1536 7.0 / 6.6).
 bool one_wave_of_half_tiles(int64_t M, int64_t N) { return M > 64 && ceil_div(M, kTileM) * ceil_div(N, 64) <= sm_count(); }
 
 // Whether they pay.  Twice the CTAs ask for the same rows of the activation at once.  Rows that straddle the 128-byte lines cost each
-// of them two: with one or two row blocks that is dearer (NVFP4 68 x 6304 x 2976 7.7 / 9.6, 128 x 8512 x 3808 10.1 / 10.8, 256 x 4640 x 3296 8.8 / 9.4).
-// So are activations of less than 128 KiB, slow to load, up to 80 rows and from eight stages on (NVFP4 65 x 9216, K of 1792 5.95 / 5.99, 2048
-// 6.33 / 6.39, 2816 7.25 / 7.62, 3840 8.52 / 9.57; of 4096, 130 KiB, 8.80 / 8.36; 88 x 9216 x 2816 7.26 / 7.23, 96 x 9216 x 3072 7.59 / 7.16).
+// of them two: with one or two row blocks that is dearer (NVFP4 68 x 6304 x 2976 7.4 / 8.9, 128 x 8512 x 3808 9.8 / 10.0, 256 x 4640 x 3296 8.6 / 8.8).
+// So are activations of less than 128 KiB, slow to load, up to 80 rows and from eight stages on (NVFP4 65 x 9216, K of 1792 5.5 / 5.8, 2048
+// 5.8 / 6.3, 2816 6.7 / 7.4, 3840 8.0 / 9.0; of 4096, 130 KiB, 8.1 / 7.7; 88 x 9216 x 2816 6.7 / 6.8, 96 x 9216 x 3072 7.0 / 6.7).
 bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
   if (!one_wave_of_half_tiles(M, N)) return false;
   if (k_bytes % kStageKBytes != 0) return M > 2 * kTileM;
@@ -48,13 +48,12 @@ bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
 
 // In a linear with a dynamic scale.  Such calls in a row are a chain of reduction, quantizer and GEMM whose launches overlap, and the quantizer's
 // few large blocks find room beside the GEMM before them only on SMs that it leaves free.  A GEMM of more, smaller CTAs gains less than
-// the quantizer then loses, unless a quarter of the SMs stays free (whole linears, us, 128 x 128 / half tiles: 200 x 4544 x 768 9.2 / 10.1, 65 x 9216 x 3072
-// 12.2 / 13.8, 1003 x 1024 x 768 9.5 / 9.9; 128 x 6848 x 3072, 107 half tiles, 13.3 / 11.8, 1003 x 576 x 352 9.3 / 8.2; pair / 128 x 128: 512 x 6848 x 768, 54 pairs,
-// 11.3 / 12.4, 1003 x 3072 x 512 11.4 / 11.8; 640 x 6848 x 768, 81 pairs on 74, 14.8 / 12.8).
+// the quantizer then loses, unless a quarter of the SMs stays free (whole linears, us, 128 x 128 / half tiles: 200 x 4544 x 768 7.5 / 8.6, 65 x 9216 x 3072
+// 11.2 / 12.9, 1003 x 1024 x 768 8.1 / 8.7; 128 x 6848 x 3072, 107 half tiles, 11.8 / 10.7, 1003 x 576 x 352 8.6 / 7.4; pair / 128 x 128: 512 x 6848 x 768, 54 pairs,
+// 10.9 / 11.7, 1003 x 3072 x 512 10.8 / 11.3; 640 x 6848 x 768, 81 pairs on 74, 14.1 / 12.4).
 struct Room {
   bool wanted;
   bool left_by_half_tiles(int64_t M, int64_t N) const { return !wanted || ceil_div(M, kTileM) * ceil_div(N, 64) * 4 <= 3 * sm_count(); }
-  bool left_by_pairs(int64_t pairs) const { return wanted && pairs * 2 <= sm_count(); }
 };
 
 // 128 x 128 tiles that take no more waves than pair tiles: a wave of them is shorter, with half the output of an SM behind its main loop.
@@ -68,20 +67,34 @@ bool tiles_in_as_few_waves(int64_t tiles, int64_t pairs, const Room& room) {
   return tile_waves <= pair_waves && tile_waves <= 3 && (!room.wanted || tile_waves > 1 || 10 * pairs >= 3 * tiles);
 }
 
+// One wave more of them, while the K is so short that a tile's time is its latencies and its epilogue, which the second accumulator of a
+// small tile hides.  us, pair / 128 x 128, two waves against one: NVFP4 512 x 9216 x 1280 7.9 / 7.2, x 1536 8.4 / 7.8, x 1792 8.7 / 8.6, x 2048 9.0 / 9.1, MXFP8 x 640
+// 7.9 / 7.1, x 768 8.3 / 7.7, x 1024 8.9 / 8.9; three against two: 1280 x 4608 x 1280 8.9 / 8.5, x 1536 9.4 / 9.3, 700 x 9216 x 1536 9.5 / 9.8; four against two: 2048 x 4608 x
+// 512 8.4 / 8.8.  The fused epilogue is the longer one: 512 x 9216 x 1536 10.8 / 10.1, x 3072 12.9 / 12.6, x 4096 14.4 / 14.8, 1024 x 6144 x 3072 16.4 / 16.0, 1152 x 7680 x
+// 3072 21.8 / 19.9, but with two waves against one and up to two stages it hides behind nothing: 208 x 12352 x 512 8.2 / 8.7, 216 x 13440 x 256 8.1 / 8.6.  Rows of K that
+// straddle 128-byte lines cost twice as many readers more (1003 x 4096 x 1248 7.7 / 8.3, MXFP8 650 x 6400 x 736 9.3 / 9.5, fused 179 x 18368 x 672 10.0 / 11.4).
+// In front of the next dynamic linear only where a sixth is padding, as above: 1003 x 6144 x 1024 14.9 / 15.3, 520 x 10240 x 1024 16.4 / 14.9.
+bool tiles_in_one_wave_more(int64_t tiles, int64_t pairs, int k_bytes, bool fused, const Room& room) {
+  const int64_t tile_waves = ceil_div(tiles, sm_count()), pair_waves = ceil_div(pairs, sm_count() / 2), k_stages = ceil_div(k_bytes, kStageKBytes);
+  const bool padded = 10 * pairs >= 3 * tiles;
+  if (tile_waves != pair_waves + 1 || tile_waves > 4) return false;
+  if (room.wanted && (tile_waves == 2 || !padded)) return false;
+  if (k_bytes % kStageKBytes != 0) return !fused && tile_waves == 2 && k_stages <= 4;
+  if (fused) return k_stages <= 12 && (k_stages >= 3 || tile_waves > 2 || padded);
+  return k_stages <= (tile_waves == 2 ? 6 : 5);
+}
+
 template <Kind KIND, typename OutT, bool FUSED>
 int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec& os, const Room& room, cudaStream_t stream) {
   int config = forced_gemm_config();
   if (config == 0) {
     const int64_t row_blocks = ceil_div(p.M, kTileM), tiles = row_blocks * ceil_div(p.N, 128);
-    const int k_stages = static_cast<int>(ceil_div(p.k_bytes, kStageKBytes));
     // The pair, from about a quarter of the SM count in pair tiles on: not where its second CTA would have no rows (us, pair / 128 x 128,
     // NVFP4 128 x 18432 x 1024 8.0 / 6.0, x 3072 11.4 / 9.4, x 8192 20.1 / 18.3, 128 x 36864 x 3072 17.1 / 15.1, MXFP8 128 x 18432 x 3072
-    // 16.4 / 14.2, the fused epilogue 128 x 12288 x 3072 12.8 / 9.8), and not for up to four stages while a CTA has at most
-    // two of the small tiles (NVFP4 512 x 9216 x 1024 7.4 / 6.7, 256 x 18432 x 1024 8.1 / 7.2, fused 512 x 8192 x 1024 9.7 / 9.4; with six
-    // stages 512 x 9216 x 1536 8.3 / 8.1 and 1003 x 3072 x 1536 7.5 / 7.6, with twelve 512 x 9216 x 3072 10.6 / 11.9).
+    // 16.5 / 13.8, the fused epilogue 128 x 12288 x 3072 12.6 / 9.1), and not where small tiles beat it (above).
     const int64_t pairs = ceil_div(p.M, 256) * ceil_div(p.N, 256);
     const bool pair = pairs * 4 >= sm_count() && row_blocks > 1 && !tiles_in_as_few_waves(tiles, pairs, room) &&
-                      (!(k_stages <= 4 && tiles <= 2 * sm_count()) || room.left_by_pairs(pairs));
+                      !tiles_in_one_wave_more(tiles, pairs, p.k_bytes, FUSED, room);
     if (pair) {
       config = 4;
     } else if (tiles * 4 <= sm_count() || (half_tiles_pay(p.M, p.N, p.k_bytes) && room.left_by_half_tiles(p.M, p.N))) {
@@ -135,9 +148,9 @@ int64_t split_workspace_bytes(int64_t M, int64_t N, const SplitPlan& plan) { ret
 // at once.  A cluster sits in one part of the chip, which can leave SMs idle that a split without clusters uses; its
 // CTAs store their partial tiles to a workspace and a second kernel adds them.  That exchange costs about four
 // thirds of a pipeline stage per partial tile, so it is taken where it saves a CTA that many.  Graph replays, us,
-// clusters / workspace: 256 x 3072 x 12288 13.3 / 11.9 with NVFP4 (24 / 16 stages, 3 partial tiles), 19.5 / 15.8 with MXFP8
-// (48 / 32), x 6144 NVFP4 9.7 / 9.4 (12 / 8), 256 x 2176 x 12288 MXFP8 14.7 / 14.0 (32 / 24, 4); but 256 x 2176 x 12288 NVFP4
-// 10.6 / 11.0 (16 / 12, 4), 256 x 1152 x 12288 MXFP8 10.6 / 11.5 (16 / 12, 8), 128 x 3712 x 16384 MXFP8 14.8 / 14.9 (32 / 26, 5).
+// clusters / workspace: 256 x 3072 x 12288 13.3 / 12.8 with NVFP4 (24 / 16 stages, 3 partial tiles), 19.5 / 16.7 with MXFP8
+// (48 / 32), x 6144 NVFP4 9.8 / 10.0 (12 / 8), 256 x 2176 x 12288 MXFP8 14.8 / 14.2 (32 / 24, 4); but 256 x 2176 x 12288 NVFP4
+// 10.7 / 11.3 (16 / 12, 4), 256 x 1152 x 12288 MXFP8 10.9 / 11.7 (16 / 12, 8), 128 x 3712 x 16384 MXFP8 17.5 / 18.1 (32 / 26, 5).
 template <Kind KIND, typename OutT>
 int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitPlan* plan) {
   const int64_t tiles = ceil_div(M, kTileM) * ceil_div(N, 128);

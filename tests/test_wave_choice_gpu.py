@@ -8,9 +8,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # one wave of tiles and of pairs: 144 tiles of three row blocks; 147 and 150 tiles; two waves of either, and three against two; padded rows; 36 and
-# 37 stages of half tiles, and columns that rule them out
+# 37 stages of half tiles, and columns that rule them out; one wave more at the last stages it is taken for and one beyond, rows that straddle lines
 SHAPES = [(300, 6144, 1312), (257, 6272, 1312), (257, 6400, 1312), (384, 12288, 1312), (384, 12672, 1312), (1152, 4096, 1344), (700, 3520, 1312),
-          (256, 4608, 36 * 128), (256, 4608, 37 * 128), (256, 4608, 36 * 256), (256, 4608, 37 * 256 - 32), (256, 4616, 30 * 128)]
+          (512, 9216, 6 * 128), (512, 9216, 6 * 256), (512, 9216, 7 * 256), (700, 6144, 5 * 256 - 32), (1100, 4608, 5 * 128), (1100, 4608, 6 * 256), (1152, 7680, 5 * 256),
+          (512, 9216, 12 * 256), (512, 9216, 2 * 256), (1100, 4608, 13 * 256), (256, 4608, 36 * 128), (256, 4608, 37 * 128), (256, 4608, 36 * 256), (256, 4608, 37 * 256 - 32), (256, 4616, 30 * 128)]
 
 
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
