@@ -147,6 +147,7 @@ struct GemmParams {
   int tiles_m, tiles_n;
   int raster;              // order in which workers walk the tiles: 0 = down the rows first, 1 = along the columns first
   int out_tma;             // the output qualifies for TMA stores (16-byte aligned base and pitch)
+  int a_box_rows;          // rows of A in a load: no more than there are
   int n_out;               // destinations of every output tile (1, or one per GPU of an all-gather)
   int splits;              // split-K: CTAs per tile (1 = off); CTA s of a tile covers pipeline stages
   int k_stages_per_split;  //   [s * k_stages_per_split, ...)
@@ -593,7 +594,7 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               tma_load_3d_pair(sfb_addr + s * Cfg::kSfbBytes, &map_sfb, bar, 0, ks * Cfg::kSfTilesPerStage, rb_b0);
             } else {
               const uint32_t sf_bytes = static_cast<uint32_t>(min(Cfg::kSfTilesPerStage, p.sf_col_tiles - ks * Cfg::kSfTilesPerStage)) * 512u;
-              mbar_arrive_expect_tx(bar, Cfg::kABytes + Cfg::kBBytes + sf_bytes * ((have_sfa ? 1 : 0) + rb_b_count));
+              mbar_arrive_expect_tx(bar, p.a_box_rows * kStageKBytes + Cfg::kBBytes + sf_bytes * ((have_sfa ? 1 : 0) + rb_b_count));
               if (first) {
                 pdl_wait();
                 CK_TRACE3(2);
@@ -1377,7 +1378,11 @@ int launch_config(const Operands& ops, GemmParams p, const OutputSpec& os, cudaS
   auto kernel = block_scaled_gemm_kernel<KIND, TILE_N, NUM_ACC, STAGES, CTAS, OutT, FUSED, OUT_STAGE, SPLIT>;
   // only the tensor maps this configuration uses are encoded (host time is visible for small problems)
   CUtensorMap map_a, map_b;
-  if (int rc = make_operand_map(&map_a, ops.a, p.M, p.k_bytes, kTileM)) return rc;
+  // No rows past M in a box where one row block has them all: filling them made a load of a small activation, less than 128 KiB, slow (us,
+  // boxes of 128 rows / of M: NVFP4 33 x 12288 x 6144 15.2 / 10.9, 33 x 9216 x 3072 7.1 / 6.4, MXFP8 33 x 9216 x 3072 11.3 / 9.5, 33 x 3072 x 3072 7.1 / 6.5;
+  // 96 x 9216 x 3072 6.5 / 6.5).  What the slot then holds of an earlier stage goes to rows of the accumulator that are not stored.
+  p.a_box_rows = CTAS == 1 && p.M < kTileM ? p.M : kTileM;
+  if (int rc = make_operand_map(&map_a, ops.a, p.M, p.k_bytes, p.a_box_rows)) return rc;
   if (int rc = make_operand_map(&map_b, ops.b, p.N, p.k_bytes, Cfg::kBRows)) return rc;
   // the dynamic shared-memory opt-in is per device: do it once for each device that launches
   static std::atomic<bool> configured[64];
