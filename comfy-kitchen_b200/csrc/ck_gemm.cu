@@ -34,16 +34,15 @@ namespace {
 
 // 128 x 64 tiles that find an SM each: half the columns to an epilogue, and more CTAs that load (us, 128 x 128 / 128 x 64: NVFP4 256 x 3072
 // x 3072 6.5 / 6.0, 128 x 9216 x 3072 7.2 / 6.8, 1003 x 1024 x 3072 6.2 / 6.1, 384 x 3072 x 2048 5.5 / 5.4, MXFP8 128 x 9216 x 1536 7.0 / 6.6).
-bool one_wave_of_half_tiles(int64_t M, int64_t N) { return M > 64 && ceil_div(M, kTileM) * ceil_div(N, 64) <= sm_count(); }
+bool one_wave_of_half_tiles(int64_t M, int64_t N) { return ceil_div(M, kTileM) * ceil_div(N, 64) <= sm_count(); }
 
 // Whether they pay.  Twice the CTAs ask for the same rows of the activation at once.  Rows that straddle the 128-byte lines cost each
 // of them two: with one or two row blocks that is dearer (NVFP4 68 x 6304 x 2976 7.4 / 8.9, 128 x 8512 x 3808 9.8 / 10.0, 256 x 4640 x 3296 8.6 / 8.8).
-// So are activations of less than 128 KiB, slow to load, up to 80 rows and from eight stages on (NVFP4 65 x 9216, K of 1792 5.5 / 5.8, 2048
-// 5.8 / 6.3, 2816 6.7 / 7.4, 3840 8.0 / 9.0; of 4096, 130 KiB, 8.1 / 7.7; 88 x 9216 x 2816 6.7 / 6.8, 96 x 9216 x 3072 7.0 / 6.7).
+// Up to 64 rows the epilogue has little to halve: from eight stages on they pay all the same (drawn sizes: 0.97 of the time up to 17 stages, 0.95 beyond, 1.05 below eight).
 bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
   if (!one_wave_of_half_tiles(M, N)) return false;
   if (k_bytes % kStageKBytes != 0) return M > 2 * kTileM;
-  return M > 80 || M * k_bytes >= (128 << 10) || k_bytes < 8 * kStageKBytes;
+  return M > 64 || k_bytes >= 8 * kStageKBytes;
 }
 
 // In a linear with a dynamic scale.  Such calls in a row are a chain of reduction, quantizer and GEMM whose launches overlap, and the quantizer's
@@ -167,8 +166,9 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
   // rows of whole 64-byte units (N of 16 bits off by 16: MXFP8 512 x 1648 x 2784 10.0 / 10.7, NVFP4 517 x 1584 x 4800 9.7 / 10.7).  us, two CTAs /
   // half tiles: linears NVFP4 256 x 4608, 24 stages, 12.9 / 11.5, 300 x 2048, 24 stages, 12.3 / 11.4, MXFP8 256 x 4608, 30 stages, 12.9 / 12.0.  Over drawn sizes of
   // both formats half tiles take 0.91 to 1.0 of the time from 24 to 35 stages, 1.0 from 36 to 41 and 1.05 from 42 on.
+  // Up to 64 rows not where those of K straddle 128-byte lines (NVFP4 40 x 8192 x 6112 10.2 / 10.8; 64 x 8192 x 6144 10.1 / 9.4, MXFP8 64 x 9216 x 3072 10.3 / 9.3).
   constexpr int kMostStages = 36;
-  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= kMostStages && N % 32 == 0 && one_wave_of_half_tiles(M, N);
+  plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= kMostStages && N % 32 == 0 && (M > 64 || k_bytes % kStageKBytes == 0) && one_wave_of_half_tiles(M, N);
   if (plan->half_tiles) splits = 1;
   plan->k_stages = static_cast<int>(ceil_div(k_stages, plan->through_workspace ? most : splits));
   plan->splits = static_cast<int>(ceil_div(k_stages, plan->k_stages));  // none without a stage
