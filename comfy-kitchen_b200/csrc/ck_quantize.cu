@@ -483,10 +483,12 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
 }
 
 // Inputs of at most this many bytes: every block of the quantizer takes the maximum of the whole input
-// itself (a few 16 KiB passes out of L2) instead of waiting for a reduction kernel.  Scale and quantizer, us, whole
-// input / reduction kernel: at the line 8 x 4096 bf16 3.5 / 4.4, 1 x 32768 bf16 4.5 / 5.3; beyond it 128 KiB 3.9 / 4.5 still, 256 KiB
-// (fp32) 4.0 / 3.8, 384 KiB 6.3 / 5.2: the line could lie near 200 KiB.
-constexpr int64_t kWholeInputBytes = 64 * 1024;
+// itself (a few 16 KiB passes out of L2) instead of waiting for a reduction kernel, which is a launch more.  Scale and quantizer, us, reduction
+// kernel / whole input: bf16 16 x 3072 (96 KiB) 4.1 / 3.4, 22 x 3072 (132 KiB) 4.0 / 3.5, 32 x 3072 (192 KiB) 4.1 / 4.1, 40 x 3072 4.1 / 4.8, fp16 64 x 1024 (128 KiB)
+// 3.9 / 3.3, fp32 12 x 3072 (144 KiB) 3.4 / 3.5; linears bf16 12 x 3072 x 3072 9.0 / 8.1, 9 x 9216 x 5120 11.7 / 10.8, 12 x 3072 x 6144 (144 KiB) 9.1 / 9.5, 64 x 9216 x 1024
+// 8.2 / 7.4.  Up to eight rows, whose quantizer blocks are narrow and many, the line
+// stays lower: 8 x 4096 (64 KiB) 4.4 / 3.5, 3 x 15360 (90 KiB) 3.6 / 3.8, 8 x 15360 4.0 / 5.6.
+constexpr int64_t whole_input_bytes(int64_t rows) { return rows > 8 ? 128 * 1024 : 64 * 1024; }
 constexpr int64_t kDynamicScratchHead = 256;
 // fp32 inputs from here on are quantized from their last rows on, which the reduction has just read.  Forwards / backwards, us: 6144 x 3072
 // (72 MiB) 24.1 / 24.3, 8192 x 3072 (96 MiB) 31.4 / 31.6, 12288 x 3072 (144 MiB) 48.0 / 46.4, 24576 x 3072 97.6 / 94.7, 36864 x 3072 147 / 143.
@@ -509,7 +511,7 @@ int launch_nvfp4_dynamic(const void* input, int dtype, float* scale_out, void* c
     ScaleSource src = {};
     src.out = scale_out;
     src.n_vecs = n / (32 / static_cast<int64_t>(sizeof(T)));
-    if (n * static_cast<int64_t>(sizeof(T)) > kWholeInputBytes) {
+    if (n * static_cast<int64_t>(sizeof(T)) > whole_input_bytes(orig_rows)) {
       // behind the arrival counter of the one-kernel reduction, which may share this scratch and wants it zero
       float* partials = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kDynamicScratchHead);
       if (int rc = launch_amax_partials(x, dtype, src.n_vecs, partials, &src.n_partials, stream)) return rc;
