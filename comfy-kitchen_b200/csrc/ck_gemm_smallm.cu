@@ -324,11 +324,11 @@ small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           }
         };
         const int n_mma = total_mma - i * kMmaPerStage;  // left from here on
-        if (n_mma >= kMmaPerStage) {
+        // one straight path for whole stages and the last one: a loop of its own for the last (code met once, and cold) cost more than the
+        // predicates (us: bf16 24 x 9216 x 3072 5.7 / 5.4, 8 x 18432 x 3072 with x dense 8.9 / 8.7, fp32 1 x 3072 x 3072 5.8 / 5.1, 4 x 6208 x 896 4.4 / 4.2)
 #pragma unroll
-          for (int kb = 0; kb < kMmaPerStage; ++kb) mma(kb);
-        } else {
-          for (int kb = 0; kb < n_mma; ++kb) mma(kb);
+        for (int kb = 0; kb < kMmaPerStage; ++kb) {
+          if (kb < n_mma) mma(kb);
         }
         tc_commit<1>(empty_addr + s * 8);
         if (i == n_stages - 1) tc_commit<1>(smem_u32(acc_bar));
