@@ -58,15 +58,21 @@ def direct_backend(*tensors):
     return _backend if _backend.is_loaded() else None
 
 
-def host_half(t):
-    """The native half of the CUDA backend's wrappers for a call on ``t``, or None: outside of any tracing, and for a plain
-    CUDA tensor, the only kind that may be asked for its size here (another kind's may be symbolic)."""
-    if torch.compiler.is_compiling() or (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter) or not t.is_cuda:
+def host_half():
+    """The native half of the CUDA backend's wrappers for a call outside of any tracing, or None."""
+    if torch.compiler.is_compiling():
         return None
     global _backend
     if _backend is None:
         from comfy_kitchen.backends import cuda as _backend
     return _backend._host
+
+
+def host_half_for(t):
+    """:func:`host_half` for a call on ``t`` that has to ask for its size: a plain CUDA tensor's (another kind's may be symbolic)."""
+    if (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter) or not t.is_cuda:
+        return None
+    return host_half()
 
 
 def crop(result: torch.Tensor, rows: int, cols: int) -> torch.Tensor:

@@ -10,7 +10,7 @@ import comfy_kitchen as ck
 from comfy_kitchen.float_utils import F4_E2M1_MAX, F8_E4M3_MAX, roundup
 
 from .base import BaseLayoutParams, QuantizedLayout
-from .blockwise import direct_backend, host_half, install_handlers
+from .blockwise import direct_backend, host_half, host_half_for, install_handlers
 
 
 class TensorCoreNVFP4Layout(QuantizedLayout):
@@ -43,7 +43,7 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
 
     @classmethod
     def quantize(cls, tensor: torch.Tensor, scale=None, **kwargs):
-        host = host_half(tensor) if cls is TensorCoreNVFP4Layout else None
+        host = host_half_for(tensor) if cls is TensorCoreNVFP4Layout else None
         if host is not None and (scale is None or type(scale) in (torch.Tensor, torch.nn.Parameter)) and tensor.dim() == 2:
             # plain eager calls (None for any other): 2 us less of host time than through the backend's wrappers
             rows, cols = shape = tuple(tensor.shape)
@@ -104,7 +104,7 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
     def scaled_mm(cls, a, b, bias, out_dtype):
         qa, sa, bsa = cls.get_plain_tensors(a)
         qb, sb, bsb = cls.get_plain_tensors(b)
-        host = host_half(qa)
+        host = host_half()
         if host is not None:  # plain eager calls (None for any other)
             y = host.scaled_mm_nvfp4(qa, qb, sa, sb, bsa, bsb, bias, out_dtype, None)
             if y is not None:

@@ -78,3 +78,14 @@ def test_padded_weight_rows_are_cut_from_the_native_result(host, layout, out_fea
     y = _layer(layout, out_features, bias=False)(torch.zeros(4, 64, dtype=torch.bfloat16))
     assert len(host.calls) == 1
     assert y.shape == (4, out_features) and torch.equal(y[3], torch.arange(float(out_features)).bfloat16())
+
+
+@pytest.mark.parametrize("layout", ["nvfp4", "mxfp8"])
+def test_layers_ask_the_backend_s_own_half(monkeypatch, layout):
+    """Without the stand-in for the function that finds it."""
+    from comfy_kitchen.backends import cuda as backend
+
+    host = _Host()
+    monkeypatch.setattr(backend, "_host", host)
+    layer = _layer(layout)
+    assert torch.equal(layer(torch.zeros(3, 64)), torch.arange(32.0).expand(3, 32)) and len(host.calls) == 1
