@@ -779,17 +779,20 @@ def _build_constraints() -> dict:
 
 
 _constraints: dict = {}  # as registered
-_stock = {name: globals()[name] for name in ("quantize_nvfp4", "quantize_mxfp8", "dequantize_nvfp4", "dequantize_mxfp8",
-                                             "scaled_mm_nvfp4", "scaled_mm_mxfp8")}
+_stock = {name: globals()[name] for name in ("quantize_nvfp4", "quantize_nvfp4_dynamic", "quantize_mxfp8", "dequantize_nvfp4",
+                                             "dequantize_mxfp8", "scaled_mm_nvfp4", "scaled_mm_mxfp8")}
+
+
+def host_function(name: str):
+    """The native half of this module's function ``name``, or None: also where somebody has put another function in its place."""
+    return getattr(_host, name) if _host is not None and globals()[name] is _stock[name] else None
 
 
 def host_operator(name: str):
     """The native half of operator ``name``, or None unless the registry would send every call that it takes to this
     module's own function anyway."""
-    if _host is None or globals()[name] is not _stock[name] or \
-            not registry.leaves_no_choice(name, _this_module, _constraints.get(name)):
-        return None
-    return getattr(_host, name)
+    host = host_function(name)
+    return host if host is not None and registry.leaves_no_choice(name, _this_module, _constraints.get(name)) else None
 
 
 def _register():

@@ -68,11 +68,16 @@ def host_half():
     return _backend._host
 
 
-def host_half_for(t):
-    """:func:`host_half` for a call on ``t`` that has to ask for its size: a plain CUDA tensor's (another kind's may be symbolic)."""
-    if (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter) or not t.is_cuda:
+def host_function(name: str, t):
+    """The native half of the CUDA backend's function ``name`` for a call on ``t``, or None: while something is traced, where that
+    function has been replaced, and for anything but a plain CUDA tensor (whose size the caller asks for; another kind's may be
+    symbolic)."""
+    if torch.compiler.is_compiling() or (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter) or not t.is_cuda:
         return None
-    return host_half()
+    global _backend
+    if _backend is None:
+        from comfy_kitchen.backends import cuda as _backend
+    return _backend.host_function(name)
 
 
 def crop(result: torch.Tensor, rows: int, cols: int) -> torch.Tensor:

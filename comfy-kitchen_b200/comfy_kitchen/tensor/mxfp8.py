@@ -10,7 +10,7 @@ import comfy_kitchen as ck
 from comfy_kitchen.float_utils import roundup
 
 from .base import BaseLayoutParams, QuantizedLayout
-from .blockwise import direct_backend, host_half, host_half_for, install_handlers
+from .blockwise import direct_backend, host_function, install_handlers
 
 
 class TensorCoreMXFP8Layout(QuantizedLayout):
@@ -33,10 +33,10 @@ class TensorCoreMXFP8Layout(QuantizedLayout):
 
     @classmethod
     def quantize(cls, tensor: torch.Tensor, **kwargs):
-        host = host_half_for(tensor) if cls is TensorCoreMXFP8Layout else None
-        if host is not None and tensor.dim() == 2:  # plain eager calls (None for any other)
+        host = host_function("quantize_mxfp8", tensor) if cls is TensorCoreMXFP8Layout and tensor.dim() == 2 else None
+        if host is not None:  # plain eager calls (None for any other)
             rows, cols = shape = tuple(tensor.shape)
-            out = host.quantize_mxfp8(tensor, (rows | cols) % 32 != 0)
+            out = host(tensor, (rows | cols) % 32 != 0)
             if out is not None:
                 return out[0], cls.Params(out[1], tensor.dtype, shape)
         if tensor.dim() != 2:
@@ -80,9 +80,9 @@ class TensorCoreMXFP8Layout(QuantizedLayout):
     def scaled_mm(cls, a, b, bias, out_dtype):
         qa, sa = cls.get_plain_tensors(a)
         qb, sb = cls.get_plain_tensors(b)
-        host = host_half()
+        host = host_function("scaled_mm_mxfp8", qa)
         if host is not None:  # plain eager calls (None for any other)
-            y = host.scaled_mm_mxfp8(qa, qb, sa, sb, bias, out_dtype)
+            y = host(qa, qb, sa, sb, bias, out_dtype)
             if y is not None:
                 return y
         backend = direct_backend(qa, qb, bias)

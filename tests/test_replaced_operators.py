@@ -53,3 +53,19 @@ def test_replacement_is_called(cuda_device):
     finally:
         lib._destroy()
     assert torch.equal(ck.quantize_nvfp4(x, g)[0], codes)
+
+
+def test_the_native_half_steps_aside_for_a_replaced_function(monkeypatch):
+    import types
+
+    from comfy_kitchen.backends import cuda as backend
+
+    names = [*OPERATORS, "quantize_nvfp4_dynamic"]
+    monkeypatch.setattr(backend, "_host", types.SimpleNamespace(**{name: name for name in names}))
+    for name in names:
+        assert backend.host_function(name) == name
+        with monkeypatch.context() as m:
+            m.setattr(backend, name, lambda *args, **kwargs: None)
+            assert backend.host_function(name) is None
+            assert all(backend.host_function(other) == other for other in names if other != name)
+        assert backend.host_function(name) == name
