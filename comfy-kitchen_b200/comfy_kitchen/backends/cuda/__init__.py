@@ -284,6 +284,21 @@ def _scale_scratch_for(device, stream: int, need: int, zeros: bool = True) -> to
     return scratch
 
 
+_KEPT_SCRATCH_BYTES = 64 << 10
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
+def kept_scratch(x: torch.Tensor) -> torch.Tensor | None:
+    """The scratch of a dynamic quantization to which nothing is written (it is kept, and whoever calls on the stream shares it),
+    or None: the call's own is wanted.  Up to 64 KiB no number of rows takes a reduction kernel
+    (``ck_quantize_nvfp4_dynamic_whole_input_bytes``); larger inputs may take one, and where they do not, memory that the native
+    half allocates costs 0.5 us less than looking this one up.  Only plain CUDA tensors are asked for their size: another kind's
+    may be symbolic."""
+    if type(x) not in _PLAIN_TYPES or not x.is_cuda or x.nbytes > _KEPT_SCRATCH_BYTES:
+        return None
+    return _scale_scratch_for(x.device, _stream(x.device), 1 << 20, zeros=False)
+
+
 def nvfp4_tensor_scale(x: torch.Tensor) -> torch.Tensor:
     """0-d float32 tensor ``amax(|x|) / (448 * 6)`` (division in x's dtype), computed by one kernel.
 
@@ -305,7 +320,6 @@ def nvfp4_tensor_scale(x: torch.Tensor) -> torch.Tensor:
 
 
 _ON_CHIP = 256  # the workspace size of a GEMM that does not use one (ck_scaled_mm_workspace_bytes)
-_WHOLE_INPUT_BYTES = 64 << 10  # inputs up to here take no reduction kernel (ck_quantize_nvfp4_dynamic)
 
 
 _workspaces = threading.local()
@@ -336,10 +350,7 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     """``scale = nvfp4_tensor_scale(x)`` and ``quantize_nvfp4(x, scale)`` in one library call (same bits):
     ``(codes, block_scales, scale)``.  The reduction leaves partial maxima that the quantizer finishes."""
     if _host is not None:
-        scratch = None
-        if type(x) is torch.Tensor and x.is_cuda and x.numel() * x.element_size() <= _WHOLE_INPUT_BYTES:
-            scratch = _scale_scratch_for(x.device, _stream(x.device), 1 << 20, zeros=False)  # nothing is kept in it between two launches
-        out = _host.quantize_nvfp4_dynamic(x, pad_16x, hi_first, scratch)
+        out = _host.quantize_nvfp4_dynamic(x, pad_16x, hi_first, kept_scratch(x))
         if out is not None:
             return out
     lib = load_library()
@@ -360,9 +371,8 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     stream = _stream(x.device)
     # the smallest workspace that is kept does up to 2^31 elements: no need to ask
     need = 1 << 20 if rows * cols < 1 << 31 else _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
-    if rows * cols * size <= _WHOLE_INPUT_BYTES:
-        scratch = _scale_scratch_for(x.device, stream, need, zeros=False)  # nothing is kept in it between two launches
-    else:
+    scratch = kept_scratch(x)
+    if scratch is None:
         scratch = _workspace_for(need, x.device, stream)  # the partial maxima go from one launch to the next
     scale = torch.empty((), dtype=torch.float32, device=x.device)
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)

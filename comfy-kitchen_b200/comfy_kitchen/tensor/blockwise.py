@@ -68,11 +68,10 @@ def host_half():
     return _backend._host
 
 
-def host_function(name: str, t):
-    """The native half of the CUDA backend's function ``name`` for a call on ``t``, or None: while something is traced, where that
-    function has been replaced, and for anything but a plain CUDA tensor (whose size the caller asks for; another kind's may be
-    symbolic)."""
-    if torch.compiler.is_compiling() or (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter) or not t.is_cuda:
+def host_function(name: str):
+    """The native half of the CUDA backend's function ``name``, or None: while something is traced, and where that function has
+    been replaced."""
+    if torch.compiler.is_compiling():
         return None
     global _backend
     if _backend is None:

@@ -33,7 +33,7 @@ class TensorCoreMXFP8Layout(QuantizedLayout):
 
     @classmethod
     def quantize(cls, tensor: torch.Tensor, **kwargs):
-        host = host_function("quantize_mxfp8", tensor) if cls is TensorCoreMXFP8Layout and tensor.dim() == 2 else None
+        host = host_function("quantize_mxfp8") if cls is TensorCoreMXFP8Layout and tensor.dim() == 2 else None
         if host is not None:  # plain eager calls (None for any other)
             rows, cols = shape = tuple(tensor.shape)
             out = host(tensor, (rows | cols) % 32 != 0)
@@ -80,7 +80,7 @@ class TensorCoreMXFP8Layout(QuantizedLayout):
     def scaled_mm(cls, a, b, bias, out_dtype):
         qa, sa = cls.get_plain_tensors(a)
         qb, sb = cls.get_plain_tensors(b)
-        host = host_function("scaled_mm_mxfp8", qa)
+        host = host_function("scaled_mm_mxfp8")
         if host is not None:  # plain eager calls (None for any other)
             y = host(qa, qb, sa, sb, bias, out_dtype)
             if y is not None:

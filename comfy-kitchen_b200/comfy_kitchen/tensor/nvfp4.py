@@ -9,6 +9,7 @@ import torch
 import comfy_kitchen as ck
 from comfy_kitchen.float_utils import F4_E2M1_MAX, F8_E4M3_MAX, roundup
 
+from . import blockwise
 from .base import BaseLayoutParams, QuantizedLayout
 from .blockwise import direct_backend, host_function, install_handlers
 
@@ -45,17 +46,13 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
     def quantize(cls, tensor: torch.Tensor, scale=None, **kwargs):
         if cls is TensorCoreNVFP4Layout and (scale is None or type(scale) in (torch.Tensor, torch.nn.Parameter)) and tensor.dim() == 2:
             # plain eager calls (None for any other): 2 us less of host time than through the backend's wrappers
-            host = host_function("quantize_nvfp4_dynamic" if scale is None else "quantize_nvfp4", tensor)
-            out = None
+            host = host_function("quantize_nvfp4_dynamic" if scale is None else "quantize_nvfp4")
             if host is not None:
                 rows, cols = shape = tuple(tensor.shape)
                 pad = (rows | cols) % 16 != 0
-                if scale is not None:
-                    out = host(tensor, scale, pad, True)
-                elif tensor.nbytes > 64 * 1024:  # small inputs have a scratch of their own, which the wrapper keeps
-                    out = host(tensor, pad, True, None)
-            if out is not None:
-                return out[0], cls.Params(out[2] if scale is None else scale, tensor.dtype, shape, out[1])
+                out = host(tensor, pad, True, blockwise._backend.kept_scratch(tensor)) if scale is None else host(tensor, scale, pad, True)
+                if out is not None:
+                    return out[0], cls.Params(out[2] if scale is None else scale, tensor.dtype, shape, out[1])
         if tensor.dim() != 2:
             raise ValueError(f"NVFP4 requires 2D tensor, got {tensor.dim()}D")
         orig_shape = tuple(tensor.shape)
@@ -106,7 +103,7 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
     def scaled_mm(cls, a, b, bias, out_dtype):
         qa, sa, bsa = cls.get_plain_tensors(a)
         qb, sb, bsb = cls.get_plain_tensors(b)
-        host = host_function("scaled_mm_nvfp4", qa)
+        host = host_function("scaled_mm_nvfp4")
         if host is not None:  # plain eager calls (None for any other)
             y = host(qa, qb, sa, sb, bsa, bsb, bias, out_dtype, None)
             if y is not None:

@@ -616,6 +616,8 @@ extern "C" int64_t ck_quantize_nvfp4_dynamic_scratch_bytes(int64_t num_elements)
   return general > partials ? general : partials;
 }
 
+extern "C" int64_t ck_quantize_nvfp4_dynamic_whole_input_bytes(int64_t orig_rows) { return ck::whole_input_bytes(orig_rows); }
+
 extern "C" int ck_quantize_nvfp4_dynamic(const void* input, int input_dtype, float* scale_out, void* codes, void* block_scales,
                                          int64_t orig_rows, int64_t orig_cols, int64_t num_rows, int64_t num_cols, int hi_first,
                                          void* scratch, int64_t scratch_bytes, void* stream) {

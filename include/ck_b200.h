@@ -117,12 +117,14 @@ CK_API int ck_nvfp4_tensor_scale(const void* input, int input_dtype, int64_t num
 
 /*
  * ck_nvfp4_tensor_scale and ck_quantize_nvfp4 with that scale, bit for bit, enqueued by one call: the
- * reduction over the input leaves one partial maximum per block and the quantizer finishes it (inputs of
- * at most 64 KiB take no reduction kernel at all).  The scale goes to *scale_out (device memory).
+ * reduction over the input leaves one partial maximum per block and the quantizer finishes it (inputs of at
+ * most ck_quantize_nvfp4_dynamic_whole_input_bytes(orig_rows) bytes in the form of the streaming quantizer take no
+ * reduction kernel at all, and nothing is written to `scratch`).  The scale goes to *scale_out (device memory).
  * `scratch`: device memory, 4-byte aligned, at least ck_quantize_nvfp4_dynamic_scratch_bytes(orig_rows *
  * orig_cols) bytes, with no requirement on its contents; a first word that was zero is zero again.
  */
 CK_API int64_t ck_quantize_nvfp4_dynamic_scratch_bytes(int64_t num_elements);
+CK_API int64_t ck_quantize_nvfp4_dynamic_whole_input_bytes(int64_t orig_rows);
 CK_API int ck_quantize_nvfp4_dynamic(const void* input, int input_dtype, float* scale_out,
                       void* codes, void* block_scales,
                       int64_t orig_rows, int64_t orig_cols,

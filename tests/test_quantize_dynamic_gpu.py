@@ -11,7 +11,7 @@ from oracle import ck_oracle as oc
 
 pytestmark = pytest.mark.gpu
 
-# 64 KiB is the largest input every block reads whole (32 x 1024 of a 16-bit type, 16 x 1024 of fp32);
+# inputs that every block reads whole (up to 64 KiB with at most eight rows, else 128 KiB) and larger ones;
 # more partial maxima than threads of a block; one unit; a column chunk of one unit; rows of padding
 # only in the last group; columns that take the general kernel (16, 48: 16-bit types; 65: padded)
 SHAPES = [(1, 32), (16, 1024), (32, 1024), (33, 1024), (3, 2080), (130, 96), (1003, 3072), (2500, 4096), (40, 48), (7, 16), (33, 65)]
@@ -77,6 +77,27 @@ def test_dynamic_quantizer_leaves_a_shared_scratch_usable(backend, cuda_device, 
     assert lib.ck_quantize_nvfp4_dynamic(x.data_ptr(), code, out.data_ptr(), q.data_ptr(), s.data_ptr(), 300, 1056, 300, 1056, 1,
                                          scratch.data_ptr(), need - 1, stream) != 0
     assert f"scratch of {need - 1} bytes, {need} needed".encode() in lib.ck_last_error()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows", [1, 8, 9, 128])
+def test_inputs_that_are_read_whole_leave_the_scratch_alone(backend, cuda_device, rows, dtype):
+    """On both sides of the line that the library reports: nothing is written to the scratch up to it; beyond it there are partial
+    maxima.  What the wrappers keep and share is handed in on this side of it alone."""
+    lib = backend.load_library()
+    code, elem = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[dtype], torch.empty((), dtype=dtype).element_size()
+    line = lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(rows) // elem // rows // 32 * 32
+    for k in (line, line + 32):
+        x = _input(rows, k, dtype).to(cuda_device)
+        need = lib.ck_quantize_nvfp4_dynamic_scratch_bytes(x.numel())
+        scratch = torch.full((need,), 0xA5, dtype=torch.uint8, device=cuda_device)
+        want = backend.quantize_nvfp4_dynamic(x, pad_16x=False)
+        out, q, s = torch.empty((), device=cuda_device), torch.empty_like(want[0]), torch.empty_like(want[1])
+        assert lib.ck_quantize_nvfp4_dynamic(x.data_ptr(), code, out.data_ptr(), q.data_ptr(), s.data_ptr(), rows, k, rows, k, 1,
+                                             scratch.data_ptr(), need, torch.cuda.current_stream().cuda_stream) == 0, lib.ck_last_error()
+        assert bool((scratch == 0xA5).all()) == (k == line)
+        assert torch.equal(out, want[2]) and torch.equal(q, want[0]) and torch.equal(s.view(torch.uint8), want[1].view(torch.uint8))
+        assert k == line or backend.kept_scratch(x) is None
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])

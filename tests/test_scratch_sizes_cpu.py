@@ -1,6 +1,8 @@
 """Size queries of the C ABI (no GPU needed)."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 
 from test_abi_cpu import lib_path  # noqa: F401  (a fixture)
@@ -8,8 +10,6 @@ from test_abi_cpu import lib_path  # noqa: F401  (a fixture)
 
 @pytest.fixture(scope="module")
 def lib(lib_path):  # noqa: F811
-    import ctypes
-
     lib = ctypes.CDLL(lib_path)
     for name in ("ck_quantize_nvfp4_dynamic_scratch_bytes", "ck_nvfp4_tensor_scale_scratch_bytes"):
         getattr(lib, name).argtypes, getattr(lib, name).restype = [ctypes.c_int64], ctypes.c_int64
@@ -27,6 +27,21 @@ def test_dynamic_scratch_depends_on_the_input_alone(lib, n):
     if partials > 592:
         partials = min(-(-4 * n // 32768), 16384)
     assert lib.ck_quantize_nvfp4_dynamic_scratch_bytes(n) == max(256 + 4 * partials, lib.ck_nvfp4_tensor_scale_scratch_bytes(n))
+
+
+@pytest.mark.parametrize("rows, kib", [(1, 64), (8, 64), (9, 128), (1 << 20, 128)])
+def test_inputs_that_are_read_whole(lib, rows, kib):
+    lib.ck_quantize_nvfp4_dynamic_whole_input_bytes.argtypes = [ctypes.c_int64]
+    lib.ck_quantize_nvfp4_dynamic_whole_input_bytes.restype = ctypes.c_int64
+    assert lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(rows) == kib << 10
+
+
+def test_the_scratch_that_callers_share_is_not_written(lib):
+    """The wrappers' line is no further out than the library's, whatever the number of rows."""
+    from comfy_kitchen.backends import cuda as backend
+
+    lib.ck_quantize_nvfp4_dynamic_whole_input_bytes.restype = ctypes.c_int64
+    assert all(backend._KEPT_SCRATCH_BYTES <= lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(ctypes.c_int64(rows)) for rows in (1, 2, 8, 9, 64, 32768))
 
 
 def test_dynamic_scratch_of_nothing(lib):

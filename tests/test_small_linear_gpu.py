@@ -7,9 +7,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # rows (the last that are quantized inside, and the first that are not), ragged weights, K of less than a stage, with a short last
-# stage or an odd number of 32-element blocks, K over clusters of 4 to 8 CTAs, more tiles than SMs, x beyond 64 KiB (a reduction kernel)
+# stage or an odd number of 32-element blocks, K over clusters of 4 to 8 CTAs, more tiles than SMs, x of 128 KiB in 16 bits
+# and beyond (a reduction kernel)
 SHAPES = [(1, 8, 32), (1, 1040, 96), (2, 136, 288), (3, 264, 1056), (4, 18432, 64), (5, 136, 24 * 256 - 32), (7, 520, 544), (8, 128, 256),
-          (8, 19200, 96), (8, 3072, 6112), (9, 264, 544), (8, 1024, 8192), (12, 128, 1120), (16, 264, 4064), (16, 128, 32), (17, 136, 288)]
+          (8, 19200, 96), (8, 3072, 6112), (9, 264, 544), (8, 1024, 8192), (8, 1024, 8224), (12, 128, 1120), (16, 264, 4064), (16, 128, 32), (17, 136, 288)]
 
 
 def _x(m, k, dtype, device, seed):
