@@ -133,7 +133,7 @@ struct ScaleSource {
   int n_partials;          //   the whole (small) input, which every block then reads for itself
   int64_t n_vecs;          // 32-byte units of the input
   float* out;              // the dynamic scale for whoever needs it next
-  bool backward;           // begin with the last rows (large fp32 inputs behind their reduction)
+  bool backward;           // begin with the last rows (walk_of)
 };
 
 // amax(|x|) / (448 * 6) of the whole input, by every block for itself (all threads return it).  NaNs
@@ -182,10 +182,10 @@ __device__ __forceinline__ float block_dynamic_scale(const T* x, const ScaleSour
 // The row groups are walked in order, which is also the order of the reduction pass: walked backwards (for
 // what the reduction pass left in L2) a static scale pays 0.3 us at 1024 x 3072 (4.72 against 4.43, inputs
 // not in L2) and three layers on one 4096 x 3072 input 85.0 against 83.9.  Behind a reduction it pays for fp32 inputs that are larger than
-// L2 (kBackwardBytes); 16-bit inputs, bound by their arithmetic, gain nothing (36864 x 3072 83.2 / 83.8).
+// L2 and marked (walk_of); 16-bit inputs, bound by their arithmetic, gain nothing (36864 x 3072 83.2 / 83.8).
 //
 // kMark: the input's lines are marked first to leave L2 (evict_first), so that they make room for each other
-// and not push out the codes, which the GEMM reads next.  By the rule in launch_streaming: not for inputs that
+// and not push out the codes, which the GEMM reads next.  By the rule in walk_of: not for inputs that
 // stay in L2, where the next layer on the same activation finds them.
 //
 // Bound by HBM for large inputs and by launches and latency for small ones: finishing the dynamic scale
@@ -215,14 +215,15 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
   // warms the cache (L2 is the point of coherence: what the previous kernel still writes is seen
   // by the loads after the wait), and it takes the DRAM latency of the first loads off the
   // critical path of a kernel that only runs for a few microseconds.
-  const bool backward = kDynamic && kMark && sizeof(T) == 4 && src.backward;
+  constexpr bool kMayTurn = kDynamic && kMark && sizeof(T) == 4;  // the only form that walk_of sends backwards
+  const bool backward = kMayTurn && src.backward;
   const int first = backward ? row_groups - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
   const int step = backward ? -static_cast<int>(gridDim.x) : static_cast<int>(gridDim.x);
   if (has_data && (threadIdx.x & 1) == 0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int row = (first + i * step) * kPairRows + static_cast<int>(threadIdx.y);
-      if (row >= 0 && row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
+      if ((!kMayTurn || row >= 0) && row < data_rows) prefetch_l2(x + static_cast<int64_t>(row) * cols + pc * kElems);  // one 128-byte line per lane pair
     }
   }
   pdl_wait();  // the tensor scale and x may come from the kernel before this one
@@ -249,11 +250,11 @@ quantize_nvfp4_stream_kernel(const T* x, const ScaleSource src, uint8_t* __restr
   }
   if constexpr (!kDynamic) g = ld_f32_dependent(src.given);
   const TensorScale ts = make_tensor_scale(g);
-  for (int rg = first; rg >= 0 && rg < row_groups; rg += step) {
+  for (int rg = first; (!kMayTurn || rg >= 0) && rg < row_groups; rg += step) {
     const int row = rg * kPairRows + threadIdx.y;
     const int next_row = row + step * kPairRows;
     Vec256 an = {}, bn = {};
-    if (has_data && next_row >= 0 && next_row < data_rows) {
+    if (has_data && (!kMayTurn || next_row >= 0) && next_row < data_rows) {
       const T* at = x + static_cast<int64_t>(next_row) * cols + pc * kElems;
       an = ld_stream_unit<kMark>(at);
       bn = ld_stream_unit<kMark>(at + kElems / 2);
@@ -431,17 +432,35 @@ int launch_streaming_marked(const T* x, const ScaleSource& src, uint8_t* codes, 
   return launch_streaming_as<T, false, kMark, 16>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, kAll, stream);
 }
 
+// How a launch of the streaming quantizer goes through its input.
+struct Walk {
+  bool mark, backward;
+};
+
 // Inputs of more than a quarter of L2 are marked as long as their codes and scales fit in half of it (64 MiB:
 // 227 MiB of a 16-bit type, 455 of fp32).  Measured marked / not: three linears on one bf16 activation of
 // 24 MiB 91.6 / 89.5 us, of 48 MiB 179.7 / 181.5; fp32 weights of 144 MiB 24.7 / 28.7, of 384 MiB 71.6 / 76.6, of
 // 576 MiB 124 / 115; the reduction and quantizer on 384 MiB of bf16 184.8 / 175.4.
+//
+// Marked fp32 inputs of more than 120 MiB, so up to 455, are quantized from their last rows on, which the reduction has just read.
+// Forwards / backwards, us: 6144 x 3072 (72 MiB) 24.1 / 24.3, 8192 x 3072 (96 MiB) 31.4 / 31.6, 12288 x 3072 (144 MiB) 48.0 / 46.4, 24576 x 3072
+// 97.6 / 94.7, 36864 x 3072 147 / 143.  Marking what the reduction reads first evict_first, so that the last 64 to 96 MiB stay, gains less
+// (47.0 to 47.5 at 144 MiB).
+Walk walk_of(int elem_bytes, bool behind_reduction, int64_t orig_rows, int64_t num_rows, int64_t num_cols) {
+  const int64_t bytes = orig_rows * num_cols * elem_bytes, written = num_rows * num_cols / 16 * 9;
+  Walk w;
+  w.mark = bytes > (32ll << 20) && written <= (64ll << 20);
+  w.backward = w.mark && behind_reduction && elem_bytes == 4 && bytes > (120ll << 20);
+  return w;
+}
+
 template <typename T>
-int launch_streaming(const T* x, const ScaleSource& src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
+int launch_streaming(const T* x, ScaleSource src, uint8_t* codes, uint8_t* scales, int64_t orig_rows, int64_t num_rows,
                      int64_t num_cols, int hi_first, cudaStream_t stream) {
-  const int64_t bytes = orig_rows * num_cols * static_cast<int64_t>(sizeof(T)), written = num_rows * num_cols / 16 * 9;
-  const bool mark = bytes > (32ll << 20) && written <= (64ll << 20);
-  return mark ? launch_streaming_marked<T, true>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream)
-              : launch_streaming_marked<T, false>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream);
+  const Walk walk = walk_of(sizeof(T), src.partials != nullptr, orig_rows, num_rows, num_cols);
+  src.backward = walk.backward;
+  return walk.mark ? launch_streaming_marked<T, true>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream)
+                   : launch_streaming_marked<T, false>(x, src, codes, scales, orig_rows, num_rows, num_cols, hi_first, stream);
 }
 
 template <typename T>
@@ -490,10 +509,6 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
 // stays lower: 8 x 4096 (64 KiB) 4.4 / 3.5, 3 x 15360 (90 KiB) 3.6 / 3.8, 8 x 15360 4.0 / 5.6.
 constexpr int64_t whole_input_bytes(int64_t rows) { return rows > 8 ? 128 * 1024 : 64 * 1024; }
 constexpr int64_t kDynamicScratchHead = 256;
-// fp32 inputs from here on are quantized from their last rows on, which the reduction has just read.  Forwards / backwards, us: 6144 x 3072
-// (72 MiB) 24.1 / 24.3, 8192 x 3072 (96 MiB) 31.4 / 31.6, 12288 x 3072 (144 MiB) 48.0 / 46.4, 24576 x 3072 97.6 / 94.7, 36864 x 3072 147 / 143.
-// Marking what the reduction reads first evict_first, so that the last 64 to 96 MiB stay, gains less (47.0 to 47.5 at 144 MiB).
-constexpr int64_t kBackwardBytes = 120ll << 20;
 
 __global__ void clear_word_kernel(unsigned int* word) {
   pdl_launch_dependents();
@@ -516,7 +531,6 @@ int launch_nvfp4_dynamic(const void* input, int dtype, float* scale_out, void* c
       float* partials = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kDynamicScratchHead);
       if (int rc = launch_amax_partials(x, dtype, src.n_vecs, partials, &src.n_partials, stream)) return rc;
       src.partials = partials;
-      src.backward = sizeof(T) == 4 && n * 4 > kBackwardBytes;
     }
     return launch_streaming<T>(x, src, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), orig_rows, num_rows, num_cols,
                                hi_first, stream);
@@ -581,6 +595,13 @@ extern "C" int ck_debug_set_exact_division(int on) {
   const bool before = ck::exact_division();
   ck::g_exact_division.store(on != 0 ? 1 : 0, std::memory_order_relaxed);
   return before ? 1 : 0;
+}
+
+extern "C" int ck_debug_quantize_nvfp4_walk(int input_dtype, int dynamic, int64_t rows, int64_t cols) {
+  const bool fp32 = input_dtype == CK_DTYPE_F32;
+  const int elem = fp32 ? 4 : 2;
+  const ck::Walk w = ck::walk_of(elem, dynamic != 0 && rows * cols * elem > ck::whole_input_bytes(rows), rows, rows, cols);
+  return (w.mark ? 1 : 0) | (w.backward ? 2 : 0);
 }
 
 extern "C" int ck_quantize_nvfp4(const void* input, int input_dtype, const float* global_scale, void* codes,

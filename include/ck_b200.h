@@ -64,6 +64,11 @@ CK_API int ck_device_supported(int device);
  * it by comparing them).  Process-wide; returns the previous setting. */
 CK_API int ck_debug_set_exact_division(int on);
 
+/* Validation aid with no counterpart in the reference: how the streaming quantizer of NVFP4 goes through an input of
+ * `rows` x `cols` with a static or a dynamic scale: bit 0, its lines are marked first to leave L2; bit 1, it begins with
+ * the last rows.  Both leave the results as they are.  Needs no GPU. */
+CK_API int ck_debug_quantize_nvfp4_walk(int input_dtype, int dynamic, int64_t rows, int64_t cols);
+
 /*
  * NVFP4 quantization: [orig_rows, orig_cols] f32/f16/bf16 row-major contiguous
  * input -> packed E2M1 codes uint8 [num_rows, num_cols/2] and E4M3 block

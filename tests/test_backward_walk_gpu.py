@@ -1,5 +1,6 @@
 """fp32 inputs larger than L2 are quantized from their last rows on when the scale comes from a reduction: the same bits as with that
-scale given, on both sides of the line (120 MiB), with rows and columns that end inside a block and padded rows."""
+scale given, on both sides of both lines (120 MiB of input, 64 MiB of codes and scales), with rows and columns that end inside a block and
+padded rows.  Which inputs they are: test_quantize_walk_cpu."""
 from __future__ import annotations
 
 import pytest
@@ -8,7 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# 10240 x 3072 fp32 is 120 MiB; 38900 x 3072 has more than 64 MiB of codes and scales (no marks)
+# 10240 x 3072 fp32 is 120 MiB; 38900 x 3072 has more than 64 MiB of codes and scales (no marks, forwards)
 @pytest.mark.parametrize("rows, cols, pad", [(10240, 3072, False), (10241, 3072, True), (10255, 3088, False), (20001, 1584, True), (130, 262144, False), (38900, 3072, False)])
 def test_same_as_with_the_scale_given(cuda_device, rows, cols, pad):
     from comfy_kitchen.backends import cuda as backend
