@@ -70,16 +70,18 @@ bool tiles_in_as_few_waves(int64_t tiles, int64_t pairs, const Room& room) {
 // small tile hides.  us, pair / 128 x 128, two waves against one: NVFP4 512 x 9216 x 1280 7.9 / 7.2, x 1536 8.4 / 7.8, x 1792 8.7 / 8.6, x 2048 9.0 / 9.1, MXFP8 x 640
 // 7.9 / 7.1, x 768 8.3 / 7.7, x 1024 8.9 / 8.9; three against two: 1280 x 4608 x 1280 8.9 / 8.5, x 1536 9.4 / 9.3, 700 x 9216 x 1536 9.5 / 9.8; four against two: 2048 x 4608 x
 // 512 8.4 / 8.8.  The fused epilogue is the longer one: 512 x 9216 x 1536 10.8 / 10.1, x 3072 12.9 / 12.6, x 4096 14.4 / 14.8, 1024 x 6144 x 3072 16.4 / 16.0, 1152 x 7680 x
-// 3072 21.8 / 19.9, but with two waves against one and up to two stages it hides behind nothing: 208 x 12352 x 512 8.2 / 8.7, 216 x 13440 x 256 8.1 / 8.6.  Rows of K that
+// 3072 21.8 / 19.9, but with two waves against one and up to two stages it hides behind nothing: 208 x 12352 x 512 8.2 / 8.7, 216 x 13440 x 256 8.1 / 8.6.  In fp32 two
+// waves against one never pay: 384 x 9216 x 256 11.5 / 12.7, 640 x 4608 x 1024 12.2 / 13.1, 1024 x 4608 x 1280 13.0 / 14.0, 2048 x 2048 x 1792 13.3 / 14.5, 640 x 4608 x 3072
+// 14.9 / 15.6; three against two pay as in 16 bits, 1152 x 7680 x 1280 28.8 / 24.6, 2048 x 4608 x 3072 24.3 / 24.0.  Rows of K that
 // straddle 128-byte lines cost twice as many readers more (1003 x 4096 x 1248 7.7 / 8.3, MXFP8 650 x 6400 x 736 9.3 / 9.5, fused 179 x 18368 x 672 10.0 / 11.4).
 // In front of the next dynamic linear only where a sixth is padding, as above: 1003 x 6144 x 1024 14.9 / 15.3, 520 x 10240 x 1024 16.4 / 14.9.
-bool tiles_in_one_wave_more(int64_t tiles, int64_t pairs, int k_bytes, bool fused, const Room& room) {
+bool tiles_in_one_wave_more(int64_t tiles, int64_t pairs, int k_bytes, bool fused, bool fp32, const Room& room) {
   const int64_t tile_waves = ceil_div(tiles, sm_count()), pair_waves = ceil_div(pairs, sm_count() / 2), k_stages = ceil_div(k_bytes, kStageKBytes);
   const bool padded = 10 * pairs >= 3 * tiles;
   if (tile_waves != pair_waves + 1 || tile_waves > 4) return false;
   if (room.wanted && (tile_waves == 2 || !padded)) return false;
   if (k_bytes % kStageKBytes != 0) return !fused && tile_waves == 2 && k_stages <= 4;
-  if (fused) return k_stages <= 12 && (k_stages >= 3 || tile_waves > 2 || padded);
+  if (fused) return k_stages <= 12 && (tile_waves > 2 || (!fp32 && (k_stages >= 3 || padded)));
   return k_stages <= (tile_waves == 2 ? 6 : 5);
 }
 
@@ -93,7 +95,7 @@ int launch_for_shape(const Operands& ops, const GemmParams& p, const OutputSpec&
     // 16.5 / 13.8, the fused epilogue 128 x 12288 x 3072 12.6 / 9.1), and not where small tiles beat it (above).
     const int64_t pairs = ceil_div(p.M, 256) * ceil_div(p.N, 256);
     const bool pair = pairs * 4 >= sm_count() && row_blocks > 1 && !tiles_in_as_few_waves(tiles, pairs, room) &&
-                      !tiles_in_one_wave_more(tiles, pairs, p.k_bytes, FUSED, room);
+                      !tiles_in_one_wave_more(tiles, pairs, p.k_bytes, FUSED, sizeof(OutT) == 4, room);
     if (pair) {
       config = 4;
     } else if (tiles * 4 <= sm_count() || (half_tiles_pay(p.M, p.N, p.k_bytes) && room.left_by_half_tiles(p.M, p.N))) {

@@ -47,3 +47,21 @@ def test_same_as_128_x_128(cuda_device, monkeypatch, fmt, m, n, k):
         else:
             assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
     backend.check_device_status("wave choice")
+
+
+# fused in fp32: pairs where they take one wave and 128 x 128 tiles two; three waves of those against two up to twelve stages
+@pytest.mark.parametrize("m, n, k", [(1024, 4608, 4 * 256), (384, 9216, 256 + 32), (1000, 4672, 5 * 256), (1152, 4608, 12 * 256), (1152, 4608, 13 * 256)])
+def test_fused_fp32_same_as_128_x_128(cuda_device, monkeypatch, m, n, k):
+    from comfy_kitchen.backends import cuda as backend
+
+    gen = torch.Generator(device=cuda_device).manual_seed(m + n + k)
+    (qx, sx, gx), (qw, sw, gw) = (backend.quantize_nvfp4_dynamic(torch.randn(r, k, generator=gen, device=cuda_device).bfloat16()) for r in (m, n))
+    bias = torch.linspace(-1, 1, n, device=cuda_device)
+    call = lambda dense: backend.linear_nvfp4_fused(qx, qw, gx, gw, sx, sw, bias=bias, activation="gelu_tanh", out_dtype=torch.float32,
+                                                    requant_scale=gx, return_dense=dense)
+    got, got_alone = call(True), call(False)
+    monkeypatch.setenv("CK_GEMM_CONFIG", "1")
+    want = call(True)
+    for a, b, c in zip(want, got, (want[0], *got_alone[1:])):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)) and torch.equal(a.view(torch.uint8), c.view(torch.uint8))
+    backend.check_device_status("fused in fp32")
