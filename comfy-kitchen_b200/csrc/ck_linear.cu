@@ -14,10 +14,6 @@ struct FromFloatLayout {
   int64_t scratch_off, scale_off, codes_off, scales_off, total;
 };
 
-// Few rows, quantized inside the GEMM: up to here every CTA takes the maximum of the whole activation itself; beyond it a reduction kernel
-// leaves partial maxima.  us, reduction kernel / whole activation: bf16 6 x 3072 x 6144 (72 KiB) 7.8 / 7.4, 8 x 3072 x 6144 (96 KiB) 7.8 / 7.6, 4 x 3072 x 12288
-// (96 KiB) 9.4 / 9.2, fp32 8 x 6144 x 4096 (128 KiB) 9.4 / 8.9, bf16 6 x 3072 x 12288 (144 KiB) 9.6 / 10.1, 8 x 12288 x 15360 (240 KiB) 23.8 / 25.0.
-constexpr int64_t kSmallLinearWholeInputBytes = 128 * 1024;
 // Workspace layout: tensor-scale scratch | dynamic tensor scale | codes [M, K/2] | tiled block scales.
 constexpr int64_t kScaleScratchBytes = 256 + 256 * 1024;  // 2^30 elements: 65536 partials behind the head
 
@@ -63,7 +59,11 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
     const int64_t elem = x_dtype == CK_DTYPE_F32 ? 4 : 2;
     float* partials = nullptr;
     int n_partials = 0;
-    if (dynamic && M * K * elem > kSmallLinearWholeInputBytes) {
+    int64_t whole = 0;
+    if (dynamic) {
+      if (int rc = linear_small_m_whole_input_bytes(x_dtype, N, K, &whole)) return rc;
+    }
+    if (dynamic && M * K * elem > whole) {
       partials = reinterpret_cast<float*>(ws + l.scratch_off);
       if (int rc = launch_amax_partials(x, x_dtype, M * K * elem / 32, partials, &n_partials, static_cast<cudaStream_t>(stream))) return rc;
     }
