@@ -38,7 +38,8 @@ bool one_wave_of_half_tiles(int64_t M, int64_t N) { return ceil_div(M, kTileM) *
 
 // Whether they pay.  Twice the CTAs ask for the same rows of the activation at once.  Rows that straddle the 128-byte lines cost each
 // of them two: with one or two row blocks that is dearer (NVFP4 68 x 6304 x 2976 7.4 / 8.9, 128 x 8512 x 3808 9.8 / 10.0, 256 x 4640 x 3296 8.6 / 8.8).
-// Up to 64 rows the epilogue has little to halve: from eight stages on they pay all the same (drawn sizes: 0.97 of the time up to 17 stages, 0.95 beyond, 1.05 below eight).
+// Up to 64 rows the epilogue has little to halve: from eight stages on they pay all the same (drawn sizes: 0.97 of the time up to 17 stages, 0.95
+// beyond, 1.05 below eight).
 bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
   if (!one_wave_of_half_tiles(M, N)) return false;
   if (k_bytes % kStageKBytes != 0) return M > 2 * kTileM;
@@ -48,8 +49,8 @@ bool half_tiles_pay(int64_t M, int64_t N, int k_bytes) {
 // In a linear with a dynamic scale.  Such calls in a row are a chain of reduction, quantizer and GEMM whose launches overlap, and the quantizer's
 // few large blocks find room beside the GEMM before them only on SMs that it leaves free.  A GEMM of more, smaller CTAs gains less than
 // the quantizer then loses, unless a quarter of the SMs stays free (whole linears, us, 128 x 128 / half tiles: 200 x 4544 x 768 7.5 / 8.6, 65 x 9216 x 3072
-// 11.2 / 12.9, 1003 x 1024 x 768 8.1 / 8.7; 128 x 6848 x 3072, 107 half tiles, 11.8 / 10.7, 1003 x 576 x 352 8.6 / 7.4; pair / 128 x 128: 512 x 6848 x 768, 54 pairs,
-// 10.9 / 11.7, 1003 x 3072 x 512 10.8 / 11.3; 640 x 6848 x 768, 81 pairs on 74, 14.1 / 12.4).
+// 11.2 / 12.9, 1003 x 1024 x 768 8.1 / 8.7; 128 x 6848 x 3072, 107 half tiles, 11.8 / 10.7, 1003 x 576 x 352 8.6 / 7.4; pair / 128 x 128: 512 x 6848
+// x 768, 54 pairs, 10.9 / 11.7, 1003 x 3072 x 512 10.8 / 11.3; 640 x 6848 x 768, 81 pairs on 74, 14.1 / 12.4).
 struct Room {
   bool wanted;
   bool left_by_half_tiles(int64_t M, int64_t N) const { return !wanted || ceil_div(M, kTileM) * ceil_div(N, 64) * 4 <= 3 * sm_count(); }
@@ -58,23 +59,24 @@ struct Room {
 // 128 x 128 tiles that take no more waves than pair tiles: a wave of them is shorter, with half the output of an SM behind its main loop.
 // That is where the pairs' last rows or columns are padding, with 257 to 384 rows above all, or their last wave is nearly empty.  us, pair / 128 x 128:
 // NVFP4 300 x 6144 x 3072 (48 pairs, 144 tiles) 9.1 / 7.1, 300 x 12288 x 3072 13.7 / 11.1, 384 x 12288 x 6144 22.3 / 18.9, MXFP8 384 x 6144 x 3072
-// 13.4 / 10.5, fused 384 x 9600 x 3072 14.8 / 11.8, 1152 x 4096 x 3072 15.7 / 12.1; with one wave more 768 x 9216 x 3072 14.0 / 15.1.  In front of the next dynamic
-// linear (Room) a full wave of small tiles is not worth it, 144 x 9472 x 1792 (37 pairs, 148 tiles) 12.0 / 12.9, 832 x 2560 x 3136 (40, 140) 15.1 / 15.7, unless
-// a sixth of the pairs' tiles is padding: 282 x 5696 x 3136 (46, 135) 15.1 / 13.6.
+// 13.4 / 10.5, fused 384 x 9600 x 3072 14.8 / 11.8, 1152 x 4096 x 3072 15.7 / 12.1; with one wave more 768 x 9216 x 3072 14.0 / 15.1.  In front of
+// the next dynamic linear (Room) a full wave of small tiles is not worth it, 144 x 9472 x 1792 (37 pairs, 148 tiles) 12.0 / 12.9, 832 x 2560 x 3136
+// (40, 140) 15.1 / 15.7, unless a sixth of the pairs' tiles is padding: 282 x 5696 x 3136 (46, 135) 15.1 / 13.6.
 bool tiles_in_as_few_waves(int64_t tiles, int64_t pairs, const Room& room) {
   const int64_t tile_waves = ceil_div(tiles, sm_count()), pair_waves = ceil_div(pairs, sm_count() / 2);
   return tile_waves <= pair_waves && tile_waves <= 3 && (!room.wanted || tile_waves > 1 || 10 * pairs >= 3 * tiles);
 }
 
 // One wave more of them, while the K is so short that a tile's time is its latencies and its epilogue, which the second accumulator of a
-// small tile hides.  us, pair / 128 x 128, two waves against one: NVFP4 512 x 9216 x 1280 7.9 / 7.2, x 1536 8.4 / 7.8, x 1792 8.7 / 8.6, x 2048 9.0 / 9.1, MXFP8 x 640
-// 7.9 / 7.1, x 768 8.3 / 7.7, x 1024 8.9 / 8.9; three against two: 1280 x 4608 x 1280 8.9 / 8.5, x 1536 9.4 / 9.3, 700 x 9216 x 1536 9.5 / 9.8; four against two: 2048 x 4608 x
-// 512 8.4 / 8.8.  The fused epilogue is the longer one: 512 x 9216 x 1536 10.8 / 10.1, x 3072 12.9 / 12.6, x 4096 14.4 / 14.8, 1024 x 6144 x 3072 16.4 / 16.0, 1152 x 7680 x
-// 3072 21.8 / 19.9, but with two waves against one and up to two stages it hides behind nothing: 208 x 12352 x 512 8.2 / 8.7, 216 x 13440 x 256 8.1 / 8.6.  In fp32 two
-// waves against one never pay: 384 x 9216 x 256 11.5 / 12.7, 640 x 4608 x 1024 12.2 / 13.1, 1024 x 4608 x 1280 13.0 / 14.0, 2048 x 2048 x 1792 13.3 / 14.5, 640 x 4608 x 3072
-// 14.9 / 15.6; three against two pay as in 16 bits, 1152 x 7680 x 1280 28.8 / 24.6, 2048 x 4608 x 3072 24.3 / 24.0.  Rows of K that
-// straddle 128-byte lines cost twice as many readers more (1003 x 4096 x 1248 7.7 / 8.3, MXFP8 650 x 6400 x 736 9.3 / 9.5, fused 179 x 18368 x 672 10.0 / 11.4).
-// In front of the next dynamic linear only where a sixth is padding, as above: 1003 x 6144 x 1024 14.9 / 15.3, 520 x 10240 x 1024 16.4 / 14.9.
+// small tile hides.  us, pair / 128 x 128, two waves against one: NVFP4 512 x 9216 x 1280 7.9 / 7.2, x 1536 8.4 / 7.8, x 1792 8.7 / 8.6, x 2048 9.0 /
+// 9.1, MXFP8 x 640 7.9 / 7.1, x 768 8.3 / 7.7, x 1024 8.9 / 8.9; three against two: 1280 x 4608 x 1280 8.9 / 8.5, x 1536 9.4 / 9.3, 700 x 9216 x 1536
+// 9.5 / 9.8; four against two: 2048 x 4608 x 512 8.4 / 8.8.  The fused epilogue is the longer one: 512 x 9216 x 1536 10.8 / 10.1, x 3072 12.9 / 12.6,
+// x 4096 14.4 / 14.8, 1024 x 6144 x 3072 16.4 / 16.0, 1152 x 7680 x 3072 21.8 / 19.9, but with two waves against one and up to two stages it hides
+// behind nothing: 208 x 12352 x 512 8.2 / 8.7, 216 x 13440 x 256 8.1 / 8.6.  In fp32 two waves against one never pay: 384 x 9216 x 256 11.5 / 12.7,
+// 640 x 4608 x 1024 12.2 / 13.1, 1024 x 4608 x 1280 13.0 / 14.0, 2048 x 2048 x 1792 13.3 / 14.5, 640 x 4608 x 3072 14.9 / 15.6; three against two pay
+// as in 16 bits, 1152 x 7680 x 1280 28.8 / 24.6, 2048 x 4608 x 3072 24.3 / 24.0.  Rows of K that straddle 128-byte lines cost twice as many readers
+// more (1003 x 4096 x 1248 7.7 / 8.3, MXFP8 650 x 6400 x 736 9.3 / 9.5, fused 179 x 18368 x 672 10.0 / 11.4). In front of the next dynamic linear
+// only where a sixth is padding, as above: 1003 x 6144 x 1024 14.9 / 15.3, 520 x 10240 x 1024 16.4 / 14.9.
 bool tiles_in_one_wave_more(int64_t tiles, int64_t pairs, int k_bytes, bool fused, bool fp32, const Room& room) {
   const int64_t tile_waves = ceil_div(tiles, sm_count()), pair_waves = ceil_div(pairs, sm_count() / 2), k_stages = ceil_div(k_bytes, kStageKBytes);
   const bool padded = 10 * pairs >= 3 * tiles;
@@ -166,9 +168,10 @@ int choose_splits(int64_t M, int64_t N, int k_bytes, bool have_workspace, SplitP
   plan->through_workspace = have_workspace && 3 * (ceil_div(k_stages, splits) - ceil_div(k_stages, most)) >= 4 * most && most > 1;
   // Two CTAs to a tile: half tiles instead, while their longer K costs less than the exchange.  They end in TMA stores, which want
   // rows of whole 64-byte units (N of 16 bits off by 16: MXFP8 512 x 1648 x 2784 10.0 / 10.7, NVFP4 517 x 1584 x 4800 9.7 / 10.7).  us, two CTAs /
-  // half tiles: linears NVFP4 256 x 4608, 24 stages, 12.9 / 11.5, 300 x 2048, 24 stages, 12.3 / 11.4, MXFP8 256 x 4608, 30 stages, 12.9 / 12.0.  Over drawn sizes of
-  // both formats half tiles take 0.91 to 1.0 of the time from 24 to 35 stages, 1.0 from 36 to 41 and 1.05 from 42 on.
-  // Up to 64 rows not where those of K straddle 128-byte lines (NVFP4 40 x 8192 x 6112 10.2 / 10.8; 64 x 8192 x 6144 10.1 / 9.4, MXFP8 64 x 9216 x 3072 10.3 / 9.3).
+  // half tiles: linears NVFP4 256 x 4608, 24 stages, 12.9 / 11.5, 300 x 2048, 24 stages, 12.3 / 11.4, MXFP8 256 x 4608, 30 stages, 12.9 / 12.0.  Over
+  // drawn sizes of both formats half tiles take 0.91 to 1.0 of the time from 24 to 35 stages, 1.0 from 36 to 41 and 1.05 from 42 on. Up to 64 rows
+  // not where those of K straddle 128-byte lines (NVFP4 40 x 8192 x 6112 10.2 / 10.8; 64 x 8192 x 6144 10.1 / 9.4, MXFP8 64 x 9216 x 3072 10.3 /
+  // 9.3).
   constexpr int kMostStages = 36;
   plan->half_tiles = splits == 2 && !plan->through_workspace && k_stages <= kMostStages && N % 32 == 0 && (M > 64 || k_bytes % kStageKBytes == 0) && one_wave_of_half_tiles(M, N);
   if (plan->half_tiles) splits = 1;

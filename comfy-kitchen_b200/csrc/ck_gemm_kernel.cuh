@@ -541,8 +541,9 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // issuer took 600 cycles a stage and the producer 480 (128 x 128 tiles; the tensor pipe needs 320 with NVFP4's eight scale copies, 284
   // with MXFP8's two), so, about 400 and 370.  us, whole warps / one lane: NVFP4 64 x 3072 x 3072 6.37 / 5.86, 256 x 3072 x 3072 6.64 / 6.06, 512 x
   // 3072 x 3072 7.36 / 6.85, 256 x 3072 x 12288 13.5 / 13.1, MXFP8 512 x 3072 x 3072 10.8 / 9.8, 128 x 9216 x 3072 10.2 / 9.65.  Pairs are bound by the
-  // tensor pipe at 512 cycles, and whole warps serve them better (NVFP4 4096 x 3072 x 3072 18.8 / 19.2, 16384 x 9216 x 3072 180 / 184), except the issuer beside the
-  // fused epilogue's sixteen warps (1024 x 12288 x 3072 23.6 / 23.1).  Asking for the next stage's barrier ahead of a stage's MMAs gains nothing.
+  // tensor pipe at 512 cycles, and whole warps serve them better (NVFP4 4096 x 3072 x 3072 18.8 / 19.2, 16384 x 9216 x 3072 180 / 184), except the
+  // issuer beside the fused epilogue's sixteen warps (1024 x 12288 x 3072 23.6 / 23.1).  Asking for the next stage's barrier ahead of a stage's MMAs
+  // gains nothing.
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (!kOneLane || elect_one()) {
@@ -793,11 +794,12 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // while tile t - 1 is in its epilogue, right after the drain, with values fetched ahead of the wait for the
       // accumulator, whose latency that wait hides.
       // Plain tiles and fp32: every thread fetches one value, and the warps meet at a barrier after the drain, where they
-      // are aligned anyway; a warp then runs at most one tile ahead of the slowest, hence the third buffer.  Fused 16-bit tiles: every warp fetches the columns it reads itself (the four warps of the same columns
-      // write the same values; tile t + 3's come behind the accumulator of t + 2, which waits for all warps' drains of t, where the bias of t is
-      // read), since a barrier a tile made each of sixteen warps wait for the one with the longest chains: bf16 4608 x
-      // 8192 x 2048 47.8 / 44.8 us, 4608 x 12288 x 3072 79.7 / 77.2, fp16 80.7 / 78.4, 128 x 12288 x 3072 9.0 / 9.0.  With fp32 it lost (77.6 / 78.3),
-      // and so did plain pairs (36864 x 9216 x 3072 407 / 416).
+      // are aligned anyway; a warp then runs at most one tile ahead of the slowest, hence the third buffer.
+      // Fused 16-bit tiles: every warp fetches the columns it reads itself (the four warps of the same columns write the same
+      // values; tile t + 3's come behind the accumulator of t + 2, which waits for all warps' drains of t, where the bias of t
+      // is read), since a barrier a tile made each of sixteen warps wait for the one with the longest chains: us, barrier / so,
+      // bf16 4608 x 8192 x 2048 47.7 / 44.8, 4608 x 12288 x 3072 80.1 / 77.6 (under the power limit 93.9 / 91.5), fp16 81.1 / 78.9; one tile to
+      // a worker, 128 x 12288 x 3072, 8.95 / 8.98.  With fp32 it lost (77.6 / 78.3), and so did plain pairs (36864 x 9216 x 3072 407 / 416).
       float* bias_s = smem_bias + (tile_it % 3) * TILE_N;
       const bool with_bias = p.bias != nullptr;
       if (tile_it == 0) {

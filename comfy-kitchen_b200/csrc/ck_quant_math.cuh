@@ -103,7 +103,7 @@ __device__ __forceinline__ void nvfp4_block(const float (&v)[16], float g, bool 
   };
   bool done = false;
   if (window) {
-    // Codes from the two products that bracket the exact quotient (see nvfp4_block_packed);
+    // Codes from the two products that bracket the exact quotient (see nvfp4_blocks);
     // accepted when they agree, which is the rule for all but a few blocks in ten thousand.
     const float y = __frcp_rn(safe);
     const float y_hi = __fmul_rn(y, 0x1.000008p0f), y_lo = __fmul_rn(y, 0x1.fffffp-1f);
@@ -260,11 +260,12 @@ __device__ __forceinline__ float approximate_reciprocal(float t) {
   return y;
 }
 
-// Codes of sixteen 16-bit values divided by t: p = x y, then one correction by the residual, q = p - (t p - x) y.  For an x of
-// at most eleven significant bits the code of q is the code of RN(x / t): q is off by less than 2^-45 beside its own rounding, so the two
-// can only part where x / t lies that close to the middle between a rounding boundary and its neighbour, and x and the boundary
-// times t are then integers a few units apart; the cases there are have been gone through one by one (test_corrected_quotient_cpu),
-// with reciprocals up to two units in the last place off.  Only a significand of all ones fails, which the caller sends elsewhere.
+// Codes of sixteen 16-bit values divided by t: p = x y, then one correction by the residual, q = p - (t p - x) y.  With a y that is
+// off by e, p is off by up to e + 2^-24, and q, beside its own rounding, by that times e and the residual's rounding: (e + 2^-24)^2 at most, 1.13 x 2^-45
+// for one unit in the last place (e = 2^-23), 1.57 x 2^-44 for two.  For an x of at most eleven significant bits the code of q is the code
+// of RN(x / t): the two can only part where x / t lies that close to the middle between a rounding boundary and its neighbour, and x and the
+// boundary times t are then integers a few units apart; the cases there are have been gone through one by one (test_corrected_quotient_cpu),
+// with reciprocals up to two units off.  Only a significand of all ones fails, which the caller sends elsewhere.
 // The residual carries the sign opposite to x, so that the sum keeps a negative zero.  Per element one and a half packed
 // multiply-adds and half a conversion; two bracketing products took one multiply and one conversion, and the conversions' bytes twice.
 template <typename T, bool kHiFirst>
@@ -347,10 +348,15 @@ __device__ __noinline__ BlockCodes nvfp4_block_packed_call(uint32_t w0, uint32_t
 // ---------------------------------------------------------------------------
 // NVFP4 blocks of one thread without a branch in the common case
 // ---------------------------------------------------------------------------
-// The E4M3 scale is bracketed like the codes: s = RN(RN(amax / 6) / g) deviates from amax / (6 g) by at most 2^-23, and
+// Codes of fp32 inputs and of the fused epilogue: no quotient is computed.  The code of x / total is a monotone step function of the
+// quotient, and RN(x / total) lies strictly between x y_lo and x y_hi with y_lo = y (1 - 2^-21) and y_hi = y (1 + 2^-21), y close to
+// 1 / total: y is off by 2^-23 at most (nvfp4_block rounds it correctly, 2^-24), y_lo or y_hi, the product and the quotient itself are rounded by up to 2^-24
+// each, 1.25 x 2^-22 in all.  So where both products convert to the same codes for a whole block, two multiplies and one convert
+// an element, those are the codes of the exact quotients, and only a block in which some product straddles a rounding boundary is
+// done again with quotients.  A zero keeps its sign through the multiplication, as the reference's cast keeps it.
+// The E4M3 scale is bracketed like those codes: s = RN(RN(amax / 6) / g) deviates from amax / (6 g) by at most 2^-23, and
 // amax * s_hi and amax * s_lo lie 2^-21 on either side of it less the 2^-22 of their own four roundings; when both
-// round to the same E4M3 byte, that is the byte of s.  The codes' reciprocal is the hardware's (one unit in the last
-// place, 2^-23): with the products' roundings and the quotient's own 1.25 * 2^-22, still inside the bracket.
+// round to the same E4M3 byte, that is the byte of s.
 // Everything is computed for all of a thread's blocks before one test asks whether some bracket was split or some
 // operand lies outside the window; those blocks are done again, out of line.  Straight code lets the blocks' serial
 // chains (maximum, scale, conversion there and back, reciprocal) overlap, and has no Markstein chains in it.

@@ -13,8 +13,10 @@
 // Arithmetic contract: results are bit-identical to the reference's eager path
 // (comfy_kitchen/backends/eager/quantization.py:115-160 and :257-324), which uses true
 // IEEE fp32 divisions.  This translation unit is therefore compiled without fast-math,
-// and every division below is either __fdiv_rn or a reciprocal-FMA sequence that is
-// proven to round identically (see div_markstein).
+// and every division below is __fdiv_rn, a reciprocal-FMA sequence that is proven to round
+// identically (see div_markstein), or none at all where what it is rounded to is certain without
+// it: an E2M1 code by a corrected quotient (16-bit inputs, nvfp4_codes_corrected), a code or an E4M3
+// scale by two products on either side of the quotient (nvfp4_blocks).
 #include "ck_quant_math.cuh"
 
 #include <atomic>
@@ -503,10 +505,10 @@ int launch_nvfp4(const void* input, const float* gs, void* codes, void* scales, 
 
 // Inputs of at most this many bytes: every block of the quantizer takes the maximum of the whole input
 // itself (a few 16 KiB passes out of L2) instead of waiting for a reduction kernel, which is a launch more.  Scale and quantizer, us, reduction
-// kernel / whole input: bf16 16 x 3072 (96 KiB) 4.1 / 3.4, 22 x 3072 (132 KiB) 4.0 / 3.5, 32 x 3072 (192 KiB) 4.1 / 4.1, 40 x 3072 4.1 / 4.8, fp16 64 x 1024 (128 KiB)
-// 3.9 / 3.3, fp32 12 x 3072 (144 KiB) 3.4 / 3.5; linears bf16 12 x 3072 x 3072 9.0 / 8.1, 9 x 9216 x 5120 11.7 / 10.8, 12 x 3072 x 6144 (144 KiB) 9.1 / 9.5, 64 x 9216 x 1024
-// 8.2 / 7.4.  Up to eight rows, whose quantizer blocks are narrow and many, the line
-// stays lower: 8 x 4096 (64 KiB) 4.4 / 3.5, 3 x 15360 (90 KiB) 3.6 / 3.8, 8 x 15360 4.0 / 5.6.
+// kernel / whole input: bf16 16 x 3072 (96 KiB) 4.1 / 3.4, 22 x 3072 (132 KiB) 4.0 / 3.5, 32 x 3072 (192 KiB) 4.1 / 4.1, 40 x 3072 4.1 / 4.8, fp16 64
+// x 1024 (128 KiB) 3.9 / 3.3, fp32 12 x 3072 (144 KiB) 3.4 / 3.5; linears bf16 12 x 3072 x 3072 9.0 / 8.1, 9 x 9216 x 5120 11.7 / 10.8, 12 x 3072 x
+// 6144 (144 KiB) 9.1 / 9.5, 64 x 9216 x 1024 8.2 / 7.4.  Up to eight rows, whose quantizer blocks are narrow and many, the line stays lower: 8 x 4096
+// (64 KiB) 4.4 / 3.5, 3 x 15360 (90 KiB) 3.6 / 3.8, 8 x 15360 4.0 / 5.6.
 constexpr int64_t whole_input_bytes(int64_t rows) { return rows > 8 ? 128 * 1024 : 64 * 1024; }
 constexpr int64_t kDynamicScratchHead = 256;
 
