@@ -61,6 +61,7 @@ _SIGNATURES = {
     "ck_debug_set_exact_division": [_I],
     "ck_quantize_nvfp4": [_P, _I, _P, _P, _P, _L, _L, _L, _L, _I, _P],
     "ck_quantize_nvfp4_dynamic_scratch_bytes": [_L],
+    "ck_quantize_nvfp4_dynamic_whole_input_bytes": [_L],
     "ck_quantize_nvfp4_dynamic": [_P, _I, _P, _P, _P, _L, _L, _L, _L, _I, _P, _L, _P],
     "ck_quantize_mxfp8": [_P, _I, _P, _P, _L, _L, _L, _L, _P],
     "ck_scaled_mm_nvfp4": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _L, _L, _L, _P],
@@ -87,7 +88,7 @@ _SIGNATURES = {
     "ck_dequantize_mxfp8": [_P, _P, _P, _I, _L, _L, _P],
 }
 _RESTYPE = {"ck_last_error": ctypes.c_char_p, "ck_nvfp4_tensor_scale_scratch_bytes": ctypes.c_int64,
-            "ck_quantize_nvfp4_dynamic_scratch_bytes": ctypes.c_int64,
+            "ck_quantize_nvfp4_dynamic_scratch_bytes": ctypes.c_int64, "ck_quantize_nvfp4_dynamic_whole_input_bytes": ctypes.c_int64,
             "ck_scaled_mm_workspace_bytes": ctypes.c_int64, "ck_linear_nvfp4_from_float_workspace_bytes": ctypes.c_int64,
             "ck_linear_mxfp8_from_float_workspace_bytes": ctypes.c_int64}
 
@@ -123,8 +124,8 @@ def load_library():
     return lib
 
 
-_HOST_NAMES = ("ck_quantize_nvfp4", "ck_quantize_nvfp4_dynamic_scratch_bytes", "ck_quantize_nvfp4_dynamic", "ck_quantize_mxfp8",
-               "ck_dequantize_nvfp4", "ck_dequantize_mxfp8", "ck_scaled_mm_workspace_bytes", "ck_scaled_mm_nvfp4_ws",
+_HOST_NAMES = ("ck_quantize_nvfp4", "ck_quantize_nvfp4_dynamic_scratch_bytes", "ck_quantize_nvfp4_dynamic_whole_input_bytes",
+               "ck_quantize_nvfp4_dynamic", "ck_quantize_mxfp8", "ck_dequantize_nvfp4", "ck_dequantize_mxfp8", "ck_scaled_mm_workspace_bytes", "ck_scaled_mm_nvfp4_ws",
                "ck_scaled_mm_mxfp8_ws", "ck_linear_nvfp4_from_float_workspace_bytes", "ck_linear_nvfp4_from_float",
                "ck_linear_mxfp8_from_float_workspace_bytes", "ck_linear_mxfp8_from_float")
 
@@ -284,18 +285,10 @@ def _scale_scratch_for(device, stream: int, need: int, zeros: bool = True) -> to
     return scratch
 
 
-_KEPT_SCRATCH_BYTES = 64 << 10
-_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
-
-
-def kept_scratch(x: torch.Tensor) -> torch.Tensor | None:
-    """The scratch of a dynamic quantization to which nothing is written (it is kept, and whoever calls on the stream shares it),
-    or None: the call's own is wanted.  Up to 64 KiB no number of rows takes a reduction kernel
-    (``ck_quantize_nvfp4_dynamic_whole_input_bytes``); larger inputs may take one, and where they do not, memory that the native
-    half allocates costs 0.5 us less than looking this one up.  Only plain CUDA tensors are asked for their size: another kind's
-    may be symbolic."""
-    if type(x) not in _PLAIN_TYPES or not x.is_cuda or x.nbytes > _KEPT_SCRATCH_BYTES:
-        return None
+def kept_scratch(x: torch.Tensor) -> torch.Tensor:
+    """The scratch of a dynamic quantization to which nothing is written: it is kept, and whoever calls on the stream shares it.  The
+    native half asks for it up to the size (64 KiB) at which no number of rows takes a reduction kernel; larger inputs may take
+    one, and where they do not, memory that the native half allocates costs 0.5 us less than this."""
     return _scale_scratch_for(x.device, _stream(x.device), 1 << 20, zeros=False)
 
 
@@ -350,7 +343,7 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     """``scale = nvfp4_tensor_scale(x)`` and ``quantize_nvfp4(x, scale)`` in one library call (same bits):
     ``(codes, block_scales, scale)``.  The reduction leaves partial maxima that the quantizer finishes."""
     if _host is not None:
-        out = _host.quantize_nvfp4_dynamic(x, pad_16x, hi_first, kept_scratch(x))
+        out = _host.quantize_nvfp4_dynamic(x, pad_16x, hi_first, kept_scratch)
         if out is not None:
             return out
     lib = load_library()
@@ -371,9 +364,7 @@ def quantize_nvfp4_dynamic(x: torch.Tensor, pad_16x: bool = False,
     stream = _stream(x.device)
     # the smallest workspace that is kept does up to 2^31 elements: no need to ask
     need = 1 << 20 if rows * cols < 1 << 31 else _workspace_bytes("ck_quantize_nvfp4_dynamic_scratch_bytes", rows * cols)
-    scratch = kept_scratch(x)
-    if scratch is None:
-        scratch = _workspace_for(need, x.device, stream)  # the partial maxima go from one launch to the next
+    scratch = _workspace_for(need, x.device, stream)  # the partial maxima go from one launch to the next
     scale = torch.empty((), dtype=torch.float32, device=x.device)
     qx = torch.empty((out_rows, out_cols // 2), device=x.device, dtype=torch.uint8)
     sx = torch.empty((roundup(out_rows, 128), roundup(out_cols // 16, 4)), device=x.device, dtype=torch.float8_e4m3fn)

@@ -68,15 +68,15 @@ def host_half():
     return _backend._host
 
 
-def host_function(name: str):
-    """The native half of the CUDA backend's function ``name``, or None: while something is traced, and where that function has
-    been replaced."""
+def untraced_backend():
+    """The CUDA backend's module for a call outside of any tracing, or None.  The layouts go to the native half of one of its functions
+    while the module holds its own function of that name (``_stock``); another that somebody has put there is called instead."""
     if torch.compiler.is_compiling():
         return None
     global _backend
     if _backend is None:
         from comfy_kitchen.backends import cuda as _backend
-    return _backend.host_function(name)
+    return _backend
 
 
 def crop(result: torch.Tensor, rows: int, cols: int) -> torch.Tensor:

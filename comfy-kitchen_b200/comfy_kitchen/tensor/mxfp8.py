@@ -10,7 +10,7 @@ import comfy_kitchen as ck
 from comfy_kitchen.float_utils import roundup
 
 from .base import BaseLayoutParams, QuantizedLayout
-from .blockwise import direct_backend, host_function, install_handlers
+from .blockwise import direct_backend, install_handlers, untraced_backend
 
 
 class TensorCoreMXFP8Layout(QuantizedLayout):
@@ -33,11 +33,12 @@ class TensorCoreMXFP8Layout(QuantizedLayout):
 
     @classmethod
     def quantize(cls, tensor: torch.Tensor, **kwargs):
-        host = host_function("quantize_mxfp8") if cls is TensorCoreMXFP8Layout and tensor.dim() == 2 else None
-        if host is not None:  # plain eager calls (None for any other)
+        backend = untraced_backend()
+        if backend is not None and backend._host is not None and backend.quantize_mxfp8 is backend._stock["quantize_mxfp8"] and \
+                cls is TensorCoreMXFP8Layout and tensor.dim() == 2:
             rows, cols = shape = tuple(tensor.shape)
-            out = host(tensor, (rows | cols) % 32 != 0)
-            if out is not None:
+            out = backend._host.quantize_mxfp8(tensor, (rows | cols) % 32 != 0)
+            if out is not None:  # plain eager calls
                 return out[0], cls.Params(out[1], tensor.dtype, shape)
         if tensor.dim() != 2:
             raise ValueError(f"MXFP8 requires 2D tensor, got {tensor.dim()}D")
@@ -80,10 +81,10 @@ class TensorCoreMXFP8Layout(QuantizedLayout):
     def scaled_mm(cls, a, b, bias, out_dtype):
         qa, sa = cls.get_plain_tensors(a)
         qb, sb = cls.get_plain_tensors(b)
-        host = host_function("scaled_mm_mxfp8")
-        if host is not None:  # plain eager calls (None for any other)
-            y = host(qa, qb, sa, sb, bias, out_dtype)
-            if y is not None:
+        backend = untraced_backend()
+        if backend is not None and backend._host is not None and backend.scaled_mm_mxfp8 is backend._stock["scaled_mm_mxfp8"]:
+            y = backend._host.scaled_mm_mxfp8(qa, qb, sa, sb, bias, out_dtype)
+            if y is not None:  # plain eager calls
                 return y
         backend = direct_backend(qa, qb, bias)
         if backend is not None:

@@ -9,9 +9,8 @@ import torch
 import comfy_kitchen as ck
 from comfy_kitchen.float_utils import F4_E2M1_MAX, F8_E4M3_MAX, roundup
 
-from . import blockwise
 from .base import BaseLayoutParams, QuantizedLayout
-from .blockwise import direct_backend, host_function, install_handlers
+from .blockwise import direct_backend, install_handlers, untraced_backend
 
 
 class TensorCoreNVFP4Layout(QuantizedLayout):
@@ -44,15 +43,18 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
 
     @classmethod
     def quantize(cls, tensor: torch.Tensor, scale=None, **kwargs):
-        if cls is TensorCoreNVFP4Layout and (scale is None or type(scale) in (torch.Tensor, torch.nn.Parameter)) and tensor.dim() == 2:
-            # plain eager calls (None for any other): 2 us less of host time than through the backend's wrappers
-            host = host_function("quantize_nvfp4_dynamic" if scale is None else "quantize_nvfp4")
-            if host is not None:
-                rows, cols = shape = tuple(tensor.shape)
-                pad = (rows | cols) % 16 != 0
-                out = host(tensor, pad, True, blockwise._backend.kept_scratch(tensor)) if scale is None else host(tensor, scale, pad, True)
-                if out is not None:
-                    return out[0], cls.Params(out[2] if scale is None else scale, tensor.dtype, shape, out[1])
+        backend = untraced_backend()
+        host = backend._host if backend is not None and cls is TensorCoreNVFP4Layout and tensor.dim() == 2 else None
+        if host is not None:  # plain eager calls (None for any other): 2 us less of host time than through the backend's wrappers
+            rows, cols = shape = tuple(tensor.shape)
+            pad, out = (rows | cols) % 16 != 0, None
+            if scale is None:
+                if backend.quantize_nvfp4_dynamic is backend._stock["quantize_nvfp4_dynamic"]:
+                    out = host.quantize_nvfp4_dynamic(tensor, pad, True, backend.kept_scratch)
+            elif type(scale) in (torch.Tensor, torch.nn.Parameter) and backend.quantize_nvfp4 is backend._stock["quantize_nvfp4"]:
+                out = host.quantize_nvfp4(tensor, scale, pad, True)
+            if out is not None:
+                return out[0], cls.Params(out[2] if scale is None else scale, tensor.dtype, shape, out[1])
         if tensor.dim() != 2:
             raise ValueError(f"NVFP4 requires 2D tensor, got {tensor.dim()}D")
         orig_shape = tuple(tensor.shape)
@@ -103,10 +105,10 @@ class TensorCoreNVFP4Layout(QuantizedLayout):
     def scaled_mm(cls, a, b, bias, out_dtype):
         qa, sa, bsa = cls.get_plain_tensors(a)
         qb, sb, bsb = cls.get_plain_tensors(b)
-        host = host_function("scaled_mm_nvfp4")
-        if host is not None:  # plain eager calls (None for any other)
-            y = host(qa, qb, sa, sb, bsa, bsb, bias, out_dtype, None)
-            if y is not None:
+        backend = untraced_backend()
+        if backend is not None and backend._host is not None and backend.scaled_mm_nvfp4 is backend._stock["scaled_mm_nvfp4"]:
+            y = backend._host.scaled_mm_nvfp4(qa, qb, sa, sb, bsa, bsb, bias, out_dtype, None)
+            if y is not None:  # plain eager calls
                 return y
         backend = direct_backend(qa, qb, bias)
         if backend is not None:

@@ -33,6 +33,7 @@ using at::Tensor;
 struct Library {
   int (*quantize_nvfp4)(const void*, int, const float*, void*, void*, int64_t, int64_t, int64_t, int64_t, int, void*);
   int64_t (*quantize_nvfp4_dynamic_scratch_bytes)(int64_t);
+  int64_t (*quantize_nvfp4_dynamic_whole_input_bytes)(int64_t);
   int (*quantize_nvfp4_dynamic)(const void*, int, float*, void*, void*, int64_t, int64_t, int64_t, int64_t, int, void*, int64_t, void*);
   int (*quantize_mxfp8)(const void*, int, void*, void*, int64_t, int64_t, int64_t, int64_t, void*);
   int (*dequantize_nvfp4)(const void*, const float*, const void*, void*, int, int64_t, int64_t, int, void*);
@@ -221,7 +222,9 @@ PyObject* quantize_nvfp4(PyObject*, Args a, Py_ssize_t n_args) {  // x, per_tens
   });
 }
 
-PyObject* quantize_nvfp4_dynamic(PyObject*, Args a, Py_ssize_t n_args) {  // x, pad_16x, hi_first, scratch or None
+// `kept_scratch(x)`: a buffer that is kept for the calls that write nothing to it.  Which they are is the library's to say: it is asked for up to
+// the size at which not even one row, whose line is the lowest, takes a reduction kernel.
+PyObject* quantize_nvfp4_dynamic(PyObject*, Args a, Py_ssize_t n_args) {  // x, pad_16x, hi_first, kept_scratch
   return or_none(a, n_args, 4, [&]() -> PyObject* {
     const Call c;
     const Tensor* x = matrix(a[0], c.device);
@@ -233,10 +236,15 @@ PyObject* quantize_nvfp4_dynamic(PyObject*, Args a, Py_ssize_t n_args) {  // x, 
     if (code < 0 || out_cols != cols || cols % (64 / x->element_size()) != 0 || reinterpret_cast<uintptr_t>(x->const_data_ptr()) % 32 != 0) return nullptr;
     const int64_t need = lib.quantize_nvfp4_dynamic_scratch_bytes(rows * cols);
     void* scratch = nullptr;
-    if (a[3] != Py_None) {
-      const Tensor* given = plain(a[3], c.device);
-      if (given == nullptr || given->scalar_type() != ScalarType::Byte || given->numel() < need) return nullptr;
-      scratch = given->mutable_data_ptr();
+    Tensor kept;
+    if (x->nbytes() <= static_cast<size_t>(lib.quantize_nvfp4_dynamic_whole_input_bytes(1))) {
+      PyObject* of_x = PyObject_CallOneArg(a[3], a[0]);
+      if (of_x == nullptr) return nullptr;  // an error, raised
+      const Tensor* t = plain(of_x, c.device);
+      if (t != nullptr) kept = *t;
+      Py_DECREF(of_x);
+      if (t == nullptr || kept.scalar_type() != ScalarType::Byte || kept.numel() < need) return nullptr;
+      scratch = kept.mutable_data_ptr();
     }
     Workspace ws(scratch == nullptr ? need : 0);
     if (scratch == nullptr) scratch = ws.ptr();
@@ -446,6 +454,7 @@ PyObject* bind(PyObject*, Args a, Py_ssize_t n_args) {
 #define CK_TAKE(name) take(got.name, "ck_" #name)
   CK_TAKE(quantize_nvfp4);
   CK_TAKE(quantize_nvfp4_dynamic_scratch_bytes);
+  CK_TAKE(quantize_nvfp4_dynamic_whole_input_bytes);
   CK_TAKE(quantize_nvfp4_dynamic);
   CK_TAKE(quantize_mxfp8);
   CK_TAKE(dequantize_nvfp4);

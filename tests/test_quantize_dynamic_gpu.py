@@ -81,9 +81,13 @@ def test_dynamic_quantizer_leaves_a_shared_scratch_usable(backend, cuda_device, 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows", [1, 8, 9, 128])
-def test_inputs_that_are_read_whole_leave_the_scratch_alone(backend, cuda_device, rows, dtype):
+def test_inputs_that_are_read_whole_leave_the_scratch_alone(backend, cuda_device, monkeypatch, rows, dtype):
     """On both sides of the line that the library reports: nothing is written to the scratch up to it; beyond it there are partial
-    maxima.  What the wrappers keep and share is handed in on this side of it alone."""
+    maxima.  What the wrappers keep and share is asked for on this side of the lowest line alone, by them and by the layout."""
+    from comfy_kitchen.tensor import QuantizedTensor
+
+    asked, kept = [], backend.kept_scratch
+    monkeypatch.setattr(backend, "kept_scratch", lambda t: asked.append(t.shape) or kept(t))
     lib = backend.load_library()
     code, elem = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[dtype], torch.empty((), dtype=dtype).element_size()
     line = lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(rows) // elem // rows // 32 * 32
@@ -97,7 +101,9 @@ def test_inputs_that_are_read_whole_leave_the_scratch_alone(backend, cuda_device
                                              scratch.data_ptr(), need, torch.cuda.current_stream().cuda_stream) == 0, lib.ck_last_error()
         assert bool((scratch == 0xA5).all()) == (k == line)
         assert torch.equal(out, want[2]) and torch.equal(q, want[0]) and torch.equal(s.view(torch.uint8), want[1].view(torch.uint8))
-        assert k == line or backend.kept_scratch(x) is None
+        QuantizedTensor.from_float(x, "TensorCoreNVFP4Layout")
+        assert asked == [x.shape] * (2 if x.nbytes <= lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(1) else 0)
+        asked.clear()
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])

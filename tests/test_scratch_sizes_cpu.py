@@ -36,12 +36,11 @@ def test_inputs_that_are_read_whole(lib, rows, kib):
     assert lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(rows) == kib << 10
 
 
-def test_the_scratch_that_callers_share_is_not_written(lib):
-    """The wrappers' line is no further out than the library's, whatever the number of rows."""
-    from comfy_kitchen.backends import cuda as backend
-
+def test_one_row_has_the_lowest_line(lib):
+    """Up to it the scratch is one that callers share: no number of rows may write to it."""
     lib.ck_quantize_nvfp4_dynamic_whole_input_bytes.restype = ctypes.c_int64
-    assert all(backend._KEPT_SCRATCH_BYTES <= lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(ctypes.c_int64(rows)) for rows in (1, 2, 8, 9, 64, 32768))
+    line = lambda rows: lib.ck_quantize_nvfp4_dynamic_whole_input_bytes(ctypes.c_int64(rows))
+    assert all(line(1) <= line(rows) for rows in (1, 2, 3, 7, 8, 9, 64, 1000, 32768))
 
 
 def test_dynamic_scratch_of_nothing(lib):
