@@ -49,7 +49,7 @@ int forced_gemm_config();
 bool exact_division();
 
 // One-call linears with very few activation rows (ck_gemm_smallm.cu).
-int linear_small_m_whole_input_bytes(int x_dtype, int64_t N, int64_t K, int64_t* bytes);
+int linear_small_m_reads_whole_input(int x_dtype, int64_t M, int64_t N, int64_t K, bool* whole);
 bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const void* w, const void* w_scales, int bias_dtype, const void* out,
                             int out_dtype, int64_t M, int64_t N, int64_t K);
 int linear_small_m(bool is_mxfp8, const void* x, int x_dtype, const float* x_scale, const float* partials, int n_partials, const void* w,

@@ -664,17 +664,22 @@ bool linear_small_m_applies(bool is_mxfp8, const void* x, int x_dtype, const voi
          is_float(bias_dtype) && aligned(x, 32) && aligned(w, 16) && aligned(w_scales, 16) && !exact_division() && (forced == 0 || forced == 9);
 }
 
-// NVFP4 with a dynamic scale: up to how many bytes every CTA takes the maximum of the whole activation itself; beyond, a reduction kernel
-// leaves partial maxima.  us, reduction kernel / whole activation: CTAs alone on their SMs bf16 6 x 3072 x 6144 (72 KiB) 7.8 / 7.4, 8 x 3072 x 6144
+// NVFP4 with a dynamic scale: whether every CTA takes the maximum of the whole activation itself, or a reduction kernel leaves partial
+// maxima: by the activation's bytes.  us, reduction kernel / whole activation: CTAs alone on their SMs bf16 6 x 3072 x 6144 (72 KiB) 7.8 / 7.4, 8 x 3072 x 6144
 // (96 KiB) 7.8 / 7.6, 4 x 3072 x 12288 (96 KiB) 9.4 / 9.2, fp32 8 x 6144 x 4096 (128 KiB) 9.4 / 8.9, bf16 6 x 3072 x 12288 (144 KiB) 9.6 / 10.1, 8 x
 // 12288 x 15360 (240 KiB) 23.8 / 25.0.  Where two share an SM, both want the whole activation at once: bf16 4 x 5120 x 9216 (72 KiB) 9.9 / 10.6, 6 x
 // 6144 x 8512 (100 KiB) 10.8 / 11.8, 8 x 24576 x 8128 (127 KiB) 23.5 / 25.2, fp16 2 x 4096 x 25600 (100 KiB) 15.5 / 15.8; fp32 has half the elements
 // to look at: 2 x 5120 x 9216 (72 KiB) 10.2 / 9.9, 2 x 6144 x 12800 (100 KiB) 13.2 / 12.8, 4 x 5120 x 8128 (127 KiB) 10.3 / 10.6, 8 x 24576 x 4032
 // 16.6 / 17.5.
-int linear_small_m_whole_input_bytes(int x_dtype, int64_t N, int64_t K, int64_t* bytes) {
+int linear_small_m_reads_whole_input(int x_dtype, int64_t M, int64_t N, int64_t K, bool* whole) {
+  constexpr int64_t kShared = 64 * 1024, kSharedFp32 = 112 * 1024, kAlone = 128 * 1024;
+  const bool fp32 = x_dtype == CK_DTYPE_F32;
+  const int64_t bytes = M * K * (fp32 ? 4 : 2), shared = fp32 ? kSharedFp32 : kShared;
+  *whole = bytes <= kAlone;
+  if (bytes <= shared || !*whole) return CK_OK;  // whatever the plan
   SmallPlan plan = {};
   if (int rc = choose_plan<Kind::kNvfp4>(N, static_cast<int>(K / 2), &plan)) return rc;
-  *bytes = (!plan.two_per_sm ? 128 : x_dtype == CK_DTYPE_F32 ? 112 : 64) * 1024;
+  *whole = !plan.two_per_sm;
   return CK_OK;
 }
 

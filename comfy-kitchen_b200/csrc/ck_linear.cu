@@ -59,11 +59,11 @@ extern "C" int ck_linear_nvfp4_from_float(const void* x, int x_dtype, const floa
     const int64_t elem = x_dtype == CK_DTYPE_F32 ? 4 : 2;
     float* partials = nullptr;
     int n_partials = 0;
-    int64_t whole = 0;
+    bool whole = true;
     if (dynamic) {
-      if (int rc = linear_small_m_whole_input_bytes(x_dtype, N, K, &whole)) return rc;
+      if (int rc = linear_small_m_reads_whole_input(x_dtype, M, N, K, &whole)) return rc;
     }
-    if (dynamic && M * K * elem > whole) {
+    if (!whole) {
       partials = reinterpret_cast<float*>(ws + l.scratch_off);
       if (int rc = launch_amax_partials(x, x_dtype, M * K * elem / 32, partials, &n_partials, static_cast<cudaStream_t>(stream))) return rc;
     }
