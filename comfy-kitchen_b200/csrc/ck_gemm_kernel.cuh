@@ -804,11 +804,16 @@ block_scaled_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const bool with_bias = p.bias != nullptr;
       if (tile_it == 0) {
         if constexpr (kWarpBias) {
+          // all fetched before the first is converted: one after the other, their latencies stood in front of a short main loop
+          // (us, 128 x 12288 x 256 fp16 5.60 / 5.49, 16 x 2496 x 256 5.25 / 5.10)
+          uint32_t bits[kBiasPerThread];
 #pragma unroll
           for (int i = 0; i < kBiasPerThread; ++i) {
             const int n = n0 + bias_col + 32 * i;
-            bias_s[bias_col + 32 * i] = (with_bias && n < p.N) ? load_bias(p.bias, p.bias_dtype, n) : 0.0f;
+            bits[i] = (with_bias && n < p.N) ? load_bias_bits(p.bias, p.bias_dtype, n) : 0u;
           }
+#pragma unroll
+          for (int i = 0; i < kBiasPerThread; ++i) bias_s[bias_col + 32 * i] = bias_of_bits(bits[i], p.bias_dtype);
           __syncwarp();
         } else {
           if (et < TILE_N) bias_s[et] = (with_bias && n0 + et < p.N) ? load_bias(p.bias, p.bias_dtype, n0 + et) : 0.0f;
